@@ -208,18 +208,14 @@ extern "C" int abk_short_conv_tail(const void *in, long long ld, int dtype, floa
     return ABK_LAUNCH_RESULT();
 }
 
-// ------------------------------------------------------------------ the recurrence
-// Two kernels. The first prepares every (token, head) in parallel, a warp each: the unit vectors q and k (q times
-// key^-1/2), the decays g, the value row and the write strength b, as one float32 record
+// ------------------------------------------------------------------ the tokens' records of the chunked form
+// Every (token, head) is prepared in parallel, a warp each: the unit vectors q and k (q times key^-1/2), the decays g, the
+// value row and the write strength b, as one float32 record
 //     [ k | q | g | v (vp) | b, 0, 0, 0 ]     vp = the value size padded to a multiple of 4
 // in which k, q and g each lie as `parts` runs of 32 channels with 4 floats of padding behind each run (zeros
 // beyond the key size; parts = 1, 2, 4 or 8).
-// The second walks each sequence's tokens in order (see delta_scan_kernel): the records of 8 tokens come in by
-// cp.async while the 8 before them are walked. The state comes in and goes out through shared memory, so that global
-// memory is read and written in whole lines.
-#define SCAN_ROWS 32    // key channels a thread keeps
-#define SCAN_RUN 36     // a run of 32 channels with its padding
-#define SCAN_CHUNK 8    // tokens in a stage
+#define SCAN_ROWS 32    // key channels of a run
+#define SCAN_RUN 36     // with its padding
 
 static inline int delta_parts(int key) { return key <= 32 ? 1 : key <= 64 ? 2 : key <= 128 ? 4 : 8; }
 static inline int delta_record_floats(int key, int value) { return 3 * delta_parts(key) * SCAN_RUN + ((value + 3) & ~3) + 4; }
@@ -234,9 +230,9 @@ struct DeltaPrepare {
     long long ld_beta;
     const float *a_log;     // [heads]
     const float *dt_bias;   // [heads * key]
-    float *records;         // [tokens, heads, record]
+    float *records;         // [tokens, heads, record] (or, of blocks of tokens, [blocks, heads, record])
     const int *token_seq;
-    long long pairs;        // tokens * heads
+    long long pairs;        // tokens (or blocks) * heads
     int heads, kv_heads, key, value, parts, record;
     float q_scale;          // key^-1/2
 };
@@ -284,153 +280,536 @@ template <typename T> __global__ void __launch_bounds__(128) delta_prepare_kerne
 }
 
 struct DeltaScan {
-    const float *records;   // [tokens, heads, record]
+    const float *records;   // the step's records: a token's and head's (chunks), or a block's and head's
     float *state;           // [slots, heads, value, key]
     float *out;             // [tokens, heads * value]
     const int *seq_start, *seq_slot;
     int heads, key, value, parts, record;
-    int col_warps;          // warps side by side along the columns (each 64 columns): a block has parts * col_warps warps
+    int n_seqs, tiles, longest_first;  // of the blocks' walk
+    int vec;                // the state's columns are read and written as 16-byte pieces (aligned, a multiple of 4 channels)
 };
+
+// ------------------------------------------------------------------ the recurrence, token by token and in blocks of 4
+// What the token-by-token walk waits for is the chain state -> sum over the key channels -> e -> state: with the sums
+// crossing lanes it is some 150 cycles a token whatever the arithmetic. Four tokens unrolled take the chain once. With S
+// the state before them, G_i = g_1 .. g_i the decays up to token i (elementwise over the key channels) and
+// G_ij = g_(j+1) .. g_i, everything the block reads of S are eight vectors' products with it, all at once:
+//     e_i = b_i (v_i - S^T (G_i k_i) - sum over j < i of [k_i . G_ij k_j] e_j)
+//     o_i =          S^T (G_i q_i) + sum over j <= i of [q_i . G_ij k_j] e_j      S <- G_4 S + sum over j of (G_4j k_j) e_j^T
+// (decays multiplied, never divided: every factor is at most 1). The vectors and the sixteen numbers in brackets know
+// neither the state nor the values: delta_block_prepare makes them for all blocks side by side, and delta_block_scan walks
+// the blocks. 13 multiply-adds a state element and 4 tokens where the walk token by token takes 16. Float32 throughout, the
+// same numbers in another order of sums.
+#define DB_TOKENS 4
+#define DB_STAGE 2     // blocks that come in together
+#define DB_STAGES 3    // of those in flight or in use
+
+static inline int delta_pad_key(int key) { return key <= 32 ? 32 : key <= 64 ? 64 : key <= 128 ? 128 : 256; }
+// A block's record, float32: [G_i k_i] x 4, [G_i q_i] x 4, [G_4j k_j] x 4, G_4 (each of the padded key size, zeros, or in
+// G_4 ones, beyond the key size), then b_i [k_i . G_ij k_j] (10, 20, 21, 30, 31, 32), [q_i . G_ij k_j] (00, 10, 11, 20 .. 33),
+// b (4), then the values [4][vp].
+#define DB_NUMBERS 20
+static inline long long delta_block_floats(int key, int value) { return 13LL * delta_pad_key(key) + DB_NUMBERS + DB_TOKENS * ((value + 3) & ~3); }
+
+// Which sequence has the step's block `b`, and which rows: whole warps call it. False: no sequence has.
+__device__ __forceinline__ bool delta_block_locate(const int *seq_start, int n_seqs, int b, int &row0, int &count) {
+    const int lane = threadIdx.x & 31;
+    for (int base = 0; base < n_seqs; base += 32) {
+        const int q = base + lane;
+        const int first = q < n_seqs ? seq_start[q] : 0, n = q < n_seqs ? seq_start[q + 1] - first : 0;
+        const int blocks = n > 0 ? (n + DB_TOKENS - 1) / DB_TOKENS : 0;
+        int upto = blocks;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, upto, m);
+            if (lane >= m) upto += other;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, b < upto);
+        if (hit) {
+            const int src = __ffs(hit) - 1;
+            const int at = (b - (upto - blocks)) * DB_TOKENS;
+            row0 = __shfl_sync(0xffffffffu, first + at, src);
+            count = __shfl_sync(0xffffffffu, min(DB_TOKENS, n - at), src);
+            return true;
+        }
+        b -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
+// A warp a (block, head); a lane has the channels lane, lane + 32, .. Every load is made before the first use.
+template <typename T, int J, bool PER_HEAD> __global__ void __launch_bounds__(128) delta_block_prepare_kernel(DeltaPrepare p, const int *seq_start, int n_seqs) {
+    constexpr int DP = 32 * J;
+    const long long pair = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    pdl_wait();
+    if (pair >= p.pairs) return;
+    const int b = (int)(pair / p.heads), h = (int)(pair - (long long)b * p.heads), K = p.key, V = p.value;
+    int row0, count;
+    if (!delta_block_locate(seq_start, n_seqs, b, row0, count)) return;
+    float *rec = p.records + pair * p.record;
+    const int kvh = h / (p.heads / p.kv_heads);
+    T q_in[DB_TOKENS][J], k_in[DB_TOKENS][J], b_in[DB_TOKENS], h_in[DB_TOKENS];
+    float d_in[DB_TOKENS][J], bias[J];
+#pragma unroll
+    for (int i = 0; i < DB_TOKENS; i++) {
+        const long long row = row0 + min(i, count - 1);
+        const T *qr = (const T *)p.qkv + row * p.ld_qkv + (long long)kvh * K, *kr = qr + (long long)p.kv_heads * K;
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const int c = min(lane + 32 * j, K - 1);
+            q_in[i][j] = qr[c], k_in[i][j] = kr[c];
+            if (!PER_HEAD) d_in[i][j] = ((const float *)p.decay_in)[row * p.ld_decay + (long long)h * K + c];
+        }
+        b_in[i] = ((const T *)p.beta_in)[row * p.ld_beta + h];
+        if (PER_HEAD) h_in[i] = ((const T *)p.decay_in)[row * p.ld_decay + h];
+    }
+#pragma unroll
+    for (int j = 0; j < J; j++) bias[j] = PER_HEAD ? p.dt_bias[h] : p.dt_bias[h * K + min(lane + 32 * j, K - 1)];
+    const float rate = expf(p.a_log[h]);
+    const int vp = (V + 3) & ~3;
+    float *vals = rec + 13 * DP + DB_NUMBERS;
+#pragma unroll
+    for (int i = 0; i < DB_TOKENS; i++) {
+        const T *vr = (const T *)p.qkv + (long long)(row0 + min(i, count - 1)) * p.ld_qkv + 2LL * p.kv_heads * K + (long long)h * V;
+        for (int j = lane; j < vp; j += 32) vals[i * vp + j] = i < count && j < V ? to_float(vr[j]) : 0.0f;
+    }
+    float q[DB_TOKENS][J], k[DB_TOKENS][J], g[DB_TOKENS][J], beta[DB_TOKENS];
+#pragma unroll
+    for (int i = 0; i < DB_TOKENS; i++) {
+        const bool real = i < count;
+        float qq = 0.0f, kk = 0.0f, head_decay = 1.0f;
+        if (PER_HEAD) head_decay = expf(-rate * softplus_f(to_float(h_in[i]) + bias[0]));
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const bool in = real && lane + 32 * j < K;
+            q[i][j] = in ? to_float(q_in[i][j]) : 0.0f, k[i][j] = in ? to_float(k_in[i][j]) : 0.0f;
+            const float decay = PER_HEAD ? head_decay : expf(-rate * softplus_f(d_in[i][j] + bias[j]));
+            g[i][j] = in ? decay : 1.0f;
+            qq = fmaf(q[i][j], q[i][j], qq), kk = fmaf(k[i][j], k[i][j], kk);
+        }
+        qq = warp_sum(qq), kk = warp_sum(kk);
+        const float qn = p.q_scale / sqrtf(qq + 1e-6f), kn = 1.0f / sqrtf(kk + 1e-6f);
+#pragma unroll
+        for (int j = 0; j < J; j++) q[i][j] *= qn, k[i][j] *= kn;
+        beta[i] = real ? 1.0f / (1.0f + expf(-to_float(b_in[i]))) : 0.0f;
+    }
+    float kk[6] = {}, qk[10] = {};
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+        const int c = lane + 32 * j;
+        float G = 1.0f, carried[DB_TOKENS];  // carried[s]: G_is k_s
+#pragma unroll
+        for (int i = 0; i < DB_TOKENS; i++) {
+            G *= g[i][j];
+            rec[i * DP + c] = G * k[i][j];
+            rec[(4 + i) * DP + c] = G * q[i][j];
+#pragma unroll
+            for (int s = 0; s < i; s++) {
+                carried[s] *= g[i][j];
+                kk[i * (i - 1) / 2 + s] = fmaf(k[i][j], carried[s], kk[i * (i - 1) / 2 + s]);
+            }
+            carried[i] = k[i][j];
+#pragma unroll
+            for (int s = 0; s <= i; s++) qk[i * (i + 1) / 2 + s] = fmaf(q[i][j], carried[s], qk[i * (i + 1) / 2 + s]);
+        }
+#pragma unroll
+        for (int s = 0; s < DB_TOKENS; s++) rec[(8 + s) * DP + c] = carried[s];
+        rec[12 * DP + c] = G;
+    }
+    float mine = 0.0f;  // lane n keeps number n
+#pragma unroll
+    for (int i = 1; i < DB_TOKENS; i++)
+#pragma unroll
+        for (int s = 0; s < i; s++) {
+            const float v = beta[i] * warp_sum(kk[i * (i - 1) / 2 + s]);
+            if (lane == i * (i - 1) / 2 + s) mine = v;
+        }
+#pragma unroll
+    for (int n = 0; n < 10; n++) {
+        const float v = warp_sum(qk[n]);
+        if (lane == 6 + n) mine = v;
+    }
+#pragma unroll
+    for (int i = 0; i < DB_TOKENS; i++)
+        if (lane == 16 + i) mine = beta[i];
+    if (lane < DB_NUMBERS) rec[13 * DP + lane] = mine;
+}
+
+// Two float32 at once: each half rounded as the single instruction rounds it.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
 
 __device__ __forceinline__ void scan_copy_16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// A warp has one run of 32 key channels (its part) of 64 value columns, a lane two neighbouring columns: 64 state
-// values in registers. All lanes of a warp read the token's k, q and g of the warp's run at one address. The sums
-// over the key channels meet across the block's warps through shared memory, two barriers a token.
-// MAX_THREADS: the most threads a block has (128, 256 or 512): the fewer, the more registers a thread may use.
-template <int MAX_THREADS> __global__ void __launch_bounds__(MAX_THREADS) delta_scan_kernel(DeltaScan p) {
-    extern __shared__ __align__(16) float smem[];  // records [2][SCAN_CHUNK][R] (before and after the walk: the
-                                                   // state's lines, [warps][32 * 33]), then the partial sums
-    const int parts = p.parts, region = parts * SCAN_RUN, R = p.record, cw = p.col_warps;
-    const int n_warps = parts * cw, n_threads = n_warps * 32;
-    const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int part = warp % parts, col_warp = warp / parts;
-    const int block_cols = cw * 64, col0 = blockIdx.z * block_cols;          // this block's columns
-    const int local = col_warp * 64 + 2 * lane, col = col0 + local;          // this lane's two columns: col, col + 1
-    const int K = p.key, V = p.value, vp = R - 3 * region - 4;
-    size_t front = (size_t)2 * SCAN_CHUNK * R;
-    if (front < (size_t)n_warps * 32 * 33) front = (size_t)n_warps * 32 * 33;
-    float *sums = smem + ((front + 3) & ~(size_t)3);  // [2 (token parity)][2 (seen, read)][parts][block_cols]
-    pdl_wait();
-    const int row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
-    if (n <= 0) return;
-    float *head_state = p.state + ((long long)p.seq_slot[seq] * p.heads + h) * V * K;
-    float *mine_stage = smem + warp * 32 * 33;  // 32 floats of each of 32 columns, a line at a time
-    float S0[SCAN_ROWS], S1[SCAN_ROWS];
-#pragma unroll
-    for (int half = 0; half < 2; half++) {  // the warp's even columns, then its odd ones
-#pragma unroll 8
-        for (int j = 0; j < 32; j++) {
-            const int cj = col0 + col_warp * 64 + 2 * j + half, ch = part * SCAN_ROWS + lane;
-            mine_stage[j * 33 + lane] = cj < V && ch < K ? head_state[(long long)cj * K + ch] : 0.0f;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < SCAN_ROWS; i++) {
-            if (half == 0) S0[i] = mine_stage[lane * 33 + i];
-            else S1[i] = mine_stage[lane * 33 + i];
-        }
-        __syncwarp();
+// Four of a state column's channels from `ch` on; beyond the key size, or where the column is none, zeros.
+__device__ __forceinline__ float4 delta_load_state(const float *column, int ch, int K, bool real, int vec) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (!real) return v;
+    const float *src = column + ch;
+    if (vec) {
+        if (ch < K) v = *(const float4 *)src;
+    } else {
+        if (ch < K) v.x = src[0];
+        if (ch + 1 < K) v.y = src[1];
+        if (ch + 2 < K) v.z = src[2];
+        if (ch + 3 < K) v.w = src[3];
     }
-    __syncthreads();  // the records come into the same memory
-
-    const uint32_t chunk_s = (uint32_t)__cvta_generic_to_shared(smem);
-    auto fetch = [&](int base, int stage_index) {  // the records of tokens [base, base + count) of this head
-        const int count = n - base < SCAN_CHUNK ? n - base : SCAN_CHUNK;
-        const int per = R / 4;
-        for (int e = tid; e < count * per; e += n_threads) {
-            const int c = e / per, q = e - c * per;
-            scan_copy_16(chunk_s + ((stage_index * SCAN_CHUNK + c) * R + q * 4) * 4,
-                         p.records + ((long long)(row0 + base + c) * p.heads + h) * R + q * 4);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    fetch(0, 0);
-    int token = 0;
-    for (int base = 0, it = 0; base < n; base += SCAN_CHUNK, it++) {
-        const int count = n - base < SCAN_CHUNK ? n - base : SCAN_CHUNK;
-        if (base + SCAN_CHUNK < n) {  // the next tokens into the other stage (its readers passed the barrier below)
-            fetch(base + SCAN_CHUNK, (it + 1) & 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const float *records = smem + (it & 1) * SCAN_CHUNK * R;
-        for (int c = 0; c < count; c++, token++) {
-            const float *rec = records + c * R;
-            const float4 *k4 = (const float4 *)(rec + part * SCAN_RUN);
-            const float4 *q4 = (const float4 *)(rec + region + part * SCAN_RUN);
-            const float4 *g4 = (const float4 *)(rec + 2 * region + part * SCAN_RUN);
-            float *seen_s = sums + (size_t)(token & 1) * 2 * parts * block_cols, *read_s = seen_s + parts * block_cols;
-            float a0 = 0.0f, a1 = 0.0f, b0 = 0.0f, b1 = 0.0f;
-#pragma unroll
-            for (int i = 0; i < SCAN_ROWS / 4; i++) {
-                const float4 g = g4[i], k = k4[i];
-                S0[4 * i] *= g.x, S0[4 * i + 1] *= g.y, S0[4 * i + 2] *= g.z, S0[4 * i + 3] *= g.w;
-                S1[4 * i] *= g.x, S1[4 * i + 1] *= g.y, S1[4 * i + 2] *= g.z, S1[4 * i + 3] *= g.w;
-                a0 = fmaf(S0[4 * i], k.x, a0), a1 = fmaf(S0[4 * i + 1], k.y, a1);
-                a0 = fmaf(S0[4 * i + 2], k.z, a0), a1 = fmaf(S0[4 * i + 3], k.w, a1);
-                b0 = fmaf(S1[4 * i], k.x, b0), b1 = fmaf(S1[4 * i + 1], k.y, b1);
-                b0 = fmaf(S1[4 * i + 2], k.z, b0), b1 = fmaf(S1[4 * i + 3], k.w, b1);
-            }
-            *(float2 *)(seen_s + part * block_cols + local) = make_float2(a0 + a1, b0 + b1);
-            __syncthreads();
-            float seen0 = 0.0f, seen1 = 0.0f;
-            for (int o = 0; o < parts; o++) {
-                const float2 t = *(const float2 *)(seen_s + o * block_cols + local);
-                seen0 += t.x, seen1 += t.y;
-            }
-            const float beta = rec[3 * region + vp];
-            const float e0 = beta * (rec[3 * region + (col < V ? col : 0)] - seen0);
-            const float e1 = beta * (rec[3 * region + (col + 1 < V ? col + 1 : 0)] - seen1);
-            a0 = a1 = b0 = b1 = 0.0f;
-#pragma unroll
-            for (int i = 0; i < SCAN_ROWS / 4; i++) {
-                const float4 k = k4[i], q = q4[i];
-                S0[4 * i] = fmaf(k.x, e0, S0[4 * i]), S0[4 * i + 1] = fmaf(k.y, e0, S0[4 * i + 1]);
-                S0[4 * i + 2] = fmaf(k.z, e0, S0[4 * i + 2]), S0[4 * i + 3] = fmaf(k.w, e0, S0[4 * i + 3]);
-                S1[4 * i] = fmaf(k.x, e1, S1[4 * i]), S1[4 * i + 1] = fmaf(k.y, e1, S1[4 * i + 1]);
-                S1[4 * i + 2] = fmaf(k.z, e1, S1[4 * i + 2]), S1[4 * i + 3] = fmaf(k.w, e1, S1[4 * i + 3]);
-                a0 = fmaf(S0[4 * i], q.x, a0), a1 = fmaf(S0[4 * i + 1], q.y, a1);
-                a0 = fmaf(S0[4 * i + 2], q.z, a0), a1 = fmaf(S0[4 * i + 3], q.w, a1);
-                b0 = fmaf(S1[4 * i], q.x, b0), b1 = fmaf(S1[4 * i + 1], q.y, b1);
-                b0 = fmaf(S1[4 * i + 2], q.z, b0), b1 = fmaf(S1[4 * i + 3], q.w, b1);
-            }
-            *(float2 *)(read_s + part * block_cols + local) = make_float2(a0 + a1, b0 + b1);
-            __syncthreads();
-            if (part == 0) {  // the warps of the first run add up what the token reads
-                float r0 = 0.0f, r1 = 0.0f;
-                for (int o = 0; o < parts; o++) {
-                    const float2 t = *(const float2 *)(read_s + o * block_cols + local);
-                    r0 += t.x, r1 += t.y;
-                }
-                float *dst = p.out + (long long)(row0 + base + c) * p.heads * V + (long long)h * V;
-                if (col < V) dst[col] = r0;
-                if (col + 1 < V) dst[col + 1] = r1;
-            }
-        }
-        __syncthreads();  // the stage is filled again by the iteration after next (and, at the end, by the state)
-    }
-#pragma unroll
-    for (int half = 0; half < 2; half++) {
-#pragma unroll
-        for (int i = 0; i < SCAN_ROWS; i++) mine_stage[lane * 33 + i] = half == 0 ? S0[i] : S1[i];
-        __syncwarp();
-#pragma unroll 8
-        for (int j = 0; j < 32; j++) {
-            const int cj = col0 + col_warp * 64 + 2 * j + half, ch = part * SCAN_ROWS + lane;
-            if (cj < V && ch < K) head_state[(long long)cj * K + ch] = mine_stage[j * 33 + lane];
-        }
-        __syncwarp();
+    return v;
+}
+__device__ __forceinline__ void delta_store_state(float *column, int ch, int K, float4 v, int vec) {
+    float *dst = column + ch;
+    if (vec) {
+        if (ch < K) *(float4 *)dst = v;
+    } else {
+        if (ch < K) dst[0] = v.x;
+        if (ch + 1 < K) dst[1] = v.y;
+        if (ch + 2 < K) dst[2] = v.z;
+        if (ch + 3 < K) dst[3] = v.w;
     }
 }
 
-// Floats of scratch memory the recurrence needs for n_tokens tokens (its records).
-extern "C" long long abk_delta_scan_scratch(int n_tokens, int heads, int key, int value) {
-    return (long long)n_tokens * heads * delta_record_floats(key, value);
+// The sequence that comes `place`-th when the step's are ordered from the longest to the shortest; whole warps call it, up
+// to 64 sequences.
+__device__ __forceinline__ int delta_place(const int *seq_start, int n_seqs, int place) {
+    const int lane = threadIdx.x & 31;
+    const int a = lane < n_seqs ? seq_start[lane + 1] - seq_start[lane] : -1;
+    const int b = lane + 32 < n_seqs ? seq_start[lane + 33] - seq_start[lane + 32] : -1;
+    int before_a = 0, before_b = 0;  // how many come before this lane's two
+    for (int j = 0; j < n_seqs; j++) {
+        const int other = __shfl_sync(0xffffffffu, j < 32 ? a : b, j & 31);
+        before_a += other > a || (other == a && j < lane), before_b += other > b || (other == b && j < lane + 32);
+    }
+    const unsigned hit_a = __ballot_sync(0xffffffffu, lane < n_seqs && before_a == place);
+    const unsigned hit_b = __ballot_sync(0xffffffffu, lane + 32 < n_seqs && before_b == place);
+    return hit_a ? __ffs(hit_a) - 1 : 31 + __ffs(hit_b);
+}
+
+// P lanes share a value column, each with 4 J of its key channels (lane p: 4 p .. 4 p + 3 of every 4 P, so that together
+// they read a vector as whole lines); a lane has C columns, 4 J C numbers of state in registers, and every piece of a
+// vector it reads serves them all: a 16-byte read costs the warp four cycles of shared memory whatever the lanes share, so
+// C, not the columns of a warp (32 C / P), decides what shared memory costs a column. A block: its eight vectors against
+// the columns; the 8 C partial sums of a lane meet by shuffles that hand half of them over at each of the first steps, so
+// that at the end a lane has one column's four sums with the keys or with the queries; the lanes with the first solve for
+// e, all get it, the lanes with the others write o. The CTA's last warp does nothing but bring the records in, so that the
+// others' instructions are the recurrence's alone.
+// Bound by the chain where sequences are few: one prompt of 1,999 tokens, 16 heads of 128 x 128: 298 us, 1,110 cycles a
+// block at one walking warp a scheduler (the walk token by token with two barriers a token, which stood here: 1,560 us);
+// towards the multiply-adds where they are many: 8 prompts, 5,672 tokens, 32 heads, 701 us.
+template <int P, int J, int C>
+__global__ void __launch_bounds__(160) delta_block_scan_kernel(DeltaScan p) {
+    extern __shared__ __align__(16) float smem[];  // [DB_STAGES][DB_STAGE] records, of the values this CTA's columns
+    constexpr int DP = 4 * P * J, HEAD = 13 * DP + DB_NUMBERS;
+    const int walkers = blockDim.x - 32, cols = walkers / P * C, vp = (p.value + 3) & ~3;  // this CTA's columns
+    const int RS = HEAD + DB_TOKENS * cols;
+    const int tid = threadIdx.x, lane = tid & 31, part = lane & (P - 1);
+    const int h = blockIdx.x % p.heads, tile = blockIdx.x / p.heads % p.tiles, place = blockIdx.x / p.heads / p.tiles;
+    const int col0 = tile * cols, first_col = col0 + tid / P * C;  // this lane's columns: first_col ..
+    const int K = p.key, V = p.value;
+    pdl_wait();
+    const int seq = p.longest_first ? delta_place(p.seq_start, p.n_seqs, place) : place;
+    const int row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
+    if (n <= 0) return;
+    const int n_blocks = (n + DB_TOKENS - 1) / DB_TOKENS;
+    if (tid >= walkers) {  // the records: a stage ahead of the walkers, two in flight
+        int first_block = 0;
+        for (int q = lane; q < seq; q += 32) first_block += (max(p.seq_start[q + 1] - p.seq_start[q], 0) + DB_TOKENS - 1) / DB_TOKENS;
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) first_block += __shfl_xor_sync(0xffffffffu, first_block, m);
+        const uint32_t base_s = (uint32_t)__cvta_generic_to_shared(smem);
+        const int own = min(cols, vp - col0);  // columns whose values the record holds (a multiple of 4)
+        auto fetch = [&](int first) {          // blocks first .. first + DB_STAGE - 1
+            const int count = min(DB_STAGE, n_blocks - first), stage = first / DB_STAGE % DB_STAGES;
+            for (int b = 0; b < count; b++) {
+                const float *rec = p.records + ((long long)(first_block + first + b) * p.heads + h) * p.record;
+                const uint32_t dst = base_s + (stage * DB_STAGE + b) * RS * 4;
+                for (int e = lane; e < HEAD / 4; e += 32) scan_copy_16(dst + e * 16, rec + e * 4);
+                for (int e = lane; e < own; e += 32) {  // own / 4 pieces of each of the four tokens
+                    const int t = e / (own / 4), c = e - t * (own / 4);
+                    scan_copy_16(dst + (HEAD + t * cols + c * 4) * 4, rec + HEAD + t * vp + col0 + c * 4);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");  // (a group each time, empty beyond the last block)
+        };
+        fetch(0);
+        fetch(DB_STAGE);
+        for (int b0 = 0; b0 < n_blocks; b0 += DB_STAGE) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();  // this stage is here, and the one before it has been read by all: its place is filled again
+            fetch(b0 + 2 * DB_STAGE);
+        }
+        return;
+    }
+    float *head_state = p.state + ((long long)p.seq_slot[seq] * p.heads + h) * V * K;
+    f32x2 S[C][2 * J];
+#pragma unroll
+    for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const float4 v = delta_load_state(head_state + (long long)(first_col + c) * K, 4 * (P * j + part), K, first_col + c < V, p.vec);
+            S[c][2 * j] = pack2(v.x, v.y), S[c][2 * j + 1] = pack2(v.z, v.w);
+        }
+    // every lane's place after the shuffles: its column, and whether its sums are with the queries
+    constexpr int COL_STEPS = C == 4 ? 2 : C == 2 ? 1 : 0;
+    constexpr int SPLIT = P >> (COL_STEPS + 1);   // the lane bit that tells sums with queries from sums with keys
+    static_assert(SPLIT >= 1, "a lane has a column to itself at the end");
+    const int my_c = part / (2 * SPLIT);          // (the first steps' bits, highest first, count the columns)
+    const bool reads = (part & SPLIT) != 0;
+    const int my_col = first_col + my_c;
+    const long long hv = (long long)p.heads * V;
+    float *out = p.out + (long long)row0 * hv + (long long)h * V + my_col;
+
+    for (int b0 = 0, stage = 0; b0 < n_blocks; b0 += DB_STAGE, stage = stage == DB_STAGES - 1 ? 0 : stage + 1) {
+        __syncthreads();
+        const int count = min(DB_STAGE, n_blocks - b0);
+        for (int b = 0; b < count; b++, out += DB_TOKENS * hv) {
+            const float *rec = smem + (stage * DB_STAGE + b) * RS;
+            const float *vec = rec + 4 * part;
+            float sums[C][8];
+#pragma unroll
+            for (int r = 0; r < 8; r++) {
+                f32x2 a[C];
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    const ulonglong2 w = *(const ulonglong2 *)(vec + r * DP + 4 * P * j);
+#pragma unroll
+                    for (int c = 0; c < C; c++) {
+                        a[c] = j == 0 ? mul2(w.x, S[c][0]) : fma2(w.x, S[c][2 * j], a[c]);
+                        a[c] = fma2(w.y, S[c][2 * j + 1], a[c]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    const float2 x = unpack2(a[c]);
+                    sums[c][r] = x.x + x.y;
+                }
+            }
+            // what does not wait for the sums: the state's decay, the block's numbers and values, and (few channels a lane)
+            // the vectors of the update, read while the shuffles are under way
+            constexpr bool AHEAD = J <= 2;
+            ulonglong2 u[AHEAD ? 4 : 1][J];
+            if constexpr (AHEAD) {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < J; j++) u[i][j] = *(const ulonglong2 *)(vec + (8 + i) * DP + 4 * P * j);
+            }
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const ulonglong2 w = *(const ulonglong2 *)(vec + 12 * DP + 4 * P * j);
+#pragma unroll
+                for (int c = 0; c < C; c++) S[c][2 * j] = mul2(w.x, S[c][2 * j]), S[c][2 * j + 1] = mul2(w.y, S[c][2 * j + 1]);
+            }
+            const float4 n0 = *(const float4 *)(rec + 13 * DP), n1 = *(const float4 *)(rec + 13 * DP + 4), n2 = *(const float4 *)(rec + 13 * DP + 8);
+            const float4 n3 = *(const float4 *)(rec + 13 * DP + 12), bt = *(const float4 *)(rec + 13 * DP + 16);
+            const float *vv = rec + HEAD + my_col - col0;
+            const float v0 = vv[0], v1 = vv[cols], v2 = vv[2 * cols], v3 = vv[3 * cols];
+            // hand over: columns first, then keys' sums against queries', then plain sums
+#pragma unroll
+            for (int step = 0; step < COL_STEPS; step++) {
+                const int half = C >> (step + 1), bit = P >> (step + 1);
+                const bool up = part & bit;
+#pragma unroll
+                for (int c = 0; c < half; c++)
+#pragma unroll
+                    for (int r = 0; r < 8; r++) {
+                        const float give = up ? sums[c][r] : sums[c + half][r], keep = up ? sums[c + half][r] : sums[c][r];
+                        sums[c][r] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                    }
+            }
+            float mine[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float give = reads ? sums[0][i] : sums[0][4 + i], keep = reads ? sums[0][4 + i] : sums[0][i];
+                mine[i] = keep + __shfl_xor_sync(0xffffffffu, give, SPLIT);
+            }
+#pragma unroll
+            for (int m = SPLIT >> 1; m > 0; m >>= 1)
+#pragma unroll
+                for (int i = 0; i < 4; i++) mine[i] += __shfl_xor_sync(0xffffffffu, mine[i], m);
+            float e[4];  // (meant where the sums are with the keys)
+            e[0] = bt.x * (v0 - mine[0]);
+            e[1] = fmaf(-n0.x, e[0], bt.y * (v1 - mine[1]));
+            e[2] = fmaf(-n0.z, e[1], fmaf(-n0.y, e[0], bt.z * (v2 - mine[2])));
+            e[3] = fmaf(-n1.y, e[2], fmaf(-n1.x, e[1], fmaf(-n0.w, e[0], bt.w * (v3 - mine[3]))));
+            float all[C][4], mine_e[4];
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const int src = (lane & ~(P - 1)) | c * 2 * SPLIT;
+#pragma unroll
+                for (int i = 0; i < 4; i++) all[c][i] = __shfl_sync(0xffffffffu, e[i], src);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                f32x2 ee[C];
+#pragma unroll
+                for (int c = 0; c < C; c++) ee[c] = pack2(all[c][i], all[c][i]);
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    const ulonglong2 w = AHEAD ? u[AHEAD ? i : 0][j] : *(const ulonglong2 *)(vec + (8 + i) * DP + 4 * P * j);
+#pragma unroll
+                    for (int c = 0; c < C; c++) S[c][2 * j] = fma2(w.x, ee[c], S[c][2 * j]), S[c][2 * j + 1] = fma2(w.y, ee[c], S[c][2 * j + 1]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                float x = all[0][i];
+#pragma unroll
+                for (int c = 1; c < C; c++) x = my_c == c ? all[c][i] : x;
+                mine_e[i] = x;
+            }
+            float o[4];
+            o[0] = fmaf(n1.z, mine_e[0], mine[0]);
+            o[1] = fmaf(n2.x, mine_e[1], fmaf(n1.w, mine_e[0], mine[1]));
+            o[2] = fmaf(n2.w, mine_e[2], fmaf(n2.z, mine_e[1], fmaf(n2.y, mine_e[0], mine[2])));
+            o[3] = fmaf(n3.w, mine_e[3], fmaf(n3.z, mine_e[2], fmaf(n3.y, mine_e[1], fmaf(n3.x, mine_e[0], mine[3]))));
+            const int left = n - (b0 + b) * DB_TOKENS;
+            if (reads && my_col < V) {  // SPLIT lanes have the same column: each writes its share of the four tokens
+                if constexpr (SPLIT >= 4) {
+                    const float lo = part & 1 ? o[1] : o[0], hi = part & 1 ? o[3] : o[2];
+                    if ((part & (SPLIT - 1)) < 4 && (part & 3) < left) out[(part & 3) * hv] = part & 2 ? hi : lo;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if ((i & (SPLIT - 1)) == (part & (SPLIT - 1)) && i < left) out[i * hv] = o[i];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            if (first_col + c >= V) continue;
+            const float2 x = unpack2(S[c][2 * j]), y = unpack2(S[c][2 * j + 1]);
+            delta_store_state(head_state + (long long)(first_col + c) * K, 4 * (P * j + part), K, make_float4(x.x, x.y, y.x, y.y), p.vec);
+        }
+}
+
+// A step of one token a sequence: the state comes and goes once, and that is all there is to do, so the preparation is in
+// the same kernel. A CTA has one (sequence, head) and some of its columns; it makes the token's k, q, g, b in shared memory
+// (its columns' CTAs each for themselves: a few hundred channels), then every warp takes 8 columns at a time, LPC lanes a
+// column with 4 J channels each: with a = g k and r = g q as above, S^T a and S^T r, then S <- g S + k e. (A sequence that
+// brings several tokens after all is walked token by token.) Bound by HBM: 64 sequences, 32 heads of 128 x 128, 268 MB of
+// state in 61 us with its wait (the walk above's general form and its preparation: 103 us).
+template <typename T, int LPC, int J>
+__global__ void __launch_bounds__(256) delta_step_kernel(DeltaPrepare p, DeltaScan q) {
+    constexpr int DP = LPC * 4 * J, SIDE = 32 / LPC, ROUNDS = 8 / SIDE;  // columns side by side, and one after another
+    __shared__ __align__(16) float ks[DP], qs[DP], gs[DP];
+    __shared__ float meet[2][8], numbers[2];
+    const int seq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = p.key, V = p.value;
+    const int n_warps = blockDim.x >> 5;
+    pdl_wait();
+    const int row0 = q.seq_start[seq], n = q.seq_start[seq + 1] - row0;
+    if (n <= 0) return;
+    float *head_state = q.state + ((long long)q.seq_slot[seq] * p.heads + h) * V * K;
+    const int kvh = h / (p.heads / p.kv_heads), part = lane % LPC, side = lane / LPC;
+    const float rate = expf(p.a_log[h]);
+    for (int t = 0; t < n; t++) {
+        const long long row = row0 + t;
+        const T *qr = (const T *)p.qkv + row * p.ld_qkv + (long long)kvh * K, *kr = qr + (long long)p.kv_heads * K;
+        const T *vr = (const T *)p.qkv + row * p.ld_qkv + 2LL * p.kv_heads * K + (long long)h * V;
+        const float beta = 1.0f / (1.0f + expf(-to_float(((const T *)p.beta_in)[row * p.ld_beta + h])));
+        float qq = 0.0f, kk = 0.0f;
+        for (int c = tid; c < DP; c += blockDim.x) {
+            const float qv = c < K ? to_float(qr[c]) : 0.0f, kv = c < K ? to_float(kr[c]) : 0.0f;
+            float g = 1.0f;
+            if (p.per_head) g = expf(-rate * softplus_f(to_float(((const T *)p.decay_in)[row * p.ld_decay + h]) + p.dt_bias[h]));
+            else if (c < K) g = expf(-rate * softplus_f(((const float *)p.decay_in)[row * p.ld_decay + (long long)h * K + c] + p.dt_bias[h * K + c]));
+            qs[c] = qv, ks[c] = kv, gs[c] = g;
+            qq = fmaf(qv, qv, qq), kk = fmaf(kv, kv, kk);
+        }
+        qq = warp_sum(qq), kk = warp_sum(kk);
+        if (lane == 0) meet[0][warp] = qq, meet[1][warp] = kk;
+        __syncthreads();
+        if (tid == 0) {
+            qq = kk = 0.0f;
+            for (int w = 0; w < n_warps; w++) qq += meet[0][w], kk += meet[1][w];
+            numbers[0] = p.q_scale / sqrtf(qq + 1e-6f), numbers[1] = 1.0f / sqrtf(kk + 1e-6f);
+        }
+        __syncthreads();
+        const float qn = numbers[0], kn = numbers[1];
+        float4 k4[J], g4[J], a4[J], r4[J];
+        float kq = 0.0f;
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const int c = 4 * (part + LPC * j);
+            const float4 kv = *(const float4 *)(ks + c), qv = *(const float4 *)(qs + c), g = *(const float4 *)(gs + c);
+            k4[j] = make_float4(kv.x * kn, kv.y * kn, kv.z * kn, kv.w * kn), g4[j] = g;
+            const float4 r = make_float4(qv.x * qn, qv.y * qn, qv.z * qn, qv.w * qn);
+            kq = fmaf(k4[j].x, r.x, fmaf(k4[j].y, r.y, fmaf(k4[j].z, r.z, fmaf(k4[j].w, r.w, kq))));
+            a4[j] = make_float4(g.x * k4[j].x, g.y * k4[j].y, g.z * k4[j].z, g.w * k4[j].w);
+            r4[j] = make_float4(g.x * r.x, g.y * r.y, g.z * r.z, g.w * r.w);
+        }
+#pragma unroll
+        for (int m = 1; m < LPC; m <<= 1) kq += __shfl_xor_sync(0xffffffffu, kq, m);
+        for (int col0 = (blockIdx.z * n_warps + warp) * 8; col0 < V; col0 += gridDim.z * n_warps * 8) {
+            float4 s[ROUNDS][J];
+            float vv[ROUNDS], a[ROUNDS], r[ROUNDS];
+#pragma unroll
+            for (int u = 0; u < ROUNDS; u++) {
+                const int col = col0 + u * SIDE + side;
+#pragma unroll
+                for (int j = 0; j < J; j++) s[u][j] = delta_load_state(head_state + (long long)col * K, 4 * (part + LPC * j), K, col < V, q.vec);
+                vv[u] = col < V ? to_float(vr[col]) : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < ROUNDS; u++) {
+                a[u] = r[u] = 0.0f;
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    a[u] = fmaf(a4[j].x, s[u][j].x, fmaf(a4[j].y, s[u][j].y, fmaf(a4[j].z, s[u][j].z, fmaf(a4[j].w, s[u][j].w, a[u]))));
+                    r[u] = fmaf(r4[j].x, s[u][j].x, fmaf(r4[j].y, s[u][j].y, fmaf(r4[j].z, s[u][j].z, fmaf(r4[j].w, s[u][j].w, r[u]))));
+                }
+            }
+#pragma unroll
+            for (int m = 1; m < LPC; m <<= 1)
+#pragma unroll
+                for (int u = 0; u < ROUNDS; u++) a[u] += __shfl_xor_sync(0xffffffffu, a[u], m), r[u] += __shfl_xor_sync(0xffffffffu, r[u], m);
+#pragma unroll
+            for (int u = 0; u < ROUNDS; u++) {
+                const int col = col0 + u * SIDE + side;
+                if (col >= V) continue;
+                const float e = beta * (vv[u] - a[u]);
+                if (part == u % LPC) q.out[row * p.heads * V + (long long)h * V + col] = fmaf(kq, e, r[u]);
+#pragma unroll
+                for (int j = 0; j < J; j++)
+                    delta_store_state(head_state + (long long)col * K, 4 * (part + LPC * j), K,
+                                      make_float4(fmaf(k4[j].x, e, g4[j].x * s[u][j].x), fmaf(k4[j].y, e, g4[j].y * s[u][j].y),
+                                                  fmaf(k4[j].z, e, g4[j].z * s[u][j].z), fmaf(k4[j].w, e, g4[j].w * s[u][j].w)), q.vec);
+            }
+        }
+        __syncthreads();  // (a further token's k, q, g come into the same memory)
+    }
+}
+
+// Floats of scratch memory the recurrence needs for n_tokens tokens of n_seqs sequences: the blocks' records, none where no
+// sequence brings more than a token; chunks: the tokens' records of abk_delta_chunks.
+extern "C" long long abk_delta_scan_scratch(int n_tokens, int n_seqs, int heads, int key, int value, int chunks) {
+    if (chunks) return (long long)n_tokens * heads * delta_record_floats(key, value);
+    if (n_tokens <= n_seqs) return 0;
+    return ((long long)n_tokens / DB_TOKENS + n_seqs) * heads * delta_block_floats(key, value);
 }
 
 extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, const void *decay_in, long long ld_decay, int per_head, const void *beta_in,
@@ -442,46 +821,92 @@ extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, cons
     if (key < 1 || key > 256) ABK_REFUSE("delta rule: key size %d, the kernel takes 1 to 256", key);
     if (kv_heads < 1 || heads % kv_heads) ABK_REFUSE("delta rule: %d heads do not divide into %d key heads", heads, kv_heads);
     if (heads > 65535 || value > 65535 * 16) ABK_REFUSE("delta rule: %d heads of %d values are more than a grid takes", heads, value);
-    const int parts = delta_parts(key), record = delta_record_floats(key, value);
-    if ((long long)n_tokens * heads * record > records_floats || ((uintptr_t)records & 15))
-        ABK_REFUSE("delta rule: the scratch memory holds %lld floats, the step needs %lld (16-byte aligned)", records_floats,
-                   (long long)n_tokens * heads * record);
-    // 64 columns a warp; two warps side by side where they fit a block and the step has (sequence, head) pairs enough
-    // to fill the GPU without the halves of a head going to different SMs
-    const int col_warps = parts <= 4 && value > 64 && (long long)n_seqs * heads * ((value + 63) / 64) > 2LL * abk_sm_count() ? 2 : 1;
-    const int n_warps = parts * col_warps, block_cols = 64 * col_warps;
-    size_t front = (size_t)2 * SCAN_CHUNK * record;
-    if (front < (size_t)n_warps * 32 * 33) front = (size_t)n_warps * 32 * 33;
-    const size_t smem = (((front + 3) & ~(size_t)3) + (size_t)4 * parts * block_cols) * 4;
-    if (smem > 220 * 1024) ABK_REFUSE("delta rule: heads of %d x %d need more shared memory than an SM has", key, value);
+    const long long need = abk_delta_scan_scratch(n_tokens, n_seqs, heads, key, value, 0);
+    if (need > records_floats || (need && ((uintptr_t)records & 15)))
+        ABK_REFUSE("delta rule: the scratch memory holds %lld floats, the step needs %lld (16-byte aligned)", records_floats, need);
     cudaStream_t s = (cudaStream_t)stream;
     DeltaPrepare q;
     q.qkv = qkv, q.ld_qkv = ld_qkv, q.decay_in = decay_in, q.ld_decay = ld_decay, q.per_head = per_head, q.beta_in = beta_in, q.ld_beta = ld_beta, q.a_log = a_log;
-    q.dt_bias = dt_bias, q.records = records, q.token_seq = token_seq, q.pairs = (long long)n_tokens * heads;
-    q.heads = heads, q.kv_heads = kv_heads, q.key = key, q.value = value, q.parts = parts, q.record = record;
+    q.dt_bias = dt_bias, q.records = records, q.token_seq = token_seq, q.pairs = ((long long)n_tokens / DB_TOKENS + n_seqs) * heads;
+    q.heads = heads, q.kv_heads = kv_heads, q.key = key, q.value = value, q.parts = 0, q.record = (int)delta_block_floats(key, value);
     q.q_scale = 1.0f / sqrtf((float)key);
-    const long long blocks = (q.pairs + 3) / 4;
-    if (blocks > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld (token, head) pairs are more than a grid takes", q.pairs);
-    if (dtype == ABK_BF16) abk_launch(delta_prepare_kernel<__nv_bfloat16>, dim3((unsigned)blocks), dim3(128), 0, s, q);
-    else abk_launch(delta_prepare_kernel<float>, dim3((unsigned)blocks), dim3(128), 0, s, q);
-    int rc = ABK_LAUNCH_RESULT();
-    if (rc) return rc;
     DeltaScan p;
     p.records = records, p.state = state, p.out = out, p.seq_start = seq_start, p.seq_slot = seq_slot;
-    p.heads = heads, p.key = key, p.value = value, p.parts = parts, p.record = record;
-    p.col_warps = col_warps;
-    dim3 grid(n_seqs, heads, (value + block_cols - 1) / block_cols);
-#define SCAN_LAUNCH(MAXT)                                                                                  \
-    do {                                                                                                   \
-        if (smem > 48 * 1024) {                                                                            \
-            cudaError_t e = abk_allow_shared_memory((const void *)delta_scan_kernel<MAXT>, (int)smem);     \
-            if (e != cudaSuccess) return (int)e;                                                           \
-        }                                                                                                  \
-        abk_launch(delta_scan_kernel<MAXT>, grid, dim3(n_warps * 32), smem, s, p);                         \
+    p.heads = heads, p.key = key, p.value = value, p.parts = 0, p.record = q.record;
+    p.vec = key % 4 == 0 && !((uintptr_t)state & 15);
+    if (n_tokens <= n_seqs) {  // a token a sequence (or fewer)
+        // (a CTA a head where that fills the GPU, else one for every 64 of its columns)
+        const int slices = (long long)n_seqs * heads >= 2LL * abk_sm_count() ? 1 : (value + 63) / 64;
+        const dim3 grid(n_seqs, heads, slices < 1 ? 1 : slices > 65535 ? 65535 : slices);
+#define STEP_LAUNCH(LPC, J)                                                                                          \
+    do {                                                                                                             \
+        if (dtype == ABK_BF16) abk_launch(delta_step_kernel<__nv_bfloat16, LPC, J>, grid, dim3(256), 0, s, q, p);    \
+        else abk_launch(delta_step_kernel<float, LPC, J>, grid, dim3(256), 0, s, q, p);                              \
     } while (0)
-    if (n_warps <= 4) SCAN_LAUNCH(128);
-    else if (n_warps <= 8) SCAN_LAUNCH(256);
-    else SCAN_LAUNCH(512);
+        if (key <= 32) STEP_LAUNCH(8, 1);
+        else if (key <= 64) STEP_LAUNCH(16, 1);
+        else if (key <= 128) STEP_LAUNCH(32, 1);
+        else STEP_LAUNCH(32, 2);
+#undef STEP_LAUNCH
+        return ABK_LAUNCH_RESULT();
+    }
+    const long long blocks = (q.pairs + 3) / 4;
+    if (blocks > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld (block, head) pairs are more than a grid takes", q.pairs);
+    const int kp4 = delta_pad_key(key) / 32;
+#define PREPARE_LAUNCH_AS(T, J)                                                                                                          \
+    do {                                                                                                                                 \
+        if (per_head) abk_launch(delta_block_prepare_kernel<T, J, true>, dim3((unsigned)blocks), dim3(128), 0, s, q, seq_start, n_seqs); \
+        else abk_launch(delta_block_prepare_kernel<T, J, false>, dim3((unsigned)blocks), dim3(128), 0, s, q, seq_start, n_seqs);         \
+    } while (0)
+#define PREPARE_LAUNCH(J)                                           \
+    do {                                                            \
+        if (dtype == ABK_BF16) PREPARE_LAUNCH_AS(__nv_bfloat16, J); \
+        else PREPARE_LAUNCH_AS(float, J);                           \
+    } while (0)
+    if (kp4 == 1) PREPARE_LAUNCH(1);
+    else if (kp4 == 2) PREPARE_LAUNCH(2);
+    else if (kp4 == 4) PREPARE_LAUNCH(4);
+    else PREPARE_LAUNCH(8);
+#undef PREPARE_LAUNCH
+#undef PREPARE_LAUNCH_AS
+    int rc = ABK_LAUNCH_RESULT();
+    if (rc) return rc;
+    // A warp's columns, 4 or 8: the fewer, the more warps share the work and the less each waits for in a block; the more,
+    // the less a column costs. Heads of 128 x 128, one prompt: of 1,999 tokens and 16 heads 298 us against 366, of 1,500
+    // tokens and 32 heads 331 against 286; 8 prompts, 5,672 tokens, 32 heads: 960 against 701. Four columns therefore up to
+    // what gives every SM one CTA of them.
+    const long long columns = (long long)n_seqs * heads * value, sms = abk_sm_count();
+    const int per_warp = columns <= 16 * sms ? 4 : 8;
+    int warps = 4;
+    while (warps > 1 && warps * per_warp >= 2 * value) warps /= 2;  // (no CTA of which less than half is used)
+    const int cols = warps * per_warp;
+    size_t smem = (size_t)DB_STAGES * DB_STAGE * (13 * delta_pad_key(key) + DB_NUMBERS + DB_TOKENS * cols) * sizeof(float);
+    // The walk's CTAs start while the preparation's last ones still hold parts of the SMs, and gather where there is room
+    // (one prompt: 601 us against 383): each asks for so much shared memory that no SM takes more than its share.
+    p.tiles = (value + cols - 1) / cols, p.n_seqs = n_seqs;
+    const long long ctas = (long long)n_seqs * heads * p.tiles, share = (ctas + sms - 1) / sms;
+    const size_t least = share <= 4 ? (size_t)(228 * 1024 / (share + 1)) : 0;
+    if (smem < least) smem = least;
+    if (ctas > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld blocks are more than a grid takes", ctas);
+    // (a long walk that starts last would be walked alone: the 8 prompts above 701 us against 1,001 in the step's order)
+    p.longest_first = n_seqs > 1 && n_seqs <= 64 && share > 1;
+#define SCAN_LAUNCH(P, J, C)                                                                               \
+    do {                                                                                                   \
+        cudaError_t e = abk_allow_shared_memory((const void *)delta_block_scan_kernel<P, J, C>, (int)smem); \
+        if (e != cudaSuccess) return (int)e;                                                               \
+        abk_launch(delta_block_scan_kernel<P, J, C>, dim3((unsigned)ctas), dim3(warps * 32 + 32), smem, s, p); \
+    } while (0)
+    const int kind = (kp4 == 1 ? 0 : kp4 == 2 ? 2 : kp4 == 4 ? 4 : 6) + (per_warp == 8);
+    switch (kind) {
+    case 0: SCAN_LAUNCH(8, 1, 1); break;
+    case 1: SCAN_LAUNCH(8, 1, 2); break;
+    case 2: SCAN_LAUNCH(16, 1, 2); break;
+    case 3: SCAN_LAUNCH(16, 1, 4); break;
+    case 4: SCAN_LAUNCH(16, 2, 2); break;
+    case 5: SCAN_LAUNCH(16, 2, 4); break;
+    case 6: SCAN_LAUNCH(16, 4, 2); break;
+    default: SCAN_LAUNCH(16, 4, 4); break;
+    }
 #undef SCAN_LAUNCH
     return ABK_LAUNCH_RESULT();
 }
@@ -755,7 +1180,7 @@ extern "C" int abk_delta_chunks(const void *qkv, long long ld_qkv, int dtype, co
     if (rc) return rc;
     DeltaChunks p;
     p.s.records = records, p.s.state = state, p.s.out = out, p.s.seq_start = seq_start, p.s.seq_slot = seq_slot;
-    p.s.heads = heads, p.s.key = key, p.s.value = value, p.s.parts = parts, p.s.record = record, p.s.col_warps = 1;
+    p.s.heads = heads, p.s.key = key, p.s.value = value, p.s.parts = parts, p.s.record = record, p.s.vec = 0;
     p.work = work, p.n_seqs = n_seqs, p.max_chunks = max_chunks;
     const size_t smem_t = (size_t)(DC_TOKENS * (2 * parts * SCAN_RUN + 4) + 2 * DC_TOKENS * DC_P + 2 * DC_TOKENS) * sizeof(float);
     const size_t smem_s = (size_t)(parts * SCAN_ROWS * DC_VT + 3 * DC_TOKENS * DC_VT + DC_TOKENS * DC_TP + 2 * DC_TOKENS +

@@ -968,8 +968,8 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
     assert a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32 and a_log.numel() == n_heads
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (n_heads, value_dim, key_dim)
     assert out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == n_heads * value_dim
-    records = ws.get("delta_records", (int(lib.abk_delta_scan_scratch(_i(n), _i(n_heads), _i(key_dim), _i(value_dim))),),
-                     torch.float32)
+    records = ws.get("delta_records", (int(lib.abk_delta_scan_scratch(_i(n), _i(n_seqs), _i(n_heads), _i(key_dim), _i(value_dim),
+                                                                      _i(1 if chunks else 0))),), torch.float32)
     if chunks:
         assert per_head, "the chunked form takes one decay a head"
         max_chunks = -(-n // DELTA_CHUNK) + n_seqs

@@ -177,6 +177,29 @@ def test_delta_rule_in_an_unequal_batch_and_in_bfloat16_inputs():
     assert float(state[1].abs().max()) == 0.0 and float(state[2].abs().max()) > 0.0  # only the step's slots are touched
 
 
+@pytest.mark.parametrize("H,K,V,lens", [(3, 32, 7, (9, 1, 6)), (5, 64, 520, (3, 8)), (2, 128, 36, (13,)), (20, 128, 132, (2, 11, 5)),
+                                        (1, 200, 70, (10, 4)), (12, 256, 260, (7, 4, 1)), (40, 30, 66, (4, 5))])
+def test_delta_rule_in_blocks(H, K, V, lens):
+    """Blocks of four tokens and their remainders for every split of the work (few and many columns, every padded key
+    size), sequences of unequal lengths in any order, and the state they leave for a single further token."""
+    from abacus_b200.kernels import ops
+    from abacus_b200.parts import Workspace
+    rng = np.random.default_rng(H * K)
+    ins = [_delta_inputs(rng, n + 1, H, H, K, V) for n in lens]
+    a_log, bias = ins[0][3], ins[0][4]
+    want = [_delta_plain(i[0], i[1], i[2], a_log, bias, H, H, K, V, real=np.float64) for i in ins]
+    noise = max(np.abs(w - _delta_plain(i[0], i[1], i[2], a_log, bias, H, H, K, V)).max() for i, w in zip(ins, want))
+    state, ws = torch.zeros((len(lens), H, V, K), device=DEV), Workspace(torch.device(DEV, torch.cuda.current_device()))
+    for part, at in ((lambda i, n: i[:n], [0] * len(lens)), (lambda i, n: i[n:], list(lens))):
+        b = batch_of([(s, [0] * len(part(i[0], n)), p) for s, (i, n, p) in enumerate(zip(ins, lens, at))])
+        cat = lambda j: dev(np.concatenate([part(i[j], n) for i, n in zip(ins, lens)]))
+        out = torch.empty((cat(0).shape[0], H * V), dtype=torch.float32, device=DEV)
+        ops.delta_scan(cat(0), cat(1), cat(2), dev(a_log), dev(bias), state, out, b, H, H, K, V, ws)
+        expected = np.concatenate([part(w, n) for w, n in zip(want, lens)])
+        # sums of 4 x K products in another order than numpy's: a few times what float32 itself is off here
+        np.testing.assert_allclose(out.cpu().numpy(), expected, rtol=1e-4, atol=2e-5 + 4 * noise)
+
+
 def test_gated_head_norm():
     from abacus_b200.kernels import ops
     rng = np.random.default_rng(1)
