@@ -1,57 +1,130 @@
 // out[M, N] = x[M, K] . w[N, K]^T with float32 multiply-adds on the CUDA cores, for any M, N, K.
 //
 // This is the matrix product of the true 32-bit path (no tensor cores, no TF32), and the
-// fallback of the bfloat16 path for shapes the tensor-core kernel refuses. Every output element
-// is one thread's running sum over k = 0, 1, ..., K-1 in that order, so a row's result does not
-// depend on how many other rows are in the batch or where its tile lies.
+// fallback of the bfloat16 path for shapes the tensor-core kernel refuses. An output element is the sum of eight running
+// sums: K in pieces of 16, piece c to sum c % 8, each sum over its k in ascending order, then in pairs,
+// ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); so a row's result does not depend on how many other rows are in the
+// batch or where its tile lies.
 // Formula: src/model.c:299, 302, 307, 309, 324 (weights are [out, in] row-major, no bias).
+//
+// A CTA has one tile of outputs, and each of its eight warps one of the eight sums of all of them: a product of a few
+// hundred rows has too few outputs to fill 148 SMs with warps whose lanes hold enough of them. Shared memory gives a warp
+// a number a lane and cycle, and an SM's four schedulers share it; a lane with 16 x 8 outputs needs 24 numbers for 128
+// multiply-adds (0.75 of what the schedulers could use up), one with 8 x 8 needs 16 for 64 (all of it). A warp stages its own
+// pieces, 16 bytes at a time by cp.async (rows of 20 floats: eight rows' pieces lie in different banks), one ahead, and meets the
+// others only at the end. Measured (one launch, operands from HBM): 500 x 6144 x 1024 in 204 us and 500 x 1024 x 3072 in 98
+// (31 and 32 TFLOP/s; the kernel that stood here, tiles of 64 x 64 with one sum and 4 x 4 outputs a lane: 329 and 299 us), 1 x
+// 1024 x 3072 in 14.5 us (317). Multiply-adds of three registers alone run at 60 TFLOP/s here; the rest goes to their
+// registers' banks and to waiting for the next piece. Half the tile, twice the CTAs an SM: 259 and 134 us.
 #define ABK_DEFINE_ERROR
 #include "common.cuh"
 
-#define BM 64
-#define BN 64
-#define BK 16
+#define GS_WARPS 8
+#define GS_BK 16
+#define GS_PITCH 20     // floats of a staged row
 
-template <typename TX, typename TW, typename TO>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const TX *__restrict__ x, const TW *__restrict__ w,
-                                                        TO *__restrict__ out, int M, int N, int K, long long ldx,
-                                                        long long ldw, long long ldo) {
-    __shared__ float xs[BK][BM + 4];
-    __shared__ float ws[BK][BN + 4];
-    int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += BK) {
+__device__ __forceinline__ void gs_copy_16(float *dst, const float *src, bool real) {
+    const int bytes = real ? 16 : 0;  // 0: zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+// TM x TN: outputs a lane has, rows 4 apart and columns 8 apart; a tile has 4 TM x 8 TN. ASYNC: float32 operands whose rows
+// start on 16-byte boundaries, K a multiple of 4.
+template <typename TX, typename TW, typename TO, int TM, int TN, bool ASYNC>
+__global__ void __launch_bounds__(32 * GS_WARPS) gemm_simt_kernel(const TX *__restrict__ x, const TW *__restrict__ w, TO *__restrict__ out, int M,
+                                                                  int N, int K, long long ldx, long long ldw, long long ldo) {
+    constexpr int BM = 4 * TM, BN = 8 * TN, STAGE = (BM + BN) * GS_PITCH;
+    extern __shared__ __align__(16) float gs_smem[];  // [warps][2 stages][BM rows of x, then BN of w][20]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tx = lane & 7, ty = lane >> 3;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    float *mine = gs_smem + warp * 2 * STAGE;
+    const int r_mine = lane >> 2, c_mine = (lane & 3) * 4;  // a lane's pieces: every 8th row from here
+    const TX *x_mine = x + (long long)(m0 + r_mine) * ldx + c_mine;
+    const TW *w_mine = w + (long long)(n0 + r_mine) * ldw + c_mine;
+    pdl_wait();
+    const int pieces = (K + GS_BK - 1) / GS_BK;
+    auto fetch = [&](int piece, int stage) {
+        float *dst = mine + stage * STAGE;
+        const int k0 = piece * GS_BK;
+        if constexpr (ASYNC) {
+            const bool in = k0 + c_mine < K;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int idx = tid + i * 256, r = idx >> 4, k = idx & 15;
-            int gm = m0 + r, gn = n0 + r, gk = k0 + k;
-            xs[k][r] = (gm < M && gk < K) ? to_float(x[(long long)gm * ldx + gk]) : 0.0f;
-            ws[k][r] = (gn < N && gk < K) ? to_float(w[(long long)gn * ldw + gk]) : 0.0f;
+            for (int i = 0; i < BM / 8; i++) {
+                const bool real = in && m0 + r_mine + 8 * i < M;
+                gs_copy_16(dst + (r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)x_mine + 8 * i * ldx + k0 : (const float *)x, real);
+            }
+#pragma unroll
+            for (int i = 0; i < BN / 8; i++) {
+                const bool real = in && n0 + r_mine + 8 * i < N;
+                gs_copy_16(dst + (BM + r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)w_mine + 8 * i * ldw + k0 : (const float *)w, real);
+            }
+        } else {
+            for (int e = lane; e < (BM + BN) * GS_BK; e += 32) {
+                const int r = e / GS_BK, c = e % GS_BK, k = k0 + c;
+                float v = 0.0f;
+                if (r < BM) {
+                    if (m0 + r < M && k < K) v = to_float(x[(long long)(m0 + r) * ldx + k]);
+                } else if (n0 + r - BM < N && k < K) {
+                    v = to_float(w[(long long)(n0 + r - BM) * ldw + k]);
+                }
+                dst[r * GS_PITCH + c] = v;
+            }
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[TM][TN];
 #pragma unroll
-        for (int k = 0; k < BK; k++) {
-            float a[4], b[4];
+    for (int i = 0; i < TM; i++)
 #pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = xs[k][ty * 4 + i], b[i] = ws[k][tx * 4 + i];
+        for (int j = 0; j < TN; j++) acc[i][j] = 0.0f;
+    if (warp < pieces) fetch(warp, 0);
+    for (int piece = warp, it = 0; piece < pieces; piece += GS_WARPS, it++) {
+        if (piece + GS_WARPS < pieces) fetch(piece + GS_WARPS, (it + 1) & 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const float *xs = mine + (it & 1) * STAGE + ty * GS_PITCH, *ws = mine + (it & 1) * STAGE + (BM + tx) * GS_PITCH;
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+        for (int k = 0; k < GS_BK; k += 2) {
+            float2 a[TM], b[TN];
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            for (int j = 0; j < TN; j++) b[j] = *(const float2 *)(ws + j * 8 * GS_PITCH + k);
+#pragma unroll
+            for (int i = 0; i < TM; i++) a[i] = *(const float2 *)(xs + i * 4 * GS_PITCH + k);
+#pragma unroll
+            for (int i = 0; i < TM; i++)
+#pragma unroll
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, acc[i][j]));
         }
-        __syncthreads();
+        __syncwarp();  // the stage is filled again by the iteration after next
     }
+    __syncthreads();
+    constexpr int PITCH = BN + 8, TILE = BM * PITCH;  // (four rows' runs of eight columns lie in different banks)
+    float *sums = gs_smem;  // [warps][BM][PITCH]
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
+    for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int gn = n0 + tx * 4 + j;
-            if (gn < N) out[(long long)gm * ldo + gn] = from_float<TO>(acc[i][j]);
-        }
+        for (int j = 0; j < TN; j++) sums[warp * TILE + (ty + 4 * i) * PITCH + tx + 8 * j] = acc[i][j];
+    __syncthreads();
+    for (int e = threadIdx.x; e < BM * BN; e += 32 * GS_WARPS) {
+        const int r = e / BN, c = e % BN;
+        const float *s = sums + r * PITCH + c;
+        if (m0 + r < M && n0 + c < N)
+            out[(long long)(m0 + r) * ldo + n0 + c] = from_float<TO>(((s[0] + s[TILE]) + (s[2 * TILE] + s[3 * TILE])) + ((s[4 * TILE] + s[5 * TILE]) + (s[6 * TILE] + s[7 * TILE])));
     }
+}
+
+template <typename TX, typename TW, typename TO, int TM, int TN, bool ASYNC>
+static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int N, int K, long long ldx, long long ldw, long long ldo, cudaStream_t s) {
+    constexpr int BM = 4 * TM, BN = 8 * TN;
+    constexpr int ring = GS_WARPS * 2 * (BM + BN) * GS_PITCH * 4, sums = GS_WARPS * BM * (BN + 8) * 4, smem = ring > sums ? ring : sums;
+    const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
+    if (grid.y > 65535) ABK_REFUSE("gemm: %d output columns are more than one launch takes", N);
+    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_simt_kernel<TX, TW, TO, TM, TN, ASYNC>, smem);
+    if (e != cudaSuccess) return (int)e;
+    abk_launch(gemm_simt_kernel<TX, TW, TO, TM, TN, ASYNC>, grid, dim3(32 * GS_WARPS), smem, s, (const TX *)x, (const TW *)w, (TO *)out, M, N, K, ldx,
+               ldw, ldo);
+    return ABK_LAUNCH_RESULT();
 }
 
 // x_dtype/w_dtype/out_dtype: ABK_F32 or ABK_BF16. Supported: all-float32; bf16 x and w with bf16 or f32 out.
@@ -59,17 +132,22 @@ extern "C" int abk_gemm_simt(const void *x, int x_dtype, const void *w, int w_dt
                              int N, int K, long long ldx, long long ldw, long long ldo, void *stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) ABK_REFUSE("gemm: K = %d", K);
-    dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
-    if (grid.y > 65535) ABK_REFUSE("gemm: %d output columns are more than one launch takes", N);
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
-    if (x_dtype == ABK_F32 && w_dtype == ABK_F32 && out_dtype == ABK_F32)
-        gemm_simt_kernel<<<grid, 256, 0, s>>>((const float *)x, (const float *)w, (float *)out, M, N, K, ldx, ldw, ldo);
-    else if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_BF16)
-        gemm_simt_kernel<<<grid, 256, 0, s>>>((const bf *)x, (const bf *)w, (bf *)out, M, N, K, ldx, ldw, ldo);
-    else if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_F32)
-        gemm_simt_kernel<<<grid, 256, 0, s>>>((const bf *)x, (const bf *)w, (float *)out, M, N, K, ldx, ldw, ldo);
-    else
-        ABK_REFUSE("gemm: dtype combination x=%d w=%d out=%d is not built", x_dtype, w_dtype, out_dtype);
-    return ABK_LAUNCH_RESULT();
+    // Tiles of 64 x 64 where they fill two thirds of the SMs, else of 32 x 32 (of 16 x 16 for up to 16 rows; tiles of 64
+    // where smaller ones were more than a grid takes): 64 x 1024 x 3072, 16 large tiles or 64 of 32 x 32, in 114 or 34 us.
+    const long long large = (long long)((M + 63) / 64) * ((N + 63) / 64);
+    const int tile = large >= abk_sm_count() * 2 / 3 || N > 65535 * 16 ? 64 : M > 16 ? 32 : 16;
+#define GS_LAUNCH(TX, TW, TO, ASYNC)                                                                              \
+    (tile == 64   ? gemm_simt_launch<TX, TW, TO, 16, 8, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)              \
+     : tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)               \
+                  : gemm_simt_launch<TX, TW, TO, 4, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s))
+    if (x_dtype == ABK_F32 && w_dtype == ABK_F32 && out_dtype == ABK_F32) {
+        const bool aligned = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !(((uintptr_t)x | (uintptr_t)w) & 15);
+        return aligned ? GS_LAUNCH(float, float, float, true) : GS_LAUNCH(float, float, float, false);
+    }
+    if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_BF16) return GS_LAUNCH(bf, bf, bf, false);
+    if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_F32) return GS_LAUNCH(bf, bf, float, false);
+#undef GS_LAUNCH
+    ABK_REFUSE("gemm: dtype combination x=%d w=%d out=%d is not built", x_dtype, w_dtype, out_dtype);
 }

@@ -131,6 +131,21 @@ def test_gemm_simt(ops, m, n, k):
             out.cpu().numpy(), plain.linear(xb, wb), rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("n, k", [(900, 132), (900, 16), (1000, 300)])
+def test_gemm_simt_tiles_give_the_same_bits(ops, n, k):
+    """The tiles of 64, 32 and 16 and the loads of single elements (rows that start on no 16-byte boundary) add in one order."""
+    rng = np.random.default_rng(n + k)
+    x, w = dev(rng.standard_normal((700, k)).astype(np.float32)), dev(rng.standard_normal((n, k)).astype(np.float32))
+    shifted = [torch.empty(t.shape[0], k + 5, device="cuda")[:, 1:k + 1].copy_(t) for t in (x, w)]
+    whole, out = torch.empty(700, n, device="cuda"), torch.empty(700, n, device="cuda")
+    ops.gemm_simt(x, w, whole)
+    np.testing.assert_allclose(whole.cpu().numpy(), plain.linear(x.cpu().numpy(), w.cpu().numpy()), rtol=1e-5, atol=2e-6 * k)
+    for rows in (700, 77, 20, 16, 3):
+        for a, b in ((x, w), shifted):
+            ops.gemm_simt(a[:rows], b, out, rows)
+            assert torch.equal(out[:rows], whole[:rows])
+
+
 def test_gemm_simt_rows_do_not_depend_on_the_batch(ops):
     """The float32 product sums over k in one fixed order: a row alone equals the row in a batch, bit for bit."""
     rng = np.random.default_rng(5)
