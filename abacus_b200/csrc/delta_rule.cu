@@ -12,7 +12,7 @@
 // keeps (a part of) one column in registers and walks the sequence's tokens in order, and a prompt of any length
 // and a decode step are the same kernel. The state is stored [head, value, key], so a column is one contiguous run.
 #define ABK_DEFINE_ERROR
-#include "common.cuh"
+#include "recurrence.cuh"
 
 #define CONV_MAX_TAPS 8
 
@@ -436,29 +436,6 @@ template <typename T, int J, bool PER_HEAD> __global__ void __launch_bounds__(12
     if (lane < DB_NUMBERS) rec[13 * DP + lane] = mine;
 }
 
-// Two float32 at once: each half rounded as the single instruction rounds it.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-    return d;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-    float2 f;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-    return f;
-}
-
 __device__ __forceinline__ void scan_copy_16(uint32_t dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -490,22 +467,6 @@ __device__ __forceinline__ void delta_store_state(float *column, int ch, int K, 
     }
 }
 
-// The sequence that comes `place`-th when the step's are ordered from the longest to the shortest; whole warps call it, up
-// to 64 sequences.
-__device__ __forceinline__ int delta_place(const int *seq_start, int n_seqs, int place) {
-    const int lane = threadIdx.x & 31;
-    const int a = lane < n_seqs ? seq_start[lane + 1] - seq_start[lane] : -1;
-    const int b = lane + 32 < n_seqs ? seq_start[lane + 33] - seq_start[lane + 32] : -1;
-    int before_a = 0, before_b = 0;  // how many come before this lane's two
-    for (int j = 0; j < n_seqs; j++) {
-        const int other = __shfl_sync(0xffffffffu, j < 32 ? a : b, j & 31);
-        before_a += other > a || (other == a && j < lane), before_b += other > b || (other == b && j < lane + 32);
-    }
-    const unsigned hit_a = __ballot_sync(0xffffffffu, lane < n_seqs && before_a == place);
-    const unsigned hit_b = __ballot_sync(0xffffffffu, lane + 32 < n_seqs && before_b == place);
-    return hit_a ? __ffs(hit_a) - 1 : 31 + __ffs(hit_b);
-}
-
 // P lanes share a value column, each with 4 J of its key channels (lane p: 4 p .. 4 p + 3 of every 4 P, so that together
 // they read a vector as whole lines); a lane has C columns, 4 J C numbers of state in registers, and every piece of a
 // vector it reads serves them all: a 16-byte read costs the warp four cycles of shared memory whatever the lanes share, so
@@ -528,7 +489,7 @@ __global__ void __launch_bounds__(160) delta_block_scan_kernel(DeltaScan p) {
     const int col0 = tile * cols, first_col = col0 + tid / P * C;  // this lane's columns: first_col ..
     const int K = p.key, V = p.value;
     pdl_wait();
-    const int seq = p.longest_first ? delta_place(p.seq_start, p.n_seqs, place) : place;
+    const int seq = p.longest_first ? sequence_place(p.seq_start, p.n_seqs, place) : place;
     const int row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
     if (n <= 0) return;
     const int n_blocks = (n + DB_TOKENS - 1) / DB_TOKENS;
@@ -889,7 +850,7 @@ extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, cons
     if (smem < least) smem = least;
     if (ctas > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld blocks are more than a grid takes", ctas);
     // (a long walk that starts last would be walked alone: the 8 prompts above 701 us against 1,001 in the step's order)
-    p.longest_first = n_seqs > 1 && n_seqs <= 64 && share > 1;
+    p.longest_first = n_seqs > 1 && n_seqs <= SEQUENCE_PLACE_MAX && share > 1;
 #define SCAN_LAUNCH(P, J, C)                                                                               \
     do {                                                                                                   \
         cudaError_t e = abk_allow_shared_memory((const void *)delta_block_scan_kernel<P, J, C>, (int)smem); \

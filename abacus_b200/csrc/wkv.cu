@@ -7,14 +7,15 @@
 //                     last row of the step before, kept in its slot, for a step's first row; zeros at the start), one
 //                     plane of the output per s. In a step of one token a sequence it also leaves the new last row.
 //   token_shift_keep  the last row of every sequence of a step of prompts, into its slot.
-//   wkv_scan          a CTA walks one sequence's tokens for one head and 16 (32 for heads of up to 32 channels) value
+//   wkv_block         prompts: blocks of four tokens (below)
+//   wkv_scan          a step of one token a sequence: a CTA walks one sequence's tokens for one head and 16 (32 for heads of up to 32 channels) value
 //                     columns. Its threads are those columns x 4, 8 or 16 parts of the key channels, so a thread keeps 4
 //                     to 16 state values in registers; the parts' partial outputs of a column meet by shuffles, four
 //                     tokens at a time. Rows come 16 (8 for heads beyond 128 channels) tokens at a time: asked for a
 //                     chunk ahead into registers, the decay made from its pre-activation on the way into shared memory,
 //                     read from there as 16-byte pieces. A sequence that brings no token to the step is left alone.
 #define ABK_DEFINE_ERROR
-#include "common.cuh"
+#include "recurrence.cuh"
 
 // ---------------------------------------------------------------- the blends with the token before
 struct TokenShift {
@@ -180,53 +181,14 @@ struct WkvScan {
     float *state;        // [slots][heads][dim][dim] (key, value)
     float *out;          // [tokens][heads * dim]
     const int *seq_start, *seq_slot;
-    // A step of prompts runs in segments of `chunk` tokens, all at once (blockIdx.z counts the step's segments, sequence
-    // after sequence): phase 1 walks each segment from an empty state and leaves its sum and the product of its decays,
-    // wkv_segment_prefix turns the sums into the states at the segments' starts (and leaves the last in the slot), phase 2
-    // walks each segment again from its start state for the outputs. chunk 0 (phase 0): a CTA walks a whole sequence.
-    int chunk, phase, n_seqs;
-    float *sums;         // [segments][heads][dim][dim]
-    float *prods;        // [segments][heads][dim]
+    int n_seqs, tiles, longest_first, vec;  // of the walk in blocks
 };
-
-// The segment blockIdx.z names: its sequence, its first row and its rows (0: none). Sequences are walked in order.
-__device__ __forceinline__ void wkv_segment(const int *seq_start, int n_seqs, int chunk, int z, int &seq, int &row0, int &n) {
-    n = 0;
-    int first = 0;
-    for (seq = 0; seq < n_seqs; seq++) {
-        const int start = seq_start[seq], len = seq_start[seq + 1] - start, count = (len + chunk - 1) / chunk;
-        if (z < first + count) {
-            const int c = z - first;
-            row0 = start + c * chunk, n = len - c * chunk < chunk ? len - c * chunk : chunk;
-            return;
-        }
-        first += count;
-    }
-}
 
 // N tokens of one thread's share: r, k, w point at the thread's channels of the first token (tokens `pitch` floats
 // apart), v at its column's value (tokens `v_pitch` apart); the column's output goes to out if `writes`.
-// SUMS: the state alone moves (a segment's own sum): no r, no output.
-template <int DPT, int PARTS, int N, bool SUMS>
+template <int DPT, int PARTS, int N>
 __device__ __forceinline__ void wkv_tokens(float *s, const float *u, const float *r, const float *k, const float *w, int pitch,
                                            const float *v, int v_pitch, bool writes, float *out, long long out_pitch) {
-    if constexpr (SUMS) {
-        float vv[N];
-#pragma unroll
-        for (int n = 0; n < N; n++) vv[n] = v[n * v_pitch];
-#pragma unroll
-        for (int i = 0; i < DPT / 4; i++) {
-            float4 kk[N], ww[N];
-#pragma unroll
-            for (int n = 0; n < N; n++) kk[n] = *(const float4 *)(k + n * pitch + 4 * i), ww[n] = *(const float4 *)(w + n * pitch + 4 * i);
-#pragma unroll
-            for (int n = 0; n < N; n++) {
-                s[4 * i] = fmaf(ww[n].x, s[4 * i], kk[n].x * vv[n]), s[4 * i + 1] = fmaf(ww[n].y, s[4 * i + 1], kk[n].y * vv[n]);
-                s[4 * i + 2] = fmaf(ww[n].z, s[4 * i + 2], kk[n].z * vv[n]), s[4 * i + 3] = fmaf(ww[n].w, s[4 * i + 3], kk[n].w * vv[n]);
-            }
-        }
-        return;
-    }
     float vv[N], o[N];
 #pragma unroll
     for (int n = 0; n < N; n++) vv[n] = v[n * v_pitch], o[n] = 0.0f;
@@ -265,7 +227,7 @@ __device__ __forceinline__ void wkv_tokens(float *s, const float *u, const float
 template <typename T> __device__ __forceinline__ float wkv_decay(float z) { return expf(-expf(z)); }
 template <> __device__ __forceinline__ float wkv_decay<__nv_bfloat16>(float z) { return __expf(-__expf(z)); }
 
-template <typename T, int DPT, int PARTS, int COLS, int TOK, bool SUMS>
+template <typename T, int DPT, int PARTS, int COLS, int TOK>
 __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
     constexpr int DP = DPT * PARTS;             // key channels, padded
     constexpr int PITCH = PARTS * (DPT + 4);    // a token's channels in shared memory: a part's run, then 4 floats of
@@ -283,19 +245,15 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
         u[i] = d < p.dim ? p.bonus[(long long)h * p.dim + d] : 0.0f;
     }
     pdl_wait();
-    int seq = blockIdx.z, row0, n;
-    if (p.chunk > 0) wkv_segment(p.seq_start, p.n_seqs, p.chunk, blockIdx.z, seq, row0, n);
-    else row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
+    const int seq = blockIdx.z, row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
     if (n <= 0) return;  // (a sequence of the step's padding: its slot is someone else's)
-    float *state = p.phase == 0 ? p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * p.dim * p.dim
-                                : p.sums + ((long long)blockIdx.z * p.n_heads + h) * p.dim * p.dim;
+    float *state = p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * p.dim * p.dim;
     float s[DPT];
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
         const int d = part * DPT + i;
-        s[i] = p.phase != 1 && d < p.dim && col < p.dim ? state[(long long)d * p.dim + col] : 0.0f;
+        s[i] = d < p.dim && col < p.dim ? state[(long long)d * p.dim + col] : 0.0f;
     }
-    float decayed = 1.0f;  // phase 1: the product of this thread's staged decays (one channel, its share of the tokens)
     const T *proj = (const T *)p.proj;
     const long long hk = (long long)p.n_heads * p.dim;
     // A chunk's rows are asked for a chunk ahead and kept as they come: nothing is done to a loaded value before the
@@ -316,8 +274,7 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
             const int tok = (tid + it * THREADS) / DP;
             const long long row = row0 + c0 + (tok < cnt ? tok : cnt - 1);
             const T *r = proj + row * p.ld + my_ch;
-            if (!SUMS) rr[it] = r[p.r_at];
-            rk[it] = r[p.k_at], rz[it] = p.pre[row * hk + my_ch];
+            rr[it] = r[p.r_at], rk[it] = r[p.k_at], rz[it] = p.pre[row * hk + my_ch];
         }
 #pragma unroll
         for (int it = 0; it < PER_V; it++) {
@@ -336,9 +293,8 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
             const int tok = (tid + it * THREADS) / DP, at = (my_d / DPT) * (DPT + 4) + my_d % DPT;
             const bool in = tok < cnt && my_d < p.dim;
             const float w = wkv_decay<T>(rz[it] + my_w0);
-            if (!SUMS) r_s[tok][at] = in ? to_float(rr[it]) : 0.0f;
+            r_s[tok][at] = in ? to_float(rr[it]) : 0.0f;
             k_s[tok][at] = in ? to_float(rk[it]) : 0.0f, w_s[tok][at] = w;
-            if (in) decayed *= w;
         }
 #pragma unroll
         for (int it = 0; it < PER_V; it++) {
@@ -351,102 +307,386 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
         // multiply-adds follow one another
         const int at = part * (DPT + 4);
         float *out = p.out + (long long)(row0 + c0) * hk + (long long)h * p.dim + col;
-        const bool writes = part == 0 && col < p.dim && p.phase != 1;
+        const bool writes = part == 0 && col < p.dim;
         int tok = 0;
         for (; tok + 4 <= cnt; tok += 4)
-            wkv_tokens<DPT, PARTS, 4, SUMS>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
+            wkv_tokens<DPT, PARTS, 4>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
         for (; tok < cnt; tok++)
-            wkv_tokens<DPT, PARTS, 1, SUMS>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
+            wkv_tokens<DPT, PARTS, 1>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
     }
-    if (p.phase == 2) return;  // (the states between segments are wkv_segment_prefix's)
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
         const int d = part * DPT + i;
         if (d < p.dim && col < p.dim) state[(long long)d * p.dim + col] = s[i];
     }
-    if (p.phase == 1 && tile == 0) {
-        // every thread staged the decays of one channel: the shares of a channel meet through shared memory
-        __syncthreads();
-        float *share = &r_s[0][0];
-        share[tid] = decayed;
-        __syncthreads();
-        if (tid < DP && tid < p.dim) {
-            float all = 1.0f;
-            for (int o = tid; o < THREADS; o += DP) all *= share[o];
-            p.prods[((long long)blockIdx.z * p.n_heads + h) * p.dim + tid] = all;
-        }
-    }
 }
 
-// The states at the segments' starts from the segments' own sums: along a sequence S <- prod * S + sum, the state before
-// each segment left where its sum was, the last in the sequence's slot. A thread an element of the state; four segments'
-// loads are on their way together.
-__global__ void __launch_bounds__(256) wkv_segment_prefix_kernel(float *sums, const float *prods, float *state, const int *seq_start,
-                                                                 const int *seq_slot, int n_heads, int dim, int chunk) {
-    const int e = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, seq = blockIdx.z;
+// ---------------------------------------------------------------- the recurrence, prompts: in blocks of four tokens
+// With S the state before a block of four, G_i = w_1 .. w_i its decays up to token i (elementwise over the key channels) and
+// G_ij = w_(j+1) .. w_i,
+//     o_i = S^T (G_(i-1) r_i) + sum over j < i of [r_i . G_(i-1)j k_j] v_j + [r_i . u k_i] v_i,   S <- G_4 S + sum_j (G_4j k_j) v_j^T
+// (decays multiplied, never divided). The nine vectors and ten numbers of a block know neither the state nor the values:
+// four warps of the CTA make them, a block each, and put them into shared memory while the walking warps are at the four
+// blocks before. What a walker does to the state is nine multiply-adds an element and four tokens (twelve token by token),
+// two elements an instruction. P lanes share a value column, each with 4 J of its key channels (lane p: 4 p .. 4 p + 3 of
+// every 4 P); a lane has C columns, and a piece of a vector it reads serves them all. Float32 throughout, the same numbers
+// as token by token in another order of sums. Bound by instructions: a block costs a walker some 290 and a maker 600, and an
+// SM with one CTA runs them at half its issue rate; 3 prompts, 3,571 tokens, 40 heads of 64: 245 us (segments walked twice
+// token by token, with the states between them made from the segments' sums, took 480 + 253 + 42 us).
+#define WB_TOKENS 4
+#define WB_NUMBERS 12   // ten, and the next multiple of four
+#define WB_WALKERS 4    // warps
+#define WB_MAKERS 4     // warps, and blocks of a stage; two stages
+
+template <int BYTES> struct WkvPiece;
+template <> struct WkvPiece<2> { typedef uint16_t type; };
+template <> struct WkvPiece<4> { typedef uint32_t type; };
+template <> struct WkvPiece<8> { typedef uint2 type; };
+template <> struct WkvPiece<16> { typedef uint4 type; };
+struct __align__(16) WkvPiece32 { uint4 a, b; };
+template <> struct WkvPiece<32> { typedef WkvPiece32 type; };
+// N floats (1, 2, or a multiple of 4) as pieces of up to 16 bytes.
+template <int N> __device__ __forceinline__ void wkv_load_floats(float *dst, const float *src) {
+    if constexpr (N == 1) dst[0] = *src;
+    else if constexpr (N == 2) *(float2 *)dst = *(const float2 *)src;
+    else
+#pragma unroll
+        for (int i = 0; i < N; i += 4) *(float4 *)(dst + i) = *(const float4 *)(src + i);
+}
+template <int N> __device__ __forceinline__ void wkv_store_floats(float *dst, const float *src) {
+    if constexpr (N == 1) *dst = src[0];
+    else if constexpr (N == 2) *(float2 *)dst = make_float2(src[0], src[1]);
+    else
+#pragma unroll
+        for (int i = 0; i < N; i += 4) *(float4 *)(dst + i) = make_float4(src[i], src[i + 1], src[i + 2], src[i + 3]);
+}
+
+template <typename T, int P, int J, int C>
+__global__ void __launch_bounds__(32 * (WB_WALKERS + WB_MAKERS)) wkv_block_kernel(WkvScan p) {
+    constexpr int DP = 4 * P * J, JL = DP / 32, COLS = WB_WALKERS * 32 / P * C, HEAD = 9 * DP + WB_NUMBERS, RS = HEAD + WB_TOKENS * COLS;
+    extern __shared__ __align__(16) float wb_smem[];  // [2 stages][WB_MAKERS blocks][RS]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int h = blockIdx.x % p.n_heads, tile = blockIdx.x / p.n_heads % p.tiles, place = blockIdx.x / p.n_heads / p.tiles;
+    const int col0 = tile * COLS, D = p.dim;
+    const long long hk = (long long)p.n_heads * D;
+    const bool makes = warp >= WB_WALKERS;
+    float w0[JL], bonus[JL];
+    if (makes) {
+#pragma unroll
+        for (int j = 0; j < JL; j++) {
+            const int c = min(lane * JL + j, D - 1);
+            w0[j] = p.w0[(long long)h * D + c], bonus[j] = p.bonus[(long long)h * D + c];  // weights: ahead of the wait
+        }
+    }
     pdl_wait();
-    const int len = seq_start[seq + 1] - seq_start[seq];
-    if (len <= 0 || e >= dim * dim) return;
-    int first = 0;
-    for (int q = 0; q < seq; q++) first += (seq_start[q + 1] - seq_start[q] + chunk - 1) / chunk;
-    const int count = (len + chunk - 1) / chunk, d = e / dim;
-    float *slot = state + ((long long)seq_slot[seq] * n_heads + h) * dim * dim + e;
-    float S = *slot;
-    for (int c0 = 0; c0 < count; c0 += 4) {
-        float u[4], pr[4];
+    const int seq = p.longest_first ? sequence_place(p.seq_start, p.n_seqs, place) : place;
+    const int row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
+    if (n <= 0) return;  // (a sequence of the step's padding: its slot is someone else's)
+    const int n_blocks = (n + WB_TOKENS - 1) / WB_TOKENS, n_stages = (n_blocks + WB_MAKERS - 1) / WB_MAKERS;
+    if (makes) {
+        constexpr int VL = (WB_TOKENS * COLS + 31) / 32;  // values a lane brings
+        typedef typename WkvPiece<sizeof(T) * JL>::type TPiece;
+        const int mine = warp - WB_WALKERS;
+        const int c_mine = lane * JL < D ? lane * JL : 0, k_from_r = p.k_at - p.r_at;  // (lanes beyond the head bring what is not used)
+        const T *mine_proj = (const T *)p.proj + h * D + p.r_at + c_mine, *head_values = (const T *)p.proj + h * D + p.v_at;
+        const float *mine_pre = p.pre + h * D + c_mine;
+        struct __align__(16) Rows {  // a block's rows as they come
+            T r_in[WB_TOKENS][JL], k_in[WB_TOKENS][JL];
+            float z_in[WB_TOKENS][JL];
+            T v_in[VL];
+        } even, odd;
+        auto ask = [&](Rows &w, int block) {
+            if (block >= n_blocks) return;
+            const int t0 = block * WB_TOKENS;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const long long at = (long long)(first + (c0 + i < count ? c0 + i : count - 1)) * n_heads + h;
-            u[i] = sums[at * dim * dim + e], pr[i] = prods[at * dim + d];
+            for (int i = 0; i < WB_TOKENS; i++) {
+                const long long row = row0 + min(t0 + i, n - 1);
+                const T *src = mine_proj + row * p.ld;
+                const float *z = mine_pre + row * hk;
+                if (p.vec) {  // a lane's channels of a row as one piece
+                    *(TPiece *)w.r_in[i] = *(const TPiece *)src, *(TPiece *)w.k_in[i] = *(const TPiece *)(src + k_from_r);
+                    wkv_load_floats<JL>(w.z_in[i], z);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < JL; j++) {
+                        const int c = min(lane * JL + j, D - 1) - c_mine;
+                        w.r_in[i][j] = src[c], w.k_in[i][j] = src[k_from_r + c], w.z_in[i][j] = z[c];
+                    }
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < VL; e++) {
+                const int at = lane + 32 * e, i = at / COLS, c = col0 + at % COLS;
+                w.v_in[e] = head_values[(row0 + min(t0 + min(i, WB_TOKENS - 1), n - 1)) * p.ld + min(c, D - 1)];
+            }
+        };
+        auto make = [&](const Rows &in, int block) {
+            if (block >= n_blocks) return;
+            float *rec = wb_smem + ((block / WB_MAKERS % 2) * WB_MAKERS + mine) * RS;
+            const int count = min(WB_TOKENS, n - block * WB_TOKENS);
+            float num[16], R[WB_TOKENS][JL], U[WB_TOKENS][JL], G[JL];
+#pragma unroll
+            for (int e = 0; e < 16; e++) num[e] = 0.0f;
+#pragma unroll
+            for (int j = 0; j < JL; j++) {
+                const bool channel = lane * JL + j < D;
+                G[j] = 1.0f;  // U[s]: G_(i-1)s k_s on the way
+#pragma unroll
+                for (int i = 0; i < WB_TOKENS; i++) {
+                    const bool real = i < count && channel;
+                    const float r = real ? to_float(in.r_in[i][j]) : 0.0f, k = real ? to_float(in.k_in[i][j]) : 0.0f;
+                    const float w = real ? wkv_decay<T>(in.z_in[i][j] + w0[j]) : 1.0f;
+                    R[i][j] = G[j] * r;
+#pragma unroll
+                    for (int s = 0; s < i; s++) {
+                        num[i * (i + 1) / 2 + s] = fmaf(r, U[s][j], num[i * (i + 1) / 2 + s]);
+                        U[s][j] *= w;
+                    }
+                    num[i * (i + 1) / 2 + i] = fmaf(r * bonus[j], k, num[i * (i + 1) / 2 + i]);
+                    U[i][j] = k;
+                    G[j] *= w;
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < WB_TOKENS; i++)
+                wkv_store_floats<JL>(rec + i * DP + lane * JL, R[i]), wkv_store_floats<JL>(rec + (4 + i) * DP + lane * JL, U[i]);
+            wkv_store_floats<JL>(rec + 8 * DP + lane * JL, G);
+            // the ten sums across the warp: half of a lane's handed over at each step, so that a pair of lanes ends with one
+#pragma unroll
+            for (int half = 8, bit = 16; half > 0; half >>= 1, bit >>= 1) {
+                const bool up = lane & bit;
+#pragma unroll
+                for (int e = 0; e < half; e++) {
+                    const float give = up ? num[e] : num[e + half], keep = up ? num[e + half] : num[e];
+                    num[e] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            }
+            num[0] += __shfl_xor_sync(0xffffffffu, num[0], 1);
+            if (!(lane & 1) && (lane >> 1) < WB_NUMBERS) rec[9 * DP + (lane >> 1)] = num[0];  // (bit 16 counts eight, .., bit 2 one)
+#pragma unroll
+            for (int e = 0; e < VL; e++) {
+                const int at = lane + 32 * e, i = at / COLS, c = col0 + at % COLS;
+                if (at < WB_TOKENS * COLS) rec[HEAD + at] = i < count && c < D ? to_float(in.v_in[e]) : 0.0f;
+            }
+        };
+        ask(even, mine);
+        ask(odd, WB_MAKERS + mine);
+        make(even, mine);
+        for (int s = 0; s < n_stages; s++) {
+            // stage s is made, and stage s - 1 has been read: its place is filled again, from rows asked for a stage ago
+            __syncthreads();
+            if (s & 1) ask(odd, (s + 2) * WB_MAKERS + mine), make(even, (s + 1) * WB_MAKERS + mine);
+            else ask(even, (s + 2) * WB_MAKERS + mine), make(odd, (s + 1) * WB_MAKERS + mine);
         }
+        return;
+    }
+    const int part = lane & (P - 1), own = tid / P * C, first_col = col0 + own;
+    float *state = p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * D * D;
+    f32x2 S[C][2 * J];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            if (c0 + i >= count) break;
-            sums[((long long)(first + c0 + i) * n_heads + h) * dim * dim + e] = S;
-            S = fmaf(pr[i], S, u[i]);
+    for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            float v[4];
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                const int ch = 4 * (P * j + part) + x;
+                v[x] = ch < D && first_col + c < D ? state[(long long)ch * D + first_col + c] : 0.0f;
+            }
+            S[c][2 * j] = pack2(v[0], v[1]), S[c][2 * j + 1] = pack2(v[2], v[3]);
+        }
+    constexpr int BITS = P == 16 ? 4 : 3, COL_STEPS = C == 4 ? 2 : C == 2 ? 1 : 0, TOK_STEPS = BITS - COL_STEPS < 2 ? BITS - COL_STEPS : 2;
+    constexpr int REST = P >> (COL_STEPS + TOK_STEPS);  // lanes that end with the same sums
+    const int my_c = part >> (BITS - COL_STEPS), my_t = (part / REST) & ((1 << TOK_STEPS) - 1);  // this lane's column and tokens
+    const int my_col = first_col + my_c;
+    float *out = p.out + (long long)row0 * hk + (long long)h * D + my_col;
+    for (int s = 0; s < n_stages; s++) {
+        __syncthreads();
+#pragma unroll 1
+        for (int b = 0; b < WB_MAKERS; b++) {
+            const int left = n - (s * WB_MAKERS + b) * WB_TOKENS;
+            if (left <= 0) break;
+            const float *rec = wb_smem + ((s & 1) * WB_MAKERS + b) * RS, *vec = rec + 4 * part;
+            float sums[C][4], vv[4][C];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                f32x2 a[C];
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    const ulonglong2 w = *(const ulonglong2 *)(vec + i * DP + 4 * P * j);
+#pragma unroll
+                    for (int c = 0; c < C; c++) {
+                        a[c] = j == 0 ? mul2(w.x, S[c][0]) : fma2(w.x, S[c][2 * j], a[c]);
+                        a[c] = fma2(w.y, S[c][2 * j + 1], a[c]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < C; c++) {
+                    const float2 x = unpack2(a[c]);
+                    sums[c][i] = x.x + x.y;
+                }
+                const float *vs = rec + HEAD + i * COLS + own;
+                if constexpr (C == 4) {
+                    const float4 x = *(const float4 *)vs;
+                    vv[i][0] = x.x, vv[i][1] = x.y, vv[i][2] = x.z, vv[i][3] = x.w;
+                } else if constexpr (C == 2) {
+                    const float2 x = *(const float2 *)vs;
+                    vv[i][0] = x.x, vv[i][1] = x.y;
+                } else {
+                    vv[i][0] = vs[0];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+                const ulonglong2 w = *(const ulonglong2 *)(vec + 8 * DP + 4 * P * j);
+#pragma unroll
+                for (int c = 0; c < C; c++) S[c][2 * j] = mul2(w.x, S[c][2 * j]), S[c][2 * j + 1] = mul2(w.y, S[c][2 * j + 1]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                f32x2 vd[C];
+#pragma unroll
+                for (int c = 0; c < C; c++) vd[c] = pack2(vv[i][c], vv[i][c]);
+#pragma unroll
+                for (int j = 0; j < J; j++) {
+                    const ulonglong2 w = *(const ulonglong2 *)(vec + (4 + i) * DP + 4 * P * j);
+#pragma unroll
+                    for (int c = 0; c < C; c++) S[c][2 * j] = fma2(w.x, vd[c], S[c][2 * j]), S[c][2 * j + 1] = fma2(w.y, vd[c], S[c][2 * j + 1]);
+                }
+            }
+            // the sums across the column's lanes: columns handed over first, then tokens, then plain sums
+#pragma unroll
+            for (int step = 0; step < COL_STEPS; step++) {
+                const int half = C >> (step + 1), bit = P >> (step + 1);
+                const bool up = part & bit;
+#pragma unroll
+                for (int c = 0; c < half; c++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float give = up ? sums[c][i] : sums[c + half][i], keep = up ? sums[c + half][i] : sums[c][i];
+                        sums[c][i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                    }
+            }
+            // the block's own tokens, with the numbers: each lane for its column
+            const float4 n0 = *(const float4 *)(rec + 9 * DP), n1 = *(const float4 *)(rec + 9 * DP + 4), n2 = *(const float4 *)(rec + 9 * DP + 8);
+            float u[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                u[i] = vv[i][0];
+#pragma unroll
+                for (int c = 1; c < C; c++) u[i] = my_c == c ? vv[i][c] : u[i];
+            }
+            float add[4];
+            add[0] = n0.x * u[0], add[1] = fmaf(n0.z, u[1], n0.y * u[0]), add[2] = fmaf(n1.y, u[2], fmaf(n1.x, u[1], n0.w * u[0]));
+            add[3] = fmaf(n2.y, u[3], fmaf(n2.x, u[2], fmaf(n1.w, u[1], n1.z * u[0])));
+            float o[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) o[i] = sums[0][i];
+#pragma unroll
+            for (int step = 0; step < TOK_STEPS; step++) {
+                const int half = 2 >> step, bit = P >> (COL_STEPS + step + 1);
+                const bool up = part & bit;
+#pragma unroll
+                for (int i = 0; i < half; i++) {
+                    const float give = up ? o[i] : o[i + half], keep = up ? o[i + half] : o[i];
+                    o[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                    add[i] = up ? add[i + half] : add[i];
+                }
+            }
+#pragma unroll
+            for (int bit = REST >> 1; bit > 0; bit >>= 1)
+#pragma unroll
+                for (int i = 0; i < (4 >> TOK_STEPS); i++) o[i] += __shfl_xor_sync(0xffffffffu, o[i], bit);
+            if ((part & (REST - 1)) == 0 && my_col < D) {
+                constexpr int EACH = 4 >> TOK_STEPS;
+#pragma unroll
+                for (int i = 0; i < EACH; i++)
+                    if (my_t * EACH + i < left) out[(my_t * EACH + i) * hk] = o[i] + add[i];
+            }
+            out += WB_TOKENS * hk;
         }
     }
-    *slot = S;
+#pragma unroll
+    for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int j = 0; j < J; j++) {
+            const float2 x = unpack2(S[c][2 * j]), y = unpack2(S[c][2 * j + 1]);
+            const float v[4] = {x.x, x.y, y.x, y.y};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int ch = 4 * (P * j + part) + e;
+                if (ch < D && first_col + c < D) state[(long long)ch * D + first_col + c] = v[e];
+            }
+        }
 }
 
+template <typename T, int P, int J, int C> static int wkv_block_launch(WkvScan p, cudaStream_t s) {
+    constexpr int COLS = WB_WALKERS * 32 / P * C, RS = 9 * 4 * P * J + WB_NUMBERS + WB_TOKENS * COLS;
+    size_t smem = (size_t)2 * WB_MAKERS * RS * sizeof(float);
+    const long long sms = abk_sm_count();
+    // a lane's JL channels of a row of r, k and the pre-activations as aligned pieces
+    constexpr int JL = P * J / 8, BYTES = JL * (int)sizeof(T) > 16 ? 16 : JL * (int)sizeof(T), FLOATS = JL < 4 ? JL : 4;
+    p.vec = p.dim % JL == 0 && (p.ld * sizeof(T)) % BYTES == 0 && !(((uintptr_t)p.proj + (size_t)p.r_at * sizeof(T)) % BYTES) &&
+            !(((uintptr_t)p.proj + (size_t)p.k_at * sizeof(T)) % BYTES) && (p.dim * sizeof(T)) % BYTES == 0 &&
+            !((uintptr_t)p.pre % (4 * FLOATS)) && p.dim % FLOATS == 0;
+    p.tiles = (p.dim + COLS - 1) / COLS;
+    const long long ctas = (long long)p.n_seqs * p.n_heads * p.tiles, share = (ctas + sms - 1) / sms;
+    if (ctas > 0x7fffffffLL) ABK_REFUSE("wkv_scan: %lld CTAs are more than a grid takes", ctas);
+    // CTAs that start while the kernel before still holds parts of the SMs gather where there is room: each asks for so much
+    // shared memory that no SM takes more than its share
+    const size_t least = share <= 4 ? (size_t)(228 * 1024 / (share + 1)) : 0;
+    if (smem < least) smem = least;
+    p.longest_first = p.n_seqs > 1 && p.n_seqs <= SEQUENCE_PLACE_MAX && share > 1;  // (a long walk that starts last would be walked alone)
+    const cudaError_t e = abk_allow_shared_memory((const void *)wkv_block_kernel<T, P, J, C>, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    abk_launch(wkv_block_kernel<T, P, J, C>, dim3((unsigned)ctas), dim3(32 * (WB_WALKERS + WB_MAKERS)), smem, s, p);
+    return ABK_LAUNCH_RESULT();
+}
+
+// blocks: the step brings prompts, walked in blocks of four tokens; else (a token a sequence) each sequence token by token.
 extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at, int k_at, int v_at, int n_heads, int dim,
                             const float *pre, const float *w0, const float *bonus, float *state, float *out,
-                            const int *seq_start, const int *seq_slot, int n_seqs, int chunk, int segments, float *sums,
-                            float *prods, void *stream) {
+                            const int *seq_start, const int *seq_slot, int n_seqs, int blocks, void *stream) {
     if (n_seqs <= 0) return 0;
     if (dim < 1 || dim > 256) ABK_REFUSE("wkv_scan: %d key channels a head are not 1 to 256", dim);
     if (n_heads < 1 || n_heads > 65535 || n_seqs > 65535) ABK_REFUSE("wkv_scan: %d heads, %d sequences", n_heads, n_seqs);
     WkvScan p;
     p.proj = proj, p.ld = ld, p.r_at = r_at, p.k_at = k_at, p.v_at = v_at, p.n_heads = n_heads, p.dim = dim;
     p.pre = pre, p.w0 = w0, p.bonus = bonus, p.state = state, p.out = out, p.seq_start = seq_start, p.seq_slot = seq_slot;
-    p.chunk = chunk, p.phase = 0, p.n_seqs = n_seqs, p.sums = sums, p.prods = prods;
-    if (chunk < 0 || (chunk > 0 && (segments < 1 || segments > 65535 || !sums || !prods)))
-        ABK_REFUSE("wkv_scan: %d segments of %d tokens", segments, chunk);
+    p.n_seqs = n_seqs, p.tiles = 1, p.longest_first = 0, p.vec = 0;
     cudaStream_t s = (cudaStream_t)stream;
-    const int cols = dim <= 32 ? 32 : 16;  // value columns a CTA has
-    dim3 grid((dim + cols - 1) / cols, n_heads, chunk > 0 ? segments : n_seqs);
-#define WS_LAUNCH(T, SUMS)                                                                                  \
-    do {                                                                                                    \
-        if (dim <= 16) abk_launch(wkv_scan_kernel<T, 4, 4, 32, 16, SUMS>, grid, dim3(128), 0, s, p);        \
-        else if (dim <= 32) abk_launch(wkv_scan_kernel<T, 8, 4, 32, 16, SUMS>, grid, dim3(128), 0, s, p);   \
-        else if (dim <= 64) abk_launch(wkv_scan_kernel<T, 8, 8, 16, 16, SUMS>, grid, dim3(128), 0, s, p);   \
-        else if (dim <= 128) abk_launch(wkv_scan_kernel<T, 8, 16, 16, 16, SUMS>, grid, dim3(256), 0, s, p); \
-        else abk_launch(wkv_scan_kernel<T, 16, 16, 16, 8, SUMS>, grid, dim3(256), 0, s, p);                 \
-    } while (0)
-    if (chunk > 0) {  // the segments' sums, the states between them, the segments' outputs
-        p.phase = 1;
-        if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16, true);
-        else WS_LAUNCH(float, true);
-        int rc = ABK_LAUNCH_RESULT();
-        if (rc) return rc;
-        abk_launch(wkv_segment_prefix_kernel, dim3((dim * dim + 255) / 256, n_heads, n_seqs), dim3(256), 0, s, sums, prods, state,
-                   seq_start, seq_slot, n_heads, dim, chunk);
-        rc = ABK_LAUNCH_RESULT();
-        if (rc) return rc;
-        p.phase = 2;
+    if (blocks) {
+        // Columns a lane has. Heads of 64, a CTA then has 16, 32 or 64 of them: the makers' work is every CTA's own, so few
+        // CTAs a head are better until an SM would have two of them while others have one (3 prompts, 3,571 tokens, 40
+        // heads: 630, 679, 604 us a layer with 1, 2, 4; 8 prompts, 5,000 tokens: 885, 748, 803; one of 2,048 and 16
+        // heads: 336, 334, 352).
+        const long long columns = (long long)n_seqs * n_heads * dim, sms = abk_sm_count();
+        const int lane_columns = columns <= 32 * sms ? 1 : columns <= 64 * sms ? 4 : 2;
+#define WB_LAUNCH_AS(T, P, J)                                     \
+    (lane_columns == 1   ? wkv_block_launch<T, P, J, 1>(p, s)     \
+     : lane_columns == 2 ? wkv_block_launch<T, P, J, 2>(p, s)     \
+                         : wkv_block_launch<T, P, J, 4>(p, s))
+#define WB_LAUNCH(T)                                              \
+    (dim <= 32    ? WB_LAUNCH_AS(T, 8, 1)                         \
+     : dim <= 64  ? WB_LAUNCH_AS(T, 8, 2)                         \
+     : dim <= 128 ? WB_LAUNCH_AS(T, 16, 2)                        \
+                  : WB_LAUNCH_AS(T, 16, 4))
+        return dtype == ABK_BF16 ? WB_LAUNCH(__nv_bfloat16) : WB_LAUNCH(float);
+#undef WB_LAUNCH
+#undef WB_LAUNCH_AS
     }
-    if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16, false);
-    else WS_LAUNCH(float, false);
+    const int cols = dim <= 32 ? 32 : 16;  // value columns a CTA has
+    dim3 grid((dim + cols - 1) / cols, n_heads, n_seqs);
+#define WS_LAUNCH(T)                                                                                  \
+    do {                                                                                              \
+        if (dim <= 16) abk_launch(wkv_scan_kernel<T, 4, 4, 32, 16>, grid, dim3(128), 0, s, p);        \
+        else if (dim <= 32) abk_launch(wkv_scan_kernel<T, 8, 4, 32, 16>, grid, dim3(128), 0, s, p);   \
+        else if (dim <= 64) abk_launch(wkv_scan_kernel<T, 8, 8, 16, 16>, grid, dim3(128), 0, s, p);   \
+        else if (dim <= 128) abk_launch(wkv_scan_kernel<T, 8, 16, 16, 16>, grid, dim3(256), 0, s, p); \
+        else abk_launch(wkv_scan_kernel<T, 16, 16, 16, 8>, grid, dim3(256), 0, s, p);                 \
+    } while (0)
+    if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16);
+    else WS_LAUNCH(float);
 #undef WS_LAUNCH
     return ABK_LAUNCH_RESULT();
 }

@@ -1545,8 +1545,6 @@ def tanh_rows(src, dst, n):
                                   _i(src.shape[1]), _stream()), "tanh_rows")
 
 
-WKV_SEGMENT = 64        # tokens of a segment of the form for prompts
-WKV_SEGMENTS_FROM = 128  # rows of a step (one that is no decode step) from which its sequences are walked in segments
 
 
 def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, batch, ws=None):
@@ -1554,10 +1552,8 @@ def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, b
         o = (S + diag(bonus) k v^T)^T r;    S <- diag(exp(-exp(pre + w0))) S + k v^T
     proj [tokens, .] as stored: r, k, v of head h at columns r_at / k_at / v_at + h * dim; pre float32 [tokens, heads * dim];
     w0, bonus float32 [heads * dim]; state float32 [slots, heads, dim, dim] (key, value); out float32 [tokens, heads * dim].
-    A decode step, or a small one, walks each sequence token by token. A step of prompts (with ws, a Workspace) walks all
-    segments of WKV_SEGMENT tokens at once, twice: for each segment's own sum from an empty state, and, once the states
-    between the segments are made from the sums, for the outputs (the same numbers, summed in another order). Which way a
-    step goes depends on its rows and sequences alone, not on how long each sequence is."""
+    A step of one token a sequence walks each sequence token by token, a step of prompts in blocks of four tokens (the same
+    numbers, summed in another order); which way a step goes depends on its rows and sequences alone."""
     _need_cuda(proj, pre, w0, bonus, state, out)
     lib = load_module("wkv")
     hk = n_heads * dim
@@ -1566,19 +1562,9 @@ def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, b
     assert w0.numel() == bonus.numel() == hk and state.shape[1:] == (n_heads, dim, dim)
     assert proj.shape[1] >= max(r_at, k_at, v_at) + hk
     n_seqs = batch.seq_slot.numel()
-    chunk, segments, sums, prods = 0, 0, None, None
-    if ws is not None and not batch.is_decode and batch.n_rows >= WKV_SEGMENTS_FROM:
-        chunk = WKV_SEGMENT
-        segments = -(-batch.n_rows // chunk) + n_seqs  # (at most: every sequence's last segment may be a short one)
-        if segments <= 65535:
-            sums = ws.get("wkv_sums", (segments, n_heads, dim, dim), torch.float32)
-            prods = ws.get("wkv_prods", (segments, n_heads, dim), torch.float32)
-        else:
-            chunk = segments = 0
     _check(lib, lib.abk_wkv_scan(_p(proj), _ll(proj.stride(0)), _i(_dt(proj)), _i(r_at), _i(k_at), _i(v_at), _i(n_heads), _i(dim),
                                  _p(pre), _p(w0), _p(bonus), _p(state), _p(out), _p(batch.seq_start), _p(batch.seq_slot),
-                                 _i(n_seqs), _i(chunk), _i(segments), _p(sums), _p(prods), _stream()), "wkv_scan",
-           kernels=3 if chunk else 1)
+                                 _i(n_seqs), _i(0 if batch.is_decode else 1), _stream()), "wkv_scan")
 
 
 # ------------------------------------------------------------------ experts by a table (csrc/moe.cu)

@@ -47,6 +47,39 @@ def test_wkv_every_way(dtype, H, K, rank):
     _every_way(_wkv_run(p, d, H, K, rank, dtype), h, want, dtype, f"wkv {H} x {K}")
 
 
+@pytest.mark.parametrize("H,K,lens", [(100, 48, (9,)), (80, 30, (5, 3, 4)), (40, 128, (6,)), (30, 256, (5,)), (60, 64, (7, 1, 6)),
+                                      (170, 20, (4, 6, 1)), (80, 128, (5,)), (48, 256, (3,)), (3, 90, (2, 9)), (2, 64, (5, 130))])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_wkv_in_blocks(H, K, lens, shift):
+    """Blocks of four tokens and their remainders for every split of the work (few and many columns, every padded head size),
+    sequences of unequal lengths, rows of bfloat16 that start on no boundary (shift), and the state they leave."""
+    from abacus_b200.engine.batch import Sequence, StepBatch
+    from abacus_b200.kernels import ops
+    rng, n = np.random.default_rng(H * K), sum(lens)
+    size = H * K
+    rows = torch.from_numpy(rng.standard_normal((n, 3 * size + 8 + shift)).astype(np.float32)).to(DEV).to(torch.bfloat16)
+    proj = rows[:, shift:]
+    pre, w0 = (torch.from_numpy(rng.standard_normal(s).astype(np.float32)).to(DEV) for s in ((n, size), (size,)))
+    bonus = torch.from_numpy(rng.standard_normal(size).astype(np.float32)).to(DEV)
+    state = torch.from_numpy(rng.standard_normal((len(lens), H, K, K)).astype(np.float32)).to(DEV)
+    S, out = state.double(), torch.empty((n, size), device=DEV)
+    batch = StepBatch(n, len(lens), 1, DEV).fill([Sequence(i, [0] * m, 3, []) for i, m in enumerate(lens)], exact=True)
+    assert not batch.is_decode
+    ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch)
+    r, k, v = (proj[:, i * size:(i + 1) * size].double().view(n, H, K) for i in range(3))
+    w, u, want, at = torch.exp(-torch.exp(pre.double() + w0.double())).view(n, H, K), bonus.double().view(H, K), [], 0
+    for i, m in enumerate(lens):
+        for t in range(at, at + m):
+            new = k[t][:, :, None] * v[t][:, None, :]
+            want.append(torch.einsum("hkv,hk->hv", S[i] + u[:, :, None] * new, r[t]).reshape(-1))
+            S[i] = w[t][:, :, None] * S[i] + new
+        at += m
+    want = torch.stack(want)
+    # sums of K products of values of around one, the decays by the special-function unit: some 2^-21 of the sums' size
+    limit = 2.0 ** -20 * K ** 0.5 * 8 * max(1.0, float(S.abs().max()))
+    assert float((out.double() - want).abs().max()) <= limit and float((state.double() - S).abs().max()) <= limit
+
+
 def test_wkv_keeps_a_token_over_a_long_decoding_and_forgets_with_decays_near_nothing():
     """Decays all but one: a loud early token is read back after 400 single-token steps (and the token before it is what
     the blends saw); decays all but nothing: only the token's own bonus term and the token before are left."""
