@@ -3,7 +3,8 @@
 // This is the matrix product of the true 32-bit path (no tensor cores, no TF32), and the
 // fallback of the bfloat16 path for shapes the tensor-core kernel refuses. An output element is the sum of eight running
 // sums: K in pieces of 16, piece c to sum c % 8, each sum over its k in ascending order, then in pairs,
-// ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); so a row's result does not depend on how many other rows are in the
+// ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); up to K = 256 of one sum alone, over k in ascending order (a chain of
+// that length needs no cutting, and the small products of small models keep the order they had). So a row's result does not depend on how many other rows are in the
 // batch or where its tile lies.
 // Formula: src/model.c:299, 302, 307, 309, 324 (weights are [out, in] row-major, no bias).
 //
@@ -22,6 +23,7 @@
 #define GS_WARPS 8
 #define GS_BK 16
 #define GS_PITCH 20     // floats of a staged row
+#define GS_ONE_SUM 16   // up to this many pieces the first warp takes them all
 
 __device__ __forceinline__ void gs_copy_16(float *dst, const float *src, bool real) {
     const int bytes = real ? 16 : 0;  // 0: zeros
@@ -77,9 +79,10 @@ __global__ void __launch_bounds__(32 * GS_WARPS) gemm_simt_kernel(const TX *__re
     for (int i = 0; i < TM; i++)
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[i][j] = 0.0f;
-    if (warp < pieces) fetch(warp, 0);
-    for (int piece = warp, it = 0; piece < pieces; piece += GS_WARPS, it++) {
-        if (piece + GS_WARPS < pieces) fetch(piece + GS_WARPS, (it + 1) & 1);
+    const int step = pieces <= GS_ONE_SUM ? 1 : GS_WARPS, end = step == 1 && warp > 0 ? 0 : pieces;
+    if (warp < end) fetch(warp, 0);
+    for (int piece = warp, it = 0; piece < end; piece += step, it++) {
+        if (piece + step < end) fetch(piece + step, (it + 1) & 1);
         else asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
