@@ -62,10 +62,32 @@ class _Group:
             self.v = self.k
         else:
             self.v = guards.zeros(shape[:-1] + (need.v_head_dim or need.head_dim,), dtype, device, what="cache values")
-        # pageable on purpose: a copy from pageable memory is staged before copy_ returns, so the
-        # host may rewrite a row (a slot used again) while earlier steps are still in flight
+        # the tables as the host has them; what changes goes to the device as arguments of a kernel (no copy from a host
+        # buffer, which would have to be kept as it is, or waited for, while earlier steps are in flight)
         self.table_host = torch.zeros((max_slots, self.table_width), dtype=torch.int32)
+        self._table_rows = self.table_host.numpy()
         self.table = torch.zeros((max_slots, self.table_width), dtype=torch.int32, device=device)
+
+    def grow(self, slot, new_length):
+        """Pages for the sequence to hold new_length tokens, set in the host's table; what changed, flat: word of the table,
+        page, word, page, .."""
+        added = self.book.grow(slot, new_length)
+        if not added:
+            return []
+        first, pages = added[0][0], [page for _, page in added]
+        self._table_rows[slot, first:first + len(pages)] = pages  # (new pages follow those a slot has)
+        word = slot * self.table_width + first
+        return [x for pair in zip(range(word, word + len(pages)), pages) for x in pair]
+
+    def send(self, changes):
+        """The device's table follows; on the table's own device, in the order of the current stream."""
+        if not changes:
+            return
+        if self.table.is_cuda and self.table.get_device() == torch.cuda.current_device():
+            from ..kernels import ops
+            ops.set_words(self.table, changes)
+        else:
+            self.table.copy_(self.table_host)
 
 
 _STATE_TYPES = {"float32": torch.float32, "int32": torch.int32}
@@ -162,11 +184,7 @@ class SequenceCache:
             raise CacheFull(f"the cache lacks {short} free pages of {TOKENS_PER_PAGE} tokens for slot {slot} to hold "
                             f"{new_length} tokens")
         for g in self.groups:
-            added = g.book.grow(slot, new_length)
-            if added:
-                for logical, page in added:
-                    g.table_host[slot, logical] = page
-                g.table[slot].copy_(g.table_host[slot])
+            g.send(g.grow(slot, new_length))
 
     def reserve_all(self, wanted):
         """reserve() for several slots at once, [(slot, new_length)]: either every one gets its room or the cache
@@ -179,8 +197,8 @@ class SequenceCache:
             if need > g.book.pages.n_free:
                 raise CacheFull(f"the cache has {g.book.pages.n_free} free pages of {TOKENS_PER_PAGE} tokens; this step "
                                 f"needs {need} more")
-        for slot, new_length in wanted:
-            self.reserve(slot, new_length)
+        for g in self.groups:
+            g.send([x for slot, n in wanted for x in g.grow(slot, n)])
 
     def save_states(self, slots):
         """Copies of every per-sequence state of these slots (of the mixers' and of the frame's), for restore_states.

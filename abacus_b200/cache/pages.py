@@ -3,6 +3,7 @@
 Nothing here touches the GPU, so its invariants (no page or slot lost, held
 twice or freed twice) are tested on the CPU.
 """
+import heapq
 
 
 class CacheFull(RuntimeError):
@@ -14,13 +15,13 @@ class FreeList:
 
     def __init__(self, n, what):
         self.n, self.what = n, what
-        self._free = list(range(n - 1, -1, -1))
+        self._free = list(range(n))  # a heap: the lowest first, so that reuse is deterministic
         self._held = set()
 
     def take(self):
         if not self._free:
             raise CacheFull(f"no free {self.what} (all {self.n} are in use)")
-        i = self._free.pop()
+        i = heapq.heappop(self._free)
         self._held.add(i)
         return i
 
@@ -28,9 +29,7 @@ class FreeList:
         if i not in self._held:
             raise ValueError(f"{self.what} {i} is not in use (freed twice, or never taken)")
         self._held.remove(i)
-        self._free.append(i)
-        # keep "lowest first" so that reuse is deterministic
-        self._free.sort(reverse=True)
+        heapq.heappush(self._free, i)
 
     @property
     def n_free(self):

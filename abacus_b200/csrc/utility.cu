@@ -14,6 +14,10 @@
 // after it; abk_guard_check counts the words that no longer hold the pattern. With no memory checker on
 // the device, this is what shows a store past the end of a workspace, a scratch area or a cache pool.
 //
+// Words from the host. A few words of a table on the device change on the host's word (the pages a sequence was given):
+// abk_set_words carries them as the launch's own arguments, so that there is no host buffer that has to stay as it is, and
+// no wait, while earlier work of the stream is under way.
+//
 // A wait that runs out. Every wait of the kernels on a barrier is bounded (tc_common.cuh) and ends in a status word
 // instead of a hang. abk_wait_that_runs_out is the smallest kernel with such a wait: a barrier that expects bytes
 // nobody sends. It exists so that the way from a wait that ran out to the host's exception can be walked without
@@ -48,6 +52,32 @@ __global__ void fill_normal_kernel(T *out, long long n, long long first, unsigne
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
         out[i] = from_float<T>(__fadd_rn(mean, __fmul_rn(amplitude, unit_normal(key, (unsigned long long)(first + i)))));
+}
+
+// A copy of a row of a page table from pageable memory waited for the stream, one row after the other, and kept the host from
+// preparing a step while the step before ran. A launch carries up to this many words.
+#define SET_WORDS 480
+struct SetWords {
+    int *table, n;
+    int pairs[2 * SET_WORDS];  // word, value
+};
+__global__ void __launch_bounds__(128) set_words_kernel(const __grid_constant__ SetWords p) {
+    for (int i = threadIdx.x; i < p.n; i += 128) p.table[p.pairs[2 * i]] = p.pairs[2 * i + 1];
+}
+
+// table[pairs[2 i]] = pairs[2 i + 1] for i in [0, n); `pairs` (on the host) is read before this returns. Words all different.
+extern "C" int abk_set_words(int *table, long long size, const int *pairs, int n, void *stream) {
+    for (int i = 0; i < n; i++)
+        if (pairs[2 * i] < 0 || pairs[2 * i] >= size) ABK_REFUSE("set_words: word %d of a table of %lld", pairs[2 * i], size);
+    for (int first = 0; first < n; first += SET_WORDS) {
+        SetWords p;
+        p.table = table, p.n = n - first < SET_WORDS ? n - first : SET_WORDS;
+        for (int i = 0; i < 2 * p.n; i++) p.pairs[i] = pairs[2 * first + i];
+        set_words_kernel<<<1, 128, 0, (cudaStream_t)stream>>>(p);
+        const int rc = ABK_LAUNCH_RESULT();
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 // out[i] = mean + amplitude * z(key, first + i) for i in [0, n): element `first + i` of the tensor that `key` names.

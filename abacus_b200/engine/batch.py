@@ -22,6 +22,7 @@ The plan's words travel in the same buffer, at an address that is fixed for the 
 life (a captured graph holds it); `batch.plan[name]` gives the mixer its words on the device
 with its layout and the info of the last fill. Nothing here knows what any plan holds.
 """
+import struct
 from dataclasses import dataclass
 
 import numpy as np
@@ -44,6 +45,17 @@ class PlanView:
     layout: object
     words: torch.Tensor  # int32, on the device, at a fixed address
     info: object         # what the plan's fill returned
+
+
+def _put_words(words, at, values):
+    """words[at:at + len(values)] = values; a list of ints goes in packed (a third of what numpy takes for it)."""
+    if type(values) is list and len(values) >= 64:
+        try:
+            struct.pack_into(f"{len(values)}i", words, 4 * at, *values)
+            return
+        except struct.error:  # (something numpy converts and struct does not, or refuses in its own words)
+            pass
+    words[at:at + len(values)] = values
 
 
 CORE = ["tokens", "token_seq", "token_pos", "seq_slot", "seq_start", "seq_pos0", "seq_len_after", "logit_rows"]
@@ -96,30 +108,36 @@ class StepBatch:
         n_logits = sum(len(s.want) for s in sequences)
         if n_tokens > self.cap_rows or len(sequences) > self.cap_seqs or n_logits > self.cap_logits:
             raise ValueError("step is larger than this StepBatch")
-        h["token_seq"][:] = -1
-        h["tokens"][:] = 0
-        h["token_pos"][:] = 0
-        h["seq_slot"][:] = 0
-        h["logit_rows"][:] = 0
-        h["seq_pos0"][:] = 0
-        h["seq_len_after"][:] = 0
-        row, lr = 0, 0
-        for i, s in enumerate(sequences):
-            n = len(s.tokens)
-            h["tokens"][row:row + n] = s.tokens
-            h["token_seq"][row:row + n] = i
-            h["token_pos"][row:row + n] = np.arange(s.start, s.start + n)
-            h["seq_slot"][i] = s.slot
-            h["seq_start"][i] = row
-            h["seq_pos0"][i] = s.start
-            h["seq_len_after"][i] = s.start + n
+        n_seqs = len(sequences)
+        lens, starts = [len(s.tokens) for s in sequences], [s.start for s in sequences]
+        lens_a, starts_a = np.array(lens, dtype=np.int64), np.array(starts, dtype=np.int64)
+        ends = np.cumsum(lens_a)
+        first = ends - lens_a
+        if n_tokens == n_seqs and all(n == 1 for n in lens):  # a decode step: a row a sequence
+            h["tokens"][:n_seqs] = [s.tokens[0] for s in sequences]
+            h["token_seq"][:n_seqs] = np.arange(n_seqs)
+            h["token_pos"][:n_seqs] = starts_a
+        else:
+            for s, row in zip(sequences, first.tolist()):
+                _put_words(h["tokens"], row, s.tokens)
+            h["token_seq"][:n_tokens] = np.repeat(np.arange(n_seqs), lens_a)
+            h["token_pos"][:n_tokens] = np.arange(n_tokens) + np.repeat(starts_a - first, lens_a)
+        h["tokens"][n_tokens:] = 0
+        h["token_seq"][n_tokens:] = -1
+        h["token_pos"][n_tokens:] = 0
+        for name, values in (("seq_slot", [s.slot for s in sequences]), ("seq_pos0", starts_a), ("seq_len_after", starts_a + lens_a)):
+            h[name][:n_seqs] = values
+            h[name][n_seqs:] = 0
+        h["seq_start"][:n_seqs] = first
+        h["seq_start"][n_seqs:] = n_tokens
+        lr = 0
+        for s, n, row in zip(sequences, lens, first.tolist()):
             for wpos in s.want:
                 if not 0 <= wpos < n:
                     raise ValueError(f"wanted place {wpos} is outside the {n} tokens given")
                 h["logit_rows"][lr] = row + wpos
                 lr += 1
-            row += n
-        h["seq_start"][len(sequences):] = row
+        h["logit_rows"][lr:] = 0
         self.n_tokens, self.n_seqs, self.n_logit_rows = n_tokens, len(sequences), n_logits
         if pad_logits:
             self.n_logit_rows = self.cap_logits

@@ -5,6 +5,7 @@ library fallback. Tensors must live on the GPU and be contiguous where a kernel
 assumes it; a kernel that does not take a size raises KernelRefused with the
 reason instead of computing something else.
 """
+import array
 import ctypes
 
 import torch
@@ -71,6 +72,18 @@ def fill_normal(out, key, mean, amplitude, first=0):
     assert out.is_contiguous()
     _check(lib, lib.abk_fill_normal(_p(out), _i(_dt(out)), _ll(out.numel()), _ll(first), ctypes.c_ulonglong(key),
                                     _f(mean), _f(amplitude), _stream()), "fill_normal")
+
+
+def set_words(table, changes):
+    """table.flat[word] = value for the flat list [word, value, word, value, ..] of the host (int32; words all different).
+    The list travels as the launch's arguments: nothing is waited for and no host buffer is kept."""
+    _need_cuda(table)
+    lib = load_module("utility")
+    assert table.dtype == torch.int32 and table.is_contiguous()
+    pairs = array.array("i", changes)
+    n = len(pairs) // 2
+    _check(lib, lib.abk_set_words(_p(table), _ll(table.numel()), ctypes.c_void_p(pairs.buffer_info()[0]), _i(n), _stream()),
+           "set_words", kernels=-(-n // 480))
 
 
 def embed(tokens, table, x, status):
@@ -499,7 +512,6 @@ def attention_window(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, bat
     keys, an optional sink (float32 [n_heads]), values of v_dim, softmax weights in float32, keys seen only within the
     token's own chunk of `chunk` positions, scores capped at `softcap` (csrc/attention_window.cu)."""
     _need_cuda(qkv, out, sink)
-    lib = load_module("attention_window")
     vd = v_dim or head_dim
     heads_size = (n_heads + n_kv_heads) * head_dim + n_kv_heads * vd
     row = row or heads_size
@@ -509,6 +521,7 @@ def attention_window(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, bat
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() == n_heads)
     if batch.any_continuation:
         raise KernelRefused("attention_window reads keys from the step's rows: every sequence must start at position 0")
+    lib = load_module("attention_window")
     max_tiles = (n + 63) // 64 + n_seqs
     _check(lib, lib.abk_attention_window(_p(qkv), _ll(row), _p(out), _i(n_heads), _i(n_kv_heads), _i(head_dim), _i(vd),
                                          _i(n_heads * head_dim), _i((n_heads + n_kv_heads) * head_dim), _f(scale),

@@ -82,14 +82,14 @@ class AttentionStepPlan:
         info = {"n_halved": 0, "counts": counts, "tile_pages": {}}
         if is_decode:  # one token each: the decode kernels need no lists
             return info
-        for r in TILE_ROWS:
-            tiles, pages = tiles_of(sequences, r)
+        of_rows = {r: tiles_of(sequences, r) for r in TILE_ROWS}
+        for r, (tiles, pages) in of_rows.items():
             off = layout.offset[f"tiles{r}"]
             words[off:off + tiles.size] = tiles.reshape(-1)
             info["tile_pages"][r] = pages
             if exact:
                 counts[f"tiles{r}"] = len(tiles)
-        work, n_halved = self._work_list(sequences)
+        work, n_halved = self._work_list(sequences, of_rows[PAIRED_ROWS][0])
         off = layout.offset["work"]
         words[off:off + work.size] = work.reshape(-1)
         info["n_halved"] = n_halved
@@ -97,12 +97,11 @@ class AttentionStepPlan:
             counts["work"] = len(work)
         return info
 
-    def _work_list(self, sequences):
+    def _work_list(self, sequences, tiles):
         """The work list of the prefill attention kernel that halves long tiles. CTAs with the most pages come first."""
-        tiles, _ = tiles_of(sequences, PAIRED_ROWS)
         seq, row = tiles[:, 0].astype(np.int64), tiles[:, 1].astype(np.int64)
-        start = np.array([s.start for s in sequences], dtype=np.int64)[seq]
-        new = np.array([len(s.tokens) for s in sequences], dtype=np.int64)[seq]
+        starts, news = (np.array(v, dtype=np.int64) for v in ([s.start for s in sequences], [len(s.tokens) for s in sequences]))
+        start, new = starts[seq], news[seq]
         pages = (start + np.minimum(row + PAIRED_ROWS, new) - 1) // 64 + 1
         # With fewer CTAs than the device holds at once, the longest tiles stand twice (each time with half of
         # their pages) as long as the CTAs still fit, give or take a few: then the kernel's longest CTA is shorter.
@@ -112,28 +111,35 @@ class AttentionStepPlan:
         spare = 1.05 * slots - len(pages) * heads
         k = min(int(np.ceil(spare / heads)) if spare > 0 else 0, HALVED_PAIRS // heads, len(pages))
         split = np.zeros(len(pages), dtype=bool)
-        for i in np.argsort(-pages, kind="stable")[:k]:
-            split[i] = pages[i] >= 8
-        halved = {int(i): k for k, i in enumerate(np.flatnonzero(split))}
-        entries = [((pages[i] + 1) // 2, i, 1) for i in halved] + [(pages[i] // 2, i, 2) for i in halved]
-        entries += [(pages[i], i, 0) for i in range(len(pages)) if not split[i]]
-        entries.sort(key=lambda t: -t[0])  # the CTAs with the most pages first
-        first_row = np.array([0] + list(np.cumsum([len(s.tokens) for s in sequences])), dtype=np.int64)
+        longest = np.argsort(-pages, kind="stable")[:k]
+        split[longest] = pages[longest] >= 8
+        halved, whole = np.flatnonzero(split), np.flatnonzero(~split)
+        ids = np.zeros(len(pages), dtype=np.int64)
+        ids[halved] = np.arange(len(halved))
+        # (pages, tile, part) of every entry: the halves with earlier keys, with later keys, the whole tiles
+        tile = np.concatenate([halved, halved, whole])
+        part = np.repeat([1, 2, 0], [len(halved), len(halved), len(whole)])
+        length = np.concatenate([(pages[halved] + 1) // 2, pages[halved] // 2, pages[whole]])
+        order = np.argsort(-length, kind="stable")  # the CTAs with the most pages first
+        tile, part = tile[order], part[order]
+        of = seq[tile]
+        first_row = np.concatenate([[0], np.cumsum(news)])
         slot_of = np.array([s.slot for s in sequences], dtype=np.int64)
-        work = np.full((len(entries), WORK_INTS), -1, dtype=np.int32)
-        for k, (_, i, part) in enumerate(entries):
-            work[k] = (seq[i], row[i], part, first_row[seq[i]], start[i], new[i], slot_of[seq[i]], halved.get(i, 0))
+        work = np.stack([of, row[tile], part, first_row[of], start[tile], new[tile], slot_of[of], ids[tile]], axis=1).astype(np.int32)
         return work, len(halved)
 
 
 def tiles_of(sequences, rows_per_tile):
     """((sequence, first row among its new tokens) of every tile of `rows_per_tile` query rows, int32 [tiles, 2], the
     tiles that see the most keys first; pages of 64 keys each tile sees, in the sequences' order)."""
-    seq = np.concatenate([np.full(-(-len(s.tokens) // rows_per_tile), i, dtype=np.int32) for i, s in enumerate(sequences)])
-    row = np.concatenate([np.arange(0, len(s.tokens), rows_per_tile, dtype=np.int32) for s in sequences])
+    lengths = np.array([len(s.tokens) for s in sequences], dtype=np.int64)
+    counts = -(-lengths // rows_per_tile)
+    seq = np.repeat(np.arange(len(sequences), dtype=np.int32), counts)
+    first = np.cumsum(counts) - counts
+    row = ((np.arange(len(seq), dtype=np.int64) - first[seq]) * rows_per_tile).astype(np.int32)
     keys = np.array([s.start for s in sequences], dtype=np.int64)[seq] + row
     # tiles that see the most keys first: the long ones start early and the short ones fill the tail
     order = np.argsort(-keys, kind="stable")
-    last = np.minimum(row + rows_per_tile, np.array([len(s.tokens) for s in sequences], dtype=np.int64)[seq])
+    last = np.minimum(row + rows_per_tile, lengths[seq])
     pages = (keys + last - row - 1) // 64 + 1
     return np.stack([seq[order], row[order]], axis=1), pages

@@ -131,7 +131,7 @@ def test_gemm_simt(ops, m, n, k):
             out.cpu().numpy(), plain.linear(xb, wb), rtol=1e-5, atol=1e-5)
 
 
-@pytest.mark.parametrize("n, k", [(900, 132), (900, 16), (1000, 300)])
+@pytest.mark.parametrize("n, k", [(900, 132), (900, 16), (900, 257), (1000, 300)])
 def test_gemm_simt_tiles_give_the_same_bits(ops, n, k):
     """The tiles of 64, 32 and 16 and the loads of single elements (rows that start on no 16-byte boundary) add in one order."""
     rng = np.random.default_rng(n + k)
@@ -144,6 +144,38 @@ def test_gemm_simt_tiles_give_the_same_bits(ops, n, k):
         for a, b in ((x, w), shifted):
             ops.gemm_simt(a[:rows], b, out, rows)
             assert torch.equal(out[:rows], whole[:rows])
+
+
+@pytest.mark.parametrize("n", [1, 480, 481, 1500])
+def test_set_words(ops, n):
+    """Words carried by one launch and by several, in any order; a word outside the table is refused and changes nothing."""
+    rng = np.random.default_rng(n)
+    table = torch.arange(2000, dtype=torch.int32, device="cuda").view(40, 50)
+    want = table.cpu().numpy().reshape(-1).copy()
+    words, values = rng.permutation(2000)[:n], rng.integers(-9, 1 << 30, n)
+    want[words] = values
+    ops.set_words(table, [int(x) for pair in zip(words, values) for x in pair])
+    assert (table.cpu().numpy().reshape(-1) == want).all()
+    with pytest.raises(ops.KernelRefused):
+        ops.set_words(table, [0, 7, 2000, 1])
+    assert (table.cpu().numpy().reshape(-1) == want).all()
+
+
+def test_page_tables_on_the_device_follow_the_host():
+    from abacus_b200.cache import CacheNeed, SequenceCache
+    rng = np.random.default_rng(3)
+    cache = SequenceCache([CacheNeed(1, 8), CacheNeed(1, 8, window=100)], [None, None], 64 * 900, torch.bfloat16, "cuda", max_slots=6)
+    slots = []
+    for _ in range(60):
+        if slots and (len(slots) == 6 or rng.random() < 0.4):
+            cache.close_slot(slots.pop(int(rng.integers(len(slots)))))
+        else:
+            slots.append(cache.open_slot())
+        cache.reserve_all([(s, int(rng.integers(1, 64 * 140))) for s in slots])
+        for g in cache.groups:
+            assert torch.equal(g.table.cpu(), g.table_host)
+            held = [p for s in slots for p in g.book.of_slot[s]]
+            assert len(held) == len(set(held)) and all(g.table_host[s, :len(g.book.of_slot[s])].tolist() == g.book.of_slot[s] for s in slots)
 
 
 def test_gemm_simt_rows_do_not_depend_on_the_batch(ops):
