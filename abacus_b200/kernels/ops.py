@@ -505,12 +505,21 @@ def attention_window_takes(qkv, head_dim, v_dim, n_heads, n_kv_heads, row=None):
             and 8 <= v_dim <= 128 and row % 8 == 0 and qkv.data_ptr() % 16 == 0)
 
 
+def attention_window_tc_takes(qkv, out, n_heads, head_dim, v_dim, scale, softcap):
+    """Whether the tcgen05 kernel takes a prompt step's attention with float32 weights: heads of 64, 128 or 192, values of 64
+    or 128, no cap of the scores, a positive scale, outputs 16-byte aligned (csrc/attention_window_tc.cu). Where it takes
+    them it is used: of one launch, 16 query and 8 key heads of 128, a window of 1,024, the warp-level kernel takes 9.7 us
+    for 16 tokens against 5.4, 41 for 512 against 27, 124 for 2,048 against 67; the least it gains was 22.9 against 24.0 (512
+    tokens, heads of 64, a window of 256)."""
+    return (head_dim in (64, 128, 192) and v_dim in (64, 128) and not softcap and scale > 0 and out.data_ptr() % 16 == 0)
+
+
 def attention_window(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, batch, v_dim=None, keep_first=0, sink=None,
                      row=None, chunk=None, softcap=None):
-    """Causal attention of whole prompts (every sequence of the step from its first token) on the warp-level tensor
-    cores, keys and values from the step's own rows of qkv: an optional window that also keeps the first keep_first
+    """Causal attention of whole prompts (every sequence of the step from its first token) on the tensor cores, keys and values from the step's own rows of qkv: an optional window that also keeps the first keep_first
     keys, an optional sink (float32 [n_heads]), values of v_dim, softmax weights in float32, keys seen only within the
-    token's own chunk of `chunk` positions, scores capped at `softcap` (csrc/attention_window.cu)."""
+    token's own chunk of `chunk` positions, scores capped at `softcap` (csrc/attention_window.cu on the warp-level ones,
+    csrc/attention_window_tc.cu by tcgen05 for the sizes that takes)."""
     _need_cuda(qkv, out, sink)
     vd = v_dim or head_dim
     heads_size = (n_heads + n_kv_heads) * head_dim + n_kv_heads * vd
@@ -521,6 +530,14 @@ def attention_window(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, bat
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() == n_heads)
     if batch.any_continuation:
         raise KernelRefused("attention_window reads keys from the step's rows: every sequence must start at position 0")
+    if attention_window_tc_takes(qkv, out, n_heads, head_dim, vd, scale, softcap):
+        lib = load_module("attention_window_tc")
+        _check(lib, lib.abk_attention_window_tc(_p(qkv), _ll(row), _i(n), _p(out), _i(n_heads), _i(n_kv_heads), _i(head_dim), _i(vd),
+                                                _i(n_heads * head_dim), _i((n_heads + n_kv_heads) * head_dim), _f(scale),
+                                                _i(window or 0), _i(keep_first or 0), _p(sink), _p(batch.seq_start), _i(n_seqs),
+                                                _i(n // 256 + n_seqs), _i(chunk or 0), _p(kernel_status(qkv.device)), _stream()),
+               "attention_window_tc")
+        return
     lib = load_module("attention_window")
     max_tiles = (n + 63) // 64 + n_seqs
     _check(lib, lib.abk_attention_window(_p(qkv), _ll(row), _p(out), _i(n_heads), _i(n_kv_heads), _i(head_dim), _i(vd),

@@ -102,7 +102,7 @@ class Attention:
 
     def step_plans(self):
         """What this mixer wants made on the host for every step and sent with the step's indices."""
-        return [] if self.sigmoid or self.maps > 1 else [self.lists]  # (attention without a softmax and differential attention need none)
+        return [] if self.general else [self.lists]  # (the kernels with the general options find their tiles themselves)
 
     def step_weights(self):
         """The tensors a step reads once whatever its size (for the bytes a decode step must move)."""

@@ -330,6 +330,44 @@ def test_the_tensor_core_prompt_kernel_on_unequal_prompts(H, G, D, V, window, ke
     np.testing.assert_allclose(got, want, rtol=2 ** -8, atol=1e-3)
 
 
+@pytest.mark.parametrize("H,G,D,V,window,keep,chunk,lens", [(2, 1, 128, 128, None, 0, 0, (256, 257, 1)), (3, 3, 192, 128, None, 0, 0, (300, 128)),
+                                                            (2, 2, 192, 64, 200, 5, 0, (513,)), (2, 1, 64, 64, 64, 100, 0, (129, 385)),
+                                                            (4, 2, 64, 128, 1, 0, 0, (260, 64)), (2, 2, 128, 64, 300, 70, 0, (700, 127)),
+                                                            (2, 1, 128, 128, None, 0, 100, (390, 128)), (2, 1, 64, 64, 150, 3, 128, (511, 65))])
+def test_prompts_on_two_groups_of_rows_a_cta(H, G, D, V, window, keep, chunk, lens):
+    """The tcgen05 kernel with float32 weights: groups of 128 rows and tiles of 64 keys at their edges, tiles only one group
+    needs, kept first keys, chunks, keys loud enough that a row's reference moves late; a neighbour's rows that are no numbers
+    change nothing."""
+    from abacus_b200.kernels import ops
+    rng, scale = np.random.default_rng(D + V + len(lens)), 0.2
+    sink = rng.standard_normal(H).astype(np.float32)
+    rows, wants = [], []
+    for T in lens:
+        q, k, v = (plain.bf16_round(rng.standard_normal((T, n, d)).astype(np.float32)) for n, d in ((H, D), (G, D), (G, V)))
+        k[T // 2] = plain.bf16_round(4.0 * k[T // 2])
+        z = np.einsum("ihd,jhd->hij", q.astype(np.float64), np.repeat(k, H // G, axis=1)) * scale
+        i, j = np.arange(T)[:, None], np.arange(T)[None]
+        seen = (j <= i) & ((i - j < (window or T)) | (j < (keep if window else 0)))
+        if chunk:
+            seen &= i // chunk == j // chunk
+        z = np.concatenate([np.where(seen, z, -np.inf), np.broadcast_to(sink[:, None, None], (H, T, 1))], axis=2)
+        w = np.exp(z - z.max(-1, keepdims=True))
+        w = (w / w.sum(-1, keepdims=True))[:, :, :T]
+        wants.append(np.einsum("hij,jhv->ihv", w, np.repeat(v, H // G, axis=1)).reshape(T, H * V))
+        rows.append(np.concatenate([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], axis=1))
+    rows.append(np.full((40, rows[0].shape[1]), np.nan, dtype=np.float32))
+    b = batch_of([(i, [0] * T, 0) for i, T in enumerate(list(lens) + [40])])
+    qkv = dev(np.concatenate(rows), torch.bfloat16)
+    out = torch.empty((sum(lens) + 40, H * V), dtype=torch.bfloat16, device=DEV)
+    assert ops.attention_window_tc_takes(qkv, out, H, D, V, scale, None)
+    ops.attention_window(qkv, out, H, G, D, scale, window, b, v_dim=V, keep_first=keep, sink=dev(sink), chunk=chunk or None)
+    got = out.float().cpu().numpy()
+    # float32 weights: what is left is the rounding of the stored result
+    np.testing.assert_allclose(got[:sum(lens)], np.concatenate(wants), rtol=2 ** -8, atol=1e-3)
+    assert np.isnan(got[sum(lens):]).all()
+    assert not ops.kernel_status(torch.device(DEV, torch.cuda.current_device())).any()
+
+
 @pytest.mark.parametrize("H,G,D,V,window,keep,dtype", [(8, 1, 32, 200, None, 0, torch.bfloat16), (6, 2, 24, 40, 300, 9, torch.float32),
                                                         (16, 1, 64, 8, 130, 128, torch.bfloat16), (3, 3, 256, 130, 128, 0, torch.bfloat16)])
 def test_decoding_in_parts_in_an_unequal_batch(H, G, D, V, window, keep, dtype):
