@@ -291,6 +291,215 @@ __global__ void __launch_bounds__(GG_THREADS) gemm_grouped_kernel(const __grid_c
     }
 }
 
+// The same product on pairs of CTAs (cta_group::2). A tile of 128 x 128 asks the L2 for 32 KB every 128 cycles of the tensor
+// core, four times what an SM gets from it; a pair's tile of 256 x 256 asks for as much every 256 cycles of either SM, its CTAs
+// are persistent, and one accumulator is stored while the other is filled. The pairs' rows are two neighbouring row tiles of
+// one expert (the leader's and its peer's; an expert's odd last tile has a peer that stores nothing), listed in shared memory
+// by every CTA for itself from the row tiles' experts. Measured, 16 experts, 6,002 rows of 2,560 into 2,432 and back, the
+// shared expert's products beside them: GROUPED_FIGURES
+#define GP_BN 256
+#define GP_STAGES 6
+#define GP_MAX_TILES 4096   // row tiles the list holds
+
+struct GroupedPairSmem {
+    static constexpr int A_BYTES = GG_ROWS * GG_K * 2, B_BYTES = (GP_BN / 2) * GG_K * 2;
+    static constexpr int BYTES = GP_STAGES * (A_BYTES + B_BYTES) + 1024 /* alignment */ + 256 /* barriers */ + GP_MAX_TILES * 2;
+};
+
+template <typename TO, int ACT>
+__global__ void __launch_bounds__(GG_THREADS) gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_x,
+                                                                       const __grid_constant__ CUtensorMap map_w, GemmGrouped g, int max_tiles) {
+    using S = GroupedPairSmem;
+    extern __shared__ uint8_t gg_smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)gg_smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t *a_tiles = smem, *b_tiles = smem + GP_STAGES * S::A_BYTES;
+    uint64_t *full = (uint64_t *)(smem + GP_STAGES * (S::A_BYTES + S::B_BYTES));
+    uint64_t *empty = full + GP_STAGES, *acc_full = empty + GP_STAGES, *acc_empty = acc_full + 2;
+    uint32_t *tmem_holder = (uint32_t *)(acc_empty + 2);
+    volatile int *flags = (volatile int *)(tmem_holder + 1);  // [0]: a wait ran out, [1]: entries of the list
+    uint16_t *list = (uint16_t *)((uint8_t *)full + 256);     // first row tile * 2 + whether the next one is the expert's too
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)tc::cluster_rank();  // 0: the leader, 1: its peer
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < GP_STAGES; s++) tc::mbar_init(&full[s], 1), tc::mbar_init(&empty[s], 1);
+        for (int b = 0; b < 2; b++) tc::mbar_init(&acc_full[b], 1), tc::mbar_init(&acc_empty[b], 8);  // every storing warp of both CTAs
+        flags[0] = 0;
+        tc::mbar_init_fence();
+        tc::tma_prefetch_map(&map_x), tc::tma_prefetch_map(&map_w);
+    }
+    if (warp == 1) tc::tmem_alloc_pair(tmem_holder, 2 * GP_BN);
+    if (warp == 2) {  // the tiles' experts were written at least two launches back: they may be read at once
+        int count = 0, run_carry = 0;  // the run of one expert's tiles that reaches into these 32 from before
+        for (int base = 0; base < max_tiles; base += 32) {
+            const int t = base + lane, e = t < max_tiles ? g.tile_expert[t] : -1;
+            const bool starts = t == 0 || (t < max_tiles && g.tile_expert[t - 1] != e);
+            const unsigned run_starts = __ballot_sync(0xffffffffu, starts), upto = run_starts & (0xffffffffu >> (31 - lane));
+            const int run = upto ? base + 31 - __clz(upto) : run_carry;
+            run_carry = __shfl_sync(0xffffffffu, run, 31);
+            const bool first = e >= 0 && ((t - run) & 1) == 0;
+            const bool both = first && t + 1 < max_tiles && g.tile_expert[t + 1] == e;
+            const unsigned firsts = __ballot_sync(0xffffffffu, first);
+            if (first) list[count + __popc(firsts & ((1u << lane) - 1))] = (uint16_t)(2 * t + (both ? 1 : 0));
+            count += __popc(firsts);
+        }
+        if (lane == 0) flags[1] = count;
+    }
+    tc::fence_before_sync();
+    tc::cluster_sync();  // both CTAs' barriers are there before either signals the other's
+    tc::fence_after_sync();
+    const uint32_t tmem = *tmem_holder;
+    const int m_tiles = flags[1], n_tiles = (g.N + GP_BN - 1) / GP_BN, tiles = m_tiles * n_tiles;
+
+    if (warp == 0) {
+        if (lane == 0 && pair < tiles) {
+            // A stage is full when both CTAs' copies have landed: all of them report to the leader's barrier.
+            constexpr uint32_t STAGE_BYTES = 2 * (S::A_BYTES + S::B_BYTES);
+            const int ahead = min(GP_STAGES, g.k_blocks);
+            {   // the weights of the first tile's first stages are asked for before pdl_wait(): nobody writes them
+                const int w_row = g.tile_expert[list[pair % m_tiles] >> 1] * g.N + (pair / m_tiles) * GP_BN + rank * (GP_BN / 2);
+                for (int i = 0; i < ahead; i++) {
+                    if (rank == 0) tc::mbar_expect_tx(&full[i], STAGE_BYTES);
+                    tc::tma_load_2d_pair(b_tiles + i * S::B_BYTES, &map_w, i * GG_K, w_row, tc::peer_smem(tc::smem_addr(&full[i]), 0));
+                }
+            }
+            pdl_wait();
+            int issued = 0;
+            for (int t = pair; t < tiles && !flags[0]; t += pairs) {
+                const int first = list[t % m_tiles] >> 1;
+                // (the peer's rows of an odd last tile: the same rows again, which are there, and nothing is stored)
+                const int p0 = (first + (rank && (list[t % m_tiles] & 1) ? 1 : 0)) * GG_ROWS;
+                const int w_row = g.tile_expert[first] * g.N + (t / m_tiles) * GP_BN + rank * (GP_BN / 2);
+                for (int kb = 0; kb < g.k_blocks; kb++, issued++) {
+                    const int s = issued % GP_STAGES;
+                    const uint32_t bar = tc::peer_smem(tc::smem_addr(&full[s]), 0);
+                    if (issued >= ahead) {
+                        if (!tc::mbar_wait(&empty[s], ((issued / GP_STAGES) & 1) ^ 1)) {  // (its own: the commit reaches both)
+                            flags[0] = 1;
+                            break;
+                        }
+                        if (rank == 0) tc::mbar_expect_tx(&full[s], STAGE_BYTES);
+                        tc::tma_load_2d_pair(b_tiles + s * S::B_BYTES, &map_w, kb * GG_K, w_row, bar);
+                    }
+                    tc::tma_load_2d_pair(a_tiles + s * S::A_BYTES, &map_x, kb * GG_K, p0, bar);
+                }
+            }
+        } else if (lane == 0) {
+            pdl_wait();
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = tc::idesc_bf16_f32(2 * GG_ROWS, GP_BN);
+            int done = 0, it = 0;
+            for (int t = pair; t < tiles && !flags[0]; t += pairs, it++) {
+                const int b = it & 1;
+                if (!tc::mbar_wait(&acc_empty[b], ((it >> 1) & 1) ^ 1)) {  // both CTAs are done with this accumulator
+                    flags[0] = 1;
+                    break;
+                }
+                tc::fence_after_sync();
+                for (int kb = 0; kb < g.k_blocks; kb++, done++) {
+                    const int s = done % GP_STAGES;
+                    if (!tc::mbar_wait(&full[s], (done / GP_STAGES) & 1)) {
+                        flags[0] = 1;
+                        break;
+                    }
+                    tc::fence_after_sync();
+                    const uint32_t a = tc::smem_addr(a_tiles + s * S::A_BYTES), bq = tc::smem_addr(b_tiles + s * S::B_BYTES);
+#pragma unroll
+                    for (int k = 0; k < GG_K / 16; k++)
+                        tc::mma_ss_pair(tmem + b * GP_BN, tc::smem_desc_k_sw128(a + k * 32), tc::smem_desc_k_sw128(bq + k * 32), idesc, kb > 0 || k > 0);
+                    tc::mma_commit_pair(&empty[s]);
+                }
+                if (flags[0]) break;
+                tc::mma_commit_pair(&acc_full[b]);
+            }
+        }
+    } else {
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+        int it = 0;
+        pdl_wait();
+        for (int t = pair; t < tiles; t += pairs, it++) {
+            const int b = it & 1, entry = list[t % m_tiles], q0 = (t / m_tiles) * GP_BN;
+            const bool stores = rank == 0 || (entry & 1);
+            TO *out = (TO *)g.out + ((long long)((entry >> 1) + rank) * GG_ROWS + row) * g.ldo;
+            const bool ok = __all_sync(0xffffffffu, !flags[0] && tc::mbar_wait(&acc_full[b], (it >> 1) & 1));
+            if (!ok) {
+                flags[0] = 1;
+                break;
+            }
+            tc::fence_after_sync();
+            if constexpr (ACT >= GG_SILU_GATED) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < GP_BN; c0 += 2 * GG_TURN)  // gate and up rows come in turns of 64
+#pragma unroll 1
+                    for (int c = 0; c < GG_TURN && q0 + c0 < g.N; c += 16) {
+                        uint32_t v[16], u[16];
+                        tc::tmem_ld16(lanes + b * GP_BN + c0 + c, v);
+                        tc::tmem_ld16(lanes + b * GP_BN + c0 + GG_TURN + c, u);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {  // gate and up pass through bfloat16, as they do where they are stored in between
+                            const float gate = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[j])));
+                            const float up = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[j])));
+                            v[j] = __float_as_uint(gated_mul(ACT == GG_CLAMPED_GATED ? ABK_CLAMPED : ABK_SILU, gate, up, g.limit));
+                        }
+                        TO *dst = out + (q0 + c0) / 2 + c;
+                        if (stores && g.vec) {
+                            gg_store16(dst, v);
+                        } else if (stores) {
+#pragma unroll
+                            for (int j = 0; j < 16; j++) dst[j] = from_float<TO>(__uint_as_float(v[j]));
+                        }
+                    }
+            } else {
+#pragma unroll 1
+                for (int c0 = 0; c0 < GP_BN && q0 + c0 < g.N; c0 += 32) {
+                    uint32_t v[32];
+                    tc::tmem_ld16(lanes + b * GP_BN + c0, v);
+                    tc::tmem_ld16(lanes + b * GP_BN + c0 + 16, v + 16);
+                    tc::tmem_ld_wait();
+                    if (ACT == GG_RELU_SQUARED) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) {
+                            const float f = __uint_as_float(v[j]);
+                            v[j] = __float_as_uint(f > 0.0f ? f * f : 0.0f);
+                        }
+                    }
+#pragma unroll
+                    for (int h = 0; h < 32; h += 16) {
+                        if (stores && g.vec && q0 + c0 + h + 16 <= g.N) {
+                            gg_store16(out + q0 + c0 + h, v + h);
+                        } else if (stores) {
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                if (q0 + c0 + h + j < g.N) out[q0 + c0 + h + j] = from_float<TO>(__uint_as_float(v[h + j]));
+                        }
+                    }
+                }
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive_in_cluster(tc::peer_smem(tc::smem_addr(&acc_empty[b]), 0));
+        }
+    }
+    // Nobody leaves while the other CTA may still signal its barriers or write its tensor memory. (After a wait that ran
+    // out, copies may still be on their way into this CTA's shared memory: give them a tenth of a millisecond.)
+    if (flags[0]) {
+        const uint64_t t0 = tc::global_ns();
+        while (tc::global_ns() - t0 < 100000) __nanosleep(1000);
+    }
+    tc::fence_before_sync();
+    tc::cluster_sync();
+    if (flags[0] && threadIdx.x == 0) atomicOr(g.status + 1, 1);
+    if (warp == 1) {
+        tc::fence_after_sync();
+        tc::tmem_free_pair(tmem, 2 * GP_BN);
+    }
+}
+
 // x bfloat16 [max_tiles * 128, K] (sorted rows); w bfloat16 [experts, N, K]; out [max_tiles * 128, ldo] bfloat16 or
 // (out_f32) float32; tile_expert int32 [max_tiles]; status int32 [>= 2]. Gated: N counts gate and up rows (a multiple of 128),
 // out has N / 2 columns.
@@ -309,9 +518,28 @@ extern "C" int abk_gemm_grouped(const void *x, const void *w, void *out, long lo
     GemmGrouped g;
     g.out = out, g.ldo = ldo, g.N = N, g.K = K, g.k_blocks = (K + GG_K - 1) / GG_K, g.tile_expert = tile_expert, g.status = status, g.limit = limit;
     g.vec = ((uintptr_t)out % 16 == 0) && (ldo * (out_f32 ? 4 : 2)) % 16 == 0;
+    cudaStream_t s = (cudaStream_t)stream;
+    // Pairs of CTAs where the rows fill at least a tile an expert on average, of small experts (whose launches are short) two:
+    // 16 experts and a shared one of 1,024 x 768, top 2, 800 tokens: a feed-forward in 64.5 us a CTA a tile against 68.2 in
+    // pairs, 1,500 tokens 82.5 against 78.5; of 2,560 x 2,432, 1,500 tokens: 278 against 231, 4,000: 538 against 407.
+    const int used = max_tiles - experts;  // the rows' own tiles; padding adds up to one an expert
+    if (N >= GP_BN && max_tiles <= GP_MAX_TILES && used >= experts && (used >= 2 * experts || (long long)N * K >= 4 << 20)) {
+        const int pairs = abk_sm_count() / 2;
+#define GP_LAUNCH(TO, ACT)                                                                                                         \
+    do {                                                                                                                           \
+        if (cudaError_t e = abk_allow_shared_memory((const void *)gemm_grouped_pair_kernel<TO, ACT>, GroupedPairSmem::BYTES))      \
+            return (int)e;                                                                                                         \
+        abk_launch_clusters(gemm_grouped_pair_kernel<TO, ACT>, dim3(2 * pairs), dim3(GG_THREADS), (size_t)GroupedPairSmem::BYTES, s, 2, mx, mw, g, max_tiles); \
+    } while (0)
+        if (out_f32) { if (activation) GP_LAUNCH(float, 1); else GP_LAUNCH(float, 0); }
+        else if (activation == GG_CLAMPED_GATED) GP_LAUNCH(__nv_bfloat16, GG_CLAMPED_GATED);
+        else if (activation == GG_SILU_GATED) GP_LAUNCH(__nv_bfloat16, GG_SILU_GATED);
+        else { if (activation) GP_LAUNCH(__nv_bfloat16, 1); else GP_LAUNCH(__nv_bfloat16, 0); }
+#undef GP_LAUNCH
+        return ABK_LAUNCH_RESULT();
+    }
     dim3 grid(max_tiles, (N + GG_BN - 1) / GG_BN);
     if (grid.y > 65535) ABK_REFUSE("gemm_grouped: %d output features are more than a grid takes", N);
-    cudaStream_t s = (cudaStream_t)stream;
 #define GG_LAUNCH(TO, ACT)                                                                                          \
     do {                                                                                                            \
         if (cudaError_t e = abk_allow_shared_memory((const void *)gemm_grouped_kernel<TO, ACT>, GroupedSmem::BYTES)) \

@@ -280,6 +280,43 @@ def test_the_router_and_the_products_by_expert(dtype, E, top, d, ff):
     np.testing.assert_allclose(host(sq), rnd(plain.relu_squared(h)), rtol=1e-6, atol=1e-6)
 
 
+@pytest.mark.parametrize("counts,N,K,kind", [((300, 0, 129, 600, 256), 400, 72, 0), ((1, 128, 700, 260), 256, 64, 1), ((900, 385), 264, 200, 1),
+                                             ((257, 513, 128), 384, 64, 2), ((1300,), 512, 136, 3), ((256, 255, 400), 256, 520, 0)])
+def test_the_product_by_expert_on_pairs_of_ctas(counts, N, K, kind):
+    """Runs of rows of every length against whole tiles and pairs of them (an odd last tile, one row, no row), outputs that end
+    within a tile of 256, activations; rows of padding that are no numbers reach nothing."""
+    from abacus_b200.kernels import ops
+    rng, E, n = np.random.default_rng(sum(counts) + N), len(counts), sum(counts)
+    order = rng.permutation(n)
+    expert = torch.empty(n, dtype=torch.int32, device=DEV)
+    expert[torch.from_numpy(order).to(DEV)] = torch.from_numpy(np.repeat(np.arange(E, dtype=np.int32), counts)).to(DEV)
+    x, w = (dev(rng.standard_normal(s), torch.bfloat16) for s in ((n, K), (E, N, K)))
+    tiles = ops.grouped_tiles(n, E)
+    assert tiles - E >= 2 * E and N >= 256  # (the sizes that go in pairs)
+    scratch = torch.empty(2 * E + n, dtype=torch.int32, device=DEV)
+    place, tile_expert = torch.empty(n, dtype=torch.int32, device=DEV), torch.empty(tiles, dtype=torch.int32, device=DEV)
+    rows = torch.full((tiles * 128, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.moe_sort(x, 1, expert, None, n, E, scratch, place, tile_expert, rows)
+    gated, activation = kind >= 2, (0, ops.RELU_SQUARED, ops.SILU_GATED, ops.CLAMPED_GATED)[kind]
+    got = torch.zeros((tiles * 128, N // 2 if gated else N), dtype=torch.bfloat16 if kind else torch.float32, device=DEV)
+    ops.gemm_grouped(rows, w, got, tile_expert, activation=activation, limit=2.0)
+    want = torch.einsum("pk,pnk->pn", x.double(), w.double()[expert.long()]) if n * N * K < 1 << 27 else torch.stack(
+        [w[e].double() @ r.double() for r, e in zip(x, expert.tolist())])
+    if kind == 1:
+        want = torch.relu(want) ** 2
+    elif gated:
+        turns = want.to(torch.bfloat16).double().view(n, -1, 2, ops.GROUPED_TURN)
+        g, u = turns[:, :, 0], turns[:, :, 1]
+        if kind == 3:
+            g, u = g.clamp(max=2.0), u.clamp(-2.0, 2.0) + 1.0
+        want = (g * torch.sigmoid((1.702 if kind == 3 else 1.0) * g) * u).reshape(n, -1)
+    diff = (got[place.long()].double() - want).abs()
+    # float32: sums of K products; bfloat16 results: their rounding, and in gated ones that of gate and up (an ulp moved)
+    limit = 1e-4 * K ** 0.5 if not kind else (2.0 ** -8 if kind == 1 else 2.0 ** -5) * want.abs() + 0.05
+    assert bool((diff <= limit).all()), float((diff - limit).max())
+    assert not ops.kernel_status(x.device).any()
+
+
 # ------------------------------------------------------------------ whole models through the engine
 def _engine(tmp_path, name, dtype, **kw):
     from abacus_b200.engine import Engine, load_model
