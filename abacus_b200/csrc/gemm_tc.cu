@@ -39,6 +39,13 @@
 #define TILE_K 64
 #define GEMM_THREADS 192
 
+// What is applied to a sum where it is stored: an activation of the library's, or GEMM_RELU_SQUARED_STORED, the square of relu of
+// the sum as the storage type bfloat16 holds it (what a product and an activation behind it would leave).
+#define GEMM_RELU_SQUARED_STORED 2
+__device__ __forceinline__ float gemm_act(int act, float v) {
+    return act == GEMM_RELU_SQUARED_STORED ? out_act(ABK_OUT_RELU_SQUARED, __bfloat162float(__float2bfloat16_rn(v))) : out_act(act, v);
+}
+
 struct GemmTc {
     void *out;
     long long stride_p, stride_q;  // out element (p, q) is out[p * stride_p + q * stride_q]
@@ -176,7 +183,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
                 tc::tmem_ld_wait();
                 if (direct && g.act) {
 #pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] = __float_as_uint(out_act(g.act, __uint_as_float(v[j])));
+                    for (int j = 0; j < 16; j++) v[j] = __float_as_uint(gemm_act(g.act, __uint_as_float(v[j])));
                 }
                 if (g.in_cluster) {  // the operands' stages are free: every product has read them
                     float *at = (float *)smem + row * (BN + 4) + c0;
@@ -232,7 +239,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
                         for (int j = 0; j < 8; j++)
                             if (c0 + j < cols)
                                 out[(long long)p * g.stride_p + (long long)(q0 + c0 + j) * g.stride_q] =
-                                    from_float<TO>(out_act(g.act, sum[j]));
+                                    from_float<TO>(gemm_act(g.act, sum[j]));
                     }
                 }
                 if (threadIdx.x == 64) g.tickets[tile] = 0;
@@ -263,7 +270,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) gemm_tc_kernel(const __grid_cons
                     for (int j = 0; j < 4; j++)
                         if (q0 + gi * 4 + j < g.Q)
                             out[(long long)p * g.stride_p + (long long)(q0 + gi * 4 + j) * g.stride_q] =
-                                from_float<TO>(out_act(g.act, r4[j]));
+                                from_float<TO>(gemm_act(g.act, r4[j]));
                 }
             }
         }
@@ -558,7 +565,7 @@ __global__ void __launch_bounds__(EPI == EPI_QKV ? QKV_THREADS : GEMM_THREADS) g
                     tc::tmem_ld_wait();
                     if (g.act) {
 #pragma unroll
-                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(out_act(g.act, __uint_as_float(v[j])));
+                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(gemm_act(g.act, __uint_as_float(v[j])));
                     }
 #pragma unroll
                     for (int h = 0; h < 32; h += 16) {
@@ -752,7 +759,7 @@ __global__ void __launch_bounds__(EPI == EPI_QKV ? QKV_THREADS : GEMM_THREADS) g
                     tc::tmem_ld_wait();
                     if (g.act) {
 #pragma unroll
-                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(out_act(g.act, __uint_as_float(v[j])));
+                        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(gemm_act(g.act, __uint_as_float(v[j])));
                     }
 #pragma unroll
                     for (int h = 0; h < 32; h += 16) {
@@ -990,7 +997,8 @@ extern "C" int abk_gemm_tc_act(const void *x, const void *w, void *out, int out_
                                long long ldw, long long ldo, float *scratch, int *tickets, int *status, int force_bn,
                                int force_swap, int force_splits, int force_persistent, int act, void *stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (act != ABK_OUT_PLAIN && act != ABK_OUT_RELU_SQUARED) ABK_REFUSE("gemm_tc: activation %d is not built", act);
+    if (act != ABK_OUT_PLAIN && act != ABK_OUT_RELU_SQUARED && (act != GEMM_RELU_SQUARED_STORED || out_dtype != ABK_BF16))
+        ABK_REFUSE("gemm_tc: activation %d is not built", act);
     if (K <= 0 || K % 8 || ldx % 8 || ldw % 8)
         ABK_REFUSE("gemm_tc: K = %d and the row pitches %lld, %lld must be multiples of 8", K, ldx, ldw);
     if (((uintptr_t)x | (uintptr_t)w) & 15) ABK_REFUSE("gemm_tc: operands must be 16-byte aligned");

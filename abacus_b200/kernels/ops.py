@@ -841,7 +841,8 @@ def gemm_tc(x, w, out, m=None, tile_n=0, swap=-1, splits=0, persistent=-1, activ
     """out[:m] = x[:m] . w^T in bfloat16 on the tcgen05 tensor cores, float32 accumulation.
 
     tile_n, swap, splits and persistent pin the tile configuration (tests); 0 / -1 / 0 / -1 let the
-    kernel choose. activation: applied to the sums (OUT_ACTIVATIONS).
+    kernel choose. activation: applied to the sums (OUT_ACTIVATIONS), or (bfloat16 results) "relu_squared_stored", applied to the
+    sums as rounded for storage.
     """
     _need_cuda(x, w, out)
     lib = load_module("gemm_tc")
@@ -854,7 +855,8 @@ def gemm_tc(x, w, out, m=None, tile_n=0, swap=-1, splits=0, persistent=-1, activ
     _check(lib, lib.abk_gemm_tc_act(_p(x), _p(w), _p(out), _i(_dt(out)), _i(m), _i(n), _i(k), _ll(x.stride(0)),
                                     _ll(w.stride(0)), _ll(out.stride(0)), _p(sc.gemm_floats), _p(sc.gemm_tickets),
                                     _p(sc.status), _i(tile_n), _i(swap), _i(splits), _i(persistent),
-                                    _i(OUT_ACTIVATIONS[activation]), _stream()), "gemm_tc")
+                                    _i(2 if activation == "relu_squared_stored" else OUT_ACTIVATIONS[activation]), _stream()),
+           "gemm_tc")
 
 
 # ------------------------------------------------------------------ streams (csrc/streams.cu)

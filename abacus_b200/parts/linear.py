@@ -36,15 +36,19 @@ class Linear:
         self.out_features, self.in_features = weight.shape
 
     def forward(self, x, out, m=None, activation=None):
-        """out[:m] = act(x[:m] . W^T); activation (ops.OUT_ACTIVATIONS): in the product's epilogue where it has one."""
+        """out[:m] = act(x[:m] . W^T); activation (ops.OUT_ACTIVATIONS): in the product's epilogue where it has one.
+        "relu_squared_stored": of the product as it is stored, the same numbers whether one kernel makes them or two."""
         rows = x.shape[0] if m is None else m
+        after = activation if activation == "relu_squared_stored" else None  # (the rows kernel's epilogue has the others)
         if (self.weight.dtype == torch.bfloat16 and rows_kernel_wins(rows, self.weight)
                 and ops.gemm_rows_takes(x, self.weight, out, rows)):
-            ops.gemm_rows(x, self.weight, out, rows, activation=activation)
+            ops.gemm_rows(x, self.weight, out, rows, activation=None if after else activation)
+            if after:
+                ops.relu_squared(out, rows)
         elif self.weight.dtype == torch.bfloat16 and ops.gemm_tc_takes(x, self.weight, out):
             ops.gemm_tc(x, self.weight, out, m, activation=activation)
         else:
             ops.gemm_simt(x, self.weight, out, m)
-            if activation == "relu_squared":
+            if activation is not None:
                 ops.relu_squared(out, rows)
         return out

@@ -154,8 +154,7 @@ class RoutedMLP:
             return self.forward_weighted_sum(xn, out, expert, weight, n, pairs, ws, shared_weight)
         if self.shared_up is not None:
             shared_act = ws.get("moe_shared_act", (n, s.shared.inter), dt)
-            self.shared_up.forward(xn, shared_act, n)
-            ops.relu_squared(shared_act, n)
+            self.shared_up.forward(xn, shared_act, n, activation="relu_squared_stored")  # in the product's epilogue
             self.shared_down.forward(shared_act, out, n)
         if pairs > GROUPED_FROM and on_input and ops.grouped_takes(xn, self.up, self.down):
             tiles = ops.grouped_tiles(pairs, n_experts)
