@@ -9,8 +9,9 @@
 // float32; q, k and v come from the convolution in the model's storage type.
 //
 // A value column of S never meets another: column j needs S[:, j], v_j and the token's q, k, g, b. So a thread
-// keeps (a part of) one column in registers and walks the sequence's tokens in order, and a prompt of any length
-// and a decode step are the same kernel. The state is stored [head, value, key], so a column is one contiguous run.
+// keeps (a part of) one column in registers and walks the sequence in order: prompts in blocks of four tokens, whose
+// vectors a kernel makes ahead of the walk, and a step of one token a sequence in one kernel with its preparation. The
+// state is stored [head, value, key], so a column is one contiguous run.
 #define ABK_DEFINE_ERROR
 #include "recurrence.cuh"
 
