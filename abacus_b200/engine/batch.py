@@ -117,17 +117,23 @@ class StepBatch:
             h["tokens"][:n_seqs] = [s.tokens[0] for s in sequences]
             h["token_seq"][:n_seqs] = np.arange(n_seqs)
             h["token_pos"][:n_seqs] = starts_a
+        elif n_seqs == 1:
+            _put_words(h["tokens"], 0, sequences[0].tokens)
+            h["token_seq"][:n_tokens] = 0
+            h["token_pos"][:n_tokens] = np.arange(starts[0], starts[0] + n_tokens)
         else:
             for s, row in zip(sequences, first.tolist()):
                 _put_words(h["tokens"], row, s.tokens)
             h["token_seq"][:n_tokens] = np.repeat(np.arange(n_seqs), lens_a)
             h["token_pos"][:n_tokens] = np.arange(n_tokens) + np.repeat(starts_a - first, lens_a)
-        h["tokens"][n_tokens:] = 0
-        h["token_seq"][n_tokens:] = -1
-        h["token_pos"][n_tokens:] = 0
+        if n_tokens < self.cap_rows:
+            h["tokens"][n_tokens:] = 0
+            h["token_seq"][n_tokens:] = -1
+            h["token_pos"][n_tokens:] = 0
         for name, values in (("seq_slot", [s.slot for s in sequences]), ("seq_pos0", starts_a), ("seq_len_after", starts_a + lens_a)):
             h[name][:n_seqs] = values
-            h[name][n_seqs:] = 0
+            if n_seqs < self.cap_seqs:
+                h[name][n_seqs:] = 0
         h["seq_start"][:n_seqs] = first
         h["seq_start"][n_seqs:] = n_tokens
         lr = 0

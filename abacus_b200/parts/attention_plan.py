@@ -82,14 +82,16 @@ class AttentionStepPlan:
         info = {"n_halved": 0, "counts": counts, "tile_pages": {}}
         if is_decode:  # one token each: the decode kernels need no lists
             return info
-        of_rows = {r: tiles_of(sequences, r) for r in TILE_ROWS}
+        starts = np.array([s.start for s in sequences], dtype=np.int64)
+        lengths = np.array([len(s.tokens) for s in sequences], dtype=np.int64)
+        of_rows = {r: tiles_of(starts, lengths, r) for r in TILE_ROWS}
         for r, (tiles, pages) in of_rows.items():
             off = layout.offset[f"tiles{r}"]
             words[off:off + tiles.size] = tiles.reshape(-1)
             info["tile_pages"][r] = pages
             if exact:
                 counts[f"tiles{r}"] = len(tiles)
-        work, n_halved = self._work_list(sequences, of_rows[PAIRED_ROWS][0])
+        work, n_halved = self._work_list(sequences, starts, lengths, of_rows[PAIRED_ROWS][0])
         off = layout.offset["work"]
         words[off:off + work.size] = work.reshape(-1)
         info["n_halved"] = n_halved
@@ -97,10 +99,9 @@ class AttentionStepPlan:
             counts["work"] = len(work)
         return info
 
-    def _work_list(self, sequences, tiles):
+    def _work_list(self, sequences, starts, news, tiles):
         """The work list of the prefill attention kernel that halves long tiles. CTAs with the most pages come first."""
         seq, row = tiles[:, 0].astype(np.int64), tiles[:, 1].astype(np.int64)
-        starts, news = (np.array(v, dtype=np.int64) for v in ([s.start for s in sequences], [len(s.tokens) for s in sequences]))
         start, new = starts[seq], news[seq]
         pages = (start + np.minimum(row + PAIRED_ROWS, new) - 1) // 64 + 1
         # With fewer CTAs than the device holds at once, the longest tiles stand twice (each time with half of
@@ -110,36 +111,41 @@ class AttentionStepPlan:
         slots = self.cta_slots if self.cta_slots is not None else CTAS_PER_SM * sm_count()
         spare = 1.05 * slots - len(pages) * heads
         k = min(int(np.ceil(spare / heads)) if spare > 0 else 0, HALVED_PAIRS // heads, len(pages))
-        split = np.zeros(len(pages), dtype=bool)
-        longest = np.argsort(-pages, kind="stable")[:k]
-        split[longest] = pages[longest] >= 8
-        halved, whole = np.flatnonzero(split), np.flatnonzero(~split)
-        ids = np.zeros(len(pages), dtype=np.int64)
-        ids[halved] = np.arange(len(halved))
-        # (pages, tile, part) of every entry: the halves with earlier keys, with later keys, the whole tiles
-        tile = np.concatenate([halved, halved, whole])
-        part = np.repeat([1, 2, 0], [len(halved), len(halved), len(whole)])
-        length = np.concatenate([(pages[halved] + 1) // 2, pages[halved] // 2, pages[whole]])
-        order = np.argsort(-length, kind="stable")  # the CTAs with the most pages first
-        tile, part = tile[order], part[order]
+        if k > 0 and pages.max() >= 8:
+            split = np.zeros(len(pages), dtype=bool)
+            longest = np.argsort(-pages, kind="stable")[:k]
+            split[longest] = pages[longest] >= 8
+            halved, whole = np.flatnonzero(split), np.flatnonzero(~split)
+            ids = np.zeros(len(pages), dtype=np.int64)
+            ids[halved] = np.arange(len(halved))
+            # (pages, tile, part) of every entry: the halves with earlier keys, with later keys, the whole tiles
+            tile = np.concatenate([halved, halved, whole])
+            part = np.repeat([1, 2, 0], [len(halved), len(halved), len(whole)])
+            length = np.concatenate([(pages[halved] + 1) // 2, pages[halved] // 2, pages[whole]])
+            order = np.argsort(-length, kind="stable")  # the CTAs with the most pages first
+            tile, part = tile[order], part[order]
+            n_halved, ids = len(halved), ids[tile]
+        else:  # no tile is long enough: nothing to put together (a step of short prompts is bound by this very code)
+            tile, part, n_halved, ids = np.argsort(-pages, kind="stable"), 0, 0, 0
         of = seq[tile]
-        first_row = np.concatenate([[0], np.cumsum(news)])
         slot_of = np.array([s.slot for s in sequences], dtype=np.int64)
-        work = np.stack([of, row[tile], part, first_row[of], start[tile], new[tile], slot_of[of], ids[tile]], axis=1).astype(np.int32)
-        return work, len(halved)
+        work = np.empty((len(tile), WORK_INTS), dtype=np.int32)
+        columns = (of, row[tile], part, (np.cumsum(news) - news)[of], start[tile], new[tile], slot_of[of], ids)
+        for c, values in enumerate(columns):
+            work[:, c] = values
+        return work, n_halved
 
 
-def tiles_of(sequences, rows_per_tile):
+def tiles_of(starts, lengths, rows_per_tile):
     """((sequence, first row among its new tokens) of every tile of `rows_per_tile` query rows, int32 [tiles, 2], the
-    tiles that see the most keys first; pages of 64 keys each tile sees, in the sequences' order)."""
-    lengths = np.array([len(s.tokens) for s in sequences], dtype=np.int64)
+    tiles that see the most keys first; pages of 64 keys each tile sees, in the sequences' order) of a step whose sequences
+    bring `lengths` tokens behind their first `starts` (int64)."""
     counts = -(-lengths // rows_per_tile)
-    seq = np.repeat(np.arange(len(sequences), dtype=np.int32), counts)
-    first = np.cumsum(counts) - counts
-    row = ((np.arange(len(seq), dtype=np.int64) - first[seq]) * rows_per_tile).astype(np.int32)
-    keys = np.array([s.start for s in sequences], dtype=np.int64)[seq] + row
+    seq = np.arange(len(lengths)).repeat(counts)
+    row = (np.arange(len(seq)) - (counts.cumsum() - counts)[seq]) * rows_per_tile
+    keys = starts[seq] + row
     # tiles that see the most keys first: the long ones start early and the short ones fill the tail
-    order = np.argsort(-keys, kind="stable")
-    last = np.minimum(row + rows_per_tile, lengths[seq])
-    pages = (keys + last - row - 1) // 64 + 1
-    return np.stack([seq[order], row[order]], axis=1), pages
+    order = (-keys).argsort(kind="stable")
+    tiles = np.empty((len(seq), 2), dtype=np.int32)
+    tiles[:, 0], tiles[:, 1] = seq[order], row[order]
+    return tiles, (keys + np.minimum(rows_per_tile, lengths[seq] - row) - 1) // 64 + 1
