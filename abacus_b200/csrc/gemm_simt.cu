@@ -3,90 +3,96 @@
 // This is the matrix product of the true 32-bit path (no tensor cores, no TF32), and the
 // fallback of the bfloat16 path for shapes the tensor-core kernel refuses. An output element is the sum of eight running
 // sums: K in pieces of 16, piece c to sum c % 8, each sum over its k in ascending order, then in pairs,
-// ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); up to K = 256 of one sum alone, over k in ascending order (a chain of
-// that length needs no cutting, and the small products of small models keep the order they had). So a row's result does not depend on how many other rows are in the
-// batch or where its tile lies.
+// ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); up to K = 256 it is one sum over k in ascending order (a chain of that
+// length needs no cutting, and the small products of small models keep the order they had). So a row's result does not
+// depend on how many other rows are in the batch or where its tile lies.
 // Formula: src/model.c:299, 302, 307, 309, 324 (weights are [out, in] row-major, no bias).
 //
-// A CTA has one tile of outputs, and each of its eight warps one of the eight sums of all of them: a product of a few
-// hundred rows has too few outputs to fill 148 SMs with warps whose lanes hold enough of them. Shared memory gives a warp
-// a number a lane and cycle, and an SM's four schedulers share it; a lane with 16 x 8 outputs needs 24 numbers for 128
-// multiply-adds (0.75 of what the schedulers could use up), one with 8 x 8 needs 16 for 64 (all of it). A warp stages its own
-// pieces, 16 bytes at a time by cp.async (rows of 20 floats: eight rows' pieces lie in different banks), one ahead, and meets the
-// others only at the end. Measured (one launch, operands from HBM): 500 x 6144 x 1024 in 204 us and 500 x 1024 x 3072 in 98
-// (31 and 32 TFLOP/s; the kernel that stood here, tiles of 64 x 64 with one sum and 4 x 4 outputs a lane: 329 and 299 us), 1 x
-// 1024 x 3072 in 14.5 us (317). Multiply-adds of three registers alone run at 60 TFLOP/s here; the rest goes to their
-// registers' banks and to waiting for the next piece. Half the tile, twice the CTAs an SM: 259 and 134 us.
+// A warp has one tile of outputs and one of their sums. It stages its own pieces, 16 bytes at a time by cp.async (rows of 20
+// floats: eight rows' pieces lie in different banks), one to three ahead, and waits for no other warp on the way. With eight
+// sums a CTA's eight warps have them all of one tile, and meet at the end: a product of a few hundred rows has too few outputs
+// to fill 148 SMs with warps whose lanes hold enough of them. Shared memory gives a warp a number a lane and cycle, and an
+// SM's four schedulers share it; a lane with 16 x 8 outputs needs 24 numbers for 128 multiply-adds (0.75 of what the
+// schedulers could use up), one with 8 x 8 needs 16 for 64 (all of it). Measured (one launch, operands from HBM): 500 x 6144 x
+// 1024 in 197 us and 500 x 1024 x 3072 in 97 (32 TFLOP/s; tiles of 64 x 64 of a whole CTA with one sum and 4 x 4 outputs a
+// lane: 322 and 220 us), 1 x 1024 x 3072 in 12 us (214). Multiply-adds of three registers alone run at 60 TFLOP/s here; the
+// rest goes to their registers' banks and to waiting for the next piece. Half the tile, twice the CTAs an SM: 259 and 134 us.
+// With one sum a CTA is one warp, so that an SM holds ten of them and takes the next when one is done; small tiles, since K
+// is too short to cut and many warps must share the outputs: 2048 x 4096 x 128 in 65 us, 2048 x 4096 x 64 in 36, 1 x 8192 x 128 in
+// 3.6 (a CTA's tile of 64 x 64 and 4 x 4 outputs a lane: 98, 52 and 10.8; one warp of eight of a CTA of 160 KB: 330, 184 and 26).
 #define ABK_DEFINE_ERROR
 #include "common.cuh"
 
-#define GS_WARPS 8
+#define GS_WARPS 8      // of a CTA that cuts its sums
 #define GS_BK 16
 #define GS_PITCH 20     // floats of a staged row
-#define GS_ONE_SUM 16   // up to this many pieces the first warp takes them all
+#define GS_ONE_SUM 256  // up to this K an element is one sum
 
 __device__ __forceinline__ void gs_copy_16(float *dst, const float *src, bool real) {
     const int bytes = real ? 16 : 0;  // 0: zeros
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-// TM x TN: outputs a lane has, rows 4 apart and columns 8 apart; a tile has 4 TM x 8 TN. ASYNC: float32 operands whose rows
-// start on 16-byte boundaries, K a multiple of 4.
-template <typename TX, typename TW, typename TO, int TM, int TN, bool ASYNC>
-__global__ void __launch_bounds__(32 * GS_WARPS) gemm_simt_kernel(const TX *__restrict__ x, const TW *__restrict__ w, TO *__restrict__ out, int M,
-                                                                  int N, int K, long long ldx, long long ldw, long long ldo) {
+// TM x TN: outputs a lane has, rows 4 apart and columns 8 apart; a tile has 4 TM x 8 TN. WARPS: GS_WARPS sums an element, or 1.
+// STAGES: pieces of a warp in flight or in use. ASYNC: float32 operands whose rows start on 16-byte boundaries, K a multiple
+// of 4.
+template <typename TX, typename TW, typename TO, int TM, int TN, int WARPS, int STAGES, bool ASYNC>
+__global__ void __launch_bounds__(32 * WARPS) gemm_simt_kernel(const TX *__restrict__ x, const TW *__restrict__ w, TO *__restrict__ out, int M,
+                                                               int N, int K, long long ldx, long long ldw, long long ldo) {
     constexpr int BM = 4 * TM, BN = 8 * TN, STAGE = (BM + BN) * GS_PITCH;
-    extern __shared__ __align__(16) float gs_smem[];  // [warps][2 stages][BM rows of x, then BN of w][20]
+    extern __shared__ __align__(16) float gs_smem[];  // [warps][stages][BM rows of x, then BN of w][20]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tx = lane & 7, ty = lane >> 3;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    float *mine = gs_smem + warp * 2 * STAGE;
+    const int m_tiles = (M + BM - 1) / BM, m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
+    float *mine = gs_smem + warp * STAGES * STAGE;
     const int r_mine = lane >> 2, c_mine = (lane & 3) * 4;  // a lane's pieces: every 8th row from here
     const TX *x_mine = x + (long long)(m0 + r_mine) * ldx + c_mine;
     const TW *w_mine = w + (long long)(n0 + r_mine) * ldw + c_mine;
     pdl_wait();
     const int pieces = (K + GS_BK - 1) / GS_BK;
     auto fetch = [&](int piece, int stage) {
-        float *dst = mine + stage * STAGE;
-        const int k0 = piece * GS_BK;
-        if constexpr (ASYNC) {
-            const bool in = k0 + c_mine < K;
+        if (piece < pieces) {
+            float *dst = mine + stage * STAGE;
+            const int k0 = piece * GS_BK;
+            if constexpr (ASYNC) {
+                const bool in = k0 + c_mine < K;
 #pragma unroll
-            for (int i = 0; i < BM / 8; i++) {
-                const bool real = in && m0 + r_mine + 8 * i < M;
-                gs_copy_16(dst + (r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)x_mine + 8 * i * ldx + k0 : (const float *)x, real);
-            }
-#pragma unroll
-            for (int i = 0; i < BN / 8; i++) {
-                const bool real = in && n0 + r_mine + 8 * i < N;
-                gs_copy_16(dst + (BM + r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)w_mine + 8 * i * ldw + k0 : (const float *)w, real);
-            }
-        } else {
-            for (int e = lane; e < (BM + BN) * GS_BK; e += 32) {
-                const int r = e / GS_BK, c = e % GS_BK, k = k0 + c;
-                float v = 0.0f;
-                if (r < BM) {
-                    if (m0 + r < M && k < K) v = to_float(x[(long long)(m0 + r) * ldx + k]);
-                } else if (n0 + r - BM < N && k < K) {
-                    v = to_float(w[(long long)(n0 + r - BM) * ldw + k]);
+                for (int i = 0; i < BM / 8; i++) {
+                    const bool real = in && m0 + r_mine + 8 * i < M;
+                    gs_copy_16(dst + (r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)x_mine + 8 * i * ldx + k0 : (const float *)x, real);
                 }
-                dst[r * GS_PITCH + c] = v;
+#pragma unroll
+                for (int i = 0; i < BN / 8; i++) {
+                    const bool real = in && n0 + r_mine + 8 * i < N;
+                    gs_copy_16(dst + (BM + r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)w_mine + 8 * i * ldw + k0 : (const float *)w, real);
+                }
+            } else {
+                for (int e = lane; e < (BM + BN) * GS_BK; e += 32) {
+                    const int r = e / GS_BK, c = e % GS_BK, k = k0 + c;
+                    float v = 0.0f;
+                    if (r < BM) {
+                        if (m0 + r < M && k < K) v = to_float(x[(long long)(m0 + r) * ldx + k]);
+                    } else if (n0 + r - BM < N && k < K) {
+                        v = to_float(w[(long long)(n0 + r - BM) * ldw + k]);
+                    }
+                    dst[r * GS_PITCH + c] = v;
+                }
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");  // (a group each time, empty beyond the last piece)
     };
     float acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[i][j] = 0.0f;
-    const int step = pieces <= GS_ONE_SUM ? 1 : GS_WARPS, end = step == 1 && warp > 0 ? 0 : pieces;
-    if (warp < end) fetch(warp, 0);
-    for (int piece = warp, it = 0; piece < end; piece += step, it++) {
-        if (piece + step < end) fetch(piece + step, (it + 1) & 1);
-        else asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; s++) fetch(warp + s * WARPS, s);
+    int stage = 0;
+    for (int piece = warp; piece < pieces; piece += WARPS) {
+        fetch(piece + (STAGES - 1) * WARPS, stage == 0 ? STAGES - 1 : stage - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
         __syncwarp();
-        const float *xs = mine + (it & 1) * STAGE + ty * GS_PITCH, *ws = mine + (it & 1) * STAGE + (BM + tx) * GS_PITCH;
+        const float *xs = mine + stage * STAGE + ty * GS_PITCH, *ws = mine + stage * STAGE + (BM + tx) * GS_PITCH;
 #pragma unroll
         for (int k = 0; k < GS_BK; k += 2) {
             float2 a[TM], b[TN];
@@ -99,34 +105,44 @@ __global__ void __launch_bounds__(32 * GS_WARPS) gemm_simt_kernel(const TX *__re
 #pragma unroll
                 for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, acc[i][j]));
         }
-        __syncwarp();  // the stage is filled again by the iteration after next
+        __syncwarp();  // the next iteration fills this stage again
+        stage = stage == STAGES - 1 ? 0 : stage + 1;
     }
-    __syncthreads();
-    constexpr int PITCH = BN + 8, TILE = BM * PITCH;  // (four rows' runs of eight columns lie in different banks)
-    float *sums = gs_smem;  // [warps][BM][PITCH]
+    if constexpr (WARPS == 1) {
 #pragma unroll
-    for (int i = 0; i < TM; i++)
+        for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < TN; j++) sums[warp * TILE + (ty + 4 * i) * PITCH + tx + 8 * j] = acc[i][j];
-    __syncthreads();
-    for (int e = threadIdx.x; e < BM * BN; e += 32 * GS_WARPS) {
-        const int r = e / BN, c = e % BN;
-        const float *s = sums + r * PITCH + c;
-        if (m0 + r < M && n0 + c < N)
-            out[(long long)(m0 + r) * ldo + n0 + c] = from_float<TO>(((s[0] + s[TILE]) + (s[2 * TILE] + s[3 * TILE])) + ((s[4 * TILE] + s[5 * TILE]) + (s[6 * TILE] + s[7 * TILE])));
+            for (int j = 0; j < TN; j++)
+                if (m0 + ty + 4 * i < M && n0 + tx + 8 * j < N) out[(long long)(m0 + ty + 4 * i) * ldo + n0 + tx + 8 * j] = from_float<TO>(acc[i][j]);
+    } else {
+        __syncthreads();
+        constexpr int PITCH = BN + 8, TILE = BM * PITCH;  // (four rows' runs of eight columns lie in different banks)
+        float *sums = gs_smem;  // [warps][BM][PITCH]
+#pragma unroll
+        for (int i = 0; i < TM; i++)
+#pragma unroll
+            for (int j = 0; j < TN; j++) sums[warp * TILE + (ty + 4 * i) * PITCH + tx + 8 * j] = acc[i][j];
+        __syncthreads();
+        for (int e = threadIdx.x; e < BM * BN; e += 32 * WARPS) {
+            const int r = e / BN, c = e % BN;
+            const float *s = sums + r * PITCH + c;
+            if (m0 + r < M && n0 + c < N)
+                out[(long long)(m0 + r) * ldo + n0 + c] = from_float<TO>(((s[0] + s[TILE]) + (s[2 * TILE] + s[3 * TILE])) + ((s[4 * TILE] + s[5 * TILE]) + (s[6 * TILE] + s[7 * TILE])));
+        }
     }
 }
 
-template <typename TX, typename TW, typename TO, int TM, int TN, bool ASYNC>
+template <typename TX, typename TW, typename TO, int TM, int TN, int WARPS, int STAGES, bool ASYNC>
 static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int N, int K, long long ldx, long long ldw, long long ldo, cudaStream_t s) {
     constexpr int BM = 4 * TM, BN = 8 * TN;
-    constexpr int ring = GS_WARPS * 2 * (BM + BN) * GS_PITCH * 4, sums = GS_WARPS * BM * (BN + 8) * 4, smem = ring > sums ? ring : sums;
-    const dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
-    if (grid.y > 65535) ABK_REFUSE("gemm: %d output columns are more than one launch takes", N);
-    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_simt_kernel<TX, TW, TO, TM, TN, ASYNC>, smem);
+    constexpr int ring = WARPS * STAGES * (BM + BN) * GS_PITCH * 4, sums = WARPS == 1 ? 0 : WARPS * BM * (BN + 8) * 4, smem = ring > sums ? ring : sums;
+    const long long tiles = ((long long)M + BM - 1) / BM * (((long long)N + BN - 1) / BN);
+    if (tiles > 0x7fffffffLL) ABK_REFUSE("gemm: %d x %d outputs are more than one launch takes", M, N);
+    const dim3 grid((unsigned)tiles);
+    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_simt_kernel<TX, TW, TO, TM, TN, WARPS, STAGES, ASYNC>, smem);
     if (e != cudaSuccess) return (int)e;
-    abk_launch(gemm_simt_kernel<TX, TW, TO, TM, TN, ASYNC>, grid, dim3(32 * GS_WARPS), smem, s, (const TX *)x, (const TW *)w, (TO *)out, M, N, K, ldx,
-               ldw, ldo);
+    abk_launch(gemm_simt_kernel<TX, TW, TO, TM, TN, WARPS, STAGES, ASYNC>, grid, dim3(32 * WARPS), smem, s, (const TX *)x, (const TW *)w, (TO *)out, M, N, K,
+               ldx, ldw, ldo);
     return ABK_LAUNCH_RESULT();
 }
 
@@ -137,14 +153,19 @@ extern "C" int abk_gemm_simt(const void *x, int x_dtype, const void *w, int w_dt
     if (K <= 0) ABK_REFUSE("gemm: K = %d", K);
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
-    // Tiles of 64 x 64 where they fill two thirds of the SMs, else of 32 x 32 (of 16 x 16 for up to 16 rows; tiles of 64
-    // where smaller ones were more than a grid takes): 64 x 1024 x 3072, 16 large tiles or 64 of 32 x 32, in 114 or 34 us.
-    const long long large = (long long)((M + 63) / 64) * ((N + 63) / 64);
-    const int tile = large >= abk_sm_count() * 2 / 3 || N > 65535 * 16 ? 64 : M > 16 ? 32 : 16;
-#define GS_LAUNCH(TX, TW, TO, ASYNC)                                                                              \
-    (tile == 64   ? gemm_simt_launch<TX, TW, TO, 16, 8, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)              \
-     : tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)               \
-                  : gemm_simt_launch<TX, TW, TO, 4, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s))
+    if (N > 65535 * 64) ABK_REFUSE("gemm: %d output columns are more than one launch takes", N);
+    const bool one = K <= GS_ONE_SUM;
+    const long long large = ((M + 63LL) / 64) * ((N + 63LL) / 64), small = ((M + 15LL) / 16) * ((N + 15LL) / 16), sms = abk_sm_count();
+    // Eight sums: tiles of 64 x 64 where they fill two thirds of the SMs, else of 32 x 32 (of 16 x 16 for up to 16 rows): 64 x
+    // 1024 x 3072, 16 large tiles or 64 of 32 x 32, in 114 or 34 us. One sum: tiles of 16 x 16 while an SM has up to seven of
+    // them, else of 32 x 32: 100 x 2048 x 256 in 8.2 us against 10.8, 200 x 2048 x 256 in 16.1 against 12.6 (of 64 x 64: 56).
+    const int tile = one ? small <= 7 * sms ? 16 : 32 : large >= sms * 2 / 3 ? 64 : M > 16 ? 32 : 16;
+#define GS_LAUNCH(TX, TW, TO, ASYNC)                                                                                   \
+    (one ? tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, 1, 4, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)          \
+                      : gemm_simt_launch<TX, TW, TO, 4, 2, 1, 4, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)          \
+     : tile == 64 ? gemm_simt_launch<TX, TW, TO, 16, 8, GS_WARPS, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)      \
+     : tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, GS_WARPS, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)       \
+                  : gemm_simt_launch<TX, TW, TO, 4, 2, GS_WARPS, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s))
     if (x_dtype == ABK_F32 && w_dtype == ABK_F32 && out_dtype == ABK_F32) {
         const bool aligned = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !(((uintptr_t)x | (uintptr_t)w) & 15);
         return aligned ? GS_LAUNCH(float, float, float, true) : GS_LAUNCH(float, float, float, false);

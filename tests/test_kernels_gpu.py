@@ -146,6 +146,31 @@ def test_gemm_simt_tiles_give_the_same_bits(ops, n, k):
             assert torch.equal(out[:rows], whole[:rows])
 
 
+def us_of(fn, n=10):
+    """Device time of one fn(): the fastest of five runs of n in a row."""
+    fn()
+    best = float("inf")
+    for _ in range(5):
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        for _ in range(n):
+            fn()
+        end.record()
+        torch.cuda.synchronize()
+        best = min(best, start.elapsed_time(end) * 1e3 / n)
+    return best
+
+
+@pytest.mark.parametrize("m, n", [(2048, 6144), (1000, 8192), (500, 6144)])
+def test_gemm_simt_with_one_sum_keeps_the_gpu_busy(ops, m, n):
+    """K = 256 is one sum an element, K = 272 eight: less to multiply may not take longer (a third for luck)."""
+    times = []
+    for k in (256, 272):
+        x, w, out = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda"), torch.empty(m, n, device="cuda")
+        times.append(us_of(lambda: ops.gemm_simt(x, w, out)))
+    assert times[0] < 1.33 * times[1], times
+
+
 @pytest.mark.parametrize("n", [1, 480, 481, 1500])
 def test_set_words(ops, n):
     """Words carried by one launch and by several, in any order; a word outside the table is refused and changes nothing."""
