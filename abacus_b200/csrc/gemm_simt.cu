@@ -33,10 +33,15 @@ __device__ __forceinline__ void gs_copy_16(float *dst, const float *src, bool re
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
+// How a warp brings its pieces. GS_PIECES: float32 operands whose rows start on 16-byte boundaries, K a multiple of 4, by
+// cp.async; GS_VALUES: any others, number by number, the next piece asked for into registers while this one is multiplied.
+// (Loads that the warp waited for one after the other: 500 x 1024 x 1023 float32 in 134 us and 500 x 1024 x 1020 bfloat16 in
+// 144, now 42 and 43; 2048 x 2048 x 130 float32 954, now 45.)
+enum { GS_PIECES, GS_VALUES };
+
 // TM x TN: outputs a lane has, rows 4 apart and columns 8 apart; a tile has 4 TM x 8 TN. WARPS: GS_WARPS sums an element, or 1.
-// STAGES: pieces of a warp in flight or in use. ASYNC: float32 operands whose rows start on 16-byte boundaries, K a multiple
-// of 4.
-template <typename TX, typename TW, typename TO, int TM, int TN, int WARPS, int STAGES, bool ASYNC>
+// STAGES: pieces of a warp in flight or in use.
+template <typename TX, typename TW, typename TO, int TM, int TN, int WARPS, int STAGES, int LOADS>
 __global__ void __launch_bounds__(32 * WARPS) gemm_simt_kernel(const TX *__restrict__ x, const TW *__restrict__ w, TO *__restrict__ out, int M,
                                                                int N, int K, long long ldx, long long ldw, long long ldo) {
     constexpr int BM = 4 * TM, BN = 8 * TN, STAGE = (BM + BN) * GS_PITCH;
@@ -47,50 +52,66 @@ __global__ void __launch_bounds__(32 * WARPS) gemm_simt_kernel(const TX *__restr
     const int r_mine = lane >> 2, c_mine = (lane & 3) * 4;  // a lane's pieces: every 8th row from here
     const TX *x_mine = x + (long long)(m0 + r_mine) * ldx + c_mine;
     const TW *w_mine = w + (long long)(n0 + r_mine) * ldw + c_mine;
+    const int r_single = lane >> 4, c_single = lane & 15;  // a lane's numbers where they come one by one: every 2nd row
     pdl_wait();
     const int pieces = (K + GS_BK - 1) / GS_BK;
     auto fetch = [&](int piece, int stage) {
         if (piece < pieces) {
             float *dst = mine + stage * STAGE;
             const int k0 = piece * GS_BK;
-            if constexpr (ASYNC) {
-                const bool in = k0 + c_mine < K;
+            const bool in = k0 + c_mine < K;
 #pragma unroll
-                for (int i = 0; i < BM / 8; i++) {
-                    const bool real = in && m0 + r_mine + 8 * i < M;
-                    gs_copy_16(dst + (r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)x_mine + 8 * i * ldx + k0 : (const float *)x, real);
-                }
+            for (int i = 0; i < BM / 8; i++) {
+                const bool real = in && m0 + r_mine + 8 * i < M;
+                gs_copy_16(dst + (r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)x_mine + 8 * i * ldx + k0 : (const float *)x, real);
+            }
 #pragma unroll
-                for (int i = 0; i < BN / 8; i++) {
-                    const bool real = in && n0 + r_mine + 8 * i < N;
-                    gs_copy_16(dst + (BM + r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)w_mine + 8 * i * ldw + k0 : (const float *)w, real);
-                }
-            } else {
-                for (int e = lane; e < (BM + BN) * GS_BK; e += 32) {
-                    const int r = e / GS_BK, c = e % GS_BK, k = k0 + c;
-                    float v = 0.0f;
-                    if (r < BM) {
-                        if (m0 + r < M && k < K) v = to_float(x[(long long)(m0 + r) * ldx + k]);
-                    } else if (n0 + r - BM < N && k < K) {
-                        v = to_float(w[(long long)(n0 + r - BM) * ldw + k]);
-                    }
-                    dst[r * GS_PITCH + c] = v;
-                }
+            for (int i = 0; i < BN / 8; i++) {
+                const bool real = in && n0 + r_mine + 8 * i < N;
+                gs_copy_16(dst + (BM + r_mine + 8 * i) * GS_PITCH + c_mine, real ? (const float *)w_mine + 8 * i * ldw + k0 : (const float *)w, real);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");  // (a group each time, empty beyond the last piece)
+    };
+    TX x_next[LOADS == GS_VALUES ? BM / 2 : 1];
+    TW w_next[LOADS == GS_VALUES ? BN / 2 : 1];
+    auto ask = [&](int piece) {
+        const int k = piece * GS_BK + c_single;
+        long long x_step = 2 * ldx, w_step = 2 * ldw;
+        asm volatile("" : "+l"(x_step), "+l"(w_step));  // (or every row's address is kept in registers from piece to piece)
+        const TX *xp = x + (long long)(m0 + r_single) * ldx + k;
+        const TW *wp = w + (long long)(n0 + r_single) * ldw + k;
+#pragma unroll
+        for (int i = 0; i < BM / 2; i++, xp += x_step) x_next[i] = k < K && m0 + r_single + 2 * i < M ? *xp : from_float<TX>(0.0f);
+#pragma unroll
+        for (int i = 0; i < BN / 2; i++, wp += w_step) w_next[i] = k < K && n0 + r_single + 2 * i < N ? *wp : from_float<TW>(0.0f);
+    };
+    auto put = [&](int stage) {
+        float *dst = mine + stage * STAGE + r_single * GS_PITCH + c_single;
+#pragma unroll
+        for (int i = 0; i < BM / 2; i++) dst[2 * i * GS_PITCH] = to_float(x_next[i]);
+#pragma unroll
+        for (int i = 0; i < BN / 2; i++) dst[(BM + 2 * i) * GS_PITCH] = to_float(w_next[i]);
     };
     float acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; i++)
 #pragma unroll
         for (int j = 0; j < TN; j++) acc[i][j] = 0.0f;
+    if constexpr (LOADS == GS_VALUES) {
+        if (warp < pieces) ask(warp), put(0);
+    } else {
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; s++) fetch(warp + s * WARPS, s);
+        for (int s = 0; s < STAGES - 1; s++) fetch(warp + s * WARPS, s);
+    }
     int stage = 0;
     for (int piece = warp; piece < pieces; piece += WARPS) {
-        fetch(piece + (STAGES - 1) * WARPS, stage == 0 ? STAGES - 1 : stage - 1);
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+        if constexpr (LOADS == GS_VALUES) {
+            if (piece + WARPS < pieces) ask(piece + WARPS);
+        } else {
+            fetch(piece + (STAGES - 1) * WARPS, stage == 0 ? STAGES - 1 : stage - 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
+        }
         __syncwarp();
         const float *xs = mine + stage * STAGE + ty * GS_PITCH, *ws = mine + stage * STAGE + (BM + tx) * GS_PITCH;
 #pragma unroll
@@ -104,6 +125,9 @@ __global__ void __launch_bounds__(32 * WARPS) gemm_simt_kernel(const TX *__restr
             for (int i = 0; i < TM; i++)
 #pragma unroll
                 for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, acc[i][j]));
+        }
+        if constexpr (LOADS == GS_VALUES) {
+            if (piece + WARPS < pieces) put(stage == STAGES - 1 ? 0 : stage + 1);
         }
         __syncwarp();  // the next iteration fills this stage again
         stage = stage == STAGES - 1 ? 0 : stage + 1;
@@ -132,16 +156,20 @@ __global__ void __launch_bounds__(32 * WARPS) gemm_simt_kernel(const TX *__restr
     }
 }
 
-template <typename TX, typename TW, typename TO, int TM, int TN, int WARPS, int STAGES, bool ASYNC>
+template <typename TX, typename TW, typename TO, int TM, int TN, int WARPS, int STAGES, int LOADS>
 static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int N, int K, long long ldx, long long ldw, long long ldo, cudaStream_t s) {
     constexpr int BM = 4 * TM, BN = 8 * TN;
-    constexpr int ring = WARPS * STAGES * (BM + BN) * GS_PITCH * 4, sums = WARPS == 1 ? 0 : WARPS * BM * (BN + 8) * 4, smem = ring > sums ? ring : sums;
+    constexpr int ring = WARPS * STAGES * (BM + BN) * GS_PITCH * 4, sums = WARPS == 1 ? 0 : WARPS * BM * (BN + 8) * 4, least = ring > sums ? ring : sums;
     const long long tiles = ((long long)M + BM - 1) / BM * (((long long)N + BN - 1) / BN);
     if (tiles > 0x7fffffffLL) ABK_REFUSE("gemm: %d x %d outputs are more than one launch takes", M, N);
     const dim3 grid((unsigned)tiles);
-    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_simt_kernel<TX, TW, TO, TM, TN, WARPS, STAGES, ASYNC>, smem);
+    // One warp a CTA: those that start while the kernel before still holds parts of the SMs gather where there is room (500 x
+    // 2048 x 256, seven an SM: 25.5 us against 20.2), so each asks for so much shared memory that no SM takes more than its share.
+    const long long share = (tiles + abk_sm_count() - 1) / abk_sm_count();
+    const int even = WARPS == 1 && share <= 10 ? 228 * 1024 / (int)(share + 1) : 0, smem = even > least ? even : least;
+    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_simt_kernel<TX, TW, TO, TM, TN, WARPS, STAGES, LOADS>, smem);
     if (e != cudaSuccess) return (int)e;
-    abk_launch(gemm_simt_kernel<TX, TW, TO, TM, TN, WARPS, STAGES, ASYNC>, grid, dim3(32 * WARPS), smem, s, (const TX *)x, (const TW *)w, (TO *)out, M, N, K,
+    abk_launch(gemm_simt_kernel<TX, TW, TO, TM, TN, WARPS, STAGES, LOADS>, grid, dim3(32 * WARPS), smem, s, (const TX *)x, (const TW *)w, (TO *)out, M, N, K,
                ldx, ldw, ldo);
     return ABK_LAUNCH_RESULT();
 }
@@ -160,18 +188,19 @@ extern "C" int abk_gemm_simt(const void *x, int x_dtype, const void *w, int w_dt
     // 1024 x 3072, 16 large tiles or 64 of 32 x 32, in 114 or 34 us. One sum: tiles of 16 x 16 while an SM has up to seven of
     // them, else of 32 x 32: 100 x 2048 x 256 in 8.2 us against 10.8, 200 x 2048 x 256 in 16.1 against 12.6 (of 64 x 64: 56).
     const int tile = one ? small <= 7 * sms ? 16 : 32 : large >= sms * 2 / 3 ? 64 : M > 16 ? 32 : 16;
-#define GS_LAUNCH(TX, TW, TO, ASYNC)                                                                                   \
-    (one ? tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, 1, 4, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)          \
-                      : gemm_simt_launch<TX, TW, TO, 4, 2, 1, 4, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)          \
-     : tile == 64 ? gemm_simt_launch<TX, TW, TO, 16, 8, GS_WARPS, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)      \
-     : tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, GS_WARPS, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s)       \
-                  : gemm_simt_launch<TX, TW, TO, 4, 2, GS_WARPS, 2, ASYNC>(x, w, out, M, N, K, ldx, ldw, ldo, s))
+#define GS_LAUNCH(TX, TW, TO, LARGE, STAGES, LOADS)                                                                    \
+    (one ? tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, 1, STAGES, LOADS>(x, w, out, M, N, K, ldx, ldw, ldo, s)     \
+                      : gemm_simt_launch<TX, TW, TO, 4, 2, 1, STAGES, LOADS>(x, w, out, M, N, K, ldx, ldw, ldo, s)     \
+     : tile == 64 ? gemm_simt_launch<TX, TW, TO, LARGE, 8, GS_WARPS, 2, LOADS>(x, w, out, M, N, K, ldx, ldw, ldo, s)   \
+     : tile == 32 ? gemm_simt_launch<TX, TW, TO, 8, 4, GS_WARPS, 2, LOADS>(x, w, out, M, N, K, ldx, ldw, ldo, s)       \
+                  : gemm_simt_launch<TX, TW, TO, 4, 2, GS_WARPS, 2, LOADS>(x, w, out, M, N, K, ldx, ldw, ldo, s))
+    // (large tiles of 32 x 64 where the next piece needs room in the registers)
     if (x_dtype == ABK_F32 && w_dtype == ABK_F32 && out_dtype == ABK_F32) {
         const bool aligned = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && !(((uintptr_t)x | (uintptr_t)w) & 15);
-        return aligned ? GS_LAUNCH(float, float, float, true) : GS_LAUNCH(float, float, float, false);
+        return aligned ? GS_LAUNCH(float, float, float, 16, 4, GS_PIECES) : GS_LAUNCH(float, float, float, 8, 2, GS_VALUES);
     }
-    if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_BF16) return GS_LAUNCH(bf, bf, bf, false);
-    if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_F32) return GS_LAUNCH(bf, bf, float, false);
+    if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_BF16) return GS_LAUNCH(bf, bf, bf, 8, 2, GS_VALUES);
+    if (x_dtype == ABK_BF16 && w_dtype == ABK_BF16 && out_dtype == ABK_F32) return GS_LAUNCH(bf, bf, float, 8, 2, GS_VALUES);
 #undef GS_LAUNCH
     ABK_REFUSE("gemm: dtype combination x=%d w=%d out=%d is not built", x_dtype, w_dtype, out_dtype);
 }

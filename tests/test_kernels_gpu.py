@@ -171,6 +171,17 @@ def test_gemm_simt_with_one_sum_keeps_the_gpu_busy(ops, m, n):
     assert times[0] < 1.33 * times[1], times
 
 
+@pytest.mark.parametrize("dtype, m, n, k", [(torch.float32, 2048, 2048, 130), (torch.float32, 500, 1024, 1023), (torch.bfloat16, 500, 2048, 250),
+                                            (torch.bfloat16, 2048, 1024, 1020)])
+def test_gemm_simt_of_rows_that_start_anywhere(ops, dtype, m, n, k):
+    """Operands whose rows start on no 16-byte boundary, number by number: at most twice what aligned float32 ones take."""
+    times = []
+    for t, size in ((dtype, k), (torch.float32, -(-k // 4) * 4)):
+        x, w, out = torch.randn(m, size, device="cuda").to(t), torch.randn(n, size, device="cuda").to(t), torch.empty(m, n, device="cuda")
+        times.append(us_of(lambda: ops.gemm_simt(x, w, out)))
+    assert times[0] < 2 * times[1], times
+
+
 @pytest.mark.parametrize("n", [1, 480, 481, 1500])
 def test_set_words(ops, n):
     """Words carried by one launch and by several, in any order; a word outside the table is refused and changes nothing."""
