@@ -236,3 +236,31 @@ def test_which_steps_are_captured():
     assert (g.rows, g.position_bound) == (8, 1024) and d.get(decode) is g
     far = [Sequence(0, [5], 1024, [0])]
     assert d.get(far).position_bound == 2048 and d.get(far).rows == 1
+
+
+@pytest.mark.parametrize("options", [{}, dict(sink=True), dict(window=64), dict(window=64, keep_first=2), dict(exact_weights=True), dict(chunk=32),
+                                     dict(softcap=30.0), dict(v_head_dim=32), dict(conv_taps=4), dict(head_gate=True), dict(values="keys"),
+                                     dict(bias=True), dict(diff=0.2, exact_weights=True), dict(weights="sigmoid", exact_weights=True)])
+def test_the_c_step_serves_plain_attention_only(options):
+    """A layer with an option that the walker's structures do not carry is left to the parts, whatever the option."""
+    from types import SimpleNamespace as NS
+
+    import torch
+
+    from abacus_b200.config.specs import AttentionSpec, GatedMLPSpec
+    from abacus_b200.engine.cstep import CStep
+    from abacus_b200.parts.attention import Attention
+    from abacus_b200.parts.block import PreNormBlock
+    from abacus_b200.parts.frame import PlainFrame
+    from abacus_b200.parts.mlp import GatedMLP
+    from abacus_b200.parts.norm import RMSNorm
+
+    def part(cls, **fields):
+        made = cls.__new__(cls)
+        made.__dict__.update(fields)
+        return made
+
+    spec = AttentionSpec(hidden=128, n_heads=4, n_kv_heads=2, head_dim=64, scale=0.125, qk_norm_eps=None, position=None, **options)
+    block = part(PreNormBlock, mixer=Attention(spec), ffn=part(GatedMLP, spec=GatedMLPSpec(128, 256)), mixer_norm=part(RMSNorm), ffn_norm=part(RMSNorm))
+    model = NS(frame=part(PlainFrame, final_norm=part(RMSNorm)), blocks=[block], ctx=NS(dtype=torch.bfloat16, device=torch.device("cuda")))
+    assert CStep.serves(model) == (options in ({}, dict(window=64)))
