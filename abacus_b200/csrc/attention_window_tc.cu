@@ -21,8 +21,8 @@
 // Tensor memory: two groups of 128 columns of output and of 96 columns of scores and weights, 512 in all, so a CTA to an SM.
 // A value row beyond the sequence's end belongs to another sequence or to nothing, and a weight of zero times what is no
 // number is none: the rows are set to zero in shared memory before the tile that crosses the end is multiplied.
-// The reference of a row's exponentials follows its maximum only when that has outgrown it by 2^8, and is a whole power of
-// two, so that O is rescaled (in tensor memory, exactly) on a few early steps only; the sink joins at the end.
+// The reference of a row's exponentials follows the row's maximum only when that has outgrown it by 2^8, and is a whole power
+// of two, so that O is rescaled (in tensor memory, exactly) on a few early steps only; the sink joins at the end.
 // Every wait on an mbarrier is bounded; one that runs out sets status word 3 and the CTA winds down.
 #define ABK_DEFINE_ERROR
 #include "common.cuh"
@@ -276,9 +276,11 @@ __global__ void __launch_bounds__(WT_THREADS, 1) attention_window_tc_kernel(cons
 #pragma unroll
             for (int c = 0; c < WT_K; c += 4) top0 = fmaxf(top0, s[c]), top1 = fmaxf(top1, s[c + 1]), top2 = fmaxf(top2, s[c + 2]), top3 = fmaxf(top3, s[c + 3]);
             const float cand = fmaxf(m, ceilf(fmaxf(fmaxf(top0, top1), fmaxf(top2, top3)) * p.scale_log2));
-            const bool move = __any_sync(0xffffffffu, cand > m + 8.0f);  // (the first tile: m is -inf)
-            const float m_new = move ? cand : m, ref = m_new == -INFINITY ? 0.0f : m_new;
-            const float corr = exp2f(m - ref);  // (0 when m is still -inf)
+            // Each row for itself (the first tile: m is -inf), so that a row's bits know nothing of the rows beside it; the
+            // vote only says whether any row of the warp has outputs to rescale (those of the others by one).
+            const float m_new = cand > m + 8.0f ? cand : m, ref = m_new == -INFINITY ? 0.0f : m_new;
+            const bool move = __any_sync(0xffffffffu, m_new != m);
+            const float corr = m_new != m ? exp2f(m - ref) : 1.0f;  // (0 when m was -inf)
             m = m_new;
             float sum0 = 0.0f, sum1 = 0.0f;
 #pragma unroll

@@ -368,6 +368,26 @@ def test_prompts_on_two_groups_of_rows_a_cta(H, G, D, V, window, keep, chunk, le
     assert not ops.kernel_status(torch.device(DEV, torch.cuda.current_device())).any()
 
 
+@pytest.mark.parametrize("H,G,D,V,window,keep", [(12, 1, 64, 64, None, 0), (8, 2, 128, 128, 100, 5), (6, 3, 192, 128, None, 0)])
+def test_a_rows_bits_know_nothing_of_the_rows_beside_it(H, G, D, V, window, keep):
+    """Loud queries in later rows of the prompt and in the prompt behind it, which a warp has beside the row: the same bits."""
+    from abacus_b200.kernels import ops
+    rng, T, after = np.random.default_rng(D), 330, 40
+    row = (H + G) * D + G * V
+    quiet = plain.bf16_round(rng.standard_normal((T + after, row)).astype(np.float32))
+    b = batch_of([(0, [0] * T, 0), (1, [0] * after, 0)])
+    got = []
+    for loud_from in (None, T, 300, 70):
+        rows = quiet.copy()
+        if loud_from is not None:
+            rows[loud_from:, :H * D] *= 64.0
+        out = torch.empty((T + after, H * V), dtype=torch.bfloat16, device=DEV)
+        ops.attention_window(dev(rows, torch.bfloat16), out, H, G, D, D ** -0.5, window, b, v_dim=V, keep_first=keep)
+        got.append((loud_from or T, out))
+    for first, out in got[1:]:
+        assert torch.equal(out[:first], got[0][1][:first]), first
+
+
 @pytest.mark.parametrize("H,G,D,V,window,keep,dtype", [(8, 1, 32, 200, None, 0, torch.bfloat16), (6, 2, 24, 40, 300, 9, torch.float32),
                                                         (16, 1, 64, 8, 130, 128, torch.bfloat16), (3, 3, 256, 130, 128, 0, torch.bfloat16)])
 def test_decoding_in_parts_in_an_unequal_batch(H, G, D, V, window, keep, dtype):
