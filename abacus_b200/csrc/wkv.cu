@@ -656,12 +656,14 @@ extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at,
     p.n_seqs = n_seqs, p.tiles = 1, p.longest_first = 0, p.vec = 0;
     cudaStream_t s = (cudaStream_t)stream;
     if (blocks) {
-        // Columns a lane has. Heads of 64, a CTA then has 16, 32 or 64 of them: the makers' work is every CTA's own, so few
-        // CTAs a head are better until an SM would have two of them while others have one (3 prompts, 3,571 tokens, 40
-        // heads: 630, 679, 604 us a layer with 1, 2, 4; 8 prompts, 5,000 tokens: 885, 748, 803; one of 2,048 and 16
-        // heads: 336, 334, 352).
-        const long long columns = (long long)n_seqs * n_heads * dim, sms = abk_sm_count();
-        const int lane_columns = columns <= 32 * sms ? 1 : columns <= 64 * sms ? 4 : 2;
+        // Columns a lane has: as few as leave an SM one CTA, else as many as a head uses. The makers' work is every CTA's own,
+        // and an SM's CTAs share its issue slots. One prompt of 500, us a walk with 1, 2, 4: 40 heads of 64 65, 54, 61 (160,
+        // 80, 40 CTAs), 16 heads of 64 44, 54, 61, 32 heads of 128 261, 162, 87, 16 of 256 484, 254, 142, 80 of 32 46, 37, 53;
+        // 500, 1,023 and 2,048 tokens, 40 heads of 64: 253, 271, 241; 8 prompts of 500: 312, 206, 152.
+        const int each = dim <= 64 ? 16 : 8;  // columns a CTA has where a lane has one
+        const long long heads = (long long)n_seqs * n_heads, sms = abk_sm_count();
+        int lane_columns = 1;
+        while (lane_columns < 4 && lane_columns * each < dim && heads * ((dim + lane_columns * each - 1) / (lane_columns * each)) > sms) lane_columns *= 2;
 #define WB_LAUNCH_AS(T, P, J)                                     \
     (lane_columns == 1   ? wkv_block_launch<T, P, J, 1>(p, s)     \
      : lane_columns == 2 ? wkv_block_launch<T, P, J, 2>(p, s)     \

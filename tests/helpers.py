@@ -156,3 +156,19 @@ def assert_logits(got, want, dtype, what="", noise=0.0):
         lp, lq = log_softmax64(want), log_softmax64(got)
         kl = (np.exp(lp) * (lp - lq)).sum(-1)
         assert kl.max() <= BF16_KL, f"{what}: KL {kl.max():.3g} at row {kl.argmax()} (limit {BF16_KL})"
+
+
+def us_of(fn, n=10):
+    """Device time of one fn(): the fastest of five runs of n in a row."""
+    import torch
+    fn()
+    best = float("inf")
+    for _ in range(5):
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        for _ in range(n):
+            fn()
+        end.record()
+        torch.cuda.synchronize()
+        best = min(best, start.elapsed_time(end) * 1e3 / n)
+    return best

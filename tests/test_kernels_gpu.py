@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+from helpers import us_of
 from plain import qwen3_plain as plain
 
 pytestmark = pytest.mark.gpu
@@ -144,21 +145,6 @@ def test_gemm_simt_tiles_give_the_same_bits(ops, n, k):
         for a, b in ((x, w), shifted):
             ops.gemm_simt(a[:rows], b, out, rows)
             assert torch.equal(out[:rows], whole[:rows])
-
-
-def us_of(fn, n=10):
-    """Device time of one fn(): the fastest of five runs of n in a row."""
-    fn()
-    best = float("inf")
-    for _ in range(5):
-        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
-        start.record()
-        for _ in range(n):
-            fn()
-        end.record()
-        torch.cuda.synchronize()
-        best = min(best, start.elapsed_time(end) * 1e3 / n)
-    return best
 
 
 @pytest.mark.parametrize("m, n", [(2048, 6144), (1000, 8192), (500, 6144)])

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import tilulorn_models as tm
-from helpers import TraceRun, assert_logits
+from helpers import TraceRun, assert_logits, us_of
 from part_run import DEV, PartRun, close as _close, every_way as _every_way, f64 as _f64, rounding as _rnd
 from plain import tilulorn_plain as plain
 
@@ -48,7 +48,8 @@ def test_wkv_every_way(dtype, H, K, rank):
 
 
 @pytest.mark.parametrize("H,K,lens", [(100, 48, (9,)), (80, 30, (5, 3, 4)), (40, 128, (6,)), (30, 256, (5,)), (60, 64, (7, 1, 6)),
-                                      (170, 20, (4, 6, 1)), (80, 128, (5,)), (48, 256, (3,)), (3, 90, (2, 9)), (2, 64, (5, 130))])
+                                      (170, 20, (4, 6, 1)), (80, 128, (5,)), (48, 256, (3,)), (3, 90, (2, 9)), (2, 64, (5, 130)),
+                                      (14, 64, (9, 4, 2)), (12, 128, (7,)), (6, 256, (13,)), (2, 256, (9,)), (4, 32, (6, 3)), (5, 8, (10,))])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_wkv_in_blocks(H, K, lens, shift):
     """Blocks of four tokens and their remainders for every split of the work (few and many columns, every padded head size),
@@ -78,6 +79,20 @@ def test_wkv_in_blocks(H, K, lens, shift):
     # sums of K products of values of around one, the decays by the special-function unit: some 2^-21 of the sums' size
     limit = 2.0 ** -20 * K ** 0.5 * 8 * max(1.0, float(S.abs().max()))
     assert float((out.double() - want).abs().max()) <= limit and float((state.double() - S).abs().max()) <= limit
+
+
+@pytest.mark.parametrize("H,K,lens", [(32, 128, (500,)), (16, 256, (500,)), (40, 64, (500,)), (64, 64, (60,) * 64)])
+def test_wkv_in_blocks_takes_no_longer_than_token_by_token(H, K, lens):
+    from abacus_b200.engine.batch import Sequence, StepBatch
+    from abacus_b200.kernels import ops
+    n, size = sum(lens), H * K
+    proj, pre = torch.randn((n, 3 * size), device=DEV).to(torch.bfloat16), torch.randn((n, size), device=DEV)
+    w0, bonus = torch.randn(size, device=DEV) - 2, torch.randn(size, device=DEV)
+    state, out = torch.zeros((len(lens), H, K, K), device=DEV), torch.empty((n, size), device=DEV)
+    batch, times = StepBatch(n, len(lens), 1, DEV).fill([Sequence(i, [0] * m, 0, []) for i, m in enumerate(lens)], exact=True), []
+    for batch.is_decode in (False, True):  # (a decode step's kernel walks any number of tokens)
+        times.append(us_of(lambda: ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch)))
+    assert times[0] <= times[1], times
 
 
 def test_wkv_keeps_a_token_over_a_long_decoding_and_forgets_with_decays_near_nothing():
