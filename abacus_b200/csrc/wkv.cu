@@ -8,12 +8,14 @@
 //                     plane of the output per s. In a step of one token a sequence it also leaves the new last row.
 //   token_shift_keep  the last row of every sequence of a step of prompts, into its slot.
 //   wkv_block         prompts: blocks of four tokens (below)
-//   wkv_scan          a step of one token a sequence: a CTA walks one sequence's tokens for one head and 16 (32 for heads of up to 32 channels) value
-//                     columns. Its threads are those columns x 4, 8 or 16 parts of the key channels, so a thread keeps 4
-//                     to 16 state values in registers; the parts' partial outputs of a column meet by shuffles, four
-//                     tokens at a time. Rows come 16 (8 for heads beyond 128 channels) tokens at a time: asked for a
-//                     chunk ahead into registers, the decay made from its pre-activation on the way into shared memory,
-//                     read from there as 16-byte pieces. A sequence that brings no token to the step is left alone.
+//   wkv_scan          a step of one token or a few a sequence, and prompts of heads too few to fill the GPU, in segments
+//                     walked side by side: a CTA walks one sequence's (a segment's) tokens for one head and 16 (32 for heads
+//                     of up to 32 channels) value columns. Its threads are those columns x 4, 8 or 16 parts of the key
+//                     channels, so a thread keeps 4 to 16 state values in registers; the parts' partial outputs of a
+//                     column meet by shuffles, four tokens at a time. Rows come 16 (8 for heads beyond 128 channels) tokens
+//                     at a time: asked for a chunk ahead into registers, the decay made from its pre-activation on the way
+//                     into shared memory, read from there as 16-byte pieces. A sequence that brings no token to the step
+//                     is left alone.
 #define ABK_DEFINE_ERROR
 #include "recurrence.cuh"
 
@@ -182,13 +184,53 @@ struct WkvScan {
     float *out;          // [tokens][heads * dim]
     const int *seq_start, *seq_slot;
     int n_seqs, tiles, longest_first, vec;  // of the walk in blocks
+    // Prompts in segments of `chunk` tokens, all at once (blockIdx.z counts the step's segments, sequence after sequence):
+    // phase 1 walks each segment from an empty state and leaves its sum and the product of its decays,
+    // wkv_segment_prefix turns the sums into the states at the segments' starts (and leaves the last in the slot), phase 2
+    // walks each segment again from its start state for the outputs. chunk 0 (phase 0): a CTA walks a whole sequence.
+    int chunk, phase;
+    float *sums;         // [segments][heads][dim][dim]
+    float *prods;        // [segments][heads][dim]
 };
+
+// The segment blockIdx.z names: its sequence, its first row and its rows (0: none). Sequences are walked in order.
+__device__ __forceinline__ void wkv_segment(const int *seq_start, int n_seqs, int chunk, int z, int &seq, int &row0, int &n) {
+    n = 0;
+    int first = 0;
+    for (seq = 0; seq < n_seqs; seq++) {
+        const int start = seq_start[seq], len = seq_start[seq + 1] - start, count = (len + chunk - 1) / chunk;
+        if (z < first + count) {
+            const int c = z - first;
+            row0 = start + c * chunk, n = len - c * chunk < chunk ? len - c * chunk : chunk;
+            return;
+        }
+        first += count;
+    }
+}
 
 // N tokens of one thread's share: r, k, w point at the thread's channels of the first token (tokens `pitch` floats
 // apart), v at its column's value (tokens `v_pitch` apart); the column's output goes to out if `writes`.
-template <int DPT, int PARTS, int N>
+// SUMS: the state alone moves (a segment's own sum): no r, no output.
+template <int DPT, int PARTS, int N, bool SUMS>
 __device__ __forceinline__ void wkv_tokens(float *s, const float *u, const float *r, const float *k, const float *w, int pitch,
                                            const float *v, int v_pitch, bool writes, float *out, long long out_pitch) {
+    if constexpr (SUMS) {
+        float vv[N];
+#pragma unroll
+        for (int n = 0; n < N; n++) vv[n] = v[n * v_pitch];
+#pragma unroll
+        for (int i = 0; i < DPT / 4; i++) {
+            float4 kk[N], ww[N];
+#pragma unroll
+            for (int n = 0; n < N; n++) kk[n] = *(const float4 *)(k + n * pitch + 4 * i), ww[n] = *(const float4 *)(w + n * pitch + 4 * i);
+#pragma unroll
+            for (int n = 0; n < N; n++) {
+                s[4 * i] = fmaf(ww[n].x, s[4 * i], kk[n].x * vv[n]), s[4 * i + 1] = fmaf(ww[n].y, s[4 * i + 1], kk[n].y * vv[n]);
+                s[4 * i + 2] = fmaf(ww[n].z, s[4 * i + 2], kk[n].z * vv[n]), s[4 * i + 3] = fmaf(ww[n].w, s[4 * i + 3], kk[n].w * vv[n]);
+            }
+        }
+        return;
+    }
     float vv[N], o[N];
 #pragma unroll
     for (int n = 0; n < N; n++) vv[n] = v[n * v_pitch], o[n] = 0.0f;
@@ -227,7 +269,7 @@ __device__ __forceinline__ void wkv_tokens(float *s, const float *u, const float
 template <typename T> __device__ __forceinline__ float wkv_decay(float z) { return expf(-expf(z)); }
 template <> __device__ __forceinline__ float wkv_decay<__nv_bfloat16>(float z) { return __expf(-__expf(z)); }
 
-template <typename T, int DPT, int PARTS, int COLS, int TOK>
+template <typename T, int DPT, int PARTS, int COLS, int TOK, bool SUMS>
 __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
     constexpr int DP = DPT * PARTS;             // key channels, padded
     constexpr int PITCH = PARTS * (DPT + 4);    // a token's channels in shared memory: a part's run, then 4 floats of
@@ -245,14 +287,17 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
         u[i] = d < p.dim ? p.bonus[(long long)h * p.dim + d] : 0.0f;
     }
     pdl_wait();
-    const int seq = blockIdx.z, row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
+    int seq = blockIdx.z, row0, n;
+    if (p.chunk > 0) wkv_segment(p.seq_start, p.n_seqs, p.chunk, blockIdx.z, seq, row0, n);
+    else row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
     if (n <= 0) return;  // (a sequence of the step's padding: its slot is someone else's)
-    float *state = p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * p.dim * p.dim;
+    float *state = p.phase == 0 ? p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * p.dim * p.dim
+                                : p.sums + ((long long)blockIdx.z * p.n_heads + h) * p.dim * p.dim;
     float s[DPT];
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
         const int d = part * DPT + i;
-        s[i] = d < p.dim && col < p.dim ? state[(long long)d * p.dim + col] : 0.0f;
+        s[i] = p.phase != 1 && d < p.dim && col < p.dim ? state[(long long)d * p.dim + col] : 0.0f;
     }
     const T *proj = (const T *)p.proj;
     const long long hk = (long long)p.n_heads * p.dim;
@@ -264,6 +309,7 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
     float rz[PER];
     const int my_d = tid % DP, my_ch = h * p.dim + (my_d < p.dim ? my_d : 0);
     const float my_w0 = p.w0[my_ch];
+    float decayed = 1.0f;  // phase 1: the product of this thread's staged decays (one channel, its share of the tokens)
     auto fetch = [&](int c0) {
         const int cnt = n - c0 < TOK ? n - c0 : TOK;
 #pragma unroll
@@ -274,7 +320,8 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
             const int tok = (tid + it * THREADS) / DP;
             const long long row = row0 + c0 + (tok < cnt ? tok : cnt - 1);
             const T *r = proj + row * p.ld + my_ch;
-            rr[it] = r[p.r_at], rk[it] = r[p.k_at], rz[it] = p.pre[row * hk + my_ch];
+            if (!SUMS) rr[it] = r[p.r_at];
+            rk[it] = r[p.k_at], rz[it] = p.pre[row * hk + my_ch];
         }
 #pragma unroll
         for (int it = 0; it < PER_V; it++) {
@@ -293,7 +340,8 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
             const int tok = (tid + it * THREADS) / DP, at = (my_d / DPT) * (DPT + 4) + my_d % DPT;
             const bool in = tok < cnt && my_d < p.dim;
             const float w = wkv_decay<T>(rz[it] + my_w0);
-            r_s[tok][at] = in ? to_float(rr[it]) : 0.0f;
+            if (!SUMS) r_s[tok][at] = in ? to_float(rr[it]) : 0.0f;
+            if (in) decayed *= w;
             k_s[tok][at] = in ? to_float(rk[it]) : 0.0f, w_s[tok][at] = w;
         }
 #pragma unroll
@@ -307,18 +355,62 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
         // multiply-adds follow one another
         const int at = part * (DPT + 4);
         float *out = p.out + (long long)(row0 + c0) * hk + (long long)h * p.dim + col;
-        const bool writes = part == 0 && col < p.dim;
+        const bool writes = part == 0 && col < p.dim && p.phase != 1;
         int tok = 0;
         for (; tok + 4 <= cnt; tok += 4)
-            wkv_tokens<DPT, PARTS, 4>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
+            wkv_tokens<DPT, PARTS, 4, SUMS>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
         for (; tok < cnt; tok++)
-            wkv_tokens<DPT, PARTS, 1>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
+            wkv_tokens<DPT, PARTS, 1, SUMS>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
     }
+    if (p.phase == 2) return;  // (the states between segments are wkv_segment_prefix's)
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
         const int d = part * DPT + i;
         if (d < p.dim && col < p.dim) state[(long long)d * p.dim + col] = s[i];
     }
+    if (p.phase == 1 && tile == 0) {
+        // every thread staged the decays of one channel: the shares of a channel meet through shared memory
+        __syncthreads();
+        float *share = &r_s[0][0];
+        share[tid] = decayed;
+        __syncthreads();
+        if (tid < DP && tid < p.dim) {
+            float all = 1.0f;
+            for (int o = tid; o < THREADS; o += DP) all *= share[o];
+            p.prods[((long long)blockIdx.z * p.n_heads + h) * p.dim + tid] = all;
+        }
+    }
+}
+
+// The states at the segments' starts from the segments' own sums: along a sequence S <- prod * S + sum, the state before
+// each segment left where its sum was, the last in the sequence's slot. A thread an element of the state; four segments'
+// loads are on their way together.
+__global__ void __launch_bounds__(256) wkv_segment_prefix_kernel(float *sums, const float *prods, float *state, const int *seq_start,
+                                                                 const int *seq_slot, int n_heads, int dim, int chunk) {
+    const int e = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, seq = blockIdx.z;
+    pdl_wait();
+    const int len = seq_start[seq + 1] - seq_start[seq];
+    if (len <= 0 || e >= dim * dim) return;
+    int first = 0;
+    for (int q = 0; q < seq; q++) first += (seq_start[q + 1] - seq_start[q] + chunk - 1) / chunk;
+    const int count = (len + chunk - 1) / chunk, d = e / dim;
+    float *slot = state + ((long long)seq_slot[seq] * n_heads + h) * dim * dim + e;
+    float S = *slot;
+    for (int c0 = 0; c0 < count; c0 += 4) {
+        float u[4], pr[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const long long at = (long long)(first + (c0 + i < count ? c0 + i : count - 1)) * n_heads + h;
+            u[i] = sums[at * dim * dim + e], pr[i] = prods[at * dim + d];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (c0 + i >= count) break;
+            sums[((long long)(first + c0 + i) * n_heads + h) * dim * dim + e] = S;
+            S = fmaf(pr[i], S, u[i]);
+        }
+    }
+    *slot = S;
 }
 
 // ---------------------------------------------------------------- the recurrence, prompts: in blocks of four tokens
@@ -643,17 +735,21 @@ template <typename T, int P, int J, int C> static int wkv_block_launch(WkvScan p
     return ABK_LAUNCH_RESULT();
 }
 
-// blocks: the step brings prompts, walked in blocks of four tokens; else (a token a sequence) each sequence token by token.
+// blocks: the step's sequences are walked in blocks of four tokens; chunk > 0: in segments of so many tokens (`segments` of
+// them at most, with room for their sums and products); else token by token.
 extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at, int k_at, int v_at, int n_heads, int dim,
                             const float *pre, const float *w0, const float *bonus, float *state, float *out,
-                            const int *seq_start, const int *seq_slot, int n_seqs, int blocks, void *stream) {
+                            const int *seq_start, const int *seq_slot, int n_seqs, int blocks, int chunk, int segments, float *sums,
+                            float *prods, void *stream) {
     if (n_seqs <= 0) return 0;
     if (dim < 1 || dim > 256) ABK_REFUSE("wkv_scan: %d key channels a head are not 1 to 256", dim);
     if (n_heads < 1 || n_heads > 65535 || n_seqs > 65535) ABK_REFUSE("wkv_scan: %d heads, %d sequences", n_heads, n_seqs);
     WkvScan p;
     p.proj = proj, p.ld = ld, p.r_at = r_at, p.k_at = k_at, p.v_at = v_at, p.n_heads = n_heads, p.dim = dim;
     p.pre = pre, p.w0 = w0, p.bonus = bonus, p.state = state, p.out = out, p.seq_start = seq_start, p.seq_slot = seq_slot;
-    p.n_seqs = n_seqs, p.tiles = 1, p.longest_first = 0, p.vec = 0;
+    p.n_seqs = n_seqs, p.tiles = 1, p.longest_first = 0, p.vec = 0, p.chunk = blocks ? 0 : chunk, p.phase = 0, p.sums = sums, p.prods = prods;
+    if (chunk < 0 || (chunk > 0 && (segments < 1 || segments > 65535 || !sums || !prods)))
+        ABK_REFUSE("wkv_scan: %d segments of %d tokens", segments, chunk);
     cudaStream_t s = (cudaStream_t)stream;
     if (blocks) {
         // Columns a lane has: as few as leave an SM one CTA, else as many as a head uses. The makers' work is every CTA's own,
@@ -678,17 +774,29 @@ extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at,
 #undef WB_LAUNCH_AS
     }
     const int cols = dim <= 32 ? 32 : 16;  // value columns a CTA has
-    dim3 grid((dim + cols - 1) / cols, n_heads, n_seqs);
-#define WS_LAUNCH(T)                                                                                  \
-    do {                                                                                              \
-        if (dim <= 16) abk_launch(wkv_scan_kernel<T, 4, 4, 32, 16>, grid, dim3(128), 0, s, p);        \
-        else if (dim <= 32) abk_launch(wkv_scan_kernel<T, 8, 4, 32, 16>, grid, dim3(128), 0, s, p);   \
-        else if (dim <= 64) abk_launch(wkv_scan_kernel<T, 8, 8, 16, 16>, grid, dim3(128), 0, s, p);   \
-        else if (dim <= 128) abk_launch(wkv_scan_kernel<T, 8, 16, 16, 16>, grid, dim3(256), 0, s, p); \
-        else abk_launch(wkv_scan_kernel<T, 16, 16, 16, 8>, grid, dim3(256), 0, s, p);                 \
+    dim3 grid((dim + cols - 1) / cols, n_heads, chunk > 0 ? segments : n_seqs);
+#define WS_LAUNCH(T, SUMS)                                                                                  \
+    do {                                                                                                    \
+        if (dim <= 16) abk_launch(wkv_scan_kernel<T, 4, 4, 32, 16, SUMS>, grid, dim3(128), 0, s, p);        \
+        else if (dim <= 32) abk_launch(wkv_scan_kernel<T, 8, 4, 32, 16, SUMS>, grid, dim3(128), 0, s, p);   \
+        else if (dim <= 64) abk_launch(wkv_scan_kernel<T, 8, 8, 16, 16, SUMS>, grid, dim3(128), 0, s, p);   \
+        else if (dim <= 128) abk_launch(wkv_scan_kernel<T, 8, 16, 16, 16, SUMS>, grid, dim3(256), 0, s, p); \
+        else abk_launch(wkv_scan_kernel<T, 16, 16, 16, 8, SUMS>, grid, dim3(256), 0, s, p);                 \
     } while (0)
-    if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16);
-    else WS_LAUNCH(float);
+    if (chunk > 0) {  // the segments' sums, the states between them, the segments' outputs
+        p.phase = 1;
+        if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16, true);
+        else WS_LAUNCH(float, true);
+        int rc = ABK_LAUNCH_RESULT();
+        if (rc) return rc;
+        abk_launch(wkv_segment_prefix_kernel, dim3((dim * dim + 255) / 256, n_heads, n_seqs), dim3(256), 0, s, sums, prods, state,
+                   seq_start, seq_slot, n_heads, dim, chunk);
+        rc = ABK_LAUNCH_RESULT();
+        if (rc) return rc;
+        p.phase = 2;
+    }
+    if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16, false);
+    else WS_LAUNCH(float, false);
 #undef WS_LAUNCH
     return ABK_LAUNCH_RESULT();
 }

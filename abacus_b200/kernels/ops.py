@@ -1579,14 +1579,33 @@ def tanh_rows(src, dst, n):
 
 
 
+WKV_SEGMENT = 64  # tokens of a segment of the form for few heads
 
-def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, batch, ws=None):
+
+def wkv_form(rows, n_seqs, n_heads, dim):
+    """How a step of prompts is walked: "tokens", "blocks" of four or "segments" side by side. Up to eight tokens a sequence go
+    token by token where a step is small or its heads are (64 prompts of 8, 40 heads of 32: 20 us, in blocks 42; 16 tokens of 40
+    heads of 64: 6.7 and 5.9). Blocks are one chain along a prompt, a number of us a token; segments twice the work and two
+    kernels more, but all at once, and win where heads are few: one prompt of 2,000 tokens, us in blocks and in segments: 16 heads
+    of 30 124 and 50, 40 of 32 122 and 101, 80 of 32 149 and 189, 8 of 100 278 and 242, 16 of 64 164 and 160, 40 of 64 211 and
+    396. (Of several prompts the longest is taken for half as long again as they are on average.)"""
+    if rows <= 8 * n_seqs and (rows < 128 or dim <= 32):
+        return "tokens"
+    padded = next(p for p in (32, 64, 128, 256) if dim <= p)
+    segments_us = 15.0 + 3.5e-5 * n_heads * dim * (padded / 32) * rows
+    blocks_us = {32: 0.0625, 64: 0.082, 128: 0.13, 256: 0.25}[padded] * rows / n_seqs * (1.5 if n_seqs > 1 else 1.0)
+    few = -(-rows // WKV_SEGMENT) + n_seqs <= 65535
+    return "segments" if rows >= 128 and few and segments_us < 0.95 * blocks_us else "blocks"
+
+
+def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, batch, ws=None, form=None):
     """The recurrence of a wkv layer for every sequence of the step and every head, float32:
         o = (S + diag(bonus) k v^T)^T r;    S <- diag(exp(-exp(pre + w0))) S + k v^T
     proj [tokens, .] as stored: r, k, v of head h at columns r_at / k_at / v_at + h * dim; pre float32 [tokens, heads * dim];
     w0, bonus float32 [heads * dim]; state float32 [slots, heads, dim, dim] (key, value); out float32 [tokens, heads * dim].
-    A step of one token a sequence walks each sequence token by token, a step of prompts in blocks of four tokens (the same
-    numbers, summed in another order); which way a step goes depends on its rows and sequences alone."""
+    A step of one token a sequence walks each sequence token by token; a step of prompts goes as wkv_form says, in segments
+    only with ws, a Workspace (the same numbers, summed in another order). Which way a step goes depends on its rows and
+    sequences alone, not on how long each sequence is; form pins it (tests)."""
     _need_cuda(proj, pre, w0, bonus, state, out)
     lib = load_module("wkv")
     hk = n_heads * dim
@@ -1595,9 +1614,19 @@ def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, b
     assert w0.numel() == bonus.numel() == hk and state.shape[1:] == (n_heads, dim, dim)
     assert proj.shape[1] >= max(r_at, k_at, v_at) + hk
     n_seqs = batch.seq_slot.numel()
+    if form is None:
+        form = "tokens" if batch.is_decode or not 1 <= dim <= 256 else wkv_form(batch.n_rows, n_seqs, n_heads, dim)
+        if form == "segments" and ws is None:
+            form = "blocks"
+    segments, sums, prods = 0, None, None
+    if form == "segments":
+        segments = -(-batch.n_rows // WKV_SEGMENT) + n_seqs  # (at most: every sequence's last segment may be a short one)
+        sums = ws.get("wkv_sums", (segments, n_heads, dim, dim), torch.float32)
+        prods = ws.get("wkv_prods", (segments, n_heads, dim), torch.float32)
     _check(lib, lib.abk_wkv_scan(_p(proj), _ll(proj.stride(0)), _i(_dt(proj)), _i(r_at), _i(k_at), _i(v_at), _i(n_heads), _i(dim),
                                  _p(pre), _p(w0), _p(bonus), _p(state), _p(out), _p(batch.seq_start), _p(batch.seq_slot),
-                                 _i(n_seqs), _i(0 if batch.is_decode else 1), _stream()), "wkv_scan")
+                                 _i(n_seqs), _i(1 if form == "blocks" else 0), _i(WKV_SEGMENT if segments else 0), _i(segments),
+                                 _p(sums), _p(prods), _stream()), "wkv_scan", kernels=3 if segments else 1)
 
 
 # ------------------------------------------------------------------ experts by a table (csrc/moe.cu)

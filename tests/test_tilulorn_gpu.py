@@ -54,6 +54,26 @@ def test_wkv_every_way(dtype, H, K, rank):
 def test_wkv_in_blocks(H, K, lens, shift):
     """Blocks of four tokens and their remainders for every split of the work (few and many columns, every padded head size),
     sequences of unequal lengths, rows of bfloat16 that start on no boundary (shift), and the state they leave."""
+    _wkv_against_64_bits(H, K, lens, shift, "blocks")
+
+
+@pytest.mark.parametrize("form", ["segments", "tokens"])
+@pytest.mark.parametrize("H,K,lens", [(2, 30, (130, 1, 64, 65, 200)), (3, 64, (63, 129)), (2, 100, (150,)), (1, 256, (70, 3)), (5, 8, (128,))])
+def test_wkv_in_segments_and_token_by_token(H, K, lens, form):
+    """Segments of 64 tokens that end with their prompt, short of it and a token beyond it, for every padded head size."""
+    _wkv_against_64_bits(H, K, lens, 0, form)
+
+
+def test_how_a_step_of_wkv_prompts_goes():
+    from abacus_b200.kernels.ops import wkv_form
+    assert wkv_form(3571, 3, 40, 64) == wkv_form(500, 1, 16, 64) == wkv_form(100, 1, 2, 30) == wkv_form(4000, 8, 16, 30) == "blocks"
+    assert wkv_form(500, 1, 16, 30) == wkv_form(1000, 1, 4, 64) == wkv_form(2000, 1, 8, 100) == "segments"
+    assert wkv_form(8, 1, 40, 64) == wkv_form(512, 64, 40, 32) == "tokens" and wkv_form(512, 64, 40, 64) == "blocks"
+    assert wkv_form(65600 * 64, 40, 1, 16) == "blocks"  # (more segments than a grid takes)
+
+
+def _wkv_against_64_bits(H, K, lens, shift, form):
+    from abacus_b200.parts import Workspace
     from abacus_b200.engine.batch import Sequence, StepBatch
     from abacus_b200.kernels import ops
     rng, n = np.random.default_rng(H * K), sum(lens)
@@ -66,7 +86,7 @@ def test_wkv_in_blocks(H, K, lens, shift):
     S, out = state.double(), torch.empty((n, size), device=DEV)
     batch = StepBatch(n, len(lens), 1, DEV).fill([Sequence(i, [0] * m, 3, []) for i, m in enumerate(lens)], exact=True)
     assert not batch.is_decode
-    ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch)
+    ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch, ws=Workspace(torch.device(DEV, torch.cuda.current_device())), form=form)
     r, k, v = (proj[:, i * size:(i + 1) * size].double().view(n, H, K) for i in range(3))
     w, u, want, at = torch.exp(-torch.exp(pre.double() + w0.double())).view(n, H, K), bonus.double().view(H, K), [], 0
     for i, m in enumerate(lens):
@@ -81,18 +101,21 @@ def test_wkv_in_blocks(H, K, lens, shift):
     assert float((out.double() - want).abs().max()) <= limit and float((state.double() - S).abs().max()) <= limit
 
 
-@pytest.mark.parametrize("H,K,lens", [(32, 128, (500,)), (16, 256, (500,)), (40, 64, (500,)), (64, 64, (60,) * 64)])
-def test_wkv_in_blocks_takes_no_longer_than_token_by_token(H, K, lens):
+@pytest.mark.parametrize("H,K,lens", [(32, 128, (500,)), (16, 256, (500,)), (40, 64, (500,)), (64, 64, (60,) * 64), (16, 30, (2000,)),
+                                      (16, 30, (17, 1000)), (2, 64, (2000,)), (40, 32, (8,) * 64)])
+def test_a_step_of_wkv_prompts_takes_no_longer_than_in_another_form(H, K, lens):
     from abacus_b200.engine.batch import Sequence, StepBatch
     from abacus_b200.kernels import ops
+    from abacus_b200.parts import Workspace
     n, size = sum(lens), H * K
     proj, pre = torch.randn((n, 3 * size), device=DEV).to(torch.bfloat16), torch.randn((n, size), device=DEV)
     w0, bonus = torch.randn(size, device=DEV) - 2, torch.randn(size, device=DEV)
     state, out = torch.zeros((len(lens), H, K, K), device=DEV), torch.empty((n, size), device=DEV)
-    batch, times = StepBatch(n, len(lens), 1, DEV).fill([Sequence(i, [0] * m, 0, []) for i, m in enumerate(lens)], exact=True), []
-    for batch.is_decode in (False, True):  # (a decode step's kernel walks any number of tokens)
-        times.append(us_of(lambda: ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch)))
-    assert times[0] <= times[1], times
+    batch = StepBatch(n, len(lens), 1, DEV).fill([Sequence(i, [0] * m, 0, []) for i, m in enumerate(lens)], exact=True)
+    ws = Workspace(torch.device(DEV, torch.cuda.current_device()))
+    times = {form: us_of(lambda: ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch, ws=ws, form=form))
+             for form in (None, "tokens", "blocks", "segments")}
+    assert times[None] < 1.2 * min(times.values()), times
 
 
 def test_wkv_keeps_a_token_over_a_long_decoding_and_forgets_with_decays_near_nothing():
