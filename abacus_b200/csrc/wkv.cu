@@ -188,7 +188,7 @@ struct WkvScan {
     // phase 1 walks each segment from an empty state and leaves its sum and the product of its decays,
     // wkv_segment_prefix turns the sums into the states at the segments' starts (and leaves the last in the slot), phase 2
     // walks each segment again from its start state for the outputs. chunk 0 (phase 0): a CTA walks a whole sequence.
-    int chunk, phase;
+    int chunk;
     float *sums;         // [segments][heads][dim][dim]
     float *prods;        // [segments][heads][dim]
 };
@@ -269,8 +269,10 @@ __device__ __forceinline__ void wkv_tokens(float *s, const float *u, const float
 template <typename T> __device__ __forceinline__ float wkv_decay(float z) { return expf(-expf(z)); }
 template <> __device__ __forceinline__ float wkv_decay<__nv_bfloat16>(float z) { return __expf(-__expf(z)); }
 
-template <typename T, int DPT, int PARTS, int COLS, int TOK, bool SUMS>
+// PHASE: of a walk in segments (above), 0 where a CTA walks a whole sequence.
+template <typename T, int DPT, int PARTS, int COLS, int TOK, int PHASE>
 __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
+    constexpr bool SUMS = PHASE == 1;
     constexpr int DP = DPT * PARTS;             // key channels, padded
     constexpr int PITCH = PARTS * (DPT + 4);    // a token's channels in shared memory: a part's run, then 4 floats of
     constexpr int THREADS = PARTS * COLS;       // padding, so that the parts' 16-byte reads meet no bank twice
@@ -288,16 +290,16 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
     }
     pdl_wait();
     int seq = blockIdx.z, row0, n;
-    if (p.chunk > 0) wkv_segment(p.seq_start, p.n_seqs, p.chunk, blockIdx.z, seq, row0, n);
+    if constexpr (PHASE > 0) wkv_segment(p.seq_start, p.n_seqs, p.chunk, blockIdx.z, seq, row0, n);
     else row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
     if (n <= 0) return;  // (a sequence of the step's padding: its slot is someone else's)
-    float *state = p.phase == 0 ? p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * p.dim * p.dim
+    float *state = PHASE == 0 ? p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * p.dim * p.dim
                                 : p.sums + ((long long)blockIdx.z * p.n_heads + h) * p.dim * p.dim;
     float s[DPT];
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
         const int d = part * DPT + i;
-        s[i] = p.phase != 1 && d < p.dim && col < p.dim ? state[(long long)d * p.dim + col] : 0.0f;
+        s[i] = PHASE != 1 && d < p.dim && col < p.dim ? state[(long long)d * p.dim + col] : 0.0f;
     }
     const T *proj = (const T *)p.proj;
     const long long hk = (long long)p.n_heads * p.dim;
@@ -341,7 +343,7 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
             const bool in = tok < cnt && my_d < p.dim;
             const float w = wkv_decay<T>(rz[it] + my_w0);
             if (!SUMS) r_s[tok][at] = in ? to_float(rr[it]) : 0.0f;
-            if (in) decayed *= w;
+            if (SUMS && in) decayed *= w;
             k_s[tok][at] = in ? to_float(rk[it]) : 0.0f, w_s[tok][at] = w;
         }
 #pragma unroll
@@ -355,20 +357,20 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
         // multiply-adds follow one another
         const int at = part * (DPT + 4);
         float *out = p.out + (long long)(row0 + c0) * hk + (long long)h * p.dim + col;
-        const bool writes = part == 0 && col < p.dim && p.phase != 1;
+        const bool writes = part == 0 && col < p.dim && PHASE != 1;
         int tok = 0;
         for (; tok + 4 <= cnt; tok += 4)
             wkv_tokens<DPT, PARTS, 4, SUMS>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
         for (; tok < cnt; tok++)
             wkv_tokens<DPT, PARTS, 1, SUMS>(s, u, &r_s[tok][at], &k_s[tok][at], &w_s[tok][at], PITCH, &v_s[tok][vc], COLS, writes, out + tok * hk, hk);
     }
-    if (p.phase == 2) return;  // (the states between segments are wkv_segment_prefix's)
+    if constexpr (PHASE == 2) return;  // (the states between segments are wkv_segment_prefix's)
 #pragma unroll
     for (int i = 0; i < DPT; i++) {
         const int d = part * DPT + i;
         if (d < p.dim && col < p.dim) state[(long long)d * p.dim + col] = s[i];
     }
-    if (p.phase == 1 && tile == 0) {
+    if (PHASE == 1 && tile == 0) {
         // every thread staged the decays of one channel: the shares of a channel meet through shared memory
         __syncthreads();
         float *share = &r_s[0][0];
@@ -747,7 +749,7 @@ extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at,
     WkvScan p;
     p.proj = proj, p.ld = ld, p.r_at = r_at, p.k_at = k_at, p.v_at = v_at, p.n_heads = n_heads, p.dim = dim;
     p.pre = pre, p.w0 = w0, p.bonus = bonus, p.state = state, p.out = out, p.seq_start = seq_start, p.seq_slot = seq_slot;
-    p.n_seqs = n_seqs, p.tiles = 1, p.longest_first = 0, p.vec = 0, p.chunk = blocks ? 0 : chunk, p.phase = 0, p.sums = sums, p.prods = prods;
+    p.n_seqs = n_seqs, p.tiles = 1, p.longest_first = 0, p.vec = 0, p.chunk = chunk, p.sums = sums, p.prods = prods;
     if (chunk < 0 || (chunk > 0 && (segments < 1 || segments > 65535 || !sums || !prods)))
         ABK_REFUSE("wkv_scan: %d segments of %d tokens", segments, chunk);
     cudaStream_t s = (cudaStream_t)stream;
@@ -775,28 +777,32 @@ extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at,
     }
     const int cols = dim <= 32 ? 32 : 16;  // value columns a CTA has
     dim3 grid((dim + cols - 1) / cols, n_heads, chunk > 0 ? segments : n_seqs);
-#define WS_LAUNCH(T, SUMS)                                                                                  \
-    do {                                                                                                    \
-        if (dim <= 16) abk_launch(wkv_scan_kernel<T, 4, 4, 32, 16, SUMS>, grid, dim3(128), 0, s, p);        \
-        else if (dim <= 32) abk_launch(wkv_scan_kernel<T, 8, 4, 32, 16, SUMS>, grid, dim3(128), 0, s, p);   \
-        else if (dim <= 64) abk_launch(wkv_scan_kernel<T, 8, 8, 16, 16, SUMS>, grid, dim3(128), 0, s, p);   \
-        else if (dim <= 128) abk_launch(wkv_scan_kernel<T, 8, 16, 16, 16, SUMS>, grid, dim3(256), 0, s, p); \
-        else abk_launch(wkv_scan_kernel<T, 16, 16, 16, 8, SUMS>, grid, dim3(256), 0, s, p);                 \
+#define WS_LAUNCH_AS(T, PHASE)                                                                               \
+    do {                                                                                                     \
+        if (dim <= 16) abk_launch(wkv_scan_kernel<T, 4, 4, 32, 16, PHASE>, grid, dim3(128), 0, s, p);        \
+        else if (dim <= 32) abk_launch(wkv_scan_kernel<T, 8, 4, 32, 16, PHASE>, grid, dim3(128), 0, s, p);   \
+        else if (dim <= 64) abk_launch(wkv_scan_kernel<T, 8, 8, 16, 16, PHASE>, grid, dim3(128), 0, s, p);   \
+        else if (dim <= 128) abk_launch(wkv_scan_kernel<T, 8, 16, 16, 16, PHASE>, grid, dim3(256), 0, s, p); \
+        else abk_launch(wkv_scan_kernel<T, 16, 16, 16, 8, PHASE>, grid, dim3(256), 0, s, p);                 \
     } while (0)
-    if (chunk > 0) {  // the segments' sums, the states between them, the segments' outputs
-        p.phase = 1;
-        if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16, true);
-        else WS_LAUNCH(float, true);
-        int rc = ABK_LAUNCH_RESULT();
-        if (rc) return rc;
-        abk_launch(wkv_segment_prefix_kernel, dim3((dim * dim + 255) / 256, n_heads, n_seqs), dim3(256), 0, s, sums, prods, state,
-                   seq_start, seq_slot, n_heads, dim, chunk);
-        rc = ABK_LAUNCH_RESULT();
-        if (rc) return rc;
-        p.phase = 2;
+#define WS_LAUNCH(PHASE)                                        \
+    do {                                                        \
+        if (dtype == ABK_BF16) WS_LAUNCH_AS(__nv_bfloat16, PHASE); \
+        else WS_LAUNCH_AS(float, PHASE);                        \
+    } while (0)
+    if (chunk == 0) {
+        WS_LAUNCH(0);
+        return ABK_LAUNCH_RESULT();
     }
-    if (dtype == ABK_BF16) WS_LAUNCH(__nv_bfloat16, false);
-    else WS_LAUNCH(float, false);
+    WS_LAUNCH(1);  // the segments' sums, the states between them, the segments' outputs
+    int rc = ABK_LAUNCH_RESULT();
+    if (rc) return rc;
+    abk_launch(wkv_segment_prefix_kernel, dim3((dim * dim + 255) / 256, n_heads, n_seqs), dim3(256), 0, s, sums, prods, state,
+               seq_start, seq_slot, n_heads, dim, chunk);
+    rc = ABK_LAUNCH_RESULT();
+    if (rc) return rc;
+    WS_LAUNCH(2);
 #undef WS_LAUNCH
+#undef WS_LAUNCH_AS
     return ABK_LAUNCH_RESULT();
 }
