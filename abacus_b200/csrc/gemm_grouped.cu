@@ -502,9 +502,10 @@ __global__ void __launch_bounds__(GG_THREADS) gemm_grouped_pair_kernel(const __g
 
 // x bfloat16 [max_tiles * 128, K] (sorted rows); w bfloat16 [experts, N, K]; out [max_tiles * 128, ldo] bfloat16 or
 // (out_f32) float32; tile_expert int32 [max_tiles]; status int32 [>= 2]. Gated: N counts gate and up rows (a multiple of 128),
-// out has N / 2 columns.
+// out has N / 2 columns. in_pairs: 1 or 0 pins the kernel on pairs of CTAs or the one on single ones; -1: whichever is faster.
 extern "C" int abk_gemm_grouped(const void *x, const void *w, void *out, long long ldo, int out_f32, int activation,
-                                int max_tiles, int experts, int N, int K, const int *tile_expert, float limit, int *status, void *stream) {
+                                int max_tiles, int experts, int N, int K, const int *tile_expert, float limit, int *status, int in_pairs,
+                                void *stream) {
     if (max_tiles <= 0 || N <= 0) return 0;
     if (K <= 0 || K % 8) ABK_REFUSE("gemm_grouped: K = %d must be a multiple of 8", K);
     const bool gated = activation == GG_SILU_GATED || activation == GG_CLAMPED_GATED;
@@ -519,11 +520,20 @@ extern "C" int abk_gemm_grouped(const void *x, const void *w, void *out, long lo
     g.out = out, g.ldo = ldo, g.N = N, g.K = K, g.k_blocks = (K + GG_K - 1) / GG_K, g.tile_expert = tile_expert, g.status = status, g.limit = limit;
     g.vec = ((uintptr_t)out % 16 == 0) && (ldo * (out_f32 ? 4 : 2)) % 16 == 0;
     cudaStream_t s = (cudaStream_t)stream;
-    // Pairs of CTAs where the rows fill at least a tile an expert on average, of small experts (whose launches are short) two:
-    // 16 experts and a shared one of 1,024 x 768, top 2, 800 tokens: a feed-forward in 64.5 us a CTA a tile against 68.2 in
-    // pairs, 1,500 tokens 82.5 against 78.5; of 2,560 x 2,432, 1,500 tokens: 278 against 231, 4,000: 538 against 407.
-    const int used = max_tiles - experts;  // the rows' own tiles; padding adds up to one an expert
-    if (N >= GP_BN && max_tiles <= GP_MAX_TILES && used >= experts && (used >= 2 * experts || (long long)N * K >= 4 << 20)) {
+    // Which way: what counts is how often the GPU has to be filled, SMs with a tile of 128 x 128 each or pairs of SMs with one of
+    // 256 x 256, since a pair's turn takes about as long as an SM's, and the launch some four us more (as much as a turn where
+    // K is short). us with single CTAs and with pairs: 4 experts, 1,024 rows in all, N = K = 512: 5.7 and 9.0 (one turn either
+    // way); 8 experts, 2,048 rows, 768 x 1,024: 9.7 and 12.9 (one); 4 experts, 4,096 rows: 18 and 14 (two and one); 16 experts,
+    // 6,400 rows, 2,432 x 2,560: 139 and 91. Which expert has how many rows is not known here: half a tile of padding an expert
+    // is the usual, and since a pair has rows of one expert only, few rows an expert may leave it half empty (16 experts of 1,024 x
+    // 768, 129 rows each on average: 15.8 and 13.8, but 16 and 19 where one expert has half of all rows).
+    const long long sms = abk_sm_count(), used = max_tiles - experts, row_tiles = used + experts / 2;
+    const long long turns = (row_tiles * ((N + GG_BN - 1) / GG_BN) + sms - 1) / sms;
+    const long long pair_turns = ((row_tiles > 2 * experts ? row_tiles : 2 * experts) * ((N + GP_BN - 1) / GP_BN) + sms - 1) / sms;
+    const bool takes = N >= GP_BN && max_tiles <= GP_MAX_TILES;
+    const bool wins = (2 * used >= 3 * experts || (used >= experts && (long long)N * K >= 4 << 20)) && pair_turns + (K < 512) < turns;
+    if (in_pairs > 0 && !takes) ABK_REFUSE("gemm_grouped: pairs of CTAs take %d and more columns and up to %d row tiles", GP_BN, GP_MAX_TILES);
+    if (takes && (in_pairs < 0 ? wins : in_pairs > 0)) {
         const int pairs = abk_sm_count() / 2;
 #define GP_LAUNCH(TO, ACT)                                                                                                         \
     do {                                                                                                                           \

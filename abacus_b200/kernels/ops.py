@@ -1459,11 +1459,12 @@ def moe_sort(x, pairs_per_row, pair_expert, pair_scale, n_pairs, experts, scratc
                                  _i(max_tiles), _p(sorted_rows), _stream()), "moe_sort", kernels=3)
 
 
-def gemm_grouped(x, w, out, tile_expert, activation=0, limit=0.0):
+def gemm_grouped(x, w, out, tile_expert, activation=0, limit=0.0, in_pairs=-1):
     """out[p] = act(w[tile_expert[p // 128]] x[p]) for the sorted rows x bfloat16 [tiles * 128, K] on the tcgen05 tensor
     cores; w bfloat16 [experts, N, K]; out bfloat16 or float32 [tiles * 128, N]. Tiles whose expert is -1 are left alone.
     activation: 0 none, RELU_SQUARED, or one of GATED (w holds gate and up rows in turns of GROUPED_TURN, N a multiple of 128,
-    out bfloat16 [tiles * 128, N / 2]; limit: of CLAMPED_GATED)."""
+    out bfloat16 [tiles * 128, N / 2]; limit: of CLAMPED_GATED). in_pairs: 1 or 0 pins the kernel on pairs of CTAs or the one on
+    single ones (tests); -1 lets the library choose."""
     _need_cuda(x, w, out, tile_expert)
     lib = load_module("gemm_grouped")
     experts, n, k = w.shape
@@ -1474,7 +1475,7 @@ def gemm_grouped(x, w, out, tile_expert, activation=0, limit=0.0):
     assert out.dtype in (torch.bfloat16, torch.float32)
     _check(lib, lib.abk_gemm_grouped(_p(x), _p(w), _p(out), _ll(out.stride(0)), _i(1 if out.dtype == torch.float32 else 0),
                                      _i(activation), _i(tiles), _i(experts), _i(n), _i(k), _p(tile_expert), _f(limit),
-                                     _p(kernel_status(x.device)), _stream()), "gemm_grouped")
+                                     _p(kernel_status(x.device)), _i(in_pairs), _stream()), "gemm_grouped")
 
 
 def moe_unsort(sorted_out, place, out, n, top, add):

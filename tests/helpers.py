@@ -172,3 +172,15 @@ def us_of(fn, n=10):
         torch.cuda.synchronize()
         best = min(best, start.elapsed_time(end) * 1e3 / n)
     return best
+
+
+def graph_of(fn, n):
+    """n runs of fn() as one captured graph (kernels too short for their launches to be hidden): a function that replays it."""
+    import torch
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(n):
+            fn()
+    return graph.replay

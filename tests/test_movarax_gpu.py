@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import movarax_models as mm
-from helpers import TraceRun, assert_logits
+from helpers import TraceRun, assert_logits, graph_of, us_of
 from plain import movarax_plain as plain
 
 pytestmark = pytest.mark.gpu
@@ -282,8 +282,9 @@ def test_the_router_and_the_products_by_expert(dtype, E, top, d, ff):
 
 @pytest.mark.parametrize("counts,N,K,kind", [((300, 0, 129, 600, 256), 400, 72, 0), ((1, 128, 700, 260), 256, 64, 1), ((900, 385), 264, 200, 1),
                                              ((257, 513, 128), 384, 64, 2), ((1300,), 512, 136, 3), ((256, 255, 400), 256, 520, 0)])
-def test_the_product_by_expert_on_pairs_of_ctas(counts, N, K, kind):
-    """Runs of rows of every length against whole tiles and pairs of them (an odd last tile, one row, no row), outputs that end
+@pytest.mark.parametrize("in_pairs", [1, 0])
+def test_the_product_by_expert_on_pairs_of_ctas(counts, N, K, kind, in_pairs):
+    """On pairs and on single CTAs: runs of rows of every length against whole tiles and pairs of them (an odd last tile, one row, no row), outputs that end
     within a tile of 256, activations; rows of padding that are no numbers reach nothing."""
     from abacus_b200.kernels import ops
     rng, E, n = np.random.default_rng(sum(counts) + N), len(counts), sum(counts)
@@ -292,14 +293,14 @@ def test_the_product_by_expert_on_pairs_of_ctas(counts, N, K, kind):
     expert[torch.from_numpy(order).to(DEV)] = torch.from_numpy(np.repeat(np.arange(E, dtype=np.int32), counts)).to(DEV)
     x, w = (dev(rng.standard_normal(s), torch.bfloat16) for s in ((n, K), (E, N, K)))
     tiles = ops.grouped_tiles(n, E)
-    assert tiles - E >= 2 * E and N >= 256  # (the sizes that go in pairs)
+    assert N >= 256  # (what pairs take)
     scratch = torch.empty(2 * E + n, dtype=torch.int32, device=DEV)
     place, tile_expert = torch.empty(n, dtype=torch.int32, device=DEV), torch.empty(tiles, dtype=torch.int32, device=DEV)
     rows = torch.full((tiles * 128, K), float("nan"), dtype=torch.bfloat16, device=DEV)
     ops.moe_sort(x, 1, expert, None, n, E, scratch, place, tile_expert, rows)
     gated, activation = kind >= 2, (0, ops.RELU_SQUARED, ops.SILU_GATED, ops.CLAMPED_GATED)[kind]
     got = torch.zeros((tiles * 128, N // 2 if gated else N), dtype=torch.bfloat16 if kind else torch.float32, device=DEV)
-    ops.gemm_grouped(rows, w, got, tile_expert, activation=activation, limit=2.0)
+    ops.gemm_grouped(rows, w, got, tile_expert, activation=activation, limit=2.0, in_pairs=in_pairs)
     want = torch.einsum("pk,pnk->pn", x.double(), w.double()[expert.long()]) if n * N * K < 1 << 27 else torch.stack(
         [w[e].double() @ r.double() for r, e in zip(x, expert.tolist())])
     if kind == 1:
@@ -315,6 +316,23 @@ def test_the_product_by_expert_on_pairs_of_ctas(counts, N, K, kind):
     limit = 1e-4 * K ** 0.5 if not kind else (2.0 ** -8 if kind == 1 else 2.0 ** -5) * want.abs() + 0.05
     assert bool((diff <= limit).all()), float((diff - limit).max())
     assert not ops.kernel_status(x.device).any()
+
+
+@pytest.mark.parametrize("E,per,N,K,out", [(4, 256, 512, 512, torch.bfloat16), (8, 512, 512, 512, torch.bfloat16), (8, 256, 768, 1024, torch.bfloat16),
+                                           (4, 1024, 768, 1024, torch.bfloat16), (16, 400, 2432, 2560, torch.bfloat16),
+                                           (16, 1024, 1024, 768, torch.float32), (4, 256, 2560, 2432, torch.float32)])
+def test_the_product_by_expert_goes_the_faster_way(E, per, N, K, out):
+    from abacus_b200.kernels import ops
+    n = E * per
+    expert = torch.arange(n, dtype=torch.int32, device=DEV) % E
+    x, w = torch.randn((n, K), device=DEV).to(torch.bfloat16), torch.randn((E, N, K), device=DEV).to(torch.bfloat16)
+    tiles = ops.grouped_tiles(n, E)
+    scratch = torch.empty(2 * E + n, dtype=torch.int32, device=DEV)
+    place, tile_expert = torch.empty(n, dtype=torch.int32, device=DEV), torch.empty(tiles, dtype=torch.int32, device=DEV)
+    rows, got = torch.zeros((tiles * 128, K), dtype=torch.bfloat16, device=DEV), torch.empty((tiles * 128, N), dtype=out, device=DEV)
+    ops.moe_sort(x, 1, expert, None, n, E, scratch, place, tile_expert, rows)
+    times = {way: us_of(graph_of(lambda: ops.gemm_grouped(rows, w, got, tile_expert, in_pairs=way), 20), 1) for way in (-1, 0, 1)}
+    assert times[-1] < 1.12 * min(times[0], times[1]), times
 
 
 # ------------------------------------------------------------------ whole models through the engine

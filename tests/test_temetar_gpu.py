@@ -11,7 +11,7 @@ import pytest
 import torch
 
 import temetar_models as tm
-from helpers import ROOT, TRACE_RUN, TraceRun, assert_logits
+from helpers import ROOT, TRACE_RUN, TraceRun, assert_logits, graph_of, us_of
 from plain import temetar_plain as plain
 
 pytestmark = pytest.mark.gpu
