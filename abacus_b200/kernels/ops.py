@@ -507,19 +507,30 @@ def attention_window_takes(qkv, head_dim, v_dim, n_heads, n_kv_heads, row=None):
 
 def attention_window_tc_takes(qkv, out, n_heads, head_dim, v_dim, scale, softcap):
     """Whether the tcgen05 kernel takes a prompt step's attention with float32 weights: heads of 64, 128 or 192, values of 64
-    or 128, no cap of the scores, a positive scale, outputs 16-byte aligned (csrc/attention_window_tc.cu). Where it takes
-    them it is used: of one launch, 16 query and 8 key heads of 128, a window of 1,024, the warp-level kernel takes 9.7 us
-    for 16 tokens against 5.4, 41 for 512 against 27, 124 for 2,048 against 67; the least it gains was 22.9 against 24.0 (512
-    tokens, heads of 64, a window of 256)."""
+    or 128, no cap of the scores, a positive scale, outputs 16-byte aligned (csrc/attention_window_tc.cu)."""
     return (head_dim in (64, 128, 192) and v_dim in (64, 128) and not softcap and scale > 0 and out.data_ptr() % 16 == 0)
 
 
+def attention_window_tc_wins(rows, n_seqs, n_heads, v_dim, window, chunk):
+    """Whether it is also the faster one, by the step's rows and sequences. A CTA has 256 rows and an SM for itself, the warp-level
+    kernel's 64 rows and up to a quarter of one. us, warp level and tcgen05: 16 query and 8 key heads of 128, a window of 1,024:
+    16 tokens 9.7 and 5.4, 512 tokens 41 and 27, 2,048 tokens 124 and 67; but prompts of up to a tile of 64 rows that fill every SM,
+    40 prompts of 30 tokens and 32 heads of 128: 43 and 64, of 64 tokens 49 and 69 (of 80 tokens 86 and 85 with heads of 64); and few
+    rows that see little, 512 tokens, 16 heads of 64, a window of 64: 14 and 17, of 128: 17.4 and 19.2; 2,048 tokens, 2 heads of 128,
+    a window of 64: 17 and 19, 16 heads: 36 and 21."""
+    if rows <= 64 * n_seqs and n_seqs * n_heads > 148:
+        return False
+    sees = min(n for n in (window, chunk, max(rows, 1)) if n)
+    return not (sees * v_dim <= 8192 and rows >= 400 * n_seqs and sees * v_dim * rows * n_heads <= 77_500_000)
+
+
 def attention_window(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, batch, v_dim=None, keep_first=0, sink=None,
-                     row=None, chunk=None, softcap=None):
-    """Causal attention of whole prompts (every sequence of the step from its first token) on the tensor cores, keys and values from the step's own rows of qkv: an optional window that also keeps the first keep_first
-    keys, an optional sink (float32 [n_heads]), values of v_dim, softmax weights in float32, keys seen only within the
-    token's own chunk of `chunk` positions, scores capped at `softcap` (csrc/attention_window.cu on the warp-level ones,
-    csrc/attention_window_tc.cu by tcgen05 for the sizes that takes)."""
+                     row=None, chunk=None, softcap=None, tcgen05=None):
+    """Causal attention of whole prompts (every sequence of the step from its first token) on the tensor cores, keys and values
+    from the step's own rows of qkv: an optional window that also keeps the first keep_first keys, an optional sink (float32
+    [n_heads]), values of v_dim, softmax weights in float32, keys seen only within the token's own chunk of `chunk` positions,
+    scores capped at `softcap` (csrc/attention_window.cu on the warp-level ones, csrc/attention_window_tc.cu by tcgen05 where
+    that takes the sizes and is faster). tcgen05: True or False pins the kernel (tests)."""
     _need_cuda(qkv, out, sink)
     vd = v_dim or head_dim
     heads_size = (n_heads + n_kv_heads) * head_dim + n_kv_heads * vd
@@ -530,7 +541,10 @@ def attention_window(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, bat
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() == n_heads)
     if batch.any_continuation:
         raise KernelRefused("attention_window reads keys from the step's rows: every sequence must start at position 0")
-    if attention_window_tc_takes(qkv, out, n_heads, head_dim, vd, scale, softcap):
+    takes = attention_window_tc_takes(qkv, out, n_heads, head_dim, vd, scale, softcap)
+    if tcgen05 and not takes:
+        raise KernelRefused("attention_window: the tcgen05 kernel does not take these sizes, or capped scores")
+    if takes and (attention_window_tc_wins(n, n_seqs, n_heads, vd, window, chunk) if tcgen05 is None else tcgen05):
         lib = load_module("attention_window_tc")
         _check(lib, lib.abk_attention_window_tc(_p(qkv), _ll(row), _i(n), _p(out), _i(n_heads), _i(n_kv_heads), _i(head_dim), _i(vd),
                                                 _i(n_heads * head_dim), _i((n_heads + n_kv_heads) * head_dim), _f(scale),

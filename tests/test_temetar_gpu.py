@@ -305,10 +305,13 @@ def test_attention_with_sink_window_and_kept_first_keys_in_prompts_and_decoding(
 @pytest.mark.parametrize("H,G,D,V,window,keep,with_sink", [(4, 2, 16, 24, 12, 3, True), (6, 2, 24, 40, 70, 0, True),
                                                           (3, 3, 32, 32, None, 0, False), (2, 2, 128, 128, 100, 7, True),
                                                           (1, 1, 256, 64, 5, 0, True), (2, 1, 40, 8, 64, 64, False),
-                                                          (2, 1, 64, 128, 200, 130, True)])
-def test_the_tensor_core_prompt_kernel_on_unequal_prompts(H, G, D, V, window, keep, with_sink):
-    """Several sequences of unequal lengths in one step (one token, just under, at and just over a tile of 64 rows),
-    every row against the plain formulas; head sizes that need padding to 16, windows shorter and longer than a tile."""
+                                                          (2, 1, 64, 128, 200, 130, True), (3, 3, 192, 128, None, 0, True),
+                                                          (4, 2, 64, 64, 128, 0, False)])
+@pytest.mark.parametrize("softcap", [None, 1.5])
+def test_the_tensor_core_prompt_kernel_on_unequal_prompts(H, G, D, V, window, keep, with_sink, softcap):
+    """The warp-level kernel, with and without a cap of the scores (where there is one, no other takes the layer): several
+    sequences of unequal lengths in one step (one token, just under, at and just over a tile of 64 rows), every row against the
+    plain formulas; head sizes that need padding to 16, windows shorter and longer than a tile."""
     from abacus_b200.kernels import ops
     lens, scale = [150, 1, 37, 64, 65, 300], 0.11
     rows, wants, sink = [], [], None
@@ -317,6 +320,7 @@ def test_the_tensor_core_prompt_kernel_on_unequal_prompts(H, G, D, V, window, ke
         q, k, v = plain.bf16_round(q), plain.bf16_round(k), plain.bf16_round(v)
         sink = sk if sink is None else sink
         z = np.einsum("ihd,jhd->hij", q, np.repeat(k, H // G, axis=1)) * np.float32(scale)
+        z = np.float32(softcap) * np.tanh(z / np.float32(softcap)) if softcap else z
         w = plain.softmax_with_sink(z, sink if with_sink else np.full(H, -np.inf, dtype=np.float32), plain.visible(T, window or T, keep))
         wants.append(np.einsum("hij,jhv->ihv", w, np.repeat(v, H // G, axis=1)).reshape(T, H * V))
         rows.append(np.concatenate([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], axis=1))
@@ -324,7 +328,8 @@ def test_the_tensor_core_prompt_kernel_on_unequal_prompts(H, G, D, V, window, ke
     qkv = dev(np.concatenate(rows), torch.bfloat16)
     out = torch.empty((sum(lens), H * V), dtype=torch.bfloat16, device=DEV)
     assert ops.attention_window_takes(qkv, D, V, H, G)
-    ops.attention_window(qkv, out, H, G, D, scale, window, b, v_dim=V, keep_first=keep, sink=dev(sink) if with_sink else None)
+    ops.attention_window(qkv, out, H, G, D, scale, window, b, v_dim=V, keep_first=keep, sink=dev(sink) if with_sink else None,
+                         softcap=softcap, tcgen05=False)
     got, want = out.float().cpu().numpy(), np.concatenate(wants)
     # float32 weights: what is left is the rounding of the stored result
     np.testing.assert_allclose(got, want, rtol=2 ** -8, atol=1e-3)
@@ -359,8 +364,8 @@ def test_prompts_on_two_groups_of_rows_a_cta(H, G, D, V, window, keep, chunk, le
     b = batch_of([(i, [0] * T, 0) for i, T in enumerate(list(lens) + [40])])
     qkv = dev(np.concatenate(rows), torch.bfloat16)
     out = torch.empty((sum(lens) + 40, H * V), dtype=torch.bfloat16, device=DEV)
-    assert ops.attention_window_tc_takes(qkv, out, H, D, V, scale, None)
-    ops.attention_window(qkv, out, H, G, D, scale, window, b, v_dim=V, keep_first=keep, sink=dev(sink), chunk=chunk or None)
+    assert ops.attention_window_tc_takes(qkv, out, H, D, V, scale, None) and not ops.attention_window_tc_takes(qkv, out, H, D, V, scale, 30.0)
+    ops.attention_window(qkv, out, H, G, D, scale, window, b, v_dim=V, keep_first=keep, sink=dev(sink), chunk=chunk or None, tcgen05=True)
     got = out.float().cpu().numpy()
     # float32 weights: what is left is the rounding of the stored result
     np.testing.assert_allclose(got[:sum(lens)], np.concatenate(wants), rtol=2 ** -8, atol=1e-3)
@@ -382,10 +387,22 @@ def test_a_rows_bits_know_nothing_of_the_rows_beside_it(H, G, D, V, window, keep
         if loud_from is not None:
             rows[loud_from:, :H * D] *= 64.0
         out = torch.empty((T + after, H * V), dtype=torch.bfloat16, device=DEV)
-        ops.attention_window(dev(rows, torch.bfloat16), out, H, G, D, D ** -0.5, window, b, v_dim=V, keep_first=keep)
+        ops.attention_window(dev(rows, torch.bfloat16), out, H, G, D, D ** -0.5, window, b, v_dim=V, keep_first=keep, tcgen05=True)
         got.append((loud_from or T, out))
     for first, out in got[1:]:
         assert torch.equal(out[:first], got[0][1][:first]), first
+
+
+@pytest.mark.parametrize("H,G,D,V,window,lens", [(32, 8, 128, 128, None, (30,) * 40), (32, 8, 64, 64, None, (50,) * 40), (16, 8, 64, 64, 64, (512,)),
+                                                 (2, 2, 192, 64, 64, (2048,)), (16, 8, 128, 128, 64, (2048,)), (32, 8, 128, 128, 1024, (345, 1500)),
+                                                 (16, 8, 64, 64, None, (16,)), (8, 1, 128, 128, 256, (512,))])
+def test_prompts_with_float32_weights_go_the_faster_way(H, G, D, V, window, lens):
+    from abacus_b200.kernels import ops
+    n, b = sum(lens), batch_of([(i, [0] * T, 0) for i, T in enumerate(lens)])
+    qkv, out = torch.randn((n, (H + G) * D + G * V), device=DEV).to(torch.bfloat16), torch.empty((n, H * V), dtype=torch.bfloat16, device=DEV)
+    times = {way: us_of(graph_of(lambda: ops.attention_window(qkv, out, H, G, D, D ** -0.5, window, b, v_dim=V, tcgen05=way), 10), 1)
+             for way in (None, False, True)}
+    assert times[None] < 1.12 * min(times[False], times[True]), times
 
 
 @pytest.mark.parametrize("H,G,D,V,window,keep,dtype", [(8, 1, 32, 200, None, 0, torch.bfloat16), (6, 2, 24, 40, 300, 9, torch.float32),
