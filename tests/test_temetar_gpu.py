@@ -200,6 +200,20 @@ def test_delta_rule_in_blocks(H, K, V, lens):
         np.testing.assert_allclose(out.cpu().numpy(), expected, rtol=1e-4, atol=2e-5 + 4 * noise)
 
 
+def test_a_delta_step_of_small_heads_leaves_no_warp_idle():
+    """A head of 32 x 32 is a quarter of one of 64 x 64: with warps that have no columns it took nearly half as long."""
+    from abacus_b200.kernels import ops
+    from abacus_b200.parts import Workspace
+    n, H, times = 256, 40, []
+    b, ws = batch_of([(i, [0], 0) for i in range(n)]), Workspace(torch.device(DEV, torch.cuda.current_device()))
+    for K in (32, 64):
+        qkv, decay, beta = torch.randn((n, 3 * H * K), device=DEV).to(torch.bfloat16), torch.randn((n, H * K), device=DEV), torch.randn((n, H), device=DEV).to(torch.bfloat16)
+        state, out = torch.zeros((n, H, K, K), device=DEV), torch.empty((n, H * K), device=DEV)
+        a_log, bias = torch.zeros(H, device=DEV), torch.zeros(H * K, device=DEV)
+        times.append(us_of(lambda: ops.delta_scan(qkv, decay, beta, a_log, bias, state, out, b, H, H, K, K, ws)))
+    assert times[0] < 0.4 * times[1], times
+
+
 def test_gated_head_norm():
     from abacus_b200.kernels import ops
     rng = np.random.default_rng(1)
