@@ -254,10 +254,8 @@ template <typename T> __global__ void __launch_bounds__(128) delta_prepare_kerne
     const T *kr = qr + (long long)p.kv_heads * K;
     const T *vr = (const T *)p.qkv + row * p.ld_qkv + 2LL * p.kv_heads * K + (long long)h * V;
     const float rate = expf(p.a_log[h]);
-    float head_decay = 0.0f;  // one decay for all of the head's key channels
-    if (p.per_head)
-        head_decay = expf(-rate * softplus_f(to_float(((const T *)p.decay_in)[row * p.ld_decay + h]) + p.dt_bias[h]));
-    const float *channel_decay = (const float *)p.decay_in + row * p.ld_decay + (long long)h * K;
+    // one decay for all of the head's key channels (the chunked form takes no others)
+    const float head_decay = expf(-rate * softplus_f(to_float(((const T *)p.decay_in)[row * p.ld_decay + h]) + p.dt_bias[h]));
     float qq = 0.0f, kk = 0.0f;
     for (int i = lane; i < K; i += 32) {
         const float qv = to_float(qr[i]), kv = to_float(kr[i]);
@@ -270,7 +268,7 @@ template <typename T> __global__ void __launch_bounds__(128) delta_prepare_kerne
         const bool real = at % SCAN_RUN < SCAN_ROWS && i < K;
         rec[at] = real ? to_float(kr[i]) * kn : 0.0f;
         rec[region + at] = real ? to_float(qr[i]) * qn : 0.0f;
-        rec[2 * region + at] = !real ? 0.0f : p.per_head ? head_decay : expf(-rate * softplus_f(channel_decay[i] + p.dt_bias[h * K + i]));
+        rec[2 * region + at] = real ? head_decay : 0.0f;
     }
     const int vp = p.record - 3 * region - 4;
     for (int j = lane; j < vp; j += 32) rec[3 * region + j] = j < V ? to_float(vr[j]) : 0.0f;

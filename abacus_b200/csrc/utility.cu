@@ -65,6 +65,8 @@ __global__ void __launch_bounds__(128) set_words_kernel(const __grid_constant__ 
     for (int i = threadIdx.x; i < p.n; i += 128) p.table[p.pairs[2 * i]] = p.pairs[2 * i + 1];
 }
 
+extern "C" int abk_set_words_room() { return SET_WORDS; }
+
 // table[pairs[2 i]] = pairs[2 i + 1] for i in [0, n); `pairs` (on the host) is read before this returns. Words all different.
 extern "C" int abk_set_words(int *table, long long size, const int *pairs, int n, void *stream) {
     for (int i = 0; i < n; i++)

@@ -83,7 +83,7 @@ def set_words(table, changes):
     pairs = array.array("i", changes)
     n = len(pairs) // 2
     _check(lib, lib.abk_set_words(_p(table), _ll(table.numel()), ctypes.c_void_p(pairs.buffer_info()[0]), _i(n), _stream()),
-           "set_words", kernels=-(-n // 480))
+           "set_words", kernels=-(-n // lib.abk_set_words_room()))
 
 
 def embed(tokens, table, x, status):
