@@ -200,6 +200,37 @@ def test_delta_rule_in_blocks(H, K, V, lens):
         np.testing.assert_allclose(out.cpu().numpy(), expected, rtol=1e-4, atol=2e-5 + 4 * noise)
 
 
+@pytest.mark.parametrize("n_seqs", [33, 64, 65])
+def test_delta_rule_in_blocks_of_many_sequences(n_seqs):
+    """The order in which sequences are walked (up to 64: the longest first, over two lanes' halves) and where a block's sequence is
+    looked for (32 at a time): equal lengths, a sequence without tokens, the longest among the last; every row, every state."""
+    from abacus_b200.kernels import ops
+    from abacus_b200.parts import Workspace
+    H, K, V, rng = 8, 16, 40, np.random.default_rng(n_seqs)
+    lens = [int(n) for n in rng.integers(1, 12, n_seqs)]
+    lens[3] = lens[40 % n_seqs] = lens[n_seqs - 1] = 17
+    lens[7] = 0
+    ins = [_delta_inputs(rng, n, H, H, K, V) for n in lens]
+    a_log, bias = ins[0][3], ins[0][4]
+    want = [_delta_plain(i[0], i[1], i[2], a_log, bias, H, H, K, V, real=np.float64) for i in ins]
+    noise = max(np.abs(w - _delta_plain(i[0], i[1], i[2], a_log, bias, H, H, K, V)).max() for i, w in zip(ins, want) if len(w))
+    ws, slots = Workspace(torch.device(DEV, torch.cuda.current_device())), [int(x) for x in rng.permutation(n_seqs)]
+    cat = lambda j: dev(np.concatenate([i[j] for i in ins]))
+    states, outs = [], []
+    for order in (list(range(n_seqs)), None):  # all at once, then one after the other
+        state, out = torch.zeros((n_seqs, H, V, K), device=DEV), torch.zeros((sum(lens), H * V), device=DEV)
+        at = np.concatenate([[0], np.cumsum(lens)])
+        for group in ([order] if order else [[i] for i in range(n_seqs) if lens[i]]):
+            first, last = at[group[0]], at[group[-1] + 1]
+            b = batch_of([(slots[i], [0] * lens[i], 0) for i in group])
+            ops.delta_scan(cat(0)[first:last], cat(1)[first:last], cat(2)[first:last], dev(a_log), dev(bias), state, out[first:last], b, H, H, K, V, ws)
+        states.append(state), outs.append(out)
+    np.testing.assert_allclose(outs[0].cpu().numpy(), np.concatenate(want), rtol=1e-4, atol=2e-5 + 4 * noise)
+    # (alone a sequence may be walked with other columns a lane: sums of as many products in another order)
+    np.testing.assert_allclose(states[0].cpu().numpy(), states[1].cpu().numpy(), rtol=1e-4, atol=2e-5 + 4 * noise)
+    assert float(states[0][slots[7]].abs().max()) == 0.0
+
+
 def test_a_delta_step_of_small_heads_leaves_no_warp_idle():
     """A head of 32 x 32 is a quarter of one of 64 x 64: with warps that have no columns it took nearly half as long."""
     from abacus_b200.kernels import ops

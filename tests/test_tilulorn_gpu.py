@@ -64,6 +64,15 @@ def test_wkv_in_segments_and_token_by_token(H, K, lens, form):
     _wkv_against_64_bits(H, K, lens, 0, form)
 
 
+@pytest.mark.parametrize("n_seqs", [33, 64, 65])
+def test_wkv_in_blocks_of_many_sequences(n_seqs):
+    """The order in which sequences are walked (up to 64 the longest first): equal lengths, a sequence without tokens."""
+    lens = [int(n) for n in np.random.default_rng(n_seqs).integers(1, 8, n_seqs)]
+    lens[3] = lens[40 % n_seqs] = lens[n_seqs - 1] = 13
+    lens[7] = 0
+    _wkv_against_64_bits(9, 20, lens, 0, "blocks")
+
+
 def test_how_a_step_of_wkv_prompts_goes():
     from abacus_b200.kernels.ops import wkv_form
     assert wkv_form(3571, 3, 40, 64) == wkv_form(500, 1, 16, 64) == wkv_form(100, 1, 2, 30) == wkv_form(4000, 8, 16, 30) == "blocks"
