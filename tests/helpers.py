@@ -158,19 +158,22 @@ def assert_logits(got, want, dtype, what="", noise=0.0):
         assert kl.max() <= BF16_KL, f"{what}: KL {kl.max():.3g} at row {kl.argmax()} (limit {BF16_KL})"
 
 
-def us_of(fn, n=10):
-    """Device time of one fn(): the fastest of five runs of n in a row."""
+def us_of(ways, n=10):
+    """Device time of one call of every function in `ways` (a dict): each the fastest of seven runs of n in a row, the ways taking
+    turns, so that a clock that moves moves all of them."""
     import torch
-    fn()
-    best = float("inf")
-    for _ in range(5):
-        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
-        start.record()
-        for _ in range(n):
-            fn()
-        end.record()
-        torch.cuda.synchronize()
-        best = min(best, start.elapsed_time(end) * 1e3 / n)
+    for fn in ways.values():
+        fn()
+    best = {}
+    for _ in range(7):
+        for name, fn in ways.items():
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            for _ in range(n):
+                fn()
+            end.record()
+            torch.cuda.synchronize()
+            best[name] = min(best.get(name, float("inf")), start.elapsed_time(end) * 1e3 / n)
     return best
 
 

@@ -150,22 +150,21 @@ def test_gemm_simt_tiles_give_the_same_bits(ops, n, k):
 @pytest.mark.parametrize("m, n", [(2048, 6144), (1000, 8192), (500, 6144)])
 def test_gemm_simt_with_one_sum_keeps_the_gpu_busy(ops, m, n):
     """K = 256 is one sum an element, K = 272 eight: less to multiply may not take longer (a third for luck)."""
-    times = []
-    for k in (256, 272):
-        x, w, out = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda"), torch.empty(m, n, device="cuda")
-        times.append(us_of(lambda: ops.gemm_simt(x, w, out)))
-    assert times[0] < 1.33 * times[1], times
+    out = torch.empty(m, n, device="cuda")
+    operands = {k: (torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda")) for k in (256, 272)}
+    times = us_of({k: lambda x=x, w=w: ops.gemm_simt(x, w, out) for k, (x, w) in operands.items()})
+    assert times[256] < 1.33 * times[272], times
 
 
 @pytest.mark.parametrize("dtype, m, n, k", [(torch.float32, 2048, 2048, 130), (torch.float32, 500, 1024, 1023), (torch.bfloat16, 500, 2048, 250),
                                             (torch.bfloat16, 2048, 1024, 1020)])
 def test_gemm_simt_of_rows_that_start_anywhere(ops, dtype, m, n, k):
     """Operands whose rows start on no 16-byte boundary, number by number: at most twice what aligned float32 ones take."""
-    times = []
-    for t, size in ((dtype, k), (torch.float32, -(-k // 4) * 4)):
-        x, w, out = torch.randn(m, size, device="cuda").to(t), torch.randn(n, size, device="cuda").to(t), torch.empty(m, n, device="cuda")
-        times.append(us_of(lambda: ops.gemm_simt(x, w, out)))
-    assert times[0] < 2 * times[1], times
+    out = torch.empty(m, n, device="cuda")
+    operands = {name: (torch.randn(m, size, device="cuda").to(t), torch.randn(n, size, device="cuda").to(t))
+                for name, t, size in (("anywhere", dtype, k), ("aligned", torch.float32, -(-k // 4) * 4))}
+    times = us_of({name: lambda x=x, w=w: ops.gemm_simt(x, w, out) for name, (x, w) in operands.items()})
+    assert times["anywhere"] < 2 * times["aligned"], times
 
 
 @pytest.mark.parametrize("n", [1, 480, 481, 1500])

@@ -331,8 +331,8 @@ def test_the_product_by_expert_goes_the_faster_way(E, per, N, K, out):
     place, tile_expert = torch.empty(n, dtype=torch.int32, device=DEV), torch.empty(tiles, dtype=torch.int32, device=DEV)
     rows, got = torch.zeros((tiles * 128, K), dtype=torch.bfloat16, device=DEV), torch.empty((tiles * 128, N), dtype=out, device=DEV)
     ops.moe_sort(x, 1, expert, None, n, E, scratch, place, tile_expert, rows)
-    times = {way: us_of(graph_of(lambda: ops.gemm_grouped(rows, w, got, tile_expert, in_pairs=way), 20), 1) for way in (-1, 0, 1)}
-    assert times[-1] < 1.12 * min(times[0], times[1]), times
+    times = us_of({way: graph_of(lambda: ops.gemm_grouped(rows, w, got, tile_expert, in_pairs=way), 20) for way in (-1, 0, 1)}, 1)
+    assert times[-1] < 1.2 * min(times[0], times[1]), times
 
 
 # ------------------------------------------------------------------ whole models through the engine

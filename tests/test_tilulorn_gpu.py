@@ -122,8 +122,8 @@ def test_a_step_of_wkv_prompts_takes_no_longer_than_in_another_form(H, K, lens):
     state, out = torch.zeros((len(lens), H, K, K), device=DEV), torch.empty((n, size), device=DEV)
     batch = StepBatch(n, len(lens), 1, DEV).fill([Sequence(i, [0] * m, 0, []) for i, m in enumerate(lens)], exact=True)
     ws = Workspace(torch.device(DEV, torch.cuda.current_device()))
-    times = {form: us_of(lambda: ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch, ws=ws, form=form))
-             for form in (None, "tokens", "blocks", "segments")}
+    times = us_of({form: lambda form=form: ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch, ws=ws, form=form)
+                   for form in (None, "tokens", "blocks", "segments")})
     assert times[None] < 1.2 * min(times.values()), times
 
 
