@@ -836,9 +836,10 @@ extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, cons
     // A warp's columns, 4 or 8: the fewer, the more warps share the work and the less each waits for in a block; the more,
     // the less a column costs. Heads of 128 x 128, one prompt: of 1,999 tokens and 16 heads 298 us against 366, of 1,500
     // tokens and 32 heads 331 against 286; 8 prompts, 5,672 tokens, 32 heads: 960 against 701. Four columns therefore up to
-    // what gives every SM one CTA of them.
+    // what gives every SM one CTA of them, and where keys are long and prompts short, whose state is most of the work (100 prompts
+    // of 20 tokens, 4 heads of 256 x 512: 417 us against 482).
     const long long columns = (long long)n_seqs * heads * value, sms = abk_sm_count();
-    const int per_warp = columns <= 16 * sms ? 4 : 8;
+    const int per_warp = columns <= 16 * sms || (key > 128 && n_tokens <= 32LL * n_seqs) ? 4 : 8;
     int warps = 4;
     while (warps > 1 && warps * per_warp >= 2 * value) warps /= 2;  // (no CTA of which less than half is used)
     const int cols = warps * per_warp;
