@@ -8,8 +8,9 @@
 //                     plane of the output per s. In a step of one token a sequence it also leaves the new last row.
 //   token_shift_keep  the last row of every sequence of a step of prompts, into its slot.
 //   wkv_block         prompts: blocks of four tokens (below)
-//   wkv_scan          a step of one token or a few a sequence, and prompts of heads too few to fill the GPU, in segments
-//                     walked side by side: a CTA walks one sequence's (a segment's) tokens for one head and 16 (32 for heads
+//   wkv_step          a step of one token a sequence (below)
+//   wkv_scan          a step of a few tokens a sequence, and prompts of heads too few to fill the GPU, in segments walked
+//                     side by side: a CTA walks one sequence's (a segment's) tokens for one head and 16 (32 for heads
 //                     of up to 32 channels) value columns. Its threads are those columns x 4, 8 or 16 parts of the key
 //                     channels, so a thread keeps 4 to 16 state values in registers; the parts' partial outputs of a
 //                     column meet by shuffles, four tokens at a time. Rows come 16 (8 for heads beyond 128 channels) tokens
@@ -384,6 +385,86 @@ __global__ void __launch_bounds__(PARTS * COLS, 2) wkv_scan_kernel(WkvScan p) {
     }
 }
 
+// A step of one token a sequence: the state comes and goes once, and that is all there is to do. A CTA has one (sequence, head) and
+// 4 LPR of its value columns, a lane four of them in every 16th row (as a 16-byte piece where heads are a multiple of 4 channels),
+// all rows asked for before the token's r, k and decay are made; the rows' sums of a column meet by shuffles and across the warps.
+// (A sequence that brings several tokens after all is walked token by token.) Bound by the state's way in and out of memory: 64
+// sequences, 40 heads of 64, 84 MB of it read and written in 14 to 15 us (part of it in the L2), 20 heads of 128 in 37; 8 sequences, 40
+// heads of 64 4.3 us (wkv_scan, which has no more than a column a thread in flight: 57, 123 and 9.1).
+template <typename T, int LPR, int ROWS, bool VEC>  // lanes of a row; rows of a thread
+__global__ void __launch_bounds__(16 * LPR) wkv_step_kernel(WkvScan p) {
+    constexpr int THREADS = 16 * LPR, WARPS = THREADS / 32, COLS = 4 * LPR;
+    __shared__ float r_s[16 * ROWS], k_s[16 * ROWS], w_s[16 * ROWS], u_s[16 * ROWS];
+    __shared__ __align__(16) float meet[WARPS][COLS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = p.dim, h = blockIdx.y, row = tid / LPR;
+    const int col = blockIdx.x * COLS + tid % LPR * 4;
+    const bool mine = col < D;
+    const long long hk = (long long)p.n_heads * D;
+    pdl_wait();
+    const int seq = blockIdx.z, row0 = p.seq_start[seq], n = p.seq_start[seq + 1] - row0;
+    if (n <= 0) return;  // (a sequence of the step's padding: its slot is someone else's)
+    float *state = p.state + ((long long)p.seq_slot[seq] * p.n_heads + h) * D * D + col;
+    float4 S[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) {
+        const float *src = state + (long long)(row + 16 * i) * D;
+        S[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (!mine || row + 16 * i >= D) continue;
+        if constexpr (VEC) S[i] = *(const float4 *)src;
+        else S[i] = make_float4(src[0], col + 1 < D ? src[1] : 0.0f, col + 2 < D ? src[2] : 0.0f, col + 3 < D ? src[3] : 0.0f);
+    }
+    for (int t = 0; t < n; t++) {
+        const T *proj = (const T *)p.proj + (long long)(row0 + t) * p.ld + h * D;
+        float v[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) v[x] = col + x < D ? to_float(proj[p.v_at + col + x]) : 0.0f;
+        for (int d = tid; d < 16 * ROWS; d += THREADS) {
+            const bool in = d < D;
+            r_s[d] = in ? to_float(proj[p.r_at + d]) : 0.0f, k_s[d] = in ? to_float(proj[p.k_at + d]) : 0.0f;
+            w_s[d] = in ? wkv_decay<T>(p.pre[(row0 + t) * hk + h * D + d] + p.w0[h * D + d]) : 0.0f, u_s[d] = in ? p.bonus[h * D + d] : 0.0f;
+        }
+        __syncthreads();
+        float o[4] = {};
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) {
+            const int d = row + 16 * i;
+            const float r = r_s[d], k = k_s[d], w = w_s[d], u = u_s[d];
+            float *s = (float *)&S[i];
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                const float a = k * v[x];
+                o[x] = fmaf(r, fmaf(u, a, s[x]), o[x]), s[x] = fmaf(w, s[x], a);
+            }
+        }
+#pragma unroll
+        for (int m = LPR; m < 32; m <<= 1)
+#pragma unroll
+            for (int x = 0; x < 4; x++) o[x] += __shfl_xor_sync(0xffffffffu, o[x], m);
+        if (lane < LPR) *(float4 *)&meet[warp][4 * lane] = make_float4(o[0], o[1], o[2], o[3]);
+        __syncthreads();
+        const int c = blockIdx.x * COLS + tid;
+        if (tid < COLS && c < D) {
+            float sum = meet[0][tid];
+#pragma unroll
+            for (int w = 1; w < WARPS; w++) sum += meet[w][tid];
+            p.out[(row0 + t) * hk + (long long)h * D + c] = sum;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) {
+        float *dst = state + (long long)(row + 16 * i) * D;
+        if (!mine || row + 16 * i >= D) continue;
+        if constexpr (VEC) {
+            *(float4 *)dst = S[i];
+        } else {
+            dst[0] = S[i].x;
+            if (col + 1 < D) dst[1] = S[i].y;
+            if (col + 2 < D) dst[2] = S[i].z;
+            if (col + 3 < D) dst[3] = S[i].w;
+        }
+    }
+}
+
 // The states at the segments' starts from the segments' own sums: along a sequence S <- prod * S + sum, the state before
 // each segment left where its sum was, the last in the sequence's slot. A thread an element of the state; four segments'
 // loads are on their way together.
@@ -737,11 +818,12 @@ template <typename T, int P, int J, int C> static int wkv_block_launch(WkvScan p
     return ABK_LAUNCH_RESULT();
 }
 
-// blocks: the step's sequences are walked in blocks of four tokens; chunk > 0: in segments of so many tokens (`segments` of
-// them at most, with room for their sums and products); else token by token.
+enum { WKV_TOKENS, WKV_BLOCKS, WKV_SEGMENTS, WKV_STEP };
+// form: token by token; in blocks of four tokens; in segments of `chunk` tokens (`segments` of them at most, with room for their
+// sums and products); or a step of one token a sequence.
 extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at, int k_at, int v_at, int n_heads, int dim,
                             const float *pre, const float *w0, const float *bonus, float *state, float *out,
-                            const int *seq_start, const int *seq_slot, int n_seqs, int blocks, int chunk, int segments, float *sums,
+                            const int *seq_start, const int *seq_slot, int n_seqs, int form, int chunk, int segments, float *sums,
                             float *prods, void *stream) {
     if (n_seqs <= 0) return 0;
     if (dim < 1 || dim > 256) ABK_REFUSE("wkv_scan: %d key channels a head are not 1 to 256", dim);
@@ -750,10 +832,11 @@ extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at,
     p.proj = proj, p.ld = ld, p.r_at = r_at, p.k_at = k_at, p.v_at = v_at, p.n_heads = n_heads, p.dim = dim;
     p.pre = pre, p.w0 = w0, p.bonus = bonus, p.state = state, p.out = out, p.seq_start = seq_start, p.seq_slot = seq_slot;
     p.n_seqs = n_seqs, p.tiles = 1, p.longest_first = 0, p.vec = 0, p.chunk = chunk, p.sums = sums, p.prods = prods;
-    if (chunk < 0 || (chunk > 0 && (segments < 1 || segments > 65535 || !sums || !prods)))
+    if (form < WKV_TOKENS || form > WKV_STEP) ABK_REFUSE("wkv_scan: form %d is not built", form);
+    if (form == WKV_SEGMENTS && (chunk < 1 || segments < 1 || segments > 65535 || !sums || !prods))
         ABK_REFUSE("wkv_scan: %d segments of %d tokens", segments, chunk);
     cudaStream_t s = (cudaStream_t)stream;
-    if (blocks) {
+    if (form == WKV_BLOCKS) {
         // Columns a lane has: as few as leave an SM one CTA, else as many as a head uses. The makers' work is every CTA's own,
         // and an SM's CTAs share its issue slots. One prompt of 500, us a walk with 1, 2, 4: 40 heads of 64 65, 54, 61 (160,
         // 80, 40 CTAs), 16 heads of 64 44, 54, 61, 32 heads of 128 261, 162, 87, 16 of 256 484, 254, 142, 80 of 32 46, 37, 53;
@@ -775,8 +858,30 @@ extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at,
 #undef WB_LAUNCH
 #undef WB_LAUNCH_AS
     }
+    if (form == WKV_STEP) {
+        const bool pieces = dim % 4 == 0 && !((uintptr_t)state & 15);
+        const int wide = dim <= 32 ? 32 : 64;
+        const dim3 tiles((dim + wide - 1) / wide, n_heads, n_seqs);
+#define WST_LAUNCH_AS(T, LPR, ROWS)                                                                      \
+    do {                                                                                                 \
+        if (pieces) abk_launch(wkv_step_kernel<T, LPR, ROWS, true>, tiles, dim3(16 * LPR), 0, s, p);     \
+        else abk_launch(wkv_step_kernel<T, LPR, ROWS, false>, tiles, dim3(16 * LPR), 0, s, p);           \
+    } while (0)
+#define WST_LAUNCH(LPR, ROWS)                                       \
+    do {                                                            \
+        if (dtype == ABK_BF16) WST_LAUNCH_AS(__nv_bfloat16, LPR, ROWS); \
+        else WST_LAUNCH_AS(float, LPR, ROWS);                       \
+    } while (0)
+        if (dim <= 32) WST_LAUNCH(8, 2);
+        else if (dim <= 64) WST_LAUNCH(16, 4);
+        else if (dim <= 128) WST_LAUNCH(16, 8);
+        else WST_LAUNCH(16, 16);
+#undef WST_LAUNCH
+#undef WST_LAUNCH_AS
+        return ABK_LAUNCH_RESULT();
+    }
     const int cols = dim <= 32 ? 32 : 16;  // value columns a CTA has
-    dim3 grid((dim + cols - 1) / cols, n_heads, chunk > 0 ? segments : n_seqs);
+    dim3 grid((dim + cols - 1) / cols, n_heads, form == WKV_SEGMENTS ? segments : n_seqs);
 #define WS_LAUNCH_AS(T, PHASE)                                                                               \
     do {                                                                                                     \
         if (dim <= 16) abk_launch(wkv_scan_kernel<T, 4, 4, 32, 16, PHASE>, grid, dim3(128), 0, s, p);        \
@@ -790,7 +895,7 @@ extern "C" int abk_wkv_scan(const void *proj, long long ld, int dtype, int r_at,
         if (dtype == ABK_BF16) WS_LAUNCH_AS(__nv_bfloat16, PHASE); \
         else WS_LAUNCH_AS(float, PHASE);                        \
     } while (0)
-    if (chunk == 0) {
+    if (form != WKV_SEGMENTS) {
         WS_LAUNCH(0);
         return ABK_LAUNCH_RESULT();
     }

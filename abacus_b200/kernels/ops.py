@@ -1619,9 +1619,9 @@ def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, b
         o = (S + diag(bonus) k v^T)^T r;    S <- diag(exp(-exp(pre + w0))) S + k v^T
     proj [tokens, .] as stored: r, k, v of head h at columns r_at / k_at / v_at + h * dim; pre float32 [tokens, heads * dim];
     w0, bonus float32 [heads * dim]; state float32 [slots, heads, dim, dim] (key, value); out float32 [tokens, heads * dim].
-    A step of one token a sequence walks each sequence token by token; a step of prompts goes as wkv_form says, in segments
-    only with ws, a Workspace (the same numbers, summed in another order). Which way a step goes depends on its rows and
-    sequences alone, not on how long each sequence is; form pins it (tests)."""
+    A step of one token a sequence has a kernel of its own ("step"); a step of prompts goes as wkv_form says, in segments only
+    with ws, a Workspace (the same numbers, summed in another order). Which way a step goes depends on its rows and sequences
+    alone, not on how long each sequence is; form pins it (tests)."""
     _need_cuda(proj, pre, w0, bonus, state, out)
     lib = load_module("wkv")
     hk = n_heads * dim
@@ -1631,7 +1631,7 @@ def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, b
     assert proj.shape[1] >= max(r_at, k_at, v_at) + hk
     n_seqs = batch.seq_slot.numel()
     if form is None:
-        form = "tokens" if batch.is_decode or not 1 <= dim <= 256 else wkv_form(batch.n_rows, n_seqs, n_heads, dim)
+        form = "step" if batch.is_decode or not 1 <= dim <= 256 else wkv_form(batch.n_rows, n_seqs, n_heads, dim)
         if form == "segments" and ws is None:
             form = "blocks"
     segments, sums, prods = 0, None, None
@@ -1641,7 +1641,7 @@ def wkv_scan(proj, r_at, k_at, v_at, n_heads, dim, pre, w0, bonus, state, out, b
         prods = ws.get("wkv_prods", (segments, n_heads, dim), torch.float32)
     _check(lib, lib.abk_wkv_scan(_p(proj), _ll(proj.stride(0)), _i(_dt(proj)), _i(r_at), _i(k_at), _i(v_at), _i(n_heads), _i(dim),
                                  _p(pre), _p(w0), _p(bonus), _p(state), _p(out), _p(batch.seq_start), _p(batch.seq_slot),
-                                 _i(n_seqs), _i(1 if form == "blocks" else 0), _i(WKV_SEGMENT if segments else 0), _i(segments),
+                                 _i(n_seqs), _i(("tokens", "blocks", "segments", "step").index(form)), _i(WKV_SEGMENT), _i(segments),
                                  _p(sums), _p(prods), _stream()), "wkv_scan", kernels=3 if segments else 1)
 
 

@@ -57,10 +57,12 @@ def test_wkv_in_blocks(H, K, lens, shift):
     _wkv_against_64_bits(H, K, lens, shift, "blocks")
 
 
-@pytest.mark.parametrize("form", ["segments", "tokens"])
-@pytest.mark.parametrize("H,K,lens", [(2, 30, (130, 1, 64, 65, 200)), (3, 64, (63, 129)), (2, 100, (150,)), (1, 256, (70, 3)), (5, 8, (128,))])
+@pytest.mark.parametrize("form", ["segments", "tokens", "step"])
+@pytest.mark.parametrize("H,K,lens", [(2, 30, (130, 1, 64, 65, 200)), (3, 64, (63, 129)), (2, 100, (150,)), (1, 256, (70, 3)), (5, 8, (128,)),
+                                      (3, 36, (1, 5, 2)), (2, 132, (3, 1)), (4, 32, (1, 1, 2))])
 def test_wkv_in_segments_and_token_by_token(H, K, lens, form):
-    """Segments of 64 tokens that end with their prompt, short of it and a token beyond it, for every padded head size."""
+    """Segments of 64 tokens that end with their prompt, short of it and a token beyond it, for every padded head size; the kernel
+    for single tokens, whose tiles of columns end within a head (36, 100, 132) and which walks several tokens as well."""
     _wkv_against_64_bits(H, K, lens, 0, form)
 
 
@@ -71,6 +73,25 @@ def test_wkv_in_blocks_of_many_sequences(n_seqs):
     lens[3] = lens[40 % n_seqs] = lens[n_seqs - 1] = 13
     lens[7] = 0
     _wkv_against_64_bits(9, 20, lens, 0, "blocks")
+
+
+def test_single_wkv_tokens_have_a_kernel_of_their_own():
+    """A step of one token a sequence, twice as fast at least as the walk that prompts take, and the same numbers."""
+    from abacus_b200.engine.batch import Sequence, StepBatch
+    from abacus_b200.kernels import ops
+    n, H, K = 64, 40, 64
+    size = H * K
+    proj, pre = torch.randn((n, 3 * size), device=DEV).to(torch.bfloat16), torch.randn((n, size), device=DEV)
+    w0, bonus, first = torch.randn(size, device=DEV) - 2, torch.randn(size, device=DEV), torch.randn((n, H, K, K), device=DEV)
+    batch = StepBatch(n, n, 1, DEV).fill([Sequence(i, [0], 3, []) for i in range(n)], exact=True)
+    got, run = {}, lambda form, state, out: ops.wkv_scan(proj, 0, size, 2 * size, H, K, pre, w0, bonus, state, out, batch, form=form)
+    for form in (None, "tokens"):
+        got[form] = first.clone(), torch.empty((n, size), device=DEV)
+        run(form, *got[form])
+    # (sums of 64 products of values of around one in another order)
+    assert torch.equal(got[None][0], got["tokens"][0]) and float((got[None][1] - got["tokens"][1]).abs().max()) < 2.0 ** -24 * 64 * 64
+    times = us_of({form: lambda form=form: run(form, *got[form]) for form in got})
+    assert 2 * times[None] < times["tokens"], times
 
 
 def test_how_a_step_of_wkv_prompts_goes():
