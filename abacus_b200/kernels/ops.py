@@ -518,8 +518,8 @@ def attention_window_tc_wins(rows, n_seqs, n_heads, v_dim, window, chunk):
     40 prompts of 30 tokens and 32 heads of 128: 43 and 64, of 64 tokens 49 and 69 (of 80 tokens 86 and 85 with heads of 64); and few
     rows that see little, 512 tokens, 16 heads of 64, a window of 64: 14 and 17, of 128: 17.4 and 19.2; 2,048 tokens, 2 heads of 128,
     a window of 64: 17 and 19, 16 heads: 36 and 21. Chunks of up to a tile are that kernel's own tiles: 8 prompts of 257 tokens, 16
-    heads of 64, chunks of 64: 19 and 26 (one of 2,048: 18 and 16)."""
-    if (rows <= 64 * n_seqs and n_seqs * n_heads > 148) or (chunk and chunk <= 64 and rows <= 512 * n_seqs):
+    heads of 64, chunks of 64: 19 and 26; 2,048 tokens, 2 heads of 128: 11 and 16, 16 heads: 22 and 17."""
+    if (rows <= 64 * n_seqs and n_seqs * n_heads > 148) or (chunk and chunk <= 64 and (rows <= 512 * n_seqs or rows * n_heads <= 16384)):
         return False
     sees = min(window or rows, max(rows, 1))
     return not (sees * v_dim <= 8192 and rows >= 400 * n_seqs and sees * v_dim * rows * n_heads <= 77_500_000)
