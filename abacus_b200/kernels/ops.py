@@ -1603,7 +1603,7 @@ def wkv_form(rows, n_seqs, n_heads, dim):
     token by token where a step is small or its heads are (64 prompts of 8, 40 heads of 32: 20 us, in blocks 42; 16 tokens of 40
     heads of 64: 6.7 and 5.9). Blocks are one chain along a prompt, a number of us a token; segments twice the work and two
     kernels more, but all at once, and win where heads are few: one prompt of 2,000 tokens, us in blocks and in segments: 16 heads
-    of 30 124 and 50, 40 of 32 122 and 101, 80 of 32 149 and 189, 8 of 100 278 and 242, 16 of 64 164 and 160, 40 of 64 211 and
+    of 30 125 and 45, 40 of 32 123 and 84, 80 of 32 149 and 189, 8 of 100 278 and 242, 16 of 64 164 and 160, 40 of 64 211 and
     396. (Of several prompts the longest is taken for half as long again as they are on average.)"""
     if rows <= 8 * n_seqs and (rows < 128 or dim <= 32):
         return "tokens"
