@@ -13,7 +13,7 @@
 // sums a CTA's eight warps have them all of one tile, and meet at the end: a product of a few hundred rows has too few outputs
 // to fill 148 SMs with warps whose lanes hold enough of them. Shared memory gives a warp a number a lane and cycle, and an
 // SM's four schedulers share it; a lane with 16 x 8 outputs needs 24 numbers for 128 multiply-adds (0.75 of what the
-// schedulers could use up), one with 8 x 8 needs 16 for 64 (all of it). Measured (one launch, operands from HBM): 500 x 6144 x
+// schedulers could use up), one with 8 x 8 needs 16 for 64 (all of it). Measured (launches in a row): 500 x 6144 x
 // 1024 in 197 us and 500 x 1024 x 3072 in 97 (32 TFLOP/s; tiles of 64 x 64 of a whole CTA with one sum and 4 x 4 outputs a
 // lane: 322 and 220 us), 1 x 1024 x 3072 in 12 us (214). Multiply-adds of three registers alone run at 60 TFLOP/s here; the
 // rest goes to their registers' banks and to waiting for the next piece. Half the tile, twice the CTAs an SM: 259 and 134 us.
