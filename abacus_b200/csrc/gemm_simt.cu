@@ -1,11 +1,11 @@
-// out[M, N] = x[M, K] . w[N, K]^T with float32 multiply-adds on the CUDA cores, for any M, N, K.
+// out[M, N] = x[M, K] . w[N, K]^T with float32 multiply-adds, for any M, N, K.
 //
-// This is the matrix product of the true 32-bit path (no tensor cores, no TF32), and the
-// fallback of the bfloat16 path for shapes the tensor-core kernel refuses. An output element is the sum of eight running
+// This is the matrix product of the true 32-bit path (no TF32), and the fallback of the bfloat16 path for shapes the tensor-core
+// kernel refuses. Large float32 products go to the tensor cores without a digit less (gemm_split.cuh); here an output element is the sum of eight running
 // sums: K in pieces of 16, piece c to sum c % 8, each sum over its k in ascending order, then in pairs,
 // ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); up to K = 256 it is one sum over k in ascending order (a chain of that
 // length needs no cutting, and the small products of small models keep the order they had). So a row's result does not
-// depend on how many other rows are in the batch or where its tile lies.
+// depend on where its tile lies, nor on how many other rows are in the batch as long as the product goes the same way.
 // Formula: src/model.c:299, 302, 307, 309, 324 (weights are [out, in] row-major, no bias).
 //
 // A warp has one tile of outputs and one of their sums. It stages its own pieces, 16 bytes at a time by cp.async (rows of 20
@@ -22,6 +22,7 @@
 // 3.6 (a CTA's tile of 64 x 64 and 4 x 4 outputs a lane: 98, 52 and 10.8; one warp of eight of a CTA of 160 KB: 330, 184 and 26).
 #define ABK_DEFINE_ERROR
 #include "common.cuh"
+#include "gemm_split.cuh"
 
 #define GS_WARPS 8      // of a CTA that cuts its sums
 #define GS_BK 16
@@ -174,14 +175,36 @@ static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int 
     return ABK_LAUNCH_RESULT();
 }
 
+// The product on the tensor cores (gemm_split.cuh), float32 operands and results. bn: rows of x in a tile (32, 64, 96, 128), quarters: pairs
+// of CTAs take quarters of K; 0, 0: by size.
+extern "C" int abk_gemm_split(const void *x, const void *w, void *out, int M, int N, int K, long long ldx, long long ldw, long long ldo, int bn,
+                              int quarters, void *scratch, int *status, void *stream) {
+    const GemmSplit g = {x, w, out, ABK_F32, ABK_F32, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};
+    return gemm_split_run<float>(g, bn, quarters, scratch, (cudaStream_t)stream);
+}
+
+// Whether a product goes to the tensor cores: more than a handful of rows (up to 32 rows the plain kernel reads the weights once and writes nothing beside: 17 x 6144 x 1024 in 19 us
+// against 23), and enough to do: a long K, which is a chain in the plain kernel (33 x 64 x 2560: 28 us, in parts 17), or a hundred
+// million multiply-adds (64 x 1024 x 1024: 13.4 against 12.8; 500 x 256 x 512: 7.9 against 10.3; 1000 x 256 x 512: 12.6 and 12.1).
+static bool gemm_split_wins(int M, int N, int K) { return M > 32 && N >= 64 && K >= 512 && (K >= 2048 || (long long)M * N * K >= 100000000LL); }
+// Bytes of scratch memory with which abk_gemm_simt goes to the tensor cores (0: it does not).
+extern "C" long long abk_gemm_simt_scratch(int M, int N, int K) { return gemm_split_wins(M, N, K) ? gemm_split_scratch(M, N, K) : 0; }
+
 // x_dtype/w_dtype/out_dtype: ABK_F32 or ABK_BF16. Supported: all-float32; bf16 x and w with bf16 or f32 out.
+// scratch: at least abk_gemm_simt_scratch bytes, or null (then every product runs on the CUDA cores); status: int32 [>= 2], word 1
+// is set if a wait ran out.
 extern "C" int abk_gemm_simt(const void *x, int x_dtype, const void *w, int w_dtype, void *out, int out_dtype, int M,
-                             int N, int K, long long ldx, long long ldw, long long ldo, void *stream) {
+                             int N, int K, long long ldx, long long ldw, long long ldo, void *scratch, long long scratch_bytes, int *status,
+                             void *stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) ABK_REFUSE("gemm: K = %d", K);
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
     if (N > 65535 * 64) ABK_REFUSE("gemm: %d output columns are more than one launch takes", N);
+    if (scratch && x_dtype == w_dtype && (x_dtype == ABK_BF16 || out_dtype == ABK_F32) && gemm_split_wins(M, N, K) && scratch_bytes >= gemm_split_scratch(M, N, K)) {
+        const GemmSplit g = {x, w, out, x_dtype, out_dtype, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};
+        return x_dtype == ABK_F32 ? gemm_split_run<float>(g, 0, 0, scratch, s) : gemm_split_run<bf>(g, 0, 0, scratch, s);
+    }
     const bool one = K <= GS_ONE_SUM;
     const long long large = ((M + 63LL) / 64) * ((N + 63LL) / 64), small = ((M + 15LL) / 16) * ((N + 15LL) / 16), sms = abk_sm_count();
     // Eight sums: tiles of 64 x 64 where they fill two thirds of the SMs, else of 32 x 32 (of 16 x 16 for up to 16 rows): 64 x

@@ -1,0 +1,405 @@
+// out[M, N] = x[M, K] . w[N, K]^T of float32 operands on the tensor cores, with no digit of float32 given up.
+//
+// A float32 number is the sum of three bfloat16 numbers (8 + 8 + 8 bits, each rounded to nearest: what is left over is below
+// 2^-26 of it), x = x1 + x2 + x3, so x w is the six products x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1; the three left out are
+// below 2^-26. The tensor cores multiply bfloat16 without rounding and add in float32, but cut a sum off where float32
+// rounds it, and a sum over a long K cut off at every step drifts towards zero. So x1 w1 is added up in tensor memory over 128
+// of K only; these short sums are added in registers, rounded. The five small products have an accumulator of their own, whose
+// cuts are 2^-8 as large.
+//
+// An element is the sum of four running sums, over the quarters of K in order: ((q0 + q1) + q2) + q3, each over its pieces of
+// 128 in order, then its small products. That order goes by K alone: a row's result does not depend on how many other rows
+// are in the batch, whether a pair of CTAs walks all of K or a quarter, or where its tile lies.
+// bfloat16 operands (those that the tensor-core product proper refuses: rows that start anywhere) go the same way with one part.
+// A number that is not finite makes its products NaN in this form; an element that came out not finite is taken again with
+// plain multiply-adds. (Numbers below 1e-33 keep fewer digits: their third part is too small for bfloat16.)
+//
+// What bounds it: for thousands of rows the tensor cores under the power cap (4000 x 6144 x 1024 in 258 us, 1,230 TFLOP/s of bfloat16 products
+// at 1.63 GHz; on the CUDA cores 1,349), for some hundred the way of the parts from the L2, 6 bytes a number, at some 30 bytes
+// a cycle and SM, and the pieces that the last turn leaves empty (500 x 6144 x 1024 in 53 us, 9 of them for the parts; 195 on the
+// CUDA cores). Errors against 64 bits (2-norm, normal numbers): 1.3e-7 for K from 512 to 3072, where eight float32 sums have 1.5e-7
+// to 3.5e-7.
+//
+// Two kernels: one writes the operands' parts as three planes of bfloat16 each, the other multiplies them on pairs of CTAs. (As one kernel
+// that splits what it fetches, weights again for every column of tiles: 500 x 6144 x 1024 in 71 us, bound by the instructions
+// of the splitting and by the way of plain loads through what the stages leave of the L1.)
+#pragma once
+#include "tc_common.cuh"
+#include "tensor_map.cuh"
+
+#define GP_ADDERS 16                      // warps that add up what the tensor cores leave
+#define GP_THREADS (32 * GP_ADDERS + 64)  // one that loads, one that multiplies
+#define GP_ROWS 128                       // weight rows of a CTA: the accumulators' lanes
+#define GP_K 64                           // of K at a time
+#define GP_QUARTERS 4
+
+// BN: rows of x in a tile of a pair of CTAs; each brings half of them.
+template <int BN> struct GpShape {
+    static constexpr int STAGES = 3, X_ROWS = BN / 2;
+    static constexpr int W_PLANE = GP_ROWS * GP_K * 2, X_PLANE = X_ROWS * GP_K * 2, STAGE = 3 * (W_PLANE + X_PLANE);
+    static constexpr int BYTES = STAGES * STAGE + 1024 /* alignment */ + 256 /* barriers */;
+    static constexpr int TMEM = BN == 96 ? 512 : 4 * BN;  // two accumulators of x1 w1 and two of the small products
+    static constexpr int COLS = BN / 4;                   // of the accumulator that a warp adds up
+};
+
+template <int N> __device__ __forceinline__ void gp_tmem_ld(uint32_t taddr, uint32_t *v);
+template <> __device__ __forceinline__ void gp_tmem_ld<8>(uint32_t taddr, uint32_t *v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
+}
+
+// Two numbers as three pairs of bfloat16 (the lower half of a word: the first number).
+__device__ __forceinline__ void gp_split(float a, float b, uint32_t &p1, uint32_t &p2, uint32_t &p3) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(b), "f"(a));
+    a -= __uint_as_float(p1 << 16), b -= __uint_as_float(p1 & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(b), "f"(a));
+    a -= __uint_as_float(p2 << 16), b -= __uint_as_float(p2 & 0xffff0000u);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p3) : "f"(b), "f"(a));
+}
+
+// ------------------------------------------------------------------ the parts of the operands
+// Rows of `k` numbers, `ld` apart, as planes [rows][pitch] of bfloat16 (pitch: k up to a multiple of 8): three of float32 numbers, one of
+// bfloat16 ones, which only get rows that TMA takes.
+struct SplitRows {
+    const void *from;
+    __nv_bfloat16 *to;
+    long long ld;
+    int rows, vec;  // vec: the rows start on 16-byte boundaries, float32 ones of a multiple of four numbers
+};
+// Bound by memory: 4 bytes read and 6 written a number (6,644 rows of 1,024: 8.9 us). A thread has eight numbers of a row.
+template <typename T> __global__ void __launch_bounds__(256) gemm_split_rows_kernel(SplitRows a, SplitRows b, int k, int pitch) {
+    const int pieces = pitch / 8;
+    pdl_wait();
+    const long long na = (long long)a.rows * pieces, n = na + (long long)b.rows * pieces;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const bool first = i < na;
+        const SplitRows &o = first ? a : b;
+        const long long j = first ? i : i - na, row = j / pieces;
+        const int c = (int)(j - row * pieces) * 8;
+        const T *from = (const T *)o.from + row * o.ld + c;
+        __nv_bfloat16 *to = o.to + row * pitch + c;
+        T v[8];
+        if (sizeof(T) == 4 && o.vec) {
+            *(float4 *)v = *(const float4 *)from;
+            *(float4 *)(v + 4) = c + 4 < k ? *(const float4 *)(from + 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = c + e < k ? from[e] : from_float<T>(0.0f);
+        }
+        if constexpr (sizeof(T) == 4) {
+            uint4 p1, p2, p3;
+            gp_split(v[0], v[1], p1.x, p2.x, p3.x), gp_split(v[2], v[3], p1.y, p2.y, p3.y);
+            gp_split(v[4], v[5], p1.z, p2.z, p3.z), gp_split(v[6], v[7], p1.w, p2.w, p3.w);
+            const long long plane = (long long)o.rows * pitch;
+            *(uint4 *)to = p1, *(uint4 *)(to + plane) = p2, *(uint4 *)(to + 2 * plane) = p3;
+        } else {
+            uint32_t word[4];
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                const __nv_bfloat162 two = __halves2bfloat162(v[e], v[e + 1]);
+                word[e / 2] = *(const uint32_t *)&two;
+            }
+            *(uint4 *)to = make_uint4(word[0], word[1], word[2], word[3]);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ the product
+struct GemmSplit {
+    const void *x, *w;
+    void *out;
+    int dtype, out_dtype;  // of x and w, ABK_F32 (three parts) or ABK_BF16 (one); of out
+    int M, N, K, m_tiles, tiles;
+    long long ldx, ldw, ldo;
+    int *status;
+    float *quarters;  // [GP_QUARTERS][M][N]
+};
+
+template <typename T> __device__ __noinline__ float gp_plain(const T *x, const T *w, int K) {
+    float s = 0.0f;
+    for (int k = 0; k < K; k++) s = fmaf(to_float(x[k]), to_float(w[k]), s);
+    return s;
+}
+// An element's place in `out`, with the sum v, or, where that is not finite, with plain multiply-adds.
+__device__ __forceinline__ void gp_put(const GemmSplit &g, int m, int n, float v) {
+    if (!isfinite(v))
+        v = g.dtype == ABK_F32 ? gp_plain((const float *)g.x + m * g.ldx, (const float *)g.w + n * g.ldw, g.K)
+                               : gp_plain((const __nv_bfloat16 *)g.x + m * g.ldx, (const __nv_bfloat16 *)g.w + n * g.ldw, g.K);
+    if (g.out_dtype == ABK_F32) ((float *)g.out)[m * g.ldo + n] = v;
+    else ((__nv_bfloat16 *)g.out)[m * g.ldo + n] = __float2bfloat16_rn(v);
+}
+
+// A tile is 256 rows of w (128 of each CTA) and BN rows of x; pair c of CTAs takes items c, c + pairs, ... An item is a tile, or
+// (QUARTERS) a quarter of K of one, whose sums go to `quarters` and are added up by the kernel behind.
+// map_w, map_x: the planes, one below the other.
+template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w,
+                                                                                               const __grid_constant__ CUtensorMap map_x, GemmSplit g) {
+    using S = GpShape<BN>;
+    constexpr int STAGES = S::STAGES, COLS = S::COLS;
+    extern __shared__ uint8_t gp_smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)gp_smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t *full = (uint64_t *)(smem + STAGES * S::STAGE), *empty = full + STAGES;
+    uint64_t *sum_ready = empty + STAGES, *sum_free = sum_ready + 2, *small_free = sum_free + 2;
+    uint32_t *tmem_holder = (uint32_t *)(small_free + 2);
+    volatile int *gave_up = (volatile int *)(tmem_holder + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t half = tc::cluster_rank();  // 0: the leader
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; s++) tc::mbar_init(&full[s], 1), tc::mbar_init(&empty[s], 1);
+        // sum_free, small_free: every adding warp of both CTAs, on the leader's
+        for (int b = 0; b < 2; b++) tc::mbar_init(&sum_ready[b], 1), tc::mbar_init(&sum_free[b], 2 * GP_ADDERS), tc::mbar_init(&small_free[b], 2 * GP_ADDERS);
+        *gave_up = 0;
+        tc::mbar_init_fence();
+        tc::tma_prefetch_map(&map_w), tc::tma_prefetch_map(&map_x);
+    }
+    if (warp == GP_ADDERS) tc::tmem_alloc_pair(tmem_holder, S::TMEM);
+    tc::fence_before_sync();
+    tc::cluster_sync();
+    tc::fence_after_sync();
+    const uint32_t tmem = *tmem_holder;
+
+    const int pieces = (g.K + GP_K - 1) / GP_K, parts = g.dtype == ABK_F32 ? 3 : 1;
+    const int items = QUARTERS ? g.tiles * GP_QUARTERS : g.tiles, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const auto first_quarter = [&](int item) { return QUARTERS ? item / g.tiles : 0; };
+    const auto last_quarter = [&](int item) { return QUARTERS ? item / g.tiles : GP_QUARTERS - 1; };
+    const auto tile_of = [&](int item) { return QUARTERS ? item % g.tiles : item; };
+    const auto begin_of = [&](int quarter) { return (int)((long long)pieces * quarter / GP_QUARTERS); };
+    if (warp == GP_ADDERS) {
+        if (lane == 0) {
+            pdl_wait();
+            int i = 0;
+            bool ok = true;
+            for (int item = pair; ok && item < items; item += pairs) {
+                const int tile = tile_of(item), m0 = tile % g.m_tiles * BN + half * S::X_ROWS, n0 = (tile / g.m_tiles * 2 + half) * GP_ROWS;
+                const int end = begin_of(last_quarter(item) + 1);
+                for (int p = begin_of(first_quarter(item)); p < end; p++, i++) {
+                    const int s = i % STAGES;
+                    if (i >= STAGES && !tc::mbar_wait(&empty[s], ((i / STAGES) & 1) ^ 1)) {
+                        ok = false;
+                        break;
+                    }
+                    if (half == 0) tc::mbar_expect_tx(&full[s], parts * 2 * (S::W_PLANE + S::X_PLANE));  // both CTAs' copies report to the leader
+                    const uint32_t bar = tc::peer_smem(tc::smem_addr(&full[s]), 0);
+                    uint8_t *stage = smem + s * S::STAGE;
+                    for (int t = 0; t < parts; t++) {
+                        tc::tma_load_2d_pair(stage + t * S::W_PLANE, &map_w, p * GP_K, t * g.N + n0, bar);
+                        tc::tma_load_2d_pair(stage + 3 * S::W_PLANE + t * S::X_PLANE, &map_x, p * GP_K, t * g.M + m0, bar);
+                    }
+                }
+            }
+            if (!ok) *gave_up = 1;
+        }
+        __syncwarp();
+    } else if (warp == GP_ADDERS + 1) {
+        if (lane == 0 && half == 0) {
+            constexpr uint32_t idesc = tc::idesc_bf16_f32(2 * GP_ROWS, BN);
+            int i = 0, sum_i = 0, quarter_i = 0;  // pieces, sums and quarters so far
+            bool ok = true;
+            for (int item = pair; ok && item < items; item += pairs) {
+                for (int q = first_quarter(item); ok && q <= last_quarter(item); q++, quarter_i++) {
+                    const int q_begin = begin_of(q), q_end = begin_of(q + 1);
+                    ok = quarter_i < 2 || tc::mbar_wait(&small_free[quarter_i & 1], ((quarter_i >> 1) & 1) ^ 1);
+                    for (int p = q_begin; ok && p < q_end; p++, i++) {
+                        const int s = i % STAGES, b = sum_i & 1;
+                        const bool starts = ((p - q_begin) & 1) == 0, ends = !starts || p + 1 == q_end;
+                        if (starts) ok = sum_i < 2 || tc::mbar_wait(&sum_free[b], ((sum_i >> 1) & 1) ^ 1);
+                        ok = ok && tc::mbar_wait(&full[s], (i / STAGES) & 1);
+                        if (!ok) break;
+                        tc::fence_after_sync();
+                        const uint32_t at = tc::smem_addr(smem + s * S::STAGE);
+                        const uint64_t w1 = tc::smem_desc_k_sw128(at), w2 = w1 + (S::W_PLANE >> 4), w3 = w2 + (S::W_PLANE >> 4);
+                        const uint64_t x1 = w3 + (S::W_PLANE >> 4), x2 = x1 + (S::X_PLANE >> 4), x3 = x2 + (S::X_PLANE >> 4);
+                        const uint32_t sum = tmem + b * BN, small = tmem + (2 + (quarter_i & 1)) * BN;
+#pragma unroll
+                        for (int k = 0; k < GP_K / 16; k++) {  // (16 of K: 32 bytes of a row)
+                            tc::mma_ss_pair(sum, w1 + 2 * k, x1 + 2 * k, idesc, !starts || k > 0);
+                            if (parts == 1) continue;
+                            tc::mma_ss_pair(small, w1 + 2 * k, x2 + 2 * k, idesc, p > q_begin || k > 0);
+                            tc::mma_ss_pair(small, w2 + 2 * k, x1 + 2 * k, idesc, true);
+                            tc::mma_ss_pair(small, w2 + 2 * k, x2 + 2 * k, idesc, true);
+                            tc::mma_ss_pair(small, w1 + 2 * k, x3 + 2 * k, idesc, true);
+                            tc::mma_ss_pair(small, w3 + 2 * k, x1 + 2 * k, idesc, true);
+                        }
+                        tc::mma_commit_pair(&empty[s]);
+                        if (ends) tc::mma_commit_pair(&sum_ready[b]), sum_i++;
+                    }
+                }
+            }
+            if (!ok) *gave_up = 1;
+        }
+        __syncwarp();
+    } else {
+        pdl_wait();
+        // a warp has a quarter of the lanes (the weights' rows) and COLS columns (rows of x) of the accumulators
+        const int lane_base = (warp & 3) * 32, col0 = (warp >> 2) * COLS;
+        const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + col0;
+        float sum[COLS], total[COLS];
+#pragma unroll
+        for (int j = 0; j < COLS; j++) sum[j] = total[j] = 0.0f;
+        int sum_i = 0, quarter_i = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int item = pair; ok && item < items; item += pairs) {
+#pragma unroll 1
+            for (int q = first_quarter(item); q <= last_quarter(item); q++, quarter_i++) {
+                const int sums = (begin_of(q + 1) - begin_of(q) + 1) / 2;
+#pragma unroll 1
+                for (int n = 0; n < sums; n++, sum_i++) {
+                    const int b = sum_i & 1;
+                    ok = __all_sync(0xffffffffu, ok && tc::mbar_wait(&sum_ready[b], (sum_i >> 1) & 1));
+                    tc::fence_after_sync();
+                    uint32_t v[8];
+#pragma unroll
+                    for (int c = 0; c < COLS; c += 8) {
+                        gp_tmem_ld<8>(taddr + b * BN + c, v);
+                        tc::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 8; j++) sum[c + j] += __uint_as_float(v[j]);
+                    }
+                    if (n + 1 == sums) {
+#pragma unroll
+                        for (int c = 0; c < COLS; c += 8) {
+                            gp_tmem_ld<8>(taddr + (2 + (quarter_i & 1)) * BN + c, v);
+                            tc::tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 8; j++) total[c + j] += sum[c + j] + (parts == 1 ? 0.0f : __uint_as_float(v[j])), sum[c + j] = 0.0f;
+                        }
+                    }
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tc::mbar_arrive_in_cluster(tc::peer_smem(tc::smem_addr(&sum_free[b]), 0));
+                        if (n + 1 == sums) tc::mbar_arrive_in_cluster(tc::peer_smem(tc::smem_addr(&small_free[quarter_i & 1]), 0));
+                    }
+                }
+            }
+            if (ok) {
+                const int tile = tile_of(item), m0 = tile % g.m_tiles * BN + col0, n = (tile / g.m_tiles * 2 + half) * GP_ROWS + lane_base + lane;
+                const int cols = n < g.N ? g.M - m0 : 0;
+                if constexpr (QUARTERS) {
+                    float *out = g.quarters + ((long long)first_quarter(item) * g.M + m0) * g.N + n;
+#pragma unroll
+                    for (int j = 0; j < COLS; j++)
+                        if (j < cols) out[(long long)j * g.N] = total[j];
+                } else {
+#pragma unroll
+                    for (int j = 0; j < COLS; j++)
+                        if (j < cols) gp_put(g, m0 + j, n, total[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < COLS; j++) total[j] = 0.0f;
+            }
+        }
+        if (!ok) *gave_up = 1;
+    }
+    tc::fence_before_sync();
+    tc::cluster_sync();  // (the pair's other CTA is done with this one's memory and barriers)
+    if (*gave_up && threadIdx.x == 0) atomicOr(g.status + 1, 1);
+    if (warp == GP_ADDERS) {
+        tc::fence_after_sync();
+        tc::tmem_free_pair(tmem, S::TMEM);
+    }
+}
+
+// The four quarters' sums of every element, in order.
+__global__ void __launch_bounds__(256) gemm_split_sum_kernel(GemmSplit g) {
+    pdl_wait();
+    const long long n = (long long)g.M * g.N;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const int row = (int)(i / g.N), col = (int)(i - (long long)row * g.N);
+        gp_put(g, row, col, ((g.quarters[i] + g.quarters[i + n]) + g.quarters[i + 2 * n]) + g.quarters[i + 3 * n]);
+    }
+}
+
+template <int BN, bool QUARTERS> static int gemm_split_launch(const CUtensorMap &map_w, const CUtensorMap &map_x, GemmSplit g, cudaStream_t s) {
+    using S = GpShape<BN>;
+    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_split_kernel<BN, QUARTERS>, S::BYTES);
+    if (e != cudaSuccess) return (int)e;
+    const int pairs = abk_sm_count() / 2, items = QUARTERS ? g.tiles * GP_QUARTERS : g.tiles;
+    abk_launch_clusters(gemm_split_kernel<BN, QUARTERS>, dim3(2 * (items < pairs ? items : pairs)), dim3(GP_THREADS), S::BYTES, s, 2, map_w, map_x, g);
+    const int rc = ABK_LAUNCH_RESULT();
+    if (rc || !QUARTERS) return rc;
+    const long long blocks = ((long long)g.M * g.N + 255) / 256, most = 8LL * abk_sm_count();
+    abk_launch(gemm_split_sum_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s, g);
+    return ABK_LAUNCH_RESULT();
+}
+
+#define GP_QUARTERS_BYTES (64LL << 20)  // sums of quarters in the scratch memory at most
+static bool gp_may_quarter(int M, int N) { return 4LL * GP_QUARTERS * M * N <= GP_QUARTERS_BYTES; }
+
+// Rows of x in a tile, and whether pairs of CTAs take quarters of K: what takes least, by turns of the GPU's pairs times what a
+// piece of 64 of K takes (measured with a turn each: 1.0 us for tiles of 32 rows, 1.05, 1.15, 1.25 for 128: the way from the L2
+// counts for more than the products, 1,104 to 1,536 cycles), and the passes over the quarters' sums. 500 x 6144 x 1024 in tiles of 96:
+// 53 us, of 128: 55, of 64: 69, in quarters 69; 500 x 1024 x 3072 in quarters with tiles of 128: 30 us, of 64: 42, whole: 65.
+static void gp_choose(int M, int N, int K, bool may_quarter, int &bn, int &quarters) {
+    static const struct { int bn; float us; } tile[4] = {{32, 1.0f}, {64, 1.05f}, {96, 1.15f}, {128, 1.25f}};
+    const long long pairs = abk_sm_count() / 2;
+    const float pieces = (float)((K + GP_K - 1) / GP_K);
+    float best = 0.0f;
+    bn = 0;
+    for (const auto &t : tile) {
+        const long long tiles = ((long long)M + t.bn - 1) / t.bn * ((N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
+        for (int q = 0; q < (may_quarter ? 2 : 1); q++) {
+            const float us = q ? (float)((tiles * GP_QUARTERS + pairs - 1) / pairs) * pieces / GP_QUARTERS * t.us + 3.0f + (float)M * (float)N * 6.4e-6f
+                               : (float)((tiles + pairs - 1) / pairs) * pieces * t.us;
+            if (bn == 0 || us < best) best = us, bn = t.bn, quarters = q;
+        }
+    }
+}
+
+// The parts of this many numbers of an operand at most lie in the scratch memory at a time (96 MB); larger products go slab by slab.
+#define GP_SLAB (16 << 20)
+static int gp_slab_rows(int rows, int K, int multiple) {
+    const int most = GP_SLAB / K / multiple * multiple;
+    return rows < most ? rows : most > multiple ? most : multiple;
+}
+static long long gp_planes(int rows, int K) {  // bytes, up to a multiple of 1024
+    return (3LL * rows * ((K + 7) / 8 * 8) * 2 + 1023) / 1024 * 1024;
+}
+static long long gemm_split_scratch(int M, int N, int K) {
+    const int n_slab = gp_slab_rows(N, K, 256), m_slab = gp_slab_rows(M, K, 128);
+    return gp_planes(n_slab, K) + gp_planes(m_slab, K) + (gp_may_quarter(m_slab, n_slab) ? 4LL * GP_QUARTERS * m_slab * n_slab : 0) + 1024;
+}
+
+// Where bn is 0 the sizes choose it and whether K is walked in quarters.
+template <typename T> static int gemm_split_run(GemmSplit g, int bn, int quarters, void *scratch, cudaStream_t s) {
+    const int pitch = (g.K + 7) / 8 * 8, n_slab = gp_slab_rows(g.N, g.K, 256), m_slab = gp_slab_rows(g.M, g.K, 128), M = g.M, N = g.N;
+    const int parts = sizeof(T) == 4 ? 3 : 1, out_size = g.out_dtype == ABK_F32 ? 4 : 2;
+    __nv_bfloat16 *const w_planes = (__nv_bfloat16 *)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
+    __nv_bfloat16 *const x_planes = w_planes + gp_planes(n_slab, g.K) / 2;
+    g.quarters = (float *)(x_planes + gp_planes(m_slab, g.K) / 2);
+    const T *const x = (const T *)g.x, *const w = (const T *)g.w;
+    char *const out = (char *)g.out;
+    const bool may_quarter = gp_may_quarter(m_slab, n_slab);
+    const auto vec = [&](const T *from, long long ld) { return sizeof(T) == 4 && g.K % 4 == 0 && ld % 4 == 0 && !((uintptr_t)from & 15); };
+    for (int m = 0; m < M; m += m_slab)
+        for (int n = 0; n < N; n += n_slab) {
+            g.M = M - m < m_slab ? M - m : m_slab, g.N = N - n < n_slab ? N - n : n_slab;
+            g.x = x + m * g.ldx, g.w = w + n * g.ldw, g.out = out + (m * g.ldo + n) * out_size;
+            const SplitRows rows_w = {g.w, w_planes, g.ldw, g.N, vec((const T *)g.w, g.ldw)};
+            const SplitRows rows_x = {g.x, x_planes, g.ldx, n == 0 ? g.M : 0, vec((const T *)g.x, g.ldx)};
+            const long long pieces = ((long long)rows_w.rows + rows_x.rows) * (pitch / 8), blocks = (pieces + 255) / 256, most = 16LL * abk_sm_count();
+            abk_launch(gemm_split_rows_kernel<T>, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s, rows_w, rows_x, g.K, pitch);
+            int rc = ABK_LAUNCH_RESULT();
+            if (rc) return rc;
+            int b = bn, in_quarters = quarters;
+            if (!b) gp_choose(g.M, g.N, g.K, may_quarter, b, in_quarters);
+            if (in_quarters && !may_quarter) ABK_REFUSE("gemm: no room for the quarters of %d x %d sums", g.M, g.N);
+            g.m_tiles = (g.M + b - 1) / b, g.tiles = g.m_tiles * ((g.N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
+            CUtensorMap map_w, map_x;
+            if ((rc = tmap::bf16_rows_of_128_bytes(w_planes, (long long)parts * g.N, g.K, pitch, GP_ROWS, &map_w))) return rc;
+            if ((rc = tmap::bf16_rows_of_128_bytes(x_planes, (long long)parts * g.M, g.K, pitch, b / 2, &map_x))) return rc;
+#define GP_CASE(BN) \
+    case BN: rc = in_quarters ? gemm_split_launch<BN, true>(map_w, map_x, g, s) : gemm_split_launch<BN, false>(map_w, map_x, g, s); break
+            switch (b) {
+                GP_CASE(32);
+                GP_CASE(64);
+                GP_CASE(96);
+                GP_CASE(128);
+                default: ABK_REFUSE("gemm: tiles of %d rows are not built", b);
+            }
+#undef GP_CASE
+            if (rc) return rc;
+        }
+    return 0;
+}

@@ -29,7 +29,7 @@ typedef int (*QkvPrepFn)(void *, int, int, int, int, int, int, const int *, cons
                          const float *, const float *, float, const float *, const float *, int, int, void *, void *,
                          const int *, int, int, int, void *);
 typedef int (*GemmSimtFn)(const void *, int, const void *, int, void *, int, int, int, int, long long, long long, long long,
-                          void *);
+                          void *, long long, int *, void *);
 typedef int (*GemmRowsFn)(const void *, const void *, void *, int, int, int, int, long long, long long, long long, void *);
 typedef int (*GemmRowsSwigluFn)(const void *, const void *, void *, int, int, int, long long, long long, long long, int,
                                 void *);
@@ -138,7 +138,8 @@ struct AbkStep {
     const AbkLists *lists;
     float *x, *branch, *logits, *attention_partials;  // workspace: the stream, a branch's output, logits, decode partials
     void *xn, *qkv, *att, *act, *gate_up, *xn_final;
-    long long partial_floats;
+    void *parts;  // scratch memory of the float32 products (abk_gemm_simt_scratch)
+    long long partial_floats, parts_bytes;
     int n_rows, n_logit_rows, is_decode, any_continuation, max_len_after, position_bound, n_lists, pad;
 };
 
@@ -185,7 +186,7 @@ static bool tc_takes(const void *x, long long ldx, const AbkLinear &l) {
 }
 
 // parts/linear.py: Linear.forward. out[:rows] = x[:rows] . w^T; x in the model's dtype.
-static int linear(const AbkModel &m, const AbkLinear &l, const void *x, long long ldx, void *out, int out_dtype, long long ldo,
+static int linear(const AbkModel &m, const AbkStep &s, const AbkLinear &l, const void *x, long long ldx, void *out, int out_dtype, long long ldo,
                   int rows, void *stream) {
     const AbkFns &f = *m.fns;
     if (l.dtype == ABK_BF16 && rows_kernel_wins(rows, l, false) && rows_takes(x, ldx, l, rows))
@@ -193,7 +194,8 @@ static int linear(const AbkModel &m, const AbkLinear &l, const void *x, long lon
     if (tc_takes(x, ldx, l))
         return LAUNCH(f.gemm_tc, x, l.w, out, out_dtype, rows, l.n, l.k, ldx, l.ldw, ldo, m.gemm_scratch, m.gemm_tickets,
                          m.kernel_status, 0, -1, 0, -1, stream);
-    return LAUNCH(f.gemm_simt, x, m.dtype, l.w, l.dtype, out, out_dtype, rows, l.n, l.k, ldx, l.ldw, ldo, stream);
+    return LAUNCH(f.gemm_simt, x, m.dtype, l.w, l.dtype, out, out_dtype, rows, l.n, l.k, ldx, l.ldw, ldo, s.parts, s.parts_bytes,
+                  m.kernel_status, stream);
 }
 
 static size_t esize(int dtype) { return dtype == ABK_BF16 ? 2 : 4; }
@@ -218,8 +220,8 @@ static int attention(const AbkModel &m, const AbkAttention &a, const AbkEntry &e
                    s.token_seq, s.token_pos, s.seq_slot, a.q_norm, a.k_norm, a.eps, a.cos, a.sin, e.k, e.v, e.table, e.table_width,
                    e.tokens_per_page, m.kernel_status, stream),
             "the q/k/v product");
-    else if (writes) TRY(linear(m, a.qkv, s.xn, m.hidden, s.qkv, m.dtype, row, n, stream), "the q/k/v product");
-    else TRY(linear(m, a.q_only, s.xn, m.hidden, s.qkv, m.dtype, row, n, stream), "the q product");
+    else if (writes) TRY(linear(m, s, a.qkv, s.xn, m.hidden, s.qkv, m.dtype, row, n, stream), "the q/k/v product");
+    else TRY(linear(m, s, a.q_only, s.xn, m.hidden, s.qkv, m.dtype, row, n, stream), "the q product");
     const size_t decode_smem = (size_t)4 * 64 * hd * 2 + (size_t)4 * group * (hd + 2) * 4 + 64;
     const bool decode_takes = has_cache && (hd == 64 || hd == 128 || hd == 256) && e.tokens_per_page == 64 && decode_smem <= 200 * 1024;
     // kernels/ops.py: attention_decode_prepares
@@ -281,7 +283,7 @@ static int attention(const AbkModel &m, const AbkAttention &a, const AbkEntry &e
                                 has_cache ? e.ring_pages : 0, has_cache ? e.tokens_per_page : 1, k_step, v_step, row, stream),
             "attention");
     }
-    TRY(linear(m, a.o, s.att, q_size, s.branch, ABK_F32, m.hidden, n, stream), "the output product");
+    TRY(linear(m, s, a.o, s.att, q_size, s.branch, ABK_F32, m.hidden, n, stream), "the output product");
     return STEP_OK;
 }
 
@@ -299,10 +301,10 @@ static int gated_mlp(const AbkModel &m, const AbkMlp &p, const AbkStep &s, int e
         TRY(LAUNCH(f.gemm_tc_swiglu, s.xn, gu.w, s.act, n, p.inter, gu.k, m.hidden, gu.ldw, p.inter, m.kernel_status, stream),
             "gate/up with SwiGLU");
     } else {
-        TRY(linear(m, gu, s.xn, m.hidden, s.gate_up, m.dtype, 2ll * p.inter, n, stream), "the gate/up product");
+        TRY(linear(m, s, gu, s.xn, m.hidden, s.gate_up, m.dtype, 2ll * p.inter, n, stream), "the gate/up product");
         TRY(LAUNCH(f.swiglu, s.gate_up, s.act, m.dtype, n, p.inter, p.block, stream), "SwiGLU");
     }
-    TRY(linear(m, p.down, s.act, p.inter, s.branch, ABK_F32, m.hidden, n, stream), "the down product");
+    TRY(linear(m, s, p.down, s.act, p.inter, s.branch, ABK_F32, m.hidden, n, stream), "the down product");
     return STEP_OK;
 }
 
@@ -330,7 +332,7 @@ extern "C" int abk_step(const AbkModel *model, const AbkStep *step, void *stream
         TRY(LAUNCH(f.add_rmsnorm, s.x, pending, m.final_norm.w, s.xn_final, m.dtype, s.logit_rows, s.n_logit_rows, m.hidden,
                           m.final_norm.eps, stream),
             "the last norm");
-        TRY(linear(m, m.head, s.xn_final, m.hidden, s.logits, ABK_F32, m.vocab, s.n_logit_rows, stream), "the output matrix");
+        TRY(linear(m, s, m.head, s.xn_final, m.hidden, s.logits, ABK_F32, m.vocab, s.n_logit_rows, stream), "the output matrix");
     }
     return STEP_OK;
 }

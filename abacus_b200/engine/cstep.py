@@ -88,8 +88,8 @@ class Lists(ctypes.Structure):
 class Step(ctypes.Structure):
     _fields_ = [(n, P) for n in ("tokens", "token_seq", "token_pos", "seq_slot", "seq_start", "seq_pos0", "seq_len_after",
                                  "logit_rows", "lists", "x", "branch", "logits", "attention_partials", "xn", "qkv", "att",
-                                 "act", "gate_up", "xn_final")]
-    _fields_ += [("partial_floats", L)] + [(n, I) for n in ("n_rows", "n_logit_rows", "is_decode", "any_continuation",
+                                 "act", "gate_up", "xn_final", "parts")]
+    _fields_ += [("partial_floats", L), ("parts_bytes", L)] + [(n, I) for n in ("n_rows", "n_logit_rows", "is_decode", "any_continuation",
                                                             "max_len_after", "position_bound", "n_lists", "pad")]
 
 
@@ -183,6 +183,11 @@ class CStep:
         self.qkv_width = max((s.n_heads + 2 * s.n_kv_heads) * s.head_dim for s in specs)
         self.att_width = max(s.n_heads * s.head_dim for s in specs)
         self.inter = max(b.ffn.spec.inter for b in model.blocks)
+        # outputs and inputs of the products that may take scratch memory: the float32 ones, and those whose rows TMA cannot take
+        takes = lambda w: not bf16 or w.shape[1] % 8 != 0
+        self.products = {tuple(w.shape) for b in model.blocks for w in (b.mixer.qkv_proj.weight, b.mixer.o_proj.weight,
+                                                                       b.ffn.gate_up.weight, b.ffn.down.weight) if takes(w)}
+        self.head_product = tuple(frame.head.weight.shape) if takes(frame.head.weight) else None
         self.table_positions = min([b.mixer.cos.shape[0] for b in model.blocks if b.mixer.cos is not None] or [1 << 30])
         self.step, self.lists = Step(), (Lists * max(1, len(self.plan_names)))()
         # the tensors whose addresses the structures hold stay alive as long as this object does
@@ -248,6 +253,9 @@ class CStep:
         s.gate_up = ws.get("gate_up", (n, 2 * self.inter), dtype).data_ptr()
         s.xn_final = ws.get("xn_final", (max(r, 1), d), dtype).data_ptr()
         s.partial_floats = partial_floats
+        s.parts_bytes = max([ops.gemm_simt_scratch(n, *p) for p in self.products]
+                            + [ops.gemm_simt_scratch(r, *self.head_product) if self.head_product else 0])
+        s.parts = ws.get("parts", (s.parts_bytes,), torch.uint8).data_ptr() if s.parts_bytes else None
         s.n_rows, s.n_logit_rows, s.is_decode, s.any_continuation = n, r, int(batch.is_decode), int(batch.any_continuation)
         s.max_len_after, s.position_bound, s.n_lists = batch.max_len_after, bound, len(self.plan_names)
         rc = self.lib.abk_step(ctypes.byref(self.struct), ctypes.byref(s), ops._stream())

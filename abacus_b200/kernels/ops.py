@@ -254,16 +254,28 @@ def attention_generic(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ba
         _p(sink), _i(1 if exact_weights else 0), _i(chunk or 0), _f(softcap or 0.0), _stream()), "attention")
 
 
+def gemm_simt_scratch(m, n, k):
+    """Bytes of scratch memory with which gemm_simt runs a product of these sizes on the tensor cores (0: it does not)."""
+    lib = load_module("gemm_simt")
+    lib.abk_gemm_simt_scratch.restype = ctypes.c_longlong
+    return lib.abk_gemm_simt_scratch(_i(m), _i(n), _i(k))
+
+
 def gemm_simt(x, w, out, m=None):
-    """out[:m] = x[:m] . w^T on the CUDA cores in float32, any sizes (src/model.c:299 and the like)."""
+    """out[:m] = x[:m] . w^T in float32, any sizes (src/model.c:299 and the like): on the CUDA cores, large ones on the
+    tensor cores in parts that together hold every digit (csrc/gemm_split.cuh)."""
     _need_cuda(x, w, out)
     lib = load_module("gemm_simt")
     m = x.shape[0] if m is None else m
     n, k = w.shape
     assert x.shape[1] == k and out.shape[1] == n and x.shape[0] >= m and out.shape[0] >= m
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
+    # (of the calling stream's own: freed when this returns, and given out again behind what runs on that stream)
+    size = gemm_simt_scratch(m, n, k)
+    scratch = torch.empty(size, dtype=torch.uint8, device=x.device) if size else None
     _check(lib, lib.abk_gemm_simt(_p(x), _i(_dt(x)), _p(w), _i(_dt(w)), _p(out), _i(_dt(out)), _i(m), _i(n), _i(k),
-                                  _ll(x.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)), _stream()), "gemm_simt")
+                                  _ll(x.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)), _p(scratch), _ll(size),
+                                  _p(kernel_status(x.device)), _stream()), "gemm_simt")
 
 
 def gemm_rows_takes(x, w, out, m):
