@@ -311,12 +311,12 @@ static inline int delta_pad_key(int key) { return key <= 32 ? 32 : key <= 64 ? 6
 static inline long long delta_block_floats(int key, int value) { return 13LL * delta_pad_key(key) + DB_NUMBERS + DB_TOKENS * ((value + 3) & ~3); }
 
 // Which sequence has the step's block `b`, and which rows: whole warps call it. False: no sequence has.
-__device__ __forceinline__ bool delta_block_locate(const int *seq_start, int n_seqs, int b, int &row0, int &count) {
+template <int TOKENS> __device__ __forceinline__ bool delta_block_locate(const int *seq_start, int n_seqs, int b, int &row0, int &count) {
     const int lane = threadIdx.x & 31;
     for (int base = 0; base < n_seqs; base += 32) {
         const int q = base + lane;
         const int first = q < n_seqs ? seq_start[q] : 0, n = q < n_seqs ? seq_start[q + 1] - first : 0;
-        const int blocks = n > 0 ? (n + DB_TOKENS - 1) / DB_TOKENS : 0;
+        const int blocks = n > 0 ? (n + TOKENS - 1) / TOKENS : 0;
         int upto = blocks;
 #pragma unroll
         for (int m = 1; m < 32; m <<= 1) {
@@ -326,9 +326,9 @@ __device__ __forceinline__ bool delta_block_locate(const int *seq_start, int n_s
         const unsigned hit = __ballot_sync(0xffffffffu, b < upto);
         if (hit) {
             const int src = __ffs(hit) - 1;
-            const int at = (b - (upto - blocks)) * DB_TOKENS;
+            const int at = (b - (upto - blocks)) * TOKENS;
             row0 = __shfl_sync(0xffffffffu, first + at, src);
-            count = __shfl_sync(0xffffffffu, min(DB_TOKENS, n - at), src);
+            count = __shfl_sync(0xffffffffu, min(TOKENS, n - at), src);
             return true;
         }
         b -= __shfl_sync(0xffffffffu, upto, 31);
@@ -345,7 +345,7 @@ template <typename T, int J, bool PER_HEAD> __global__ void __launch_bounds__(12
     if (pair >= p.pairs) return;
     const int b = (int)(pair / p.heads), h = (int)(pair - (long long)b * p.heads), K = p.key, V = p.value;
     int row0, count;
-    if (!delta_block_locate(seq_start, n_seqs, b, row0, count)) return;
+    if (!delta_block_locate<DB_TOKENS>(seq_start, n_seqs, b, row0, count)) return;
     float *rec = p.records + pair * p.record;
     const int kvh = h / (p.heads / p.kv_heads);
     T q_in[DB_TOKENS][J], k_in[DB_TOKENS][J], b_in[DB_TOKENS], h_in[DB_TOKENS];
@@ -764,19 +764,78 @@ __global__ void __launch_bounds__(256) delta_step_kernel(DeltaPrepare p, DeltaSc
     }
 }
 
+#include "delta_chunk.cuh"
+
+// Whether a step's prompts go in chunks of 16 tokens (delta_chunk.cuh) rather than in blocks of four: where the walk's chain counts for more
+// than what it does, that is for prompts of a hundred tokens and more, and few of them or few columns to an SM. In us, blocks
+// against chunks, both kernels each: 16 heads of 128 x 128, one prompt of 1,999 tokens 327 and 210, of 200 43 and 34, of 50 21 and 22; three
+// prompts, 3,416 tokens, 644 and 328; 32 heads, the same three, 708 and 590; eight prompts of 709, 4 heads 161 and 145, 8 heads 261 and
+// 274; 32 heads of 64 x 64: one prompt of 1,999 265 and 241, four prompts 269 and 221, eight prompts of 709 373 and 447.
+static bool delta_in_chunks(int n_tokens, int n_seqs, int heads, int per_head, int key, int value) {
+    if (per_head || !delta_chunk_takes(key, value) || n_tokens < 100LL * n_seqs) return false;
+    const long long columns = (long long)n_seqs * heads * value, sms = abk_sm_count();
+    return columns <= 32 * sms || (n_seqs <= 4 && columns <= (key == 64 ? 60 : 140) * sms);
+}
+
+static long long delta_chunk_scratch(int n_tokens, int n_seqs, int heads, int key, int value) {
+    return ((long long)n_tokens / DK_TOKENS + n_seqs) * heads * delta_chunk_floats(key, value);
+}
+
 // Floats of scratch memory the recurrence needs for n_tokens tokens of n_seqs sequences: the blocks' records, none where no
 // sequence brings more than a token; chunks: the tokens' records of abk_delta_chunks.
 extern "C" long long abk_delta_scan_scratch(int n_tokens, int n_seqs, int heads, int key, int value, int chunks) {
     if (chunks) return (long long)n_tokens * heads * delta_record_floats(key, value);
     if (n_tokens <= n_seqs) return 0;
+    if (delta_in_chunks(n_tokens, n_seqs, heads, 0, key, value)) {
+        const long long in_chunks = delta_chunk_scratch(n_tokens, n_seqs, heads, key, value);
+        const long long in_blocks = ((long long)n_tokens / DB_TOKENS + n_seqs) * heads * delta_block_floats(key, value);
+        return in_chunks > in_blocks ? in_chunks : in_blocks;
+    }
     return ((long long)n_tokens / DB_TOKENS + n_seqs) * heads * delta_block_floats(key, value);
 }
 
+static int delta_chunk_run(DeltaPrepare q, DeltaScan p, const int *seq_start, int dtype, int n_tokens, int n_seqs, cudaStream_t s) {
+    q.record = p.record = (int)delta_chunk_floats(q.key, q.value), q.pairs = ((long long)n_tokens / DK_TOKENS + n_seqs) * q.heads;
+    if (q.pairs > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld (chunk, head) pairs are more than a grid takes", q.pairs);
+#define CHUNK_PREPARE_AS(T, J) abk_launch(delta_chunk_prepare_kernel<T, J>, dim3((unsigned)q.pairs), dim3(256), 0, s, q, seq_start, n_seqs)
+#define CHUNK_PREPARE(J)                                           \
+    do {                                                           \
+        if (dtype == ABK_BF16) CHUNK_PREPARE_AS(__nv_bfloat16, J); \
+        else CHUNK_PREPARE_AS(float, J);                           \
+    } while (0)
+    if (q.key == 64) CHUNK_PREPARE(2);
+    else CHUNK_PREPARE(4);
+#undef CHUNK_PREPARE
+#undef CHUNK_PREPARE_AS
+    const int rc = ABK_LAUNCH_RESULT();
+    if (rc) return rc;
+    const int lanes = q.key / 4, cols = DK_WARPS * 128 / lanes, sms = abk_sm_count();
+    p.tiles = (q.value + cols - 1) / cols, p.n_seqs = n_seqs;
+    const long long ctas = (long long)n_seqs * q.heads * p.tiles, share = (ctas + sms - 1) / sms;
+    if (ctas > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld blocks are more than a grid takes", ctas);
+    size_t smem = (size_t)(DK_STAGES * (49 * q.key + 32 * cols) + 16 * cols) * 4;
+    // (as the walk in blocks: no SM takes more CTAs than its share, and the longest sequence starts first)
+    const size_t least = share <= 4 ? (size_t)(228 * 1024 / (share + 1)) : 0;
+    if (smem < least) smem = least;
+    p.longest_first = n_seqs > 1 && n_seqs <= SEQUENCE_PLACE_MAX && share > 1;
+#define CHUNK_WALK(P)                                                                                        \
+    do {                                                                                                     \
+        const cudaError_t e = abk_allow_shared_memory((const void *)delta_chunk_walk_kernel<P>, (int)smem);  \
+        if (e != cudaSuccess) return (int)e;                                                                 \
+        abk_launch(delta_chunk_walk_kernel<P>, dim3((unsigned)ctas), dim3(32 * DK_WARPS + 32), smem, s, p);  \
+    } while (0)
+    if (lanes == 16) CHUNK_WALK(16);
+    else CHUNK_WALK(32);
+#undef CHUNK_WALK
+    return ABK_LAUNCH_RESULT();
+}
+
+// form: 0 by size; 4: prompts in blocks of four tokens; 16: in chunks of 16 where the keys' size and the scratch memory allow it.
 extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, const void *decay_in, long long ld_decay, int per_head, const void *beta_in,
                               long long ld_beta, const float *a_log, const float *dt_bias, float *state, float *out,
                               const int *token_seq, const int *seq_start, const int *seq_slot, int n_tokens, int n_seqs,
                               int heads, int kv_heads, int key, int value, float *records, long long records_floats,
-                              void *stream) {
+                              int form, void *stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (key < 1 || key > 256) ABK_REFUSE("delta rule: key size %d, the kernel takes 1 to 256", key);
     if (kv_heads < 1 || heads % kv_heads) ABK_REFUSE("delta rule: %d heads do not divide into %d key heads", heads, kv_heads);
@@ -812,6 +871,10 @@ extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, cons
 #undef STEP_LAUNCH
         return ABK_LAUNCH_RESULT();
     }
+    // form 4: in blocks whatever the sizes; 16: in chunks wherever they are built
+    const bool chunks = form == 16 ? !per_head && delta_chunk_takes(key, value) : form != 4 && delta_in_chunks(n_tokens, n_seqs, heads, per_head, key, value);
+    if (chunks && !((uintptr_t)state & 15) && delta_chunk_scratch(n_tokens, n_seqs, heads, key, value) <= records_floats)
+        return delta_chunk_run(q, p, seq_start, dtype, n_tokens, n_seqs, s);
     const long long blocks = (q.pairs + 3) / 4;
     if (blocks > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld (block, head) pairs are more than a grid takes", q.pairs);
     const int kp4 = delta_pad_key(key) / 32;

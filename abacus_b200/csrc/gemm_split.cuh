@@ -24,6 +24,7 @@
 // that splits what it fetches, weights again for every column of tiles: 500 x 6144 x 1024 in 71 us, bound by the instructions
 // of the splitting and by the way of plain loads through what the stages leave of the L1.)
 #pragma once
+#include "bf16_parts.cuh"
 #include "tc_common.cuh"
 #include "tensor_map.cuh"
 
@@ -46,15 +47,6 @@ template <int N> __device__ __forceinline__ void gp_tmem_ld(uint32_t taddr, uint
 template <> __device__ __forceinline__ void gp_tmem_ld<8>(uint32_t taddr, uint32_t *v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
-}
-
-// Two numbers as three pairs of bfloat16 (the lower half of a word: the first number).
-__device__ __forceinline__ void gp_split(float a, float b, uint32_t &p1, uint32_t &p2, uint32_t &p3) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(b), "f"(a));
-    a -= __uint_as_float(p1 << 16), b -= __uint_as_float(p1 & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(b), "f"(a));
-    a -= __uint_as_float(p2 << 16), b -= __uint_as_float(p2 & 0xffff0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p3) : "f"(b), "f"(a));
 }
 
 // ------------------------------------------------------------------ the parts of the operands
@@ -88,8 +80,8 @@ template <typename T> __global__ void __launch_bounds__(256) gemm_split_rows_ker
         }
         if constexpr (sizeof(T) == 4) {
             uint4 p1, p2, p3;
-            gp_split(v[0], v[1], p1.x, p2.x, p3.x), gp_split(v[2], v[3], p1.y, p2.y, p3.y);
-            gp_split(v[4], v[5], p1.z, p2.z, p3.z), gp_split(v[6], v[7], p1.w, p2.w, p3.w);
+            split_pair(v[0], v[1], p1.x, p2.x, p3.x), split_pair(v[2], v[3], p1.y, p2.y, p3.y);
+            split_pair(v[4], v[5], p1.z, p2.z, p3.z), split_pair(v[6], v[7], p1.w, p2.w, p3.w);
             const long long plane = (long long)o.rows * pitch;
             *(uint4 *)to = p1, *(uint4 *)(to + plane) = p2, *(uint4 *)(to + 2 * plane) = p3;
         } else {

@@ -1004,14 +1004,14 @@ DELTA_CHUNK = 64  # tokens of a chunk of the chunked form (one decay a head)
 
 
 def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_heads, n_kv_heads, key_dim, value_dim, ws,
-               per_head=False, chunks=False):
+               per_head=False, chunks=False, tokens_a_time=0):
     """The gated delta rule over every sequence of the step, in order, from and into the slots' states (float32
     [slots, heads, value, key]). qkv [tokens, 2 * kv_heads * key + heads * value]: q, k and v after their convolution;
     decay_in float32 [tokens, heads * key] (rows of any pitch) before bias and softplus; beta_in [tokens, >= heads] (rows of any pitch)
     before the sigmoid; out float32 [tokens, heads * value], not yet normed. per_head: one decay for all key channels of a
     head; decay_in is then [tokens, >= heads] of qkv's type and dt_bias [heads]. A step of one token a sequence is one kernel;
-    else every (block of four tokens, head) is prepared in parallel into scratch memory from ws (a parts.Workspace), then the
-    sequences are walked, a block at a time. chunks (with
+    else every (block of four tokens, head), or for few and long prompts (chunk of 16, head), is prepared in parallel into scratch memory from
+    ws (a parts.Workspace), then the sequences are walked, a block or chunk at a time (tokens_a_time 4 or 16 pins it). chunks (with
     per_head, for steps that bring prompts): the walk goes in chunks of 64 tokens, a triangular system a chunk solved
     beside the others and four products a chunk along the sequence (three kernels)."""
     _need_cuda(qkv, decay_in, beta_in, a_log, dt_bias, state, out)
@@ -1043,7 +1043,7 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
     _check(lib, lib.abk_delta_scan(_p(qkv), _ll(qkv.stride(0)), _i(_dt(qkv)), _p(decay_in), _ll(decay_in.stride(0)),
                                    _i(1 if per_head else 0), _p(beta_in), _ll(beta_in.stride(0)), _p(a_log), _p(dt_bias), _p(state), _p(out), _p(batch.token_seq),
                                    _p(batch.seq_start), _p(batch.seq_slot), _i(n), _i(n_seqs), _i(n_heads), _i(n_kv_heads),
-                                   _i(key_dim), _i(value_dim), _p(records), _ll(records.numel()), _stream()),
+                                   _i(key_dim), _i(value_dim), _p(records), _ll(records.numel()), _i(tokens_a_time), _stream()),
            "delta_scan", kernels=1 if n <= n_seqs else 2)
 
 

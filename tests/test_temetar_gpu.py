@@ -231,6 +231,39 @@ def test_delta_rule_in_blocks_of_many_sequences(n_seqs):
     assert float(states[0][slots[7]].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("H,G,K,V,lens,rate", [(4, 2, 128, 128, (100, 16, 1), -1), (2, 1, 64, 36, (17, 33), -1), (1, 1, 128, 4, (31,), 1.5), (3, 3, 64, 520, (48, 5), -4),
+                                               (2, 2, 128, 132, (1, 250), -6)])
+def test_delta_rule_in_chunks(H, G, K, V, lens, rate):
+    """Chunks of 16 tokens against 64 bits and against blocks of four: remainders, columns that no CTA fills, decays from nothing to nearly
+    one, both operand types, states that are there before, and a slot that the step does not touch."""
+    from abacus_b200.kernels import ops
+    from abacus_b200.parts import Workspace
+    rng = np.random.default_rng(H * K + V)
+    ins = [_delta_inputs(rng, n, H, G, K, V) for n in lens]
+    a_log, bias = ins[0][3] + 1 + rate, ins[0][4]
+    slots, start = [2 * i + 1 for i in range(len(lens))], torch.randn((2 * len(lens) + 1, H, V, K), device=DEV) * 0.1
+    for dtype in (torch.float32, torch.bfloat16):
+        rounded = [(plain.bf16_round(i[0]), i[1], plain.bf16_round(i[2])) if dtype == torch.bfloat16 else i[:3] for i in ins]
+        b, outs, states = batch_of([(s, [0] * n, 0) for s, n in zip(slots, lens)]), {}, {}
+        cat = lambda j, t: dev(np.concatenate([i[j] for i in rounded]), t)
+        for tokens in (16, 4):
+            state, out = start.clone(), torch.empty((sum(lens), H * V), device=DEV)
+            ws = Workspace(torch.device(DEV, torch.cuda.current_device()))
+            room = torch.empty(1 << 22, device=DEV)  # (for either form)
+            ws.get = lambda name, shape, dt: room
+            ops.delta_scan(cat(0, dtype), cat(1, torch.float32), cat(2, dtype), dev(a_log), dev(bias), state, out, b, H, G, K, V, ws, tokens_a_time=tokens)
+            outs[tokens], states[tokens] = out.cpu().double(), state.cpu().double()
+            assert torch.equal(state[::2], start[::2])
+        want = np.concatenate([_delta_plain(*x, a_log, bias, H, G, K, V, real=np.float64) for x in rounded])
+        noise = max(np.abs(_delta_plain(*x, a_log, bias, H, G, K, V) - _delta_plain(*x, a_log, bias, H, G, K, V, real=np.float64)).max() for x in rounded)
+        # sums of 4 x K products and of a chunk's tokens in another order: a few times what float32 itself is off here
+        for a in (outs, states):
+            np.testing.assert_allclose(a[16].numpy(), a[4].numpy(), rtol=1e-4, atol=2e-5 + 4 * noise)
+        state, out = torch.zeros_like(start), torch.empty((sum(lens), H * V), device=DEV)
+        ops.delta_scan(cat(0, dtype), cat(1, torch.float32), cat(2, dtype), dev(a_log), dev(bias), state, out, b, H, G, K, V, ws, tokens_a_time=16)
+        np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-4, atol=2e-5 + 4 * noise)
+
+
 def test_a_delta_step_of_small_heads_leaves_no_warp_idle():
     """A head of 32 x 32 is a quarter of one of 64 x 64: with warps that have no columns it took nearly half as long."""
     from abacus_b200.kernels import ops
