@@ -175,18 +175,21 @@ static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int 
     return ABK_LAUNCH_RESULT();
 }
 
-// The product on the tensor cores (gemm_split.cuh), float32 operands and results. bn: rows of x in a tile (32, 64, 96, 128), quarters: pairs
-// of CTAs take quarters of K; 0, 0: by size.
-extern "C" int abk_gemm_split(const void *x, const void *w, void *out, int M, int N, int K, long long ldx, long long ldw, long long ldo, int bn,
-                              int quarters, void *scratch, int *status, void *stream) {
-    const GemmSplit g = {x, w, out, ABK_F32, ABK_F32, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};
-    return gemm_split_run<float>(g, bn, quarters, scratch, (cudaStream_t)stream);
+// The product on the tensor cores (gemm_split.cuh), for any sizes. bn: rows of x in a tile (32, 64, 96, 128), quarters: pairs of CTAs take
+// quarters of K; 0, 0: by size. scratch: abk_gemm_split_scratch bytes.
+extern "C" int abk_gemm_split(const void *x, const void *w, int dtype, void *out, int out_dtype, int M, int N, int K, long long ldx, long long ldw,
+                              long long ldo, int bn, int quarters, void *scratch, int *status, void *stream) {
+    const GemmSplit g = {x, w, out, dtype, out_dtype, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};
+    return dtype == ABK_F32 ? gemm_split_run<float>(g, bn, quarters, scratch, (cudaStream_t)stream)
+                            : gemm_split_run<__nv_bfloat16>(g, bn, quarters, scratch, (cudaStream_t)stream);
 }
+extern "C" long long abk_gemm_split_scratch(int M, int N, int K) { return gemm_split_scratch(M, N, K); }
 
-// Whether a product goes to the tensor cores: more than a handful of rows (up to 32 rows the plain kernel reads the weights once and writes nothing beside: 17 x 6144 x 1024 in 19 us
-// against 23), and enough to do: a long K, which is a chain in the plain kernel (33 x 64 x 2560: 28 us, in parts 17), or a hundred
-// million multiply-adds (64 x 1024 x 1024: 13.4 against 12.8; 500 x 256 x 512: 7.9 against 10.3; 1000 x 256 x 512: 12.6 and 12.1).
-static bool gemm_split_wins(int M, int N, int K) { return M > 32 && N >= 64 && K >= 512 && (K >= 2048 || (long long)M * N * K >= 100000000LL); }
+// Whether a product goes to the tensor cores: more than a handful of rows (up to 32 rows the plain kernel reads the weights once and
+// writes nothing beside: 17 x 6144 x 1024 in 19 us against 23), and enough to do for two or three launches in place of one, whose
+// host side takes some 12 us more: 64 x 6144 x 1024 in 25 us against 32, 100 x 4096 x 1024 in 24 against 35, 500 x 1024 x 1024 in 18 against
+// 35; below that there is little to win (64 x 1024 x 1024: 12.8 against 13.4; 500 x 256 x 512: 10.3 against 7.9).
+static bool gemm_split_wins(int M, int N, int K) { return M > 32 && N >= 64 && K >= 512 && (long long)M * N * K >= 400000000LL; }
 // Bytes of scratch memory with which abk_gemm_simt goes to the tensor cores (0: it does not).
 extern "C" long long abk_gemm_simt_scratch(int M, int N, int K) { return gemm_split_wins(M, N, K) ? gemm_split_scratch(M, N, K) : 0; }
 

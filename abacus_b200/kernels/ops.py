@@ -7,6 +7,7 @@ reason instead of computing something else.
 """
 import array
 import ctypes
+import functools
 
 import torch
 
@@ -254,6 +255,7 @@ def attention_generic(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ba
         _p(sink), _i(1 if exact_weights else 0), _i(chunk or 0), _f(softcap or 0.0), _stream()), "attention")
 
 
+@functools.lru_cache(maxsize=4096)
 def gemm_simt_scratch(m, n, k):
     """Bytes of scratch memory with which gemm_simt runs a product of these sizes on the tensor cores (0: it does not)."""
     lib = load_module("gemm_simt")

@@ -1,4 +1,6 @@
 """Each kernel alone against its plain reference, at sizes the engine's tiny models do not use."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -199,49 +201,50 @@ def test_page_tables_on_the_device_follow_the_host():
             assert len(held) == len(set(held)) and all(g.table_host[s, :len(g.book.of_slot[s])].tolist() == g.book.of_slot[s] for s in slots)
 
 
-@pytest.mark.parametrize("m, n, k", [(33, 64, 2048), (33, 65, 2052), (129, 257, 4100), (100, 1024, 1024), (260, 1100, 580), (1000, 300, 2108)])
+@pytest.mark.parametrize("m, n, k", [(33, 64, 2048), (33, 65, 2052), (129, 257, 4100), (100, 1024, 1024), (260, 1100, 580), (1000, 300, 2108), (400, 1030, 1023)])
 def test_float32_product_in_parts(ops, m, n, k):
-    """Large float32 products on the tensor cores, in three bfloat16 parts an operand, in every tile and in quarters of K: one set of bits,
-    as near to 64 bits as eight float32 sums. Limits: a part is left over of 2^-26 of a number, a sum of 128 is cut off eight times by up
-    to 2^-23 of itself, and K / 128 such sums are added with 2^-24 each: below 4e-7 of the result's norm for normal numbers."""
+    """The float32 product on the tensor cores, in three bfloat16 parts an operand, in every tile and in quarters of K: one set of bits, as
+    near to 64 bits as eight float32 sums. Limits: a part is left over of 2^-26 of a number, a sum of 128 is cut off eight times by up to
+    2^-23 of itself, and K / 128 such sums are added with 2^-24 each: below 4e-7 of the result's norm for normal numbers."""
     rng = np.random.default_rng(m + n + k)
     x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
     x[m // 2, k // 3], x[3, 5], w[7, k - 1], x[m - 1, 1] = np.inf, np.nan, -np.inf, 3.4e38
-    xd, wd, status = dev(x), dev(w), ops.kernel_status(torch.device("cuda", 0))
-    whole, out, plain_out = (torch.empty(m, n, device="cuda") for _ in range(3))
-    assert ops.gemm_simt_scratch(m, n, k) > 0
-    ops.gemm_simt(xd, wd, whole)
-    exact = torch.tensor(x, dtype=torch.float64) @ torch.tensor(w, dtype=torch.float64).T
-    odd = torch.zeros(m, n, dtype=torch.bool)
-    odd[[m // 2, 3, m - 1]] = True
-    odd[:, 7] = True
-    assert ((whole.cpu().double() - exact)[~odd].norm() / exact[~odd].norm()).item() < 4e-7
-    lib, sizes = ops.load_module("gemm_simt"), [ops._i(m), ops._i(n), ops._i(k), ops._ll(k), ops._ll(k), ops._ll(n)]
-    tail = [ops._p(status), ops._stream()]
+    xd, wd, status, lib = dev(x), dev(w), ops.kernel_status(torch.device("cuda", 0)), ops.load_module("gemm_simt")
+    lib.abk_gemm_split_scratch.restype = ctypes.c_longlong
+    scratch = torch.empty(lib.abk_gemm_split_scratch(m, n, k), dtype=torch.uint8, device="cuda")
 
-    def general(a, b, o, dt, odt, scratch=None):
-        nbytes = scratch.numel() if scratch is not None else 0
-        assert lib.abk_gemm_simt(ops._p(a), ops._i(dt), ops._p(b), ops._i(dt), ops._p(o), ops._i(odt), *sizes, ops._p(scratch),
-                                 ops._ll(nbytes), *tail) == 0
+    def product(a, b, dtype, rows=0, quarters=0):
+        out = torch.full((m, n), 7, dtype=dtype, device="cuda")
+        assert lib.abk_gemm_split(ops._p(a), ops._p(b), ops._i(ops._dt(a)), ops._p(out), ops._i(ops._dt(out)), ops._i(m), ops._i(n), ops._i(k),
+                                  ops._ll(a.stride(0)), ops._ll(b.stride(0)), ops._ll(n), ops._i(rows), ops._i(quarters), ops._p(scratch),
+                                  ops._p(status), ops._stream()) == 0
+        return out
 
-    general(xd, wd, plain_out, 0, 0)  # (without scratch memory: the CUDA cores)
+    off = lambda out, want, where: ((out.cpu().double() - want)[where].norm() / want[where].norm()).item()
+    whole, exact = product(xd, wd, torch.float32), torch.tensor(x, dtype=torch.float64) @ torch.tensor(w, dtype=torch.float64).T
+    real = torch.ones(m, n, dtype=torch.bool)
+    real[[m // 2, 3, m - 1]] = False
+    real[:, 7] = False
+    assert off(whole, exact, real) < 4e-7
+    plain_out = torch.empty(m, n, device="cuda")  # (without scratch memory: the CUDA cores)
+    assert lib.abk_gemm_simt(ops._p(xd), ops._i(0), ops._p(wd), ops._i(0), ops._p(plain_out), ops._i(0), ops._i(m), ops._i(n), ops._i(k), ops._ll(k),
+                             ops._ll(k), ops._ll(n), None, ops._ll(0), ops._p(status), ops._stream()) == 0
     assert torch.equal(torch.isnan(whole), torch.isnan(plain_out)) and torch.equal(torch.isinf(whole), torch.isinf(plain_out))
-    scratch = torch.empty(ops.gemm_simt_scratch(m, n, k), dtype=torch.uint8, device="cuda")
+    same = lambda out: torch.equal(out.nan_to_num(1, 2, 3), whole.nan_to_num(1, 2, 3))
     for rows in (32, 64, 96, 128):
         for quarters in (0, 1):
-            out.fill_(7)
-            assert lib.abk_gemm_split(ops._p(xd), ops._p(wd), ops._p(out), *sizes, ops._i(rows), ops._i(quarters), ops._p(scratch), *tail) == 0
-            assert torch.equal(out.nan_to_num(1, 2, 3), whole.nan_to_num(1, 2, 3)), (rows, quarters)
-    # rows that start anywhere: the same bits; bfloat16 ones: one part, which is all there is of them
+            assert same(product(xd, wd, torch.float32, rows, quarters)), (rows, quarters)
+    # rows that start anywhere: the same bits; the way by size: the same bits, where it goes to the tensor cores
     anywhere = [torch.empty(t.shape[0], k + 5, device="cuda")[:, 1:k + 1].copy_(t) for t in (xd, wd)]
-    ops.gemm_simt(*anywhere, out)
-    assert torch.equal(out.nan_to_num(1, 2, 3), whole.nan_to_num(1, 2, 3))
-    xb, wb = bf(rng.standard_normal((m, k)).astype(np.float32)), bf(rng.standard_normal((n, k)).astype(np.float32))
-    want = torch.tensor(xb, dtype=torch.float64) @ torch.tensor(wb, dtype=torch.float64).T
-    half = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
-    for o, odt, limit in ((out, 0, 4e-7), (half, 1, 2.0 ** -8)):
-        general(dev(xb, torch.bfloat16), dev(wb, torch.bfloat16), o, 1, odt, scratch)
-        assert ((o.cpu().double() - want).norm() / want.norm()).item() < limit
+    assert same(product(*anywhere, torch.float32))
+    by_size = torch.empty(m, n, device="cuda")
+    ops.gemm_simt(xd, wd, by_size)
+    assert (m * n * k >= 4e8) == bool(ops.gemm_simt_scratch(m, n, k)) and (same(by_size) or m * n * k < 4e8)
+    # bfloat16 operands: one part, which is all there is of them
+    xb, wb = (dev(bf(rng.standard_normal(s).astype(np.float32)), torch.bfloat16) for s in ((m, k), (n, k)))
+    want = xb.cpu().double() @ wb.cpu().double().T
+    for dtype, limit in ((torch.float32, 4e-7), (torch.bfloat16, 2.0 ** -8)):
+        assert off(product(xb, wb, dtype), want, torch.ones(m, n, dtype=torch.bool)) < limit
     assert not status.any()
 
 
