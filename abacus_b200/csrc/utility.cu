@@ -65,6 +65,11 @@ __global__ void __launch_bounds__(128) set_words_kernel(const __grid_constant__ 
     for (int i = threadIdx.x; i < p.n; i += 128) p.table[p.pairs[2 * i]] = p.pairs[2 * i + 1];
 }
 
+// bytes of pinned host memory to the device in the stream's order, and `event` behind them.
+extern "C" int abk_send(void *dst, const void *src, long long bytes, void *event, void *stream) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyHostToDevice, (cudaStream_t)stream);
+    return (int)(e != cudaSuccess ? e : cudaEventRecord((cudaEvent_t)event, (cudaStream_t)stream));
+}
 extern "C" int abk_set_words_room() { return SET_WORDS; }
 
 // table[pairs[2 i]] = pairs[2 i + 1] for i in [0, n); `pairs` (on the host) is read before this returns. Words all different.

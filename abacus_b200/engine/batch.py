@@ -104,16 +104,16 @@ class StepBatch:
         h = self._h
         if self._sent is not None:
             self._sent.synchronize()  # the last copy must have read the host buffer before it is rewritten
-        n_tokens = sum(len(s.tokens) for s in sequences)
-        n_logits = sum(len(s.want) for s in sequences)
+        lens, starts, wants = [len(s.tokens) for s in sequences], [s.start for s in sequences], [s.want for s in sequences]
+        n_tokens, n_logits = sum(lens), sum(map(len, wants))
         if n_tokens > self.cap_rows or len(sequences) > self.cap_seqs or n_logits > self.cap_logits:
             raise ValueError("step is larger than this StepBatch")
         n_seqs = len(sequences)
-        lens, starts = [len(s.tokens) for s in sequences], [s.start for s in sequences]
         lens_a, starts_a = np.array(lens, dtype=np.int64), np.array(starts, dtype=np.int64)
         ends = np.cumsum(lens_a)
         first = ends - lens_a
-        if n_tokens == n_seqs and all(n == 1 for n in lens):  # a decode step: a row a sequence
+        one_each = n_tokens == n_seqs and (n_seqs == 0 or min(lens) == 1)
+        if one_each:  # a decode step: a row a sequence
             h["tokens"][:n_seqs] = [s.tokens[0] for s in sequences]
             h["token_seq"][:n_seqs] = np.arange(n_seqs)
             h["token_pos"][:n_seqs] = starts_a
@@ -130,43 +130,53 @@ class StepBatch:
             h["tokens"][n_tokens:] = 0
             h["token_seq"][n_tokens:] = -1
             h["token_pos"][n_tokens:] = 0
-        for name, values in (("seq_slot", [s.slot for s in sequences]), ("seq_pos0", starts_a), ("seq_len_after", starts_a + lens_a)):
+        lens_after = starts_a + lens_a
+        for name, values in (("seq_slot", [s.slot for s in sequences]), ("seq_pos0", starts_a), ("seq_len_after", lens_after)):
             h[name][:n_seqs] = values
             if n_seqs < self.cap_seqs:
                 h[name][n_seqs:] = 0
         h["seq_start"][:n_seqs] = first
         h["seq_start"][n_seqs:] = n_tokens
-        lr = 0
-        for s, n, row in zip(sequences, lens, first.tolist()):
-            for wpos in s.want:
-                if not 0 <= wpos < n:
-                    raise ValueError(f"wanted place {wpos} is outside the {n} tokens given")
-                h["logit_rows"][lr] = row + wpos
-                lr += 1
-        h["logit_rows"][lr:] = 0
+        logit_rows = []
+        if n_logits:
+            for want, n, row in zip(wants, lens, first.tolist()):
+                for wpos in want:
+                    if not 0 <= wpos < n:
+                        raise ValueError(f"wanted place {wpos} is outside the {n} tokens given")
+                    logit_rows.append(row + wpos)
+            h["logit_rows"][:n_logits] = logit_rows
+        h["logit_rows"][n_logits:] = 0
         self.n_tokens, self.n_seqs, self.n_logit_rows = n_tokens, len(sequences), n_logits
         if pad_logits:
             self.n_logit_rows = self.cap_logits
         if exact:
             self.n_rows = n_tokens
-            n_seqs = len(sequences)
             for name, n in (("tokens", n_tokens), ("token_seq", n_tokens), ("token_pos", n_tokens), ("seq_slot", n_seqs),
                             ("seq_start", n_seqs + 1), ("seq_pos0", n_seqs), ("seq_len_after", n_seqs),
                             ("logit_rows", max(1, n_logits))):
-                setattr(self, name, self._parts[name][:n])
+                whole = self._parts[name]
+                setattr(self, name, whole if whole.shape[0] == n else whole[:n])
         self.sequences = list(sequences)  # host view, for mixers that walk the sequences themselves
-        self.is_decode = all(len(s.tokens) == 1 for s in sequences)
+        self.is_decode = one_each
         for name, p in self.plans.items():
             info = p.fill(self._layouts[name], self.sequences, h[f"plan:{name}"], self.is_decode, exact)
             self.plan[name] = PlanView(p, self._layouts[name], self._parts[f"plan:{name}"], info)
-        self.max_position = max((s.start + len(s.tokens) - 1 for s in sequences), default=0)
+        self.max_position = int(lens_after.max()) - 1 if n_seqs else 0
         self.max_len_after = self.max_position + 1
-        self.any_continuation = any(s.start > 0 for s in sequences)
+        self.any_continuation = n_seqs > 0 and max(starts) > 0
+        self._send()
+        return self
+
+    def _send(self):
+        """The host's words to the device, in the order of the device's current stream."""
+        if self._sent is not None and self._dev.get_device() == torch.cuda.current_device():
+            from ..kernels import ops
+            ops.send_words(self._dev, self._host, self._sent)  # (a copy and an event by torch cost the host four times as long)
+            return
         self._dev.copy_(self._host, non_blocking=True)
         if self.device.type == "cuda":
-            self._sent = torch.cuda.Event()
+            self._sent = self._sent or torch.cuda.Event()
             self._sent.record()
-        return self
 
     def advance_on_device(self):
         """Every sequence moves one position on (a decode step follows a decode step); the tokens are

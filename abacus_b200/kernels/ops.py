@@ -40,7 +40,26 @@ def _p(t):
 def _stream():
     # torch's current stream as a raw handle (the public torch.cuda.current_stream() builds a Stream object
     # for it and takes fifty times as long: a few microseconds on every launch)
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return ctypes.c_void_p(_raw_stream())
+
+
+def _raw_stream():
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+_KINDS = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
+
+
+def _typed(fn, kinds):
+    """The launcher `fn` with its argument types told once (a letter each: p, i, l, f), so that a call takes plain numbers and
+    addresses: an object made for each argument is a third of what a call of twenty costs the host."""
+    if fn.argtypes is None:
+        fn.argtypes = [_KINDS[k] for k in kinds]
+    return fn
+
+
+def _at(t):
+    return t.data_ptr() if t is not None else None
 
 
 def _need_cuda(*tensors):
@@ -73,6 +92,14 @@ def fill_normal(out, key, mean, amplitude, first=0):
     assert out.is_contiguous()
     _check(lib, lib.abk_fill_normal(_p(out), _i(_dt(out)), _ll(out.numel()), _ll(first), ctypes.c_ulonglong(key),
                                     _f(mean), _f(amplitude), _stream()), "fill_normal")
+
+
+def send_words(dst, src, event):
+    """dst, int32 on the current device, becomes a copy of src, pinned, in the order of the current stream; `event` (a torch.cuda.Event that was
+    recorded before) is recorded behind it."""
+    lib = load_module("utility")
+    fn = _typed(lib.abk_send, "pplpp")
+    _check(lib, fn(dst.data_ptr(), src.data_ptr(), 4 * src.numel(), event.cuda_event, _raw_stream()), "send_words", kernels=0)
 
 
 def set_words(table, changes):
@@ -675,13 +702,12 @@ def _attention_decode_mma(qkv, out, n_heads, n_kv_heads, head_dim, scale, window
         cos = prepare["cos"]
         if cos is not None and batch.max_position >= cos.shape[0]:
             raise KernelError(f"position {batch.max_position} is beyond the rotary table of {cos.shape[0]} positions")
-        _check(lib, lib.abk_attention_decode_ring_prepare(
-            _p(qkv), _ll(row), _p(out), _i(n), _i(n_heads), _i(n_kv_heads), _i(head_dim), _f(scale), _i(window or 0),
-            _p(batch.token_seq), _p(batch.token_pos), _p(batch.seq_slot), _p(cache.k), _p(cache.v), _ll(pool_rows),
-            _p(cache.page_table), _i(cache.table_width), _i(cache.ring_pages), _i(cache.tokens_per_page),
-            _i(max_positions), _p(prepare["q_norm"]), _p(prepare["k_norm"]), _f(prepare["eps"] or 0.0), _p(cos),
-            _p(prepare["sin"]), _i(1 if prepare["keep"] else 0), _p(kernel_status(qkv.device)), _stream()),
-            "attention_decode_mma")
+        fn = _typed(lib.abk_attention_decode_ring_prepare, "plpiiiifippppplpiiiippfppipp")
+        _check(lib, fn(qkv.data_ptr(), row, out.data_ptr(), n, n_heads, n_kv_heads, head_dim, scale, window or 0, batch.token_seq.data_ptr(),
+                       batch.token_pos.data_ptr(), batch.seq_slot.data_ptr(), cache.k.data_ptr(), cache.v.data_ptr(), pool_rows,
+                       cache.page_table.data_ptr(), cache.table_width, cache.ring_pages, cache.tokens_per_page, max_positions,
+                       _at(prepare["q_norm"]), _at(prepare["k_norm"]), prepare["eps"] or 0.0, _at(cos), _at(prepare["sin"]),
+                       1 if prepare["keep"] else 0, kernel_status(qkv.device).data_ptr(), _raw_stream()), "attention_decode_mma")
         return
     _check(lib, lib.abk_attention_decode_ring(
         _p(qkv), _ll(row), _p(out), _i(n), _i(n_heads), _i(n_kv_heads), _i(head_dim), _f(scale), _i(window or 0),
@@ -881,11 +907,10 @@ def gemm_tc(x, w, out, m=None, tile_n=0, swap=-1, splits=0, persistent=-1, activ
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
     assert x.shape[1] == k and out.shape[1] == n and x.shape[0] >= m and out.shape[0] >= m
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
-    _check(lib, lib.abk_gemm_tc_act(_p(x), _p(w), _p(out), _i(_dt(out)), _i(m), _i(n), _i(k), _ll(x.stride(0)),
-                                    _ll(w.stride(0)), _ll(out.stride(0)), _p(sc.gemm_floats), _p(sc.gemm_tickets),
-                                    _p(sc.status), _i(tile_n), _i(swap), _i(splits), _i(persistent),
-                                    _i(2 if activation == "relu_squared_stored" else OUT_ACTIVATIONS[activation]), _stream()),
-           "gemm_tc")
+    fn = _typed(lib.abk_gemm_tc_act, "pppiiiilllpppiiiiip")
+    _check(lib, fn(x.data_ptr(), w.data_ptr(), out.data_ptr(), _dt(out), m, n, k, x.stride(0), w.stride(0), out.stride(0),
+                   sc.gemm_floats.data_ptr(), sc.gemm_tickets.data_ptr(), sc.status.data_ptr(), tile_n, swap, splits, persistent,
+                   2 if activation == "relu_squared_stored" else OUT_ACTIVATIONS[activation], _raw_stream()), "gemm_tc")
 
 
 # ------------------------------------------------------------------ streams (csrc/streams.cu)
@@ -985,9 +1010,10 @@ def short_conv(x, channels, weight, tail, out, batch, update_tail=False, plain=F
     assert x.stride(1) == 1 and x.shape[1] >= channels and out.is_contiguous() and out.shape[1] == channels
     assert out.dtype == x.dtype and weight.dtype == torch.float32 and weight.shape == (channels, taps) and weight.is_contiguous()
     assert tail.dtype == torch.float32 and tail.shape[1:] == (max(taps - 1, 0), channels) and tail.is_contiguous()
-    _check(lib, lib.abk_short_conv(_p(x), _ll(x.stride(0)), _p(out), _i(_dt(x)), _p(weight), _p(tail), _p(batch.token_seq),
-                                   _p(batch.token_pos), _p(batch.seq_slot), _p(batch.seq_pos0), _i(n), _i(channels),
-                                   _i(taps), _i(1 if update_tail else 0), _i(1 if plain else 0), _stream()), "short_conv")
+    fn = _typed(lib.abk_short_conv, "plpippppppiiiiip")
+    _check(lib, fn(x.data_ptr(), x.stride(0), out.data_ptr(), _dt(x), weight.data_ptr(), tail.data_ptr(), batch.token_seq.data_ptr(),
+                   batch.token_pos.data_ptr(), batch.seq_slot.data_ptr(), batch.seq_pos0.data_ptr(), n, channels, taps,
+                   1 if update_tail else 0, 1 if plain else 0, _raw_stream()), "short_conv")
 
 
 def short_conv_tail(x, channels, taps, tail, batch):
@@ -1005,6 +1031,13 @@ def short_conv_tail(x, channels, taps, tail, batch):
 DELTA_CHUNK = 64  # tokens of a chunk of the chunked form (one decay a head)
 
 
+@functools.lru_cache(maxsize=4096)
+def _delta_scan_scratch(n, n_seqs, n_heads, key_dim, value_dim, chunks):
+    lib = load_module("delta_rule")
+    lib.abk_delta_scan_scratch.restype = ctypes.c_longlong
+    return int(lib.abk_delta_scan_scratch(_i(n), _i(n_seqs), _i(n_heads), _i(key_dim), _i(value_dim), _i(chunks)))
+
+
 def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_heads, n_kv_heads, key_dim, value_dim, ws,
                per_head=False, chunks=False, tokens_a_time=0):
     """The gated delta rule over every sequence of the step, in order, from and into the slots' states (float32
@@ -1018,7 +1051,6 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
     beside the others and four products a chunk along the sequence (three kernels)."""
     _need_cuda(qkv, decay_in, beta_in, a_log, dt_bias, state, out)
     lib = load_module("delta_rule")
-    lib.abk_delta_scan_scratch.restype = ctypes.c_longlong
     n, n_seqs = batch.n_rows, batch.seq_slot.numel()
     assert qkv.is_contiguous() and qkv.shape[1] == 2 * n_kv_heads * key_dim + n_heads * value_dim and qkv.shape[0] >= n
     if per_head:
@@ -1030,8 +1062,7 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
     assert a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32 and a_log.numel() == n_heads
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (n_heads, value_dim, key_dim)
     assert out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == n_heads * value_dim
-    records = ws.get("delta_records", (int(lib.abk_delta_scan_scratch(_i(n), _i(n_seqs), _i(n_heads), _i(key_dim), _i(value_dim),
-                                                                      _i(1 if chunks else 0))),), torch.float32)
+    records = ws.get("delta_records", (_delta_scan_scratch(n, n_seqs, n_heads, key_dim, value_dim, 1 if chunks else 0),), torch.float32)
     if chunks:
         assert per_head, "the chunked form takes one decay a head"
         max_chunks = -(-n // DELTA_CHUNK) + n_seqs
@@ -1042,11 +1073,11 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
             _p(batch.seq_slot), _i(n), _i(n_seqs), _i(n_heads), _i(n_kv_heads), _i(key_dim), _i(value_dim), _p(records),
             _ll(records.numel()), _i(max_chunks), _p(work), _ll(work.numel()), _stream()), "delta_chunks", kernels=3)
         return
-    _check(lib, lib.abk_delta_scan(_p(qkv), _ll(qkv.stride(0)), _i(_dt(qkv)), _p(decay_in), _ll(decay_in.stride(0)),
-                                   _i(1 if per_head else 0), _p(beta_in), _ll(beta_in.stride(0)), _p(a_log), _p(dt_bias), _p(state), _p(out), _p(batch.token_seq),
-                                   _p(batch.seq_start), _p(batch.seq_slot), _i(n), _i(n_seqs), _i(n_heads), _i(n_kv_heads),
-                                   _i(key_dim), _i(value_dim), _p(records), _ll(records.numel()), _i(tokens_a_time), _stream()),
-           "delta_scan", kernels=1 if n <= n_seqs else 2)
+    fn = _typed(lib.abk_delta_scan, "plipliplpppppppiiiiiiplip")
+    _check(lib, fn(qkv.data_ptr(), qkv.stride(0), _dt(qkv), decay_in.data_ptr(), decay_in.stride(0), 1 if per_head else 0, beta_in.data_ptr(),
+                   beta_in.stride(0), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(), batch.token_seq.data_ptr(),
+                   batch.seq_start.data_ptr(), batch.seq_slot.data_ptr(), n, n_seqs, n_heads, n_kv_heads, key_dim, value_dim,
+                   records.data_ptr(), records.numel(), tokens_a_time, _raw_stream()), "delta_scan", kernels=1 if n <= n_seqs else 2)
 
 
 def gated_head_norm(o, gate, weight, out, n_tokens, n_heads, value_dim, eps, silu=False):
@@ -1058,10 +1089,9 @@ def gated_head_norm(o, gate, weight, out, n_tokens, n_heads, value_dim, eps, sil
     assert o.dtype == torch.float32 and gate.dtype in (torch.float32, out.dtype) and weight.dtype == torch.float32
     assert o.is_contiguous() and gate.stride(1) == 1 and out.is_contiguous() and weight.numel() in (value_dim, n_heads * value_dim)
     assert o.shape[1] == gate.shape[1] == out.shape[1] == n_heads * value_dim
-    _check(lib, lib.abk_gated_head_norm(_p(o), _p(gate), _ll(gate.stride(0)), _i(0 if gate.dtype == torch.float32 else 1), _p(weight),
-                                        _p(out), _i(_dt(out)), _i(n_tokens), _i(n_heads), _i(value_dim), _f(eps),
-                                        _i(1 if silu else 0), _i(1 if weight.numel() != value_dim else 0), _stream()),
-           "gated_head_norm")
+    fn = _typed(lib.abk_gated_head_norm, "pplippiiiifiip")
+    _check(lib, fn(o.data_ptr(), gate.data_ptr(), gate.stride(0), 0 if gate.dtype == torch.float32 else 1, weight.data_ptr(), out.data_ptr(), _dt(out),
+                   n_tokens, n_heads, value_dim, eps, 1 if silu else 0, 1 if weight.numel() != value_dim else 0, _raw_stream()), "gated_head_norm")
 
 
 # ------------------------------------------------------------------ latent attention (csrc/latent.cu)
