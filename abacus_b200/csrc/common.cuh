@@ -171,6 +171,14 @@ __device__ __forceinline__ float silu_mul_fast(float gate, float up) {
     return gate * r * up;
 }
 
+// sigmoid(z) as above, for results that are stored in bfloat16.
+__device__ __forceinline__ float sigmoid_fast(float z) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return r;
+}
+
 // The activation of a gated feed-forward times its up value: ABK_SILU (above), ABK_RELU, or ABK_CLAMPED, which bounds both
 // first, g = min(gate, limit), u = clamp(up, -limit, limit), and gives g * sigmoid(1.702 g) * (u + 1).
 enum { ABK_SILU = 0, ABK_RELU = 1, ABK_CLAMPED = 2 };

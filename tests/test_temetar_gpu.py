@@ -667,3 +667,47 @@ def test_trace_replay_of_a_model_folder(tmp_path):
     assert_logits(got, np.stack([wa[0], wa[65], wb[7]]), "float32", "replayed prompt", noise)
     assert_logits(more[0].reshape(2, -1), np.stack([wa[66], wb[8]]), "float32", "replayed decode", noise)
     assert_logits(np.stack([m.reshape(-1, raw["vocab"])[0] for m in more[1:]]), wa[67:70], "float32", "replayed decode", noise)
+
+
+@pytest.mark.parametrize("T,H,V,silu", [(3, 5, 32, False), (2, 41, 64, True), (4, 3, 128, False), (5, 2, 256, True), (2, 3, 512, False), (3, 2, 96, True)])
+def test_gated_head_norm_of_every_head_size(T, H, V, silu):
+    """Heads in pieces of four, one CTA's heads and a remainder, gates of either type and rows of any pitch, and a head size that goes
+    number by number."""
+    from abacus_b200.kernels import ops
+    rng = np.random.default_rng(H * V)
+    o, rows = rng.standard_normal((T, H * V)).astype(np.float32), (4 * rng.standard_normal((T, H * V + 12))).astype(np.float32)
+    w = (1 + 0.1 * rng.standard_normal(H * V)).astype(np.float32)
+    for dtype, stored in ((torch.float32, False), (torch.bfloat16, False), (torch.bfloat16, True)):
+        gates = plain.bf16_round(rows) if stored else rows
+        for first in (0, 4, 1):  # (1: not aligned)
+            gate = gates[:, first:first + H * V].astype(np.float64)
+            want = plain.norm_plain(o.astype(np.float64).reshape(T, H, V), w.reshape(H, V).astype(np.float64), 1e-5).reshape(T, H * V) / (1 + np.exp(-gate)) * (gate if silu else 1)
+            out = torch.empty((T, H * V), dtype=dtype, device=DEV)
+            ops.gated_head_norm(dev(o), dev(gates, torch.bfloat16 if stored else torch.float32)[:, first:first + H * V], dev(w), out, T, H, V, 1e-5, silu=silu)
+            # bfloat16: half a unit of its eight bits, 2^-8 of a number at most
+            np.testing.assert_allclose(out.float().cpu().numpy(), want, rtol=2e-5 if dtype == torch.float32 else 2.0 ** -8, atol=2e-5)
+
+
+@pytest.mark.parametrize("lens,C,taps", [((1030,), 16, 4), ((700, 2, 1, 3, 330), 24, 3), ((1025, 1), 8, 2), ((3, 1, 2), 16, 4)])
+def test_short_convolution_of_several_tokens_a_thread(lens, C, taps):
+    """Groups of tokens that cross from sequence to sequence, rows before a sequence's start and from its slot's tail, both types."""
+    from abacus_b200.kernels import ops
+    rng = np.random.default_rng(C + taps)
+    w = rng.standard_normal((C, taps)).astype(np.float32)
+    tails = rng.standard_normal((len(lens), taps - 1, C)).astype(np.float32)
+    starts = [0 if i % 2 else 5 for i in range(len(lens))]
+    for dtype in (torch.float32, torch.bfloat16):
+        x = rng.standard_normal((sum(lens), C)).astype(np.float32)
+        x = plain.bf16_round(x) if dtype == torch.bfloat16 else x
+        b = batch_of([(i, [0] * n, s) for i, (n, s) in enumerate(zip(lens, starts))])
+        want, at = [], 0
+        for n, s, tail in zip(lens, starts, tails):
+            seen = np.concatenate([tail if s else np.zeros_like(tail), x[at:at + n]]).astype(np.float64)
+            want.append(sum(seen[j:j + n] * w[:, j] for j in range(taps)))
+            at += n
+        want = np.concatenate(want)
+        for plainly in (False, True):
+            out = torch.empty((sum(lens), C), dtype=dtype, device=DEV)
+            ops.short_conv(dev(x, dtype), C, dev(w), dev(tails), out, b, plain=plainly)
+            np.testing.assert_allclose(out.float().cpu().numpy(), want if plainly else want / (1 + np.exp(-want)),
+                                       rtol=2e-5 if dtype == torch.float32 else 2.0 ** -8, atol=2e-5)
