@@ -711,3 +711,20 @@ def test_short_convolution_of_several_tokens_a_thread(lens, C, taps):
             ops.short_conv(dev(x, dtype), C, dev(w), dev(tails), out, b, plain=plainly)
             np.testing.assert_allclose(out.float().cpu().numpy(), want if plainly else want / (1 + np.exp(-want)),
                                        rtol=2e-5 if dtype == torch.float32 else 2.0 ** -8, atol=2e-5)
+
+
+@pytest.mark.parametrize("lens,d,blends", [((1030,), 16, 5), ((700, 2, 1, 3, 330), 2048 + 8, 3), ((1025, 3), 24, 8), ((2, 5), 16, 1)])
+def test_token_shift_of_several_tokens_a_thread(lens, d, blends):
+    """Groups of tokens that cross from sequence to sequence; the rows that sequences left before, and those they leave."""
+    from abacus_b200.kernels import ops
+    rng = np.random.default_rng(d + blends)
+    x, mu, kept = rng.standard_normal((sum(lens), d)).astype(np.float32), rng.standard_normal((blends, d)).astype(np.float32), rng.standard_normal((len(lens), d)).astype(np.float32)
+    x, b, firsts = plain.bf16_round(x), batch_of([(i, [0] * n, 3) for i, n in enumerate(lens)]), np.cumsum((0,) + lens[:-1])
+    before = np.concatenate([kept[:1], x[:-1]])
+    before[firsts] = kept
+    last, out = dev(kept), torch.empty((blends, sum(lens), d), dtype=torch.bfloat16, device=DEV)
+    ops.token_shift(dev(x, torch.bfloat16), dev(mu), last, out, b)
+    want = x.astype(np.float64) + (before.astype(np.float64) - x) * mu[:, None].astype(np.float64)
+    # the difference and the blend rounded in float32, the result by half a unit of eight bits
+    np.testing.assert_allclose(out.float().cpu().numpy(), want, rtol=2.0 ** -8, atol=2e-6)
+    np.testing.assert_array_equal(last.cpu().numpy(), x[firsts + np.array(lens) - 1])
