@@ -15,9 +15,11 @@
 //   warps 2-9  a thread a query row (four warps a group): reads its row of S, masks (only in tiles that some row does not
 //              see whole), follows the row's maximum, and writes the three parts of the row's weights over its scores.
 // While one group's rows are in the softmax the tensor cores work for the other. Bound by the softmax warps: 995 instructions a
-// warp and tile, two warps to a scheduler, where the products of both groups take 1,100 cycles (tensor pipe 29 % of active
-// cycles). Measured: 3 prompts, 3,893 tokens, 32 query and 8 key heads of 128, a window of 1,024: 158 us (the warp-level kernel
-// 377); 32 heads of 192 with values of 128, no window: 191 (506).
+// warp and tile one weight at a time, two warps to a scheduler, where the products of both groups take 1,100 cycles (tensor pipe
+// 29 % of active cycles). Two weights at a time need one multiply-add, sum or remainder for both and give the same bits. Measured one
+// weight at a time: 3 prompts, 3,893 tokens, 32 query and 8 key heads of 128, a window of 1,024: 158 us (the warp-level kernel 377);
+// 32 heads of 192 with values of 128, no window: 191 (506); two at a time the whole layers, products and all, go from 398 to 392 and
+// from 416 to 411 us.
 // Tensor memory: two groups of 128 columns of output and of 96 columns of scores and weights, 512 in all, so a CTA to an SM.
 // A value row beyond the sequence's end belongs to another sequence or to nothing, and a weight of zero times what is no
 // number is none: the rows are set to zero in shared memory before the tile that crosses the end is multiplied.
@@ -26,6 +28,7 @@
 // Every wait on an mbarrier is bounded; one that runs out sets status word 3 and the CTA winds down.
 #define ABK_DEFINE_ERROR
 #include "common.cuh"
+#include "recurrence.cuh"
 #include "tc_common.cuh"
 #include "tensor_map.cuh"
 
@@ -282,26 +285,32 @@ __global__ void __launch_bounds__(WT_THREADS, 1) attention_window_tc_kernel(cons
             const bool move = __any_sync(0xffffffffu, m_new != m);
             const float corr = m_new != m ? exp2f(m - ref) : 1.0f;  // (0 when m was -inf)
             m = m_new;
-            float sum0 = 0.0f, sum1 = 0.0f;
+            // two weights at a time: an instruction for both where there is one (the same numbers, fewer to issue)
+            const f32x2 scale2 = pack2(p.scale_log2, p.scale_log2), ref2 = pack2(-ref, -ref), minus = pack2(-1.0f, -1.0f);
+            f32x2 sum2 = pack2(0.0f, 0.0f);
 #pragma unroll
             for (int c0 = 0; c0 < WT_K; c0 += 32) {
                 uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
                 for (int c = 0; c < 32; c += 2) {
-                    float x0 = wt_ex2(fmaf(s[c0 + c], p.scale_log2, -ref)), x1 = wt_ex2(fmaf(s[c0 + c + 1], p.scale_log2, -ref));
-                    sum0 += x0, sum1 += x1;
-                    __nv_bfloat162 b = __floats2bfloat162_rn(x0, x1);
+                    float2 x = unpack2(fma2(pack2(s[c0 + c], s[c0 + c + 1]), scale2, ref2));
+                    x.x = wt_ex2(x.x), x.y = wt_ex2(x.y);
+                    f32x2 x2 = pack2(x.x, x.y);
+                    sum2 = add2(sum2, x2);
+                    __nv_bfloat162 b = __floats2bfloat162_rn(x.x, x.y);
                     hi[c / 2] = *(const uint32_t *)&b;
-                    x0 -= __uint_as_float(hi[c / 2] << 16), x1 -= __uint_as_float(hi[c / 2] & 0xffff0000u);
-                    b = __floats2bfloat162_rn(x0, x1);
+                    x2 = fma2(pack2(__uint_as_float(hi[c / 2] << 16), __uint_as_float(hi[c / 2] & 0xffff0000u)), minus, x2);
+                    x = unpack2(x2);
+                    b = __floats2bfloat162_rn(x.x, x.y);
                     mid[c / 2] = *(const uint32_t *)&b;
-                    x0 -= __uint_as_float(mid[c / 2] << 16), x1 -= __uint_as_float(mid[c / 2] & 0xffff0000u);
-                    b = __floats2bfloat162_rn(x0, x1);
+                    x = unpack2(fma2(pack2(__uint_as_float(mid[c / 2] << 16), __uint_as_float(mid[c / 2] & 0xffff0000u)), minus, x2));
+                    b = __floats2bfloat162_rn(x.x, x.y);
                     lo[c / 2] = *(const uint32_t *)&b;
                 }
                 wt_tmem_st16(scores + c0 / 2, hi), wt_tmem_st16(scores + 32 + c0 / 2, mid), wt_tmem_st16(scores + 64 + c0 / 2, lo);
             }
-            l = l * corr + (sum0 + sum1);
+            const float2 sums = unpack2(sum2);
+            l = l * corr + (sums.x + sums.y);
             if (done > 0 && move) {  // (the second product of the tile before is done: the first product of this one waited for it)
 #pragma unroll 1
                 for (int c0 = 0; c0 < VB * 64; c0 += 16) {
