@@ -93,7 +93,7 @@ class StepBatch:
         self.max_len_after = 0
         self.is_decode = False
         self.any_continuation = False
-        self._sent = None
+        self._sent, self._sent_on = None, set()
 
     def fill(self, sequences, pad_logits=False, exact=False):
         """Write the step described by `sequences` (list of Sequence) and send it to the device.
@@ -169,10 +169,16 @@ class StepBatch:
 
     def _send(self):
         """The host's words to the device, in the order of the device's current stream."""
-        if self._sent is not None and self._dev.get_device() == torch.cuda.current_device():
-            from ..kernels import ops
-            ops.send_words(self._dev, self._host, self._sent)  # (a copy and an event by torch cost the host four times as long)
-            return
+        # The first copy on a stream is torch's: its allocator then keeps the pinned words, should they be freed, until that stream has read
+        # them. A copy and an event by torch cost the host four times as long, so the later ones go straight to the runtime.
+        index = self._dev.get_device()
+        if index >= 0:
+            stream = torch._C._cuda_getCurrentRawStream(index)
+            if stream in self._sent_on and index == torch.cuda.current_device():
+                from ..kernels import ops
+                ops.send_words(self._dev, self._host, self._sent)
+                return
+            self._sent_on.add(stream)
         self._dev.copy_(self._host, non_blocking=True)
         if self.device.type == "cuda":
             self._sent = self._sent or torch.cuda.Event()

@@ -568,6 +568,21 @@ def test_refusals_are_errors_not_results(ops):
         ops.swiglu(torch.zeros(2, 4), torch.zeros(2, 2))
 
 
+def test_a_steps_words_are_made_known_to_each_stream_that_copies_them(ops, monkeypatch):
+    """torch's allocator has to hear of every stream that reads the pinned words: the first copy on a stream is torch's, the
+    others go straight to the runtime."""
+    from abacus_b200.engine.batch import Sequence, StepBatch
+    sent, straight = [], ops.send_words
+    monkeypatch.setattr(ops, "send_words", lambda dst, src, event: (sent.append(1), straight(dst, src, event)))
+    batch, streams = StepBatch(4, 2, 0, "cuda"), [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for n, (stream, straight_so_far) in enumerate([(0, 0), (0, 1), (1, 1), (1, 2), (0, 3)]):
+        with torch.cuda.stream(streams[stream]):
+            batch.fill([Sequence(1, [n, 7], n, []), Sequence(0, [n + 9], 3, [])])
+            assert batch.tokens.tolist() == [n, 7, n + 9, 0] and batch.token_pos[:3].tolist() == [n, n + 1, 3]
+        assert len(sent) == straight_so_far
+
+
 # ------------------------------------------------------------------ tensor-core matrix product
 
 def product_tolerance(want, k, out_dtype):
