@@ -1,7 +1,7 @@
 // out[M, N] = x[M, K] . w[N, K]^T with float32 multiply-adds, for any M, N, K.
 //
 // This is the matrix product of the true 32-bit path (no TF32), and the fallback of the bfloat16 path for shapes the tensor-core
-// kernel refuses. Large float32 products go to the tensor cores without a digit less (gemm_split.cuh); here an output element is the sum of eight running
+// kernel refuses. Large products go to the tensor cores, with smaller errors (gemm_split.cuh); here an output element is the sum of eight running
 // sums: K in pieces of 16, piece c to sum c % 8, each sum over its k in ascending order, then in pairs,
 // ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); up to K = 256 it is one sum over k in ascending order (a chain of that
 // length needs no cutting, and the small products of small models keep the order they had). So a row's result does not
@@ -176,7 +176,7 @@ static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int 
 }
 
 // The product on the tensor cores (gemm_split.cuh), for any sizes. bn: rows of x in a tile (32, 64, 96, 128), quarters: pairs of CTAs take
-// quarters of K; 0, 0: by size. scratch: abk_gemm_split_scratch bytes.
+// quarters of K (of float32 operands only); 0, 0: by size. scratch: abk_gemm_split_scratch bytes.
 extern "C" int abk_gemm_split(const void *x, const void *w, int dtype, void *out, int out_dtype, int M, int N, int K, long long ldx, long long ldw,
                               long long ldo, int bn, int quarters, void *scratch, int *status, void *stream) {
     const GemmSplit g = {x, w, out, dtype, out_dtype, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};
@@ -187,9 +187,13 @@ extern "C" long long abk_gemm_split_scratch(int M, int N, int K) { return gemm_s
 
 // Whether a product goes to the tensor cores: more than a handful of rows (up to 32 rows the plain kernel reads the weights once and
 // writes nothing beside: 17 x 6144 x 1024 in 19 us against 23), and enough to do for two or three launches in place of one, whose
-// host side takes some 12 us more: 64 x 6144 x 1024 in 25 us against 32, 100 x 4096 x 1024 in 24 against 35, 500 x 1024 x 1024 in 18 against
-// 35; below that there is little to win (64 x 1024 x 1024: 12.8 against 13.4; 500 x 256 x 512: 10.3 against 7.9).
-static bool gemm_split_wins(int M, int N, int K) { return M > 32 && N >= 64 && K >= 512 && (long long)M * N * K >= 400000000LL; }
+// host side takes some 12 us more: 64 x 6144 x 1024 in 27 us against 32, 100 x 4096 x 1024 in 21 against 36, 500 x 1024 x 1024 in 20 against
+// 35; below that there is little to win (64 x 1024 x 1024: 12.8 against 13.4; 500 x 256 x 512: 10.3 against 7.9). 64 columns are one of the plain
+// kernel's tiles and a quarter of a pair's: 6300 x 64 x 1024 in 39 us against 36, x 72 in 39 against 67. Up to 64 rows are one of its tiles too, and
+// weights beyond the L2 are written and read again as parts: 33 x 40960 x 1024 in 145 against 157, x 65536 in 231 against 223.
+static bool gemm_split_wins(int M, int N, int K) {
+    return M > 32 && N > 64 && K >= 512 && (long long)M * N * K >= 400000000LL && (M > 64 || N < 65536);
+}
 // Bytes of scratch memory with which abk_gemm_simt goes to the tensor cores (0: it does not).
 extern "C" long long abk_gemm_simt_scratch(int M, int N, int K) { return gemm_split_wins(M, N, K) ? gemm_split_scratch(M, N, K) : 0; }
 

@@ -1,30 +1,40 @@
-// out[M, N] = x[M, K] . w[N, K]^T of float32 operands on the tensor cores, with no digit of float32 given up.
+// out[M, N] = x[M, K] . w[N, K]^T of float32 operands on the tensor cores, with errors below those of eight float32 sums.
 //
 // A float32 number is the sum of three bfloat16 numbers (8 + 8 + 8 bits, each rounded to nearest: what is left over is below
 // 2^-26 of it), x = x1 + x2 + x3, so x w is the six products x1 w1, x1 w2, x2 w1, x2 w2, x1 w3, x3 w1; the three left out are
 // below 2^-26. The tensor cores multiply bfloat16 without rounding and add in float32, but cut a sum off where float32
-// rounds it, and a sum over a long K cut off at every step drifts towards zero. So x1 w1 is added up in tensor memory over 128
-// of K only; these short sums are added in registers, rounded. The five small products have an accumulator of their own, whose
+// rounds it, and a sum over a long K cut off at every step of 16 drifts towards zero. So x1 w1 is added up in tensor memory over a few
+// steps only; these short sums are added in registers, rounded. The five small products have an accumulator of their own, whose
 // cuts are 2^-8 as large.
 //
-// An element is the sum of four running sums, over the quarters of K in order: ((q0 + q1) + q2) + q3, each over its pieces of
-// 128 in order, then its small products. That order goes by K alone: a row's result does not depend on how many other rows
+// Errors against 64 bits (2-norm, in units of 1e-8; K = 512, 768, 1024, 2048, 3072, 9728) with sums over 16, 32 and 64 of K, and of the eight
+// rounded sums on the CUDA cores:
+//     numbers of either sign   16: 7.5 8.2 9.0 11.6 13.7 23.3   32: 7.4 7.9 8.4  9.9 11.2 17.5   64: 8.6 8.9 9.1 9.9 10.6 14.5   15.2 18.3 20.9 29.1 35.5 62.5
+//     their magnitudes         16: 5.1 4.8 5.5  6.2  6.0 10.2   32: 5.9 5.6 6.0  6.4  6.0  8.5   64: 9.0 8.8 9.0 9.0  8.8  9.8    5.9  6.0  7.4  9.6  9.9 18.8
+// (numbers of one sign: the cuts all go one way, 1.6, 3.7 and 7.7e-8 too small, and 17e-8 with sums over 128). So the short sums grow with K, as
+// the CUDA cores' errors do: over 16 below K = 1024, over 32 below 2048, else over 64, below the CUDA cores' in every one of these.
+//
+// An element is the sum of four running sums, over the quarters of K in order: ((q0 + q1) + q2) + q3, each over its short sums in
+// order, then its small products. That order goes by K alone: a row's result does not depend on how many other rows
 // are in the batch, whether a pair of CTAs walks all of K or a quarter, or where its tile lies.
-// bfloat16 operands (those that the tensor-core product proper refuses: rows that start anywhere) go the same way with one part.
+// bfloat16 operands (those that the tensor-core product proper refuses: rows that start anywhere) have one part. Their eight sums on the CUDA
+// cores lose less, a product being exact there too, so their short sums, over 16, are added in one running sum with what each addition rounds off
+// beside it (Knuth's two-sum), added at the end. (In float32 that takes 2048 x 1024 x 1020 from 22 us, with errors of 1.3e-7, to 68, with 0.35e-7;
+// the CUDA cores 148, 0.9e-7.)
 // A number that is not finite makes its products NaN in this form; an element that came out not finite is taken again with
 // plain multiply-adds. (Numbers below 1e-33 keep fewer digits: their third part is too small for bfloat16.)
 //
-// What bounds it: for thousands of rows the tensor cores under the power cap (4000 x 6144 x 1024 in 258 us, 1,230 TFLOP/s of bfloat16 products
-// at 1.63 GHz; on the CUDA cores 1,349), for some hundred the way of the parts from the L2, 6 bytes a number, at some 30 bytes
-// a cycle and SM, and the pieces that the last turn leaves empty (500 x 6144 x 1024 in 53 us, 9 of them for the parts; 195 on the
-// CUDA cores). Errors against 64 bits (2-norm, normal numbers): 1.3e-7 for K from 512 to 3072, where eight float32 sums have 1.5e-7
-// to 3.5e-7.
+// What bounds it: the chain between the tensor cores and the warps that add up (0.3 us a short sum), and the way of the parts from
+// the L2, 6 bytes a number, at some 30 bytes a cycle and SM (500 x 6144 x 1024 in 65 us, 9 of them for the parts; sums of 128 53, the CUDA
+// cores 197; 4000 x 6144 x 1024 in 333 us, 253, 1,349). The adding warps report to their own CTA's barrier and the pair's idle warp passes
+// that on: 16 warps' words to the other CTA's barrier, one by one, took 72 us for 63.
 //
 // Two kernels: one writes the operands' parts as three planes of bfloat16 each, the other multiplies them on pairs of CTAs. (As one kernel
 // that splits what it fetches, weights again for every column of tiles: 500 x 6144 x 1024 in 71 us, bound by the instructions
 // of the splitting and by the way of plain loads through what the stages leave of the L1.)
 #pragma once
 #include "bf16_parts.cuh"
+#include "recurrence.cuh"
 #include "tc_common.cuh"
 #include "tensor_map.cuh"
 
@@ -39,7 +49,11 @@ template <int BN> struct GpShape {
     static constexpr int STAGES = 3, X_ROWS = BN / 2;
     static constexpr int W_PLANE = GP_ROWS * GP_K * 2, X_PLANE = X_ROWS * GP_K * 2, STAGE = 3 * (W_PLANE + X_PLANE);
     static constexpr int BYTES = STAGES * STAGE + 1024 /* alignment */ + 256 /* barriers */;
-    static constexpr int TMEM = BN == 96 ? 512 : 4 * BN;  // two accumulators of x1 w1 and two of the small products
+    // accumulators of x1 w1 (three or four in turn where they fit: 63.3 -> 62.4 us with tiles of 96; two with 128: 65.4 against 70.0)
+    // and two of the small products
+    static constexpr int SUMS = BN == 128 ? 2 : BN == 96 ? 3 : 4, SMALLS = 2, ACCUMULATORS = SUMS + SMALLS;
+    static constexpr int TMEM = BN == 32 ? 256 : 512;
+    static_assert(ACCUMULATORS * BN <= TMEM, "the accumulators fill tensor memory");
     static constexpr int COLS = BN / 4;                   // of the accumulator that a warp adds up
 };
 
@@ -100,7 +114,7 @@ template <typename T> __global__ void __launch_bounds__(256) gemm_split_rows_ker
 struct GemmSplit {
     const void *x, *w;
     void *out;
-    int dtype, out_dtype;  // of x and w, ABK_F32 (three parts) or ABK_BF16 (one); of out
+    int dtype, out_dtype;  // of x and w, ABK_F32 or ABK_BF16; of out
     int M, N, K, m_tiles, tiles;
     long long ldx, ldw, ldo;
     int *status;
@@ -123,23 +137,25 @@ __device__ __forceinline__ void gp_put(const GemmSplit &g, int m, int n, float v
 
 // A tile is 256 rows of w (128 of each CTA) and BN rows of x; pair c of CTAs takes items c, c + pairs, ... An item is a tile, or
 // (QUARTERS) a quarter of K of one, whose sums go to `quarters` and are added up by the kernel behind.
-// map_w, map_x: the planes, one below the other.
-template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w,
+// map_w, map_x: the planes, one below the other; PARTS: 3 of float32 operands, 1 of bfloat16 ones; STEPS: of 16 of K in a
+// short sum, 1, 2 or 4.
+template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_bounds__(GP_THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                                                const __grid_constant__ CUtensorMap map_x, GemmSplit g) {
     using S = GpShape<BN>;
-    constexpr int STAGES = S::STAGES, COLS = S::COLS;
+    constexpr int STAGES = S::STAGES, COLS = S::COLS, SUMS = S::SUMS, SMALLS = S::SMALLS;
     extern __shared__ uint8_t gp_smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)gp_smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = (uint64_t *)(smem + STAGES * S::STAGE), *empty = full + STAGES;
-    uint64_t *sum_ready = empty + STAGES, *sum_free = sum_ready + 2, *small_free = sum_free + 2;
-    uint32_t *tmem_holder = (uint32_t *)(small_free + 2);
+    uint64_t *sum_ready = empty + STAGES, *sum_free = sum_ready + SUMS, *small_free = sum_free + SUMS;
+    uint32_t *tmem_holder = (uint32_t *)(small_free + SMALLS);
     volatile int *gave_up = (volatile int *)(tmem_holder + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t half = tc::cluster_rank();  // 0: the leader
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) tc::mbar_init(&full[s], 1), tc::mbar_init(&empty[s], 1);
-        // sum_free, small_free: every adding warp of both CTAs, on the leader's
-        for (int b = 0; b < 2; b++) tc::mbar_init(&sum_ready[b], 1), tc::mbar_init(&sum_free[b], 2 * GP_ADDERS), tc::mbar_init(&small_free[b], 2 * GP_ADDERS);
+        // sum_free, small_free: every adding warp of the CTA, and, on the leader's, the peer's word that all of its own have
+        for (int b = 0; b < SUMS; b++) tc::mbar_init(&sum_ready[b], 1), tc::mbar_init(&sum_free[b], GP_ADDERS + (half == 0));
+        for (int b = 0; b < SMALLS; b++) tc::mbar_init(&small_free[b], GP_ADDERS + (half == 0));
         *gave_up = 0;
         tc::mbar_init_fence();
         tc::tma_prefetch_map(&map_w), tc::tma_prefetch_map(&map_x);
@@ -150,7 +166,8 @@ template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1
     tc::fence_after_sync();
     const uint32_t tmem = *tmem_holder;
 
-    const int pieces = (g.K + GP_K - 1) / GP_K, parts = g.dtype == ABK_F32 ? 3 : 1;
+    const int pieces = (g.K + GP_K - 1) / GP_K;
+    constexpr int sums_a_piece = GP_K / 16 / STEPS;
     const int items = QUARTERS ? g.tiles * GP_QUARTERS : g.tiles, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const auto first_quarter = [&](int item) { return QUARTERS ? item / g.tiles : 0; };
     const auto last_quarter = [&](int item) { return QUARTERS ? item / g.tiles : GP_QUARTERS - 1; };
@@ -170,10 +187,10 @@ template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1
                         ok = false;
                         break;
                     }
-                    if (half == 0) tc::mbar_expect_tx(&full[s], parts * 2 * (S::W_PLANE + S::X_PLANE));  // both CTAs' copies report to the leader
+                    if (half == 0) tc::mbar_expect_tx(&full[s], PARTS * 2 * (S::W_PLANE + S::X_PLANE));  // both CTAs' copies report to the leader
                     const uint32_t bar = tc::peer_smem(tc::smem_addr(&full[s]), 0);
                     uint8_t *stage = smem + s * S::STAGE;
-                    for (int t = 0; t < parts; t++) {
+                    for (int t = 0; t < PARTS; t++) {
                         tc::tma_load_2d_pair(stage + t * S::W_PLANE, &map_w, p * GP_K, t * g.N + n0, bar);
                         tc::tma_load_2d_pair(stage + 3 * S::W_PLANE + t * S::X_PLANE, &map_x, p * GP_K, t * g.M + m0, bar);
                     }
@@ -185,36 +202,55 @@ template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1
     } else if (warp == GP_ADDERS + 1) {
         if (lane == 0 && half == 0) {
             constexpr uint32_t idesc = tc::idesc_bf16_f32(2 * GP_ROWS, BN);
-            int i = 0, sum_i = 0, quarter_i = 0;  // pieces, sums and quarters so far
+            int i = 0, sum_i = 0, quarter_i = 0;  // pieces, short sums and quarters so far
             bool ok = true;
             for (int item = pair; ok && item < items; item += pairs) {
                 for (int q = first_quarter(item); ok && q <= last_quarter(item); q++, quarter_i++) {
                     const int q_begin = begin_of(q), q_end = begin_of(q + 1);
-                    ok = quarter_i < 2 || tc::mbar_wait(&small_free[quarter_i & 1], ((quarter_i >> 1) & 1) ^ 1);
+                    const uint32_t small = tmem + (SUMS + quarter_i % SMALLS) * BN;
+                    if (PARTS == 3) ok = quarter_i < SMALLS || tc::mbar_wait(&small_free[quarter_i % SMALLS], ((quarter_i / SMALLS) & 1) ^ 1);
                     for (int p = q_begin; ok && p < q_end; p++, i++) {
-                        const int s = i % STAGES, b = sum_i & 1;
-                        const bool starts = ((p - q_begin) & 1) == 0, ends = !starts || p + 1 == q_end;
-                        if (starts) ok = sum_i < 2 || tc::mbar_wait(&sum_free[b], ((sum_i >> 1) & 1) ^ 1);
-                        ok = ok && tc::mbar_wait(&full[s], (i / STAGES) & 1);
-                        if (!ok) break;
+                        const int s = i % STAGES;
+                        if (!(ok = tc::mbar_wait(&full[s], (i / STAGES) & 1))) break;
                         tc::fence_after_sync();
                         const uint32_t at = tc::smem_addr(smem + s * S::STAGE);
                         const uint64_t w1 = tc::smem_desc_k_sw128(at), w2 = w1 + (S::W_PLANE >> 4), w3 = w2 + (S::W_PLANE >> 4);
                         const uint64_t x1 = w3 + (S::W_PLANE >> 4), x2 = x1 + (S::X_PLANE >> 4), x3 = x2 + (S::X_PLANE >> 4);
-                        const uint32_t sum = tmem + b * BN, small = tmem + (2 + (quarter_i & 1)) * BN;
 #pragma unroll
-                        for (int k = 0; k < GP_K / 16; k++) {  // (16 of K: 32 bytes of a row)
-                            tc::mma_ss_pair(sum, w1 + 2 * k, x1 + 2 * k, idesc, !starts || k > 0);
-                            if (parts == 1) continue;
-                            tc::mma_ss_pair(small, w1 + 2 * k, x2 + 2 * k, idesc, p > q_begin || k > 0);
-                            tc::mma_ss_pair(small, w2 + 2 * k, x1 + 2 * k, idesc, true);
-                            tc::mma_ss_pair(small, w2 + 2 * k, x2 + 2 * k, idesc, true);
-                            tc::mma_ss_pair(small, w1 + 2 * k, x3 + 2 * k, idesc, true);
-                            tc::mma_ss_pair(small, w3 + 2 * k, x1 + 2 * k, idesc, true);
+                        for (int k0 = 0; k0 < GP_K / 16; k0 += STEPS) {  // (16 of K: 32 bytes of a row)
+                            const int b = sum_i % SUMS;
+#pragma unroll
+                            for (int k = k0; k < k0 + STEPS; k++) {
+                                if (PARTS == 1) continue;  // (ahead of the wait: they keep the tensor cores busy while a sum is read)
+                                tc::mma_ss_pair(small, w1 + 2 * k, x2 + 2 * k, idesc, p > q_begin || k > 0);
+                                tc::mma_ss_pair(small, w2 + 2 * k, x1 + 2 * k, idesc, true);
+                                tc::mma_ss_pair(small, w2 + 2 * k, x2 + 2 * k, idesc, true);
+                                tc::mma_ss_pair(small, w1 + 2 * k, x3 + 2 * k, idesc, true);
+                                tc::mma_ss_pair(small, w3 + 2 * k, x1 + 2 * k, idesc, true);
+                            }
+                            if (!(ok = sum_i < SUMS || tc::mbar_wait(&sum_free[b], ((sum_i / SUMS) & 1) ^ 1))) break;
+                            tc::fence_after_sync();
+#pragma unroll
+                            for (int k = k0; k < k0 + STEPS; k++) tc::mma_ss_pair(tmem + b * BN, w1 + 2 * k, x1 + 2 * k, idesc, k > k0);
+                            tc::mma_commit_pair(&sum_ready[b]), sum_i++;
                         }
-                        tc::mma_commit_pair(&empty[s]);
-                        if (ends) tc::mma_commit_pair(&sum_ready[b]), sum_i++;
+                        if (ok) tc::mma_commit_pair(&empty[s]);
                     }
+                }
+            }
+            if (!ok) *gave_up = 1;
+        } else if (lane == 0) {  // the peer: what its adding warps have read, passed on to the leader
+            int sum_i = 0, quarter_i = 0;
+            bool ok = true;
+            for (int item = pair; ok && item < items; item += pairs) {
+                for (int q = first_quarter(item); ok && q <= last_quarter(item); q++, quarter_i++) {
+                    const int sums = (begin_of(q + 1) - begin_of(q)) * sums_a_piece;
+                    for (int n = 0; ok && n < sums; n++, sum_i++) {
+                        ok = tc::mbar_wait(&sum_free[sum_i % SUMS], (sum_i / SUMS) & 1);
+                        if (ok) tc::mbar_arrive_in_cluster(tc::peer_smem(tc::smem_addr(&sum_free[sum_i % SUMS]), 0));
+                    }
+                    if (PARTS == 3) ok = ok && tc::mbar_wait(&small_free[quarter_i % SMALLS], (quarter_i / SMALLS) & 1);
+                    if (PARTS == 3 && ok) tc::mbar_arrive_in_cluster(tc::peer_smem(tc::smem_addr(&small_free[quarter_i % SMALLS]), 0));
                 }
             }
             if (!ok) *gave_up = 1;
@@ -225,7 +261,8 @@ template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1
         // a warp has a quarter of the lanes (the weights' rows) and COLS columns (rows of x) of the accumulators
         const int lane_base = (warp & 3) * 32, col0 = (warp >> 2) * COLS;
         const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + col0;
-        float sum[COLS], total[COLS];
+        float sum[COLS], total[COLS];  // of the quarter, of those before; PARTS 1: of all, and what its additions rounded off
+        const f32x2 minus = pack2(-1.0f, -1.0f);
 #pragma unroll
         for (int j = 0; j < COLS; j++) sum[j] = total[j] = 0.0f;
         int sum_i = 0, quarter_i = 0;
@@ -234,11 +271,11 @@ template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1
         for (int item = pair; ok && item < items; item += pairs) {
 #pragma unroll 1
             for (int q = first_quarter(item); q <= last_quarter(item); q++, quarter_i++) {
-                const int sums = (begin_of(q + 1) - begin_of(q) + 1) / 2;
+                const int sums = (begin_of(q + 1) - begin_of(q)) * sums_a_piece;
 #pragma unroll 1
                 for (int n = 0; n < sums; n++, sum_i++) {
-                    const int b = sum_i & 1;
-                    ok = __all_sync(0xffffffffu, ok && tc::mbar_wait(&sum_ready[b], (sum_i >> 1) & 1));
+                    const int b = sum_i % SUMS;
+                    ok = __all_sync(0xffffffffu, ok && tc::mbar_wait(&sum_ready[b], (sum_i / SUMS) & 1));
                     tc::fence_after_sync();
                     uint32_t v[8];
 #pragma unroll
@@ -246,22 +283,32 @@ template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1
                         gp_tmem_ld<8>(taddr + b * BN + c, v);
                         tc::tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 8; j++) sum[c + j] += __uint_as_float(v[j]);
+                        for (int j = 0; j < 8; j += 2) {
+                            float *const s2 = sum + c + j, *const t2 = total + c + j;
+                            if constexpr (PARTS == 3) {
+                                s2[0] += __uint_as_float(v[j]), s2[1] += __uint_as_float(v[j + 1]);
+                            } else {
+                                const f32x2 a = pack2(s2[0], s2[1]), b2 = pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+                                const f32x2 both = add2(a, b2), of_b = fma2(a, minus, both), of_a = fma2(of_b, minus, both);
+                                const float2 r = unpack2(both), lost = unpack2(add2(pack2(t2[0], t2[1]), add2(fma2(of_a, minus, a), fma2(of_b, minus, b2))));
+                                s2[0] = r.x, s2[1] = r.y, t2[0] = lost.x, t2[1] = lost.y;
+                            }
+                        }
                     }
-                    if (n + 1 == sums) {
+                    if (PARTS == 3 && n + 1 == sums) {
 #pragma unroll
                         for (int c = 0; c < COLS; c += 8) {
-                            gp_tmem_ld<8>(taddr + (2 + (quarter_i & 1)) * BN + c, v);
+                            gp_tmem_ld<8>(taddr + (SUMS + quarter_i % SMALLS) * BN + c, v);
                             tc::tmem_ld_wait();
 #pragma unroll
-                            for (int j = 0; j < 8; j++) total[c + j] += sum[c + j] + (parts == 1 ? 0.0f : __uint_as_float(v[j])), sum[c + j] = 0.0f;
+                            for (int j = 0; j < 8; j++) total[c + j] += sum[c + j] + __uint_as_float(v[j]), sum[c + j] = 0.0f;
                         }
                     }
                     tc::fence_before_sync();
                     __syncwarp();
                     if (lane == 0) {
-                        tc::mbar_arrive_in_cluster(tc::peer_smem(tc::smem_addr(&sum_free[b]), 0));
-                        if (n + 1 == sums) tc::mbar_arrive_in_cluster(tc::peer_smem(tc::smem_addr(&small_free[quarter_i & 1]), 0));
+                        tc::mbar_arrive(&sum_free[b]);
+                        if (PARTS == 3 && n + 1 == sums) tc::mbar_arrive(&small_free[quarter_i % SMALLS]);
                     }
                 }
             }
@@ -276,10 +323,10 @@ template <int BN, bool QUARTERS> __global__ void __launch_bounds__(GP_THREADS, 1
                 } else {
 #pragma unroll
                     for (int j = 0; j < COLS; j++)
-                        if (j < cols) gp_put(g, m0 + j, n, total[j]);
+                        if (j < cols) gp_put(g, m0 + j, n, PARTS == 3 ? total[j] : sum[j] + total[j]);
                 }
 #pragma unroll
-                for (int j = 0; j < COLS; j++) total[j] = 0.0f;
+                for (int j = 0; j < COLS; j++) sum[j] = total[j] = 0.0f;
             }
         }
         if (!ok) *gave_up = 1;
@@ -303,12 +350,12 @@ __global__ void __launch_bounds__(256) gemm_split_sum_kernel(GemmSplit g) {
     }
 }
 
-template <int BN, bool QUARTERS> static int gemm_split_launch(const CUtensorMap &map_w, const CUtensorMap &map_x, GemmSplit g, cudaStream_t s) {
+template <int BN, bool QUARTERS, int PARTS, int STEPS> static int gemm_split_launch(const CUtensorMap &map_w, const CUtensorMap &map_x, GemmSplit g, cudaStream_t s) {
     using S = GpShape<BN>;
-    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_split_kernel<BN, QUARTERS>, S::BYTES);
+    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_split_kernel<BN, QUARTERS, PARTS, STEPS>, S::BYTES);
     if (e != cudaSuccess) return (int)e;
     const int pairs = abk_sm_count() / 2, items = QUARTERS ? g.tiles * GP_QUARTERS : g.tiles;
-    abk_launch_clusters(gemm_split_kernel<BN, QUARTERS>, dim3(2 * (items < pairs ? items : pairs)), dim3(GP_THREADS), S::BYTES, s, 2, map_w, map_x, g);
+    abk_launch_clusters(gemm_split_kernel<BN, QUARTERS, PARTS, STEPS>, dim3(2 * (items < pairs ? items : pairs)), dim3(GP_THREADS), S::BYTES, s, 2, map_w, map_x, g);
     const int rc = ABK_LAUNCH_RESULT();
     if (rc || !QUARTERS) return rc;
     const long long blocks = ((long long)g.M * g.N + 255) / 256, most = 8LL * abk_sm_count();
@@ -319,17 +366,22 @@ template <int BN, bool QUARTERS> static int gemm_split_launch(const CUtensorMap 
 #define GP_QUARTERS_BYTES (64LL << 20)  // sums of quarters in the scratch memory at most
 static bool gp_may_quarter(int M, int N) { return 4LL * GP_QUARTERS * M * N <= GP_QUARTERS_BYTES; }
 
+// Steps of 16 of K in a short sum of float32 operands' parts.
+static int gp_steps(int K) { return K < 1024 ? 1 : K < 2048 ? 2 : 4; }
+
 // Rows of x in a tile, and whether pairs of CTAs take quarters of K: what takes least, by turns of the GPU's pairs times what a
-// piece of 64 of K takes (measured with a turn each: 1.0 us for tiles of 32 rows, 1.05, 1.15, 1.25 for 128: the way from the L2
-// counts for more than the products, 1,104 to 1,536 cycles), and the passes over the quarters' sums. 500 x 6144 x 1024 in tiles of 96:
-// 53 us, of 128: 55, of 64: 69, in quarters 69; 500 x 1024 x 3072 in quarters with tiles of 128: 30 us, of 64: 42, whole: 65.
-static void gp_choose(int M, int N, int K, bool may_quarter, int &bn, int &quarters) {
-    static const struct { int bn; float us; } tile[4] = {{32, 1.0f}, {64, 1.05f}, {96, 1.15f}, {128, 1.25f}};
+// piece of 64 of K takes (measured with a turn each: 1.2 us for tiles of 32 rows, 1.25, 1.35, 1.5 for 128 with sums over 64, a fifth more
+// over 32, half as much again over 16: the way from the L2 and the chain count for more than the products, 1,104 to 1,536 cycles), and the passes over the quarters'
+// sums. 500 x 6144 x 1024 in tiles of 96: 62 us, of 128: 65, of 64: 81, in quarters 79; 500 x 1024 x 3072 in quarters with tiles of 128: 30 us, of
+// 64: 41, whole: 63.
+static void gp_choose(int M, int N, int K, int parts, bool may_quarter, int &bn, int &quarters) {
+    static const struct { int bn; float us; } tile[4] = {{32, 1.2f}, {64, 1.25f}, {96, 1.35f}, {128, 1.5f}};
     const long long pairs = abk_sm_count() / 2;
-    const float pieces = (float)((K + GP_K - 1) / GP_K);
+    const float pieces = (float)((K + GP_K - 1) / GP_K) * (gp_steps(K) == 4 ? 1.0f : gp_steps(K) == 2 ? 1.2f : 1.6f);  // (in those of sums over 64)
     float best = 0.0f;
     bn = 0;
     for (const auto &t : tile) {
+        if (parts == 1 && t.bn == 128) continue;  // (not built: two numbers an output in registers)
         const long long tiles = ((long long)M + t.bn - 1) / t.bn * ((N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
         for (int q = 0; q < (may_quarter ? 2 : 1); q++) {
             const float us = q ? (float)((tiles * GP_QUARTERS + pairs - 1) / pairs) * pieces / GP_QUARTERS * t.us + 3.0f + (float)M * (float)N * 6.4e-6f
@@ -356,13 +408,14 @@ static long long gemm_split_scratch(int M, int N, int K) {
 // Where bn is 0 the sizes choose it and whether K is walked in quarters.
 template <typename T> static int gemm_split_run(GemmSplit g, int bn, int quarters, void *scratch, cudaStream_t s) {
     const int pitch = (g.K + 7) / 8 * 8, n_slab = gp_slab_rows(g.N, g.K, 256), m_slab = gp_slab_rows(g.M, g.K, 128), M = g.M, N = g.N;
-    const int parts = sizeof(T) == 4 ? 3 : 1, out_size = g.out_dtype == ABK_F32 ? 4 : 2;
+    constexpr int parts = sizeof(T) == 4 ? 3 : 1;
+    const int out_size = g.out_dtype == ABK_F32 ? 4 : 2;
     __nv_bfloat16 *const w_planes = (__nv_bfloat16 *)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
     __nv_bfloat16 *const x_planes = w_planes + gp_planes(n_slab, g.K) / 2;
     g.quarters = (float *)(x_planes + gp_planes(m_slab, g.K) / 2);
     const T *const x = (const T *)g.x, *const w = (const T *)g.w;
     char *const out = (char *)g.out;
-    const bool may_quarter = gp_may_quarter(m_slab, n_slab);
+    const bool may_quarter = parts == 3 && gp_may_quarter(m_slab, n_slab);
     const auto vec = [&](const T *from, long long ld) { return sizeof(T) == 4 && g.K % 4 == 0 && ld % 4 == 0 && !((uintptr_t)from & 15); };
     for (int m = 0; m < M; m += m_slab)
         for (int n = 0; n < N; n += n_slab) {
@@ -375,14 +428,21 @@ template <typename T> static int gemm_split_run(GemmSplit g, int bn, int quarter
             int rc = ABK_LAUNCH_RESULT();
             if (rc) return rc;
             int b = bn, in_quarters = quarters;
-            if (!b) gp_choose(g.M, g.N, g.K, may_quarter, b, in_quarters);
+            if (!b) gp_choose(g.M, g.N, g.K, parts, may_quarter, b, in_quarters);
             if (in_quarters && !may_quarter) ABK_REFUSE("gemm: no room for the quarters of %d x %d sums", g.M, g.N);
             g.m_tiles = (g.M + b - 1) / b, g.tiles = g.m_tiles * ((g.N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
+            const int steps = gp_steps(g.K);
             CUtensorMap map_w, map_x;
             if ((rc = tmap::bf16_rows_of_128_bytes(w_planes, (long long)parts * g.N, g.K, pitch, GP_ROWS, &map_w))) return rc;
             if ((rc = tmap::bf16_rows_of_128_bytes(x_planes, (long long)parts * g.M, g.K, pitch, b / 2, &map_x))) return rc;
-#define GP_CASE(BN) \
-    case BN: rc = in_quarters ? gemm_split_launch<BN, true>(map_w, map_x, g, s) : gemm_split_launch<BN, false>(map_w, map_x, g, s); break
+#define GP_CASE(BN)                                                                                                                        \
+    case BN:                                                                                                                               \
+        if constexpr (parts == 3)                                                                                                          \
+            rc = steps == 1 ? GP_AS(BN, 1) : steps == 2 ? GP_AS(BN, 2) : GP_AS(BN, 4);                                                     \
+        else if constexpr (BN < 128) rc = gemm_split_launch<BN, false, 1, 1>(map_w, map_x, g, s);                                          \
+        else ABK_REFUSE("gemm: tiles of %d rows of bfloat16 numbers are not built", BN);                                                   \
+        break
+#define GP_AS(BN, STEPS) (in_quarters ? gemm_split_launch<BN, true, 3, STEPS>(map_w, map_x, g, s) : gemm_split_launch<BN, false, 3, STEPS>(map_w, map_x, g, s))
             switch (b) {
                 GP_CASE(32);
                 GP_CASE(64);
@@ -391,6 +451,7 @@ template <typename T> static int gemm_split_run(GemmSplit g, int bn, int quarter
                 default: ABK_REFUSE("gemm: tiles of %d rows are not built", b);
             }
 #undef GP_CASE
+#undef GP_AS
             if (rc) return rc;
         }
     return 0;

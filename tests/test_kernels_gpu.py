@@ -204,8 +204,8 @@ def test_page_tables_on_the_device_follow_the_host():
 @pytest.mark.parametrize("m, n, k", [(33, 64, 2048), (33, 65, 2052), (129, 257, 4100), (100, 1024, 1024), (260, 1100, 580), (1000, 300, 2108), (400, 1030, 1023)])
 def test_float32_product_in_parts(ops, m, n, k):
     """The float32 product on the tensor cores, in three bfloat16 parts an operand, in every tile and in quarters of K: one set of bits, as
-    near to 64 bits as eight float32 sums. Limits: a part is left over of 2^-26 of a number, a sum of 128 is cut off eight times by up to
-    2^-23 of itself, and K / 128 such sums are added with 2^-24 each: below 4e-7 of the result's norm for normal numbers."""
+    near to 64 bits as eight float32 sums. Limits: a part is left over of 2^-26 of a number, a short sum is cut off up to four times by up to
+    2^-23 of itself, and K / 16 to K / 64 such sums are added with 2^-24 each: below 4e-7 of the result's norm for normal numbers."""
     rng = np.random.default_rng(m + n + k)
     x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
     x[m // 2, k // 3], x[3, 5], w[7, k - 1], x[m - 1, 1] = np.inf, np.nan, -np.inf, 3.4e38
@@ -245,6 +245,30 @@ def test_float32_product_in_parts(ops, m, n, k):
     want = xb.cpu().double() @ wb.cpu().double().T
     for dtype, limit in ((torch.float32, 4e-7), (torch.bfloat16, 2.0 ** -8)):
         assert off(product(xb, wb, dtype), want, torch.ones(m, n, dtype=torch.bool)) < limit
+    assert not status.any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("k", [512, 1023, 1024, 2047, 2048, 3072])
+def test_float32_sums_on_the_tensor_cores_are_no_further_off(ops, k, dtype):
+    """Against 64 bits, for numbers of both signs and of one (where every cut-off goes the same way): no further off than the eight running
+    sums of the CUDA cores, and no sum systematically too small by more than half a unit of float32's last place (2^-24). Limit: a twentieth
+    for the draw (the two norms over 256 x 500 results differ by less than a hundredth from draw to draw)."""
+    gen, lib, status = torch.Generator(device="cuda").manual_seed(k), ops.load_module("gemm_simt"), ops.kernel_status(torch.device("cuda", 0))
+    m, n = 256, 3500 if k > 512 else 7000  # (large enough for the tensor cores)
+    assert ops.gemm_simt_scratch(m, n, k) or dtype == torch.bfloat16
+    draws = {"normal": lambda s: torch.randn(s, generator=gen, device="cuda"), "magnitudes": lambda s: torch.randn(s, generator=gen, device="cuda").abs(),
+             "0 to 1": lambda s: torch.rand(s, generator=gen, device="cuda")}
+    for name, draw in draws.items():
+        x, w = draw((m, k)).to(dtype), draw((n, k)).to(dtype)
+        exact, out, plain_out = x.double() @ w.double().T, torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+        ops.gemm_simt(x, w, out)
+        assert lib.abk_gemm_simt(ops._p(x), ops._i(ops._dt(x)), ops._p(w), ops._i(ops._dt(w)), ops._p(plain_out), ops._i(0), ops._i(m), ops._i(n),
+                                 ops._i(k), ops._ll(k), ops._ll(k), ops._ll(n), None, ops._ll(0), ops._p(status), ops._stream()) == 0
+        off = lambda a: ((a.double() - exact).norm() / exact.norm()).item()
+        assert off(out) <= 1.05 * off(plain_out), (name, off(out), off(plain_out))
+        if name != "normal":
+            assert abs(((out.double() - exact) / exact).mean().item()) < (2 ** -24 if k < 2048 else 2 ** -23), name
     assert not status.any()
 
 
