@@ -21,8 +21,10 @@
 // cores lose less, a product being exact there too, so their short sums, over 16, are added in one running sum with what each addition rounds off
 // beside it (Knuth's two-sum), added at the end. (In float32 that takes 2048 x 1024 x 1020 from 22 us, with errors of 1.3e-7, to 68, with 0.35e-7;
 // the CUDA cores 148, 0.9e-7.)
-// A number that is not finite makes its products NaN in this form; an element that came out not finite is taken again with
-// plain multiply-adds. (Numbers below 1e-33 keep fewer digits: their third part is too small for bfloat16.)
+// A number that is not finite makes its products NaN in this form, and one below 1e-33 keeps fewer digits (its third part is too small for
+// bfloat16): an element that came out not finite, or below 2^-96 but not zero, is taken again with the CUDA cores' eight sums, a tile at a time and
+// behind all waits, so that no wait runs out meanwhile: 2000 x 6144 x 1024 in 170 us, with one row of NaN 400, with nothing but NaN 3,600 (the CUDA
+// cores 691). What is left: factors below 1e-33 whose partners are beyond 2^14, so that the element is not small.
 //
 // What bounds it: the chain between the tensor cores and the warps that add up (0.3 us a short sum), and the way of the parts from
 // the L2, 6 bytes a number, at some 30 bytes a cycle and SM (500 x 6144 x 1024 in 65 us, 9 of them for the parts; sums of 128 53, the CUDA
@@ -37,6 +39,7 @@
 #include "recurrence.cuh"
 #include "tc_common.cuh"
 #include "tensor_map.cuh"
+#include <float.h>
 
 #define GP_ADDERS 16                      // warps that add up what the tensor cores leave
 #define GP_THREADS (32 * GP_ADDERS + 64)  // one that loads, one that multiplies
@@ -121,26 +124,102 @@ struct GemmSplit {
     float *quarters;  // [GP_QUARTERS][M][N]
 };
 
-template <typename T> __device__ __noinline__ float gp_plain(const T *x, const T *w, int K) {
-    float s = 0.0f;
-    for (int k = 0; k < K; k++) s = fmaf(to_float(x[k]), to_float(w[k]), s);
-    return s;
-}
-// An element's place in `out`, with the sum v, or, where that is not finite, with plain multiply-adds.
-__device__ __forceinline__ void gp_put(const GemmSplit &g, int m, int n, float v) {
-    if (!isfinite(v))
-        v = g.dtype == ABK_F32 ? gp_plain((const float *)g.x + m * g.ldx, (const float *)g.w + n * g.ldw, g.K)
-                               : gp_plain((const __nv_bfloat16 *)g.x + m * g.ldx, (const __nv_bfloat16 *)g.w + n * g.ldw, g.K);
-    if (g.out_dtype == ABK_F32) ((float *)g.out)[m * g.ldo + n] = v;
+template <typename T> __device__ __forceinline__ void gp_put(const GemmSplit &g, int m, int n, float v) {
+    if (sizeof(T) == 4 || g.out_dtype == ABK_F32) ((float *)g.out)[m * g.ldo + n] = v;
     else ((__nv_bfloat16 *)g.out)[m * g.ldo + n] = __float2bfloat16_rn(v);
 }
+template <typename T> __device__ __forceinline__ float gp_stored(const GemmSplit &g, int m, int n) {
+    if (sizeof(T) == 4 || g.out_dtype == ABK_F32) return __ldcg((const float *)g.out + m * g.ldo + n);
+    return __bfloat162float(__ldcg((const __nv_bfloat16 *)g.out + m * g.ldo + n));
+}
+// Whether a sum has to be taken again.
+__device__ __forceinline__ bool gp_again(float v) { return !(fabsf(v) >= 0x1p-96f && fabsf(v) <= FLT_MAX) && v != 0.0f; }
+
+// The elements of a tile of THREADS / 16 rows of x from m0 on and 128 rows of w from n0 on that have to be taken again, as gemm_simt.cu adds
+// them up: eight sums, pieces of 16 of K, piece c to sum c % 8, in ascending order, then in pairs (up to K = 256 one sum). All threads of
+// the CTA call it and THREADS of them work, one for a row of w and eight rows of x; bad: bit j for the thread's j-th. smem: GP_REDO_FLOATS.
+#define GP_REDO_PITCH 20  // (eight rows' runs of four numbers lie in different banks)
+#define GP_REDO_FLOATS(THREADS) ((128 + (THREADS) / 16) * GP_REDO_PITCH)
+template <typename T, int THREADS> __device__ __forceinline__ void gp_redo(const GemmSplit &g, int m0, int n0, uint32_t bad, float *smem) {
+    const int tid = threadIdx.x, n = tid & 127, row = tid / 128 * 8, sums = g.K <= 256 ? 1 : 8, pieces = (g.K + 15) / 16;
+    const float *const ws = smem + n * GP_REDO_PITCH, *const xs = smem + (128 + row) * GP_REDO_PITCH;
+    constexpr int MINE = (128 + THREADS / 16) * 16 / THREADS;  // numbers of a piece that a thread brings: asked for while the one before is multiplied
+    float a[8], b[8], c[8], sum[8], next[MINE];
+    auto ask = [&](int piece) {
+        if (tid >= THREADS) return;
+#pragma unroll
+        for (int i = 0; i < MINE; i++) {
+            const int e = tid + i * THREADS, r = e / 16, k = piece * 16 + e % 16;
+            const bool of_w = r < 128, real = k < g.K && (of_w ? n0 + r < g.N : m0 + r - 128 < g.M);
+            const T *from = of_w ? (const T *)g.w + (n0 + r) * g.ldw : (const T *)g.x + (m0 + r - 128) * g.ldx;
+            next[i] = real ? to_float(from[k]) : 0.0f;
+        }
+    };
+    for (int s = 0; s < sums; s++) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) sum[j] = 0.0f;
+        ask(s);
+        for (int piece = s; piece < pieces; piece += sums) {
+            __syncthreads();
+            if (tid < THREADS) {
+#pragma unroll
+                for (int i = 0; i < MINE; i++) smem[(tid + i * THREADS) / 16 * GP_REDO_PITCH + (tid + i * THREADS) % 16] = next[i];
+            }
+            __syncthreads();
+            if (piece + sums < pieces) ask(piece + sums);
+            if (tid < THREADS) {
+#pragma unroll
+                for (int k = 0; k < 16; k += 4) {
+                    const float4 v = *(const float4 *)(ws + k);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const float4 u = *(const float4 *)(xs + j * GP_REDO_PITCH + k);
+                        sum[j] = fmaf(u.w, v.w, fmaf(u.z, v.z, fmaf(u.y, v.y, fmaf(u.x, v.x, sum[j]))));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {  // ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7))
+            if (s == 0) a[j] = sum[j];
+            else if (s == 1) a[j] += sum[j];
+            else if (s == 2 || s == 4) b[j] = sum[j];
+            else if (s == 3) a[j] += b[j] + sum[j];
+            else if (s == 5) b[j] += sum[j];
+            else if (s == 6) c[j] = sum[j];
+            else a[j] += b[j] + (c[j] + sum[j]);
+        }
+    }
+    __syncthreads();  // (the next tile is staged in the same place)
+    if (tid < THREADS)
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (bad >> j & 1) gp_put<T>(g, m0 + row + j, n0 + n, a[j]);
+}
+
+// The same for the tiles of a pair's CTA (item pair, pair + pairs, ...).
+template <typename T, int BN> __device__ __noinline__ void gp_redo_items(const GemmSplit &g, int pair, int pairs, int items, int half, float *smem) {
+    constexpr int THREADS = 32 * GP_ADDERS, ROWS = THREADS / 16;
+    for (int item = pair; item < items; item += pairs) {
+        const int m_end = min((item % g.m_tiles + 1) * BN, g.M), n0 = (item / g.m_tiles * 2 + half) * GP_ROWS, n = n0 + (threadIdx.x & 127);
+        for (int m0 = item % g.m_tiles * BN; m0 < m_end; m0 += ROWS) {
+            uint32_t bad = 0;
+            if (threadIdx.x < THREADS && n < g.N)
+                for (int j = 0, m = m0 + threadIdx.x / 128 * 8; j < 8 && m < m_end; j++, m++) bad |= (uint32_t)gp_again(gp_stored<T>(g, m, n)) << j;
+            if (__syncthreads_or(bad)) gp_redo<T, THREADS>(g, m0, n0, bad, smem);
+        }
+    }
+}
+
+template <int PARTS> struct GpOperand { typedef float T; };
+template <> struct GpOperand<1> { typedef __nv_bfloat16 T; };
 
 // A tile is 256 rows of w (128 of each CTA) and BN rows of x; pair c of CTAs takes items c, c + pairs, ... An item is a tile, or
 // (QUARTERS) a quarter of K of one, whose sums go to `quarters` and are added up by the kernel behind.
 // map_w, map_x: the planes, one below the other; PARTS: 3 of float32 operands, 1 of bfloat16 ones; STEPS: of 16 of K in a
 // short sum, 1, 2 or 4.
 template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_bounds__(GP_THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w,
-                                                                                               const __grid_constant__ CUtensorMap map_x, GemmSplit g) {
+                                                                                               const __grid_constant__ CUtensorMap map_x, const __grid_constant__ GemmSplit g) {
     using S = GpShape<BN>;
     constexpr int STAGES = S::STAGES, COLS = S::COLS, SUMS = S::SUMS, SMALLS = S::SMALLS;
     extern __shared__ uint8_t gp_smem_raw[];
@@ -148,7 +227,8 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
     uint64_t *full = (uint64_t *)(smem + STAGES * S::STAGE), *empty = full + STAGES;
     uint64_t *sum_ready = empty + STAGES, *sum_free = sum_ready + SUMS, *small_free = sum_free + SUMS;
     uint32_t *tmem_holder = (uint32_t *)(small_free + SMALLS);
-    volatile int *gave_up = (volatile int *)(tmem_holder + 1);
+    volatile int *gave_up = (volatile int *)(tmem_holder + 1), *again = gave_up + 1;  // again: some element has to be taken again
+    typedef typename GpOperand<PARTS>::T T;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t half = tc::cluster_rank();  // 0: the leader
     if (threadIdx.x == 0) {
@@ -156,7 +236,7 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
         // sum_free, small_free: every adding warp of the CTA, and, on the leader's, the peer's word that all of its own have
         for (int b = 0; b < SUMS; b++) tc::mbar_init(&sum_ready[b], 1), tc::mbar_init(&sum_free[b], GP_ADDERS + (half == 0));
         for (int b = 0; b < SMALLS; b++) tc::mbar_init(&small_free[b], GP_ADDERS + (half == 0));
-        *gave_up = 0;
+        *gave_up = *again = 0;
         tc::mbar_init_fence();
         tc::tma_prefetch_map(&map_w), tc::tma_prefetch_map(&map_x);
     }
@@ -266,7 +346,7 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
 #pragma unroll
         for (int j = 0; j < COLS; j++) sum[j] = total[j] = 0.0f;
         int sum_i = 0, quarter_i = 0;
-        bool ok = true;
+        bool ok = true, redo = false;
 #pragma unroll 1
         for (int item = pair; ok && item < items; item += pairs) {
 #pragma unroll 1
@@ -323,13 +403,17 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
                 } else {
 #pragma unroll
                     for (int j = 0; j < COLS; j++)
-                        if (j < cols) gp_put(g, m0 + j, n, PARTS == 3 ? total[j] : sum[j] + total[j]);
+                        if (j < cols) {
+                            const float v = PARTS == 3 ? total[j] : sum[j] + total[j];
+                            gp_put<T>(g, m0 + j, n, v), redo |= gp_again(v);
+                        }
                 }
 #pragma unroll
                 for (int j = 0; j < COLS; j++) sum[j] = total[j] = 0.0f;
             }
         }
         if (!ok) *gave_up = 1;
+        if (redo) *again = 1;
     }
     tc::fence_before_sync();
     tc::cluster_sync();  // (the pair's other CTA is done with this one's memory and barriers)
@@ -338,15 +422,31 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
         tc::fence_after_sync();
         tc::tmem_free_pair(tmem, S::TMEM);
     }
+    if (!QUARTERS && *again && !*gave_up) gp_redo_items<T, BN>(g, pair, pairs, items, half, (float *)smem);
 }
 
-// The four quarters' sums of every element, in order.
-__global__ void __launch_bounds__(256) gemm_split_sum_kernel(GemmSplit g) {
+// The four quarters' sums of every element, in order: a CTA has tiles of 16 rows and 128 columns, a thread a column and eight rows.
+#define GP_SUM_THREADS 256
+__global__ void __launch_bounds__(GP_SUM_THREADS) gemm_split_sum_kernel(const __grid_constant__ GemmSplit g) {
+    __shared__ __align__(16) float smem[GP_REDO_FLOATS(GP_SUM_THREADS)];
+    constexpr int ROWS = GP_SUM_THREADS / 16;
+    const long long plane = (long long)g.M * g.N;
+    const int m_tiles = (g.M + ROWS - 1) / ROWS, tiles = m_tiles * ((g.N + 127) / 128);
     pdl_wait();
-    const long long n = (long long)g.M * g.N;
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
-        const int row = (int)(i / g.N), col = (int)(i - (long long)row * g.N);
-        gp_put(g, row, col, ((g.quarters[i] + g.quarters[i + n]) + g.quarters[i + 2 * n]) + g.quarters[i + 3 * n]);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int m0 = tile % m_tiles * ROWS, n0 = tile / m_tiles * 128, m = m0 + threadIdx.x / 128 * 8, n = n0 + (threadIdx.x & 127);
+        float q[8][GP_QUARTERS];
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+#pragma unroll
+            for (int i = 0; i < GP_QUARTERS; i++) q[j][i] = m + j < g.M && n < g.N ? g.quarters[i * plane + (long long)(m + j) * g.N + n] : 0.0f;
+        uint32_t bad = 0;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const float v = ((q[j][0] + q[j][1]) + q[j][2]) + q[j][3];
+            if (m + j < g.M && n < g.N) gp_put<float>(g, m + j, n, v), bad |= (uint32_t)gp_again(v) << j;
+        }
+        if (__syncthreads_or(bad)) gp_redo<float, GP_SUM_THREADS>(g, m0, n0, bad, smem);
     }
 }
 
@@ -358,8 +458,8 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> static int gemm_split_lau
     abk_launch_clusters(gemm_split_kernel<BN, QUARTERS, PARTS, STEPS>, dim3(2 * (items < pairs ? items : pairs)), dim3(GP_THREADS), S::BYTES, s, 2, map_w, map_x, g);
     const int rc = ABK_LAUNCH_RESULT();
     if (rc || !QUARTERS) return rc;
-    const long long blocks = ((long long)g.M * g.N + 255) / 256, most = 8LL * abk_sm_count();
-    abk_launch(gemm_split_sum_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s, g);
+    const long long blocks = ((long long)g.M + 15) / 16 * ((g.N + 127) / 128), most = 8LL * abk_sm_count();
+    abk_launch(gemm_split_sum_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(GP_SUM_THREADS), 0, s, g);
     return ABK_LAUNCH_RESULT();
 }
 

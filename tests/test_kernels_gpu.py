@@ -249,6 +249,52 @@ def test_float32_product_in_parts(ops, m, n, k):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m, n, k", [(150, 300, 700), (129, 257, 1027), (40, 129, 2500)])
+def test_sums_in_parts_that_are_no_numbers_or_too_small_are_taken_again(ops, m, n, k, dtype):
+    """Rows with infinities, NaNs, numbers whose bfloat16 part overflows and numbers whose third part underflows: the bits of the CUDA cores'
+    kernel. The other rows are what they are without them, in every tile and in quarters."""
+    gen, lib, status = torch.Generator(device="cuda").manual_seed(k), ops.load_module("gemm_simt"), ops.kernel_status(torch.device("cuda", 0))
+    x, w = torch.randn((m, k), generator=gen, device="cuda"), torch.randn((n, k), generator=gen, device="cuda")
+    clean, planted = x.clone(), [0, 1, 31, 32, 33, m - 3, m - 2, m - 1]
+    x[0] = float("nan")
+    x[1, 11] = float("inf")
+    x[31, 3], x[31, 5] = float("inf"), float("-inf")
+    x[32, 2], x[32, 400], x[33, 9] = 3.4e38, -3.4e38, 3.4e38
+    x[m - 3] *= 1e-35
+    x[m - 2] *= 1e-37
+    x[m - 1] = 0
+    x, w, clean = x.to(dtype), w.to(dtype), clean.to(dtype)
+    scratch = torch.empty(lib.abk_gemm_split_scratch(m, n, k), dtype=torch.uint8, device="cuda")
+
+    def product(a, rows=0, quarters=0):
+        out = torch.full((m, n), 7.0, device="cuda")
+        assert lib.abk_gemm_split(ops._p(a), ops._p(w), ops._i(ops._dt(a)), ops._p(out), ops._i(0), ops._i(m), ops._i(n), ops._i(k), ops._ll(k), ops._ll(k),
+                                  ops._ll(n), ops._i(rows), ops._i(quarters), ops._p(scratch), ops._p(status), ops._stream()) == 0
+        return out
+
+    want, plain_out, others = product(clean), torch.empty(m, n, device="cuda"), [i for i in range(m) if i not in planted]
+    assert lib.abk_gemm_simt(ops._p(x), ops._i(ops._dt(x)), ops._p(w), ops._i(ops._dt(w)), ops._p(plain_out), ops._i(0), ops._i(m), ops._i(n), ops._i(k),
+                             ops._ll(k), ops._ll(k), ops._ll(n), None, ops._ll(0), ops._p(status), ops._stream()) == 0
+    for rows, quarters in [(0, 0)] + [(r, q) for r in (32, 64, 96, 128) for q in (0, 1) if dtype == torch.float32 or (r < 128 and not q)]:
+        out = product(x, rows, quarters)
+        assert torch.equal(out[others], want[others]), (rows, quarters)
+        for i in planted:
+            assert torch.equal(out[i].nan_to_num(1, 2, 3), plain_out[i].nan_to_num(1, 2, 3)) and torch.equal(out[i].isnan(), plain_out[i].isnan()), (i, rows, quarters)
+    assert plain_out[0].isnan().all() and plain_out[1].isinf().any() and 0 < plain_out[m - 2].abs().max() < 1e-34 and not status.any()
+
+
+def test_a_product_of_nothing_but_nan_takes_no_milliseconds(ops):
+    """Eight times what it takes on the CUDA cores at most: the tiles are taken again by the CTAs that made them, one after the other."""
+    m, n, k = 500, 6144, 1024
+    x, w, out = torch.full((m, k), float("nan"), device="cuda"), torch.randn(n, k, device="cuda"), torch.empty(m, n, device="cuda")
+    lib, status = ops.load_module("gemm_simt"), ops.kernel_status(torch.device("cuda", 0))
+    cores = lambda: lib.abk_gemm_simt(ops._p(x), ops._i(0), ops._p(w), ops._i(0), ops._p(out), ops._i(0), ops._i(m), ops._i(n), ops._i(k), ops._ll(k), ops._ll(k),
+                                      ops._ll(n), None, ops._ll(0), ops._p(status), ops._stream())
+    times = us_of({"parts": lambda: ops.gemm_simt(x, w, out), "cores": cores}, 3)
+    assert out.isnan().all() and times["parts"] < 8 * times["cores"], times
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("k", [512, 1023, 1024, 2047, 2048, 3072])
 def test_float32_sums_on_the_tensor_cores_are_no_further_off(ops, k, dtype):
     """Against 64 bits, for numbers of both signs and of one (where every cut-off goes the same way): no further off than the eight running
