@@ -175,7 +175,7 @@ static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int 
     return ABK_LAUNCH_RESULT();
 }
 
-// The product on the tensor cores (gemm_split.cuh), for any sizes. bn: rows of x in a tile (32, 64, 96, 128), quarters: pairs of CTAs take
+// The product on the tensor cores (gemm_split.cuh), for any M and N and K from 193 on (every quarter of K has a piece of 64). bn: rows of x in a tile (32, 64, 96, 128), quarters: pairs of CTAs take
 // quarters of K (of float32 operands only); 0, 0: by size. scratch: abk_gemm_split_scratch bytes.
 extern "C" int abk_gemm_split(const void *x, const void *w, int dtype, void *out, int out_dtype, int M, int N, int K, long long ldx, long long ldw,
                               long long ldo, int bn, int quarters, void *scratch, int *status, void *stream) {

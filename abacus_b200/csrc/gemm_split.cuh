@@ -509,6 +509,7 @@ static long long gemm_split_scratch(int M, int N, int K) {
 template <typename T> static int gemm_split_run(GemmSplit g, int bn, int quarters, void *scratch, cudaStream_t s) {
     const int pitch = (g.K + 7) / 8 * 8, n_slab = gp_slab_rows(g.N, g.K, 256), m_slab = gp_slab_rows(g.M, g.K, 128), M = g.M, N = g.N;
     constexpr int parts = sizeof(T) == 4 ? 3 : 1;
+    if (g.K <= (GP_QUARTERS - 1) * GP_K) ABK_REFUSE("gemm: K = %d is too short for four quarters on the tensor cores", g.K);
     const int out_size = g.out_dtype == ABK_F32 ? 4 : 2;
     __nv_bfloat16 *const w_planes = (__nv_bfloat16 *)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
     __nv_bfloat16 *const x_planes = w_planes + gp_planes(n_slab, g.K) / 2;

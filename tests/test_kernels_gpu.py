@@ -283,6 +283,20 @@ def test_sums_in_parts_that_are_no_numbers_or_too_small_are_taken_again(ops, m, 
     assert plain_out[0].isnan().all() and plain_out[1].isinf().any() and 0 < plain_out[m - 2].abs().max() < 1e-34 and not status.any()
 
 
+@pytest.mark.parametrize("k", [1, 64, 128, 192, 193])
+def test_products_in_parts_refuse_a_k_without_four_quarters(ops, k):
+    """Up to K = 192 some quarter has no piece, and a wait for it would run out: refused on the host. 193 is the shortest that runs."""
+    m, n = 70, 140
+    x, w, out = torch.ones(m, k, device="cuda"), torch.ones(n, k, device="cuda"), torch.full((m, n), 7.0, device="cuda")
+    lib, status = ops.load_module("gemm_simt"), ops.kernel_status(torch.device("cuda", 0))
+    lib.abk_gemm_split_scratch.restype = ctypes.c_longlong
+    scratch = torch.empty(lib.abk_gemm_split_scratch(m, n, k), dtype=torch.uint8, device="cuda")
+    for rows, quarters in ((0, 0), (32, 1)):
+        rc = lib.abk_gemm_split(ops._p(x), ops._p(w), ops._i(0), ops._p(out), ops._i(0), ops._i(m), ops._i(n), ops._i(k), ops._ll(k), ops._ll(k), ops._ll(n),
+                                ops._i(rows), ops._i(quarters), ops._p(scratch), ops._p(status), ops._stream())
+        assert rc == (-1 if k < 193 else 0) and bool((out == (7.0 if k < 193 else k)).all()) and not status.any()
+
+
 def test_a_product_of_nothing_but_nan_takes_no_milliseconds(ops):
     """Eight times what it takes on the CUDA cores at most: the tiles are taken again by the CTAs that made them, one after the other."""
     m, n, k = 500, 6144, 1024
