@@ -208,7 +208,9 @@ extern "C" int abk_gemm_simt(const void *x, int x_dtype, const void *w, int w_dt
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
     if (N > 65535 * 64) ABK_REFUSE("gemm: %d output columns are more than one launch takes", N);
-    if (scratch && x_dtype == w_dtype && (x_dtype == ABK_BF16 || out_dtype == ABK_F32) && gemm_split_wins(M, N, K) && scratch_bytes >= gemm_split_scratch(M, N, K)) {
+    if (scratch && x_dtype == w_dtype && (x_dtype == ABK_BF16 || out_dtype == ABK_F32) && gemm_split_wins(M, N, K)) {
+        if (scratch_bytes < gemm_split_scratch(M, N, K))
+            ABK_REFUSE("gemm: %lld bytes of scratch memory for %d x %d x %d, which takes %lld", scratch_bytes, M, N, K, gemm_split_scratch(M, N, K));
         const GemmSplit g = {x, w, out, x_dtype, out_dtype, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};
         return x_dtype == ABK_F32 ? gemm_split_run<float>(g, 0, 0, scratch, s) : gemm_split_run<bf>(g, 0, 0, scratch, s);
     }

@@ -184,9 +184,12 @@ class CStep:
         self.att_width = max(s.n_heads * s.head_dim for s in specs)
         self.inter = max(b.ffn.spec.inter for b in model.blocks)
         # outputs and inputs of the products that may take scratch memory: the float32 ones, and those whose rows TMA cannot take
-        takes = lambda w: not bf16 or w.shape[1] % 8 != 0
-        self.products = {tuple(w.shape) for b in model.blocks for w in (b.mixer.qkv_proj.weight, b.mixer.o_proj.weight,
-                                                                       b.ffn.gate_up.weight, b.ffn.down.weight) if takes(w)}
+        takes = lambda w: not bf16 or w.shape[1] % 8 != 0 or w.data_ptr() % 16 != 0
+        owns = {e.layer for i, e in enumerate(model.schedule) if cache.views[i].owns_storage}
+        reads = {e.layer for i, e in enumerate(model.schedule) if not cache.views[i].owns_storage}
+        self.products = {tuple(w.shape) for i, b in enumerate(model.blocks)
+                         for w in [b.mixer.qkv_proj.weight] * (i in owns) + [b.mixer.q_proj.weight] * (i in reads)
+                         + [b.mixer.o_proj.weight, b.ffn.gate_up.weight, b.ffn.down.weight] if takes(w)}
         self.head_product = tuple(frame.head.weight.shape) if takes(frame.head.weight) else None
         self.table_positions = min([b.mixer.cos.shape[0] for b in model.blocks if b.mixer.cos is not None] or [1 << 30])
         self.step, self.lists = Step(), (Lists * max(1, len(self.plan_names)))()
@@ -253,6 +256,7 @@ class CStep:
         s.gate_up = ws.get("gate_up", (n, 2 * self.inter), dtype).data_ptr()
         s.xn_final = ws.get("xn_final", (max(r, 1), d), dtype).data_ptr()
         s.partial_floats = partial_floats
+        # (a smaller matrix can need more: with few columns the sums of quarters of K fit too)
         s.parts_bytes = max([ops.gemm_simt_scratch(n, *p) for p in self.products]
                             + [ops.gemm_simt_scratch(r, *self.head_product) if self.head_product else 0])
         s.parts = ws.get("parts", (s.parts_bytes,), torch.uint8).data_ptr() if s.parts_bytes else None

@@ -244,6 +244,36 @@ def test_the_step_function_in_c_launches_what_the_parts_would(tmp_path, name, dt
 
 
 
+@pytest.mark.parametrize("rows", [1536, 1600, 2048])
+def test_a_layer_that_reads_anothers_cache_goes_the_same_way_in_c(tmp_path, rows):
+    """Its q product is smaller than the other products and needs more scratch memory for its sums of quarters than any of them: the C walker
+    has to have room for it, or its bits are not the parts'."""
+    import dataclasses
+    from abacus_b200.config import ScheduleEntry, load_config
+    from abacus_b200.engine import Engine
+    from abacus_b200.kernels import ops
+    from abacus_b200.models import Model
+    from abacus_b200.weights import load_folder
+    folder = folder_of(tmp_path, "B", hidden_size=1024, intermediate_size=3072, num_attention_heads=16, num_key_value_heads=8, head_dim=128,
+                       max_position_embeddings=4096)
+    arch, cfg = load_config(folder)
+    spec = dataclasses.replace(cfg.to_spec(), schedule=(ScheduleEntry(0), ScheduleEntry(1, source=0)))
+    tensors = load_folder(folder, lambda names: arch.tensor_names(spec, names))
+    model = Model(spec, arch.layout(spec), tensors, torch.float32, torch.device("cuda", 0))
+    need = {p: ops.gemm_simt_scratch(rows, *p) for p in ((2048, 1024), (4096, 1024), (1024, 2048), (6144, 1024), (1024, 3072))}
+    assert rows == 1536 or need[2048, 1024] == max(need.values()) > need[4096, 1024]
+    tokens, logits = random_tokens(np.random.default_rng(rows), rows, TINY["B"]["cfg"]["vocab_size"]), []
+    for c_step in (True, False):
+        engine = Engine(model, max_tokens=4096, use_graphs=False)
+        assert engine.cstep is not None
+        if not c_step:
+            engine.cstep = None
+        slot = engine.open()
+        logits.append(engine.step([(slot, tokens, [0, rows // 2, rows - 1])]).clone())
+        engine.check_status()
+    assert torch.equal(*logits)
+
+
 def test_preparing_q_k_v_in_the_neighbouring_kernels_changes_no_bit(tmp_path, monkeypatch):
     """In bfloat16 the step between the q/k/v product and attention (per-head norm, rotation, cache write) runs in the
     product's epilogue for long prompt steps and inside the attention kernel for decode steps. With both switched off
