@@ -785,32 +785,37 @@ __global__ void __launch_bounds__(256) delta_step_kernel(DeltaPrepare p, DeltaSc
 
 #include "delta_chunk.cuh"
 
-// Whether a step's prompts go in chunks of 16 tokens (delta_chunk.cuh) rather than in blocks of four: where the walk's chain counts for more
-// than what it does, that is for prompts of a hundred tokens and more, and few of them or few columns to an SM. In us, blocks
-// against chunks, both kernels each: 16 heads of 128 x 128, one prompt of 1,999 tokens 327 and 210, of 200 43 and 34, of 50 21 and 22; three
-// prompts, 3,416 tokens, 644 and 328; 32 heads, the same three, 708 and 590; eight prompts of 709, 4 heads 161 and 145, 8 heads 261 and
-// 274; 32 heads of 64 x 64: one prompt of 1,999 265 and 241, four prompts 269 and 221, eight prompts of 709 373 and 447.
-static bool delta_in_chunks(int n_tokens, int n_seqs, int heads, int per_head, int key, int value) {
-    if (per_head || !delta_chunk_takes(key, value) || n_tokens < 100LL * n_seqs) return false;
-    const long long columns = (long long)n_seqs * heads * value, sms = abk_sm_count();
-    return columns <= 32 * sms || (n_seqs <= 4 && columns <= (key == 64 ? 60 : 140) * sms);
+// Whether a step's prompts go in chunks of 16 tokens (delta_chunk.cuh) rather than in blocks of four: where the longest prompt's chain counts
+// for more than what the GPU has to do meanwhile, that is by the value columns an SM has on average while the longest walks. In us, blocks
+// against chunks, both kernels each, keys and values of 128 (limit 48 columns), columns in brackets: 16 heads, one prompt of 1,999 tokens (14) 325
+// and 208; prompts of 167, 32, 32 and 1,998 (15) 562 and 253; three of 900 (42) 309 and 265; 8 heads, six of 800 (42) 280 and 235, seven
+// of 700 (48) 253 and 255, eight of 101 (55) 46 and 55; 32 heads, two of 250 (55) 95 and 106; 16 heads, four of 700 (55) 255 and 266.
+// Of 64 (limit 24): 32 heads, one of 1,999 (14) 263 and 238; 8 heads, seven of 700 (24) 120 and 109; 32 heads, 35, 699, 1,223, 135, 71, 111 and
+// 28 (26) 273 and 297; 32 heads, three of 900 (42) 229 and 241, four of 700 (55) 191 and 216. And prompts of 48 tokens on: 16 heads of 128, one of 50
+// 21 and 22, of 100 28 and 25. Over 225 steps of one to eight prompts of 16 to 2,048 tokens this takes 31.3 ms, the faster form each time 31.2;
+// none of them is more than 3 % slower than blocks, which take 39.4.
+static bool delta_in_chunks(int n_tokens, int longest, int heads, int per_head, int key, int value) {
+    if (per_head || !delta_chunk_takes(key, value) || longest < 48) return false;
+    return (long long)heads * value * n_tokens <= (long long)(key == 64 ? 24 : 48) * abk_sm_count() * longest;
 }
 
 static long long delta_chunk_scratch(int n_tokens, int n_seqs, int heads, int key, int value) {
     return ((long long)n_tokens / DK_TOKENS + n_seqs) * heads * delta_chunk_floats(key, value);
 }
 
-// Floats of scratch memory the recurrence needs for n_tokens tokens of n_seqs sequences: the blocks' records, none where no
-// sequence brings more than a token; chunks: the tokens' records of abk_delta_chunks.
-extern "C" long long abk_delta_scan_scratch(int n_tokens, int n_seqs, int heads, int key, int value, int chunks) {
+static long long delta_block_scratch(int n_tokens, int n_seqs, int heads, int key, int value) {
+    return ((long long)n_tokens / DB_TOKENS + n_seqs) * heads * delta_block_floats(key, value);
+}
+
+// Floats of scratch memory the recurrence needs for n_tokens tokens of n_seqs sequences, the longest of `longest`: the records of the blocks or
+// chunks (form as in abk_delta_scan), none where no sequence brings more than a token; chunks: the tokens' records of abk_delta_chunks.
+extern "C" long long abk_delta_scan_scratch(int n_tokens, int n_seqs, int longest, int heads, int key, int value, int chunks, int form) {
     if (chunks) return (long long)n_tokens * heads * delta_record_floats(key, value);
     if (n_tokens <= n_seqs) return 0;
-    if (delta_in_chunks(n_tokens, n_seqs, heads, 0, key, value)) {
-        const long long in_chunks = delta_chunk_scratch(n_tokens, n_seqs, heads, key, value);
-        const long long in_blocks = ((long long)n_tokens / DB_TOKENS + n_seqs) * heads * delta_block_floats(key, value);
-        return in_chunks > in_blocks ? in_chunks : in_blocks;
-    }
-    return ((long long)n_tokens / DB_TOKENS + n_seqs) * heads * delta_block_floats(key, value);
+    const long long in_chunks = delta_chunk_scratch(n_tokens, n_seqs, heads, key, value), in_blocks = delta_block_scratch(n_tokens, n_seqs, heads, key, value);
+    if (form == 16) return in_chunks;
+    // (a state that is not 16-byte aligned goes in blocks whatever the sizes)
+    return form != 4 && in_chunks > in_blocks && delta_in_chunks(n_tokens, longest, heads, 0, key, value) ? in_chunks : in_blocks;
 }
 
 static int delta_chunk_run(DeltaPrepare q, DeltaScan p, const int *seq_start, int dtype, int n_tokens, int n_seqs, cudaStream_t s) {
@@ -849,17 +854,19 @@ static int delta_chunk_run(DeltaPrepare q, DeltaScan p, const int *seq_start, in
     return ABK_LAUNCH_RESULT();
 }
 
-// form: 0 by size; 4: prompts in blocks of four tokens; 16: in chunks of 16 where the keys' size and the scratch memory allow it.
+// longest: tokens of the longest sequence. form: 0 by size; 4: prompts in blocks of four tokens; 16: in chunks of 16 (refused where they are not built).
 extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, const void *decay_in, long long ld_decay, int per_head, const void *beta_in,
                               long long ld_beta, const float *a_log, const float *dt_bias, float *state, float *out,
                               const int *token_seq, const int *seq_start, const int *seq_slot, int n_tokens, int n_seqs,
                               int heads, int kv_heads, int key, int value, float *records, long long records_floats,
-                              int form, void *stream) {
+                              int longest, int form, void *stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
     if (key < 1 || key > 256) ABK_REFUSE("delta rule: key size %d, the kernel takes 1 to 256", key);
     if (kv_heads < 1 || heads % kv_heads) ABK_REFUSE("delta rule: %d heads do not divide into %d key heads", heads, kv_heads);
     if (heads > 65535 || value > 65535 * 16) ABK_REFUSE("delta rule: %d heads of %d values are more than a grid takes", heads, value);
-    const long long need = abk_delta_scan_scratch(n_tokens, n_seqs, heads, key, value, 0);
+    if (form == 16 && (per_head || !delta_chunk_takes(key, value) || ((uintptr_t)state & 15)))
+        ABK_REFUSE("delta rule: no chunks of 16 tokens for keys of %d and values of %d%s", key, value, per_head ? " with one decay a head" : "");
+    const long long need = abk_delta_scan_scratch(n_tokens, n_seqs, longest, heads, key, value, 0, form);
     if (need > records_floats || (need && ((uintptr_t)records & 15)))
         ABK_REFUSE("delta rule: the scratch memory holds %lld floats, the step needs %lld (16-byte aligned)", records_floats, need);
     cudaStream_t s = (cudaStream_t)stream;
@@ -890,9 +897,7 @@ extern "C" int abk_delta_scan(const void *qkv, long long ld_qkv, int dtype, cons
 #undef STEP_LAUNCH
         return ABK_LAUNCH_RESULT();
     }
-    // form 4: in blocks whatever the sizes; 16: in chunks wherever they are built
-    const bool chunks = form == 16 ? !per_head && delta_chunk_takes(key, value) : form != 4 && delta_in_chunks(n_tokens, n_seqs, heads, per_head, key, value);
-    if (chunks && !((uintptr_t)state & 15) && delta_chunk_scratch(n_tokens, n_seqs, heads, key, value) <= records_floats)
+    if (form == 16 || (form == 0 && delta_in_chunks(n_tokens, longest, heads, per_head, key, value) && !((uintptr_t)state & 15)))
         return delta_chunk_run(q, p, seq_start, dtype, n_tokens, n_seqs, s);
     const long long blocks = (q.pairs + 3) / 4;
     if (blocks > 0x7fffffffLL) ABK_REFUSE("delta rule: %lld (block, head) pairs are more than a grid takes", q.pairs);

@@ -91,6 +91,7 @@ class StepBatch:
         self.n_tokens = self.n_seqs = self.n_logit_rows = 0
         self.max_position = 0
         self.max_len_after = 0
+        self.longest = 0  # tokens of the sequence that brings most
         self.is_decode = False
         self.any_continuation = False
         self._sent, self._sent_on = None, set()
@@ -158,6 +159,7 @@ class StepBatch:
                 setattr(self, name, whole if whole.shape[0] == n else whole[:n])
         self.sequences = list(sequences)  # host view, for mixers that walk the sequences themselves
         self.is_decode = one_each
+        self.longest = max(lens, default=0)
         for name, p in self.plans.items():
             info = p.fill(self._layouts[name], self.sequences, h[f"plan:{name}"], self.is_decode, exact)
             self.plan[name] = PlanView(p, self._layouts[name], self._parts[f"plan:{name}"], info)

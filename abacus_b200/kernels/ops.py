@@ -1032,10 +1032,10 @@ DELTA_CHUNK = 64  # tokens of a chunk of the chunked form (one decay a head)
 
 
 @functools.lru_cache(maxsize=4096)
-def _delta_scan_scratch(n, n_seqs, n_heads, key_dim, value_dim, chunks):
+def _delta_scan_scratch(n, n_seqs, longest, n_heads, key_dim, value_dim, chunks, form):
     lib = load_module("delta_rule")
     lib.abk_delta_scan_scratch.restype = ctypes.c_longlong
-    return int(lib.abk_delta_scan_scratch(_i(n), _i(n_seqs), _i(n_heads), _i(key_dim), _i(value_dim), _i(chunks)))
+    return int(lib.abk_delta_scan_scratch(_i(n), _i(n_seqs), _i(longest), _i(n_heads), _i(key_dim), _i(value_dim), _i(chunks), _i(form)))
 
 
 def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_heads, n_kv_heads, key_dim, value_dim, ws,
@@ -1046,7 +1046,8 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
     before the sigmoid; out float32 [tokens, heads * value], not yet normed. per_head: one decay for all key channels of a
     head; decay_in is then [tokens, >= heads] of qkv's type and dt_bias [heads]. A step of one token a sequence is one kernel;
     else every (block of four tokens, head), or for few and long prompts (chunk of 16, head), is prepared in parallel into scratch memory from
-    ws (a parts.Workspace), then the sequences are walked, a block or chunk at a time (tokens_a_time 4 or 16 pins it). chunks (with
+    ws (a parts.Workspace), then the sequences are walked, a block or chunk at a time (tokens_a_time 4 or 16 pins it; refused where it is not
+    built). chunks (with
     per_head, for steps that bring prompts): the walk goes in chunks of 64 tokens, a triangular system a chunk solved
     beside the others and four products a chunk along the sequence (three kernels)."""
     _need_cuda(qkv, decay_in, beta_in, a_log, dt_bias, state, out)
@@ -1062,7 +1063,8 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
     assert a_log.dtype == torch.float32 and dt_bias.dtype == torch.float32 and a_log.numel() == n_heads
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (n_heads, value_dim, key_dim)
     assert out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == n_heads * value_dim
-    records = ws.get("delta_records", (_delta_scan_scratch(n, n_seqs, n_heads, key_dim, value_dim, 1 if chunks else 0),), torch.float32)
+    records = ws.get("delta_records", (_delta_scan_scratch(n, n_seqs, batch.longest, n_heads, key_dim, value_dim, 1 if chunks else 0, tokens_a_time),),
+                     torch.float32)
     if chunks:
         assert per_head, "the chunked form takes one decay a head"
         max_chunks = -(-n // DELTA_CHUNK) + n_seqs
@@ -1073,11 +1075,11 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
             _p(batch.seq_slot), _i(n), _i(n_seqs), _i(n_heads), _i(n_kv_heads), _i(key_dim), _i(value_dim), _p(records),
             _ll(records.numel()), _i(max_chunks), _p(work), _ll(work.numel()), _stream()), "delta_chunks", kernels=3)
         return
-    fn = _typed(lib.abk_delta_scan, "plipliplpppppppiiiiiiplip")
+    fn = _typed(lib.abk_delta_scan, "plipliplpppppppiiiiiipliip")
     _check(lib, fn(qkv.data_ptr(), qkv.stride(0), _dt(qkv), decay_in.data_ptr(), decay_in.stride(0), 1 if per_head else 0, beta_in.data_ptr(),
                    beta_in.stride(0), a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), out.data_ptr(), batch.token_seq.data_ptr(),
                    batch.seq_start.data_ptr(), batch.seq_slot.data_ptr(), n, n_seqs, n_heads, n_kv_heads, key_dim, value_dim,
-                   records.data_ptr(), records.numel(), tokens_a_time, _raw_stream()), "delta_scan", kernels=1 if n <= n_seqs else 2)
+                   records.data_ptr(), records.numel(), batch.longest, tokens_a_time, _raw_stream()), "delta_scan", kernels=1 if n <= n_seqs else 2)
 
 
 def gated_head_norm(o, gate, weight, out, n_tokens, n_heads, value_dim, eps, silu=False):

@@ -249,19 +249,40 @@ def test_delta_rule_in_chunks(H, G, K, V, lens, rate):
         for tokens in (16, 4):
             state, out = start.clone(), torch.empty((sum(lens), H * V), device=DEV)
             ws = Workspace(torch.device(DEV, torch.cuda.current_device()))
-            room = torch.empty(1 << 22, device=DEV)  # (for either form)
-            ws.get = lambda name, shape, dt: room
             ops.delta_scan(cat(0, dtype), cat(1, torch.float32), cat(2, dtype), dev(a_log), dev(bias), state, out, b, H, G, K, V, ws, tokens_a_time=tokens)
             outs[tokens], states[tokens] = out.cpu().double(), state.cpu().double()
             assert torch.equal(state[::2], start[::2])
         want = np.concatenate([_delta_plain(*x, a_log, bias, H, G, K, V, real=np.float64) for x in rounded])
         noise = max(np.abs(_delta_plain(*x, a_log, bias, H, G, K, V) - _delta_plain(*x, a_log, bias, H, G, K, V, real=np.float64)).max() for x in rounded)
+        assert not torch.equal(outs[16], outs[4])  # (two forms ran)
         # sums of 4 x K products and of a chunk's tokens in another order: a few times what float32 itself is off here
         for a in (outs, states):
             np.testing.assert_allclose(a[16].numpy(), a[4].numpy(), rtol=1e-4, atol=2e-5 + 4 * noise)
         state, out = torch.zeros_like(start), torch.empty((sum(lens), H * V), device=DEV)
         ops.delta_scan(cat(0, dtype), cat(1, torch.float32), cat(2, dtype), dev(a_log), dev(bias), state, out, b, H, G, K, V, ws, tokens_a_time=16)
         np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-4, atol=2e-5 + 4 * noise)
+
+
+@pytest.mark.parametrize("H,K,lens,form", [(2, 128, (100,), 16), (16, 128, (50, 300), 16), (2, 64, (47, 30), 4), (2, 64, (48, 30), 16), (32, 64, (200,) * 4, 4),
+                                           (32, 128, (120,) * 2, 4), (32, 128, (10, 400), 16), (2, 32, (100,), 4), (3, 128, (1, 1, 2), 4)])
+def test_the_form_of_the_delta_rule_by_size(H, K, lens, form):
+    """Which of the two forms a step takes by itself, in the workspace that the library sizes for it; a form that is not built is refused."""
+    from abacus_b200.kernels import ops
+    from abacus_b200.parts import Workspace
+    n, gen = sum(lens), torch.Generator(device=DEV).manual_seed(K)
+    randn = lambda *s: torch.randn(s, generator=gen, device=DEV)
+    args = randn(n, 3 * H * K), randn(n, H * K), randn(n, H), randn(H), randn(H * K)
+    start, b, got = randn(len(lens), H, K, K), batch_of([(i, [0] * m, 0) for i, m in enumerate(lens)]), []
+    for pinned in (0, form, 20 - form):
+        state, out = start.clone(), torch.empty((n, H * K), device=DEV)
+        try:
+            ops.delta_scan(*args, state, out, b, H, H, K, K, Workspace(torch.device(DEV, torch.cuda.current_device())), tokens_a_time=pinned)
+        except ops.KernelRefused:
+            assert pinned == 16 and K == 32
+            continue
+        got.append((out, state))
+    assert all(torch.equal(a, c) for a, c in zip(got[0], got[1])) and (len(got) < 3 or not torch.equal(got[0][0], got[2][0]))
+    assert b.longest == max(lens)
 
 
 def test_a_delta_step_of_small_heads_leaves_no_warp_idle():
