@@ -64,7 +64,9 @@ template <typename T> __global__ void __launch_bounds__(128) short_conv_kernel(S
 // The same with VEC channels a thread (16 bytes of the storage type), for channel counts and row pitches that are
 // multiples of VEC with everything 16-byte aligned, for 2 to 4 taps. A thread has TOKENS tokens of its channels: the weights and
 // the rows that its tokens share are read once, and all of its loads are in flight together. Long steps take four tokens (two in
-// float32), short ones one. 1,999 tokens of 4,096 bfloat16 channels, four taps: 20.4 us, 5,672 tokens 57; with each token's rows fetched
+// float32, and from 2,400 CTAs on two such turns, the weights read once for both: 5,672 tokens of 4,096 float32 channels 50 us, with one turn
+// 60, token by token 58; 1,024 of 1,024, 1,024 CTAs, 4.5, 4.1 and 5.6), short ones one: 1,016 tokens of 4,096 bfloat16 channels by one
+// 21 us, 1,024 by four 11; float32 15 and 11. 1,999 tokens of 4,096 bfloat16 channels, four taps: 20.4 us, 5,672 tokens 57; with each token's rows fetched
 // one token after the other, and the division in full, 23.1 and 60.
 #define CONV_TOKENS 4
 template <typename T, int VEC> struct ConvVector;
@@ -92,8 +94,8 @@ template <> struct ConvVector<float, 4> {
     static __device__ __forceinline__ void store(float *p, const float *v) { *(float4 *)p = make_float4(v[0], v[1], v[2], v[3]); }
 };
 
-template <typename T, int VEC, int TAPS, int TOKENS> __global__ void __launch_bounds__(128) short_conv_vec_kernel(ShortConv p) {
-    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC, t0 = blockIdx.x * TOKENS;
+template <typename T, int VEC, int TAPS, int TOKENS, int TURNS> __global__ void __launch_bounds__(128) short_conv_vec_kernel(ShortConv p) {
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
     float w[VEC * TAPS];  // this thread's weights lie together: VEC channels of TAPS taps, a multiple of 16 bytes
     if (c < p.channels) {
 #pragma unroll
@@ -104,53 +106,57 @@ template <typename T, int VEC, int TAPS, int TOKENS> __global__ void __launch_bo
     }
     pdl_wait();
     if (c >= p.channels) return;
-    int seq[TOKENS], pos[TOKENS], pos0[TOKENS];
-    uint4 rows[TOKENS + TAPS - 1];  // rows t0 - (TAPS - 1) .. t0 + TOKENS - 1 of the step
+    for (int turn = 0; turn < TURNS; turn++) {
+        const int t0 = (blockIdx.x * TURNS + turn) * TOKENS;
+        if (t0 >= p.n_tokens) return;
+        int seq[TOKENS], pos[TOKENS], pos0[TOKENS];
+        uint4 rows[TOKENS + TAPS - 1];  // rows t0 - (TAPS - 1) .. t0 + TOKENS - 1 of the step
 #pragma unroll
-    for (int i = 0; i < TOKENS; i++) {
-        seq[i] = t0 + i < p.n_tokens ? p.token_seq[t0 + i] : -1;
-        pos[i] = t0 + i < p.n_tokens ? p.token_pos[t0 + i] : 0;
-    }
-#pragma unroll
-    for (int i = 0; i < TOKENS + TAPS - 1; i++) {
-        const int t = t0 + i - (TAPS - 1);
-        rows[i] = make_uint4(0, 0, 0, 0);
-        if (t >= 0 && t < p.n_tokens) rows[i] = *(const uint4 *)((const T *)p.in + (long long)t * p.ld + c);
-    }
-#pragma unroll
-    for (int i = 0; i < TOKENS; i++) pos0[i] = seq[i] >= 0 ? p.seq_pos0[seq[i]] : 0;
-#pragma unroll
-    for (int i = 0; i < TOKENS; i++) {
-        if (t0 + i >= p.n_tokens) break;
-        float acc[VEC];
-#pragma unroll
-        for (int u = 0; u < VEC; u++) acc[u] = 0.0f;
-        if (seq[i] >= 0) {
-            const float *tail = p.tail + (p.new_tail || pos[i] - pos0[i] < TAPS - 1 ? (long long)p.seq_slot[seq[i]] * (TAPS - 1) * p.channels + c : 0);
-#pragma unroll
-            for (int j = 0; j < TAPS; j++) {
-                const int back = TAPS - 1 - j, at = pos[i] - back;
-                float v[VEC];
-                if (at >= pos0[i]) ConvVector<T, VEC>::open(rows[i + j], v);
-                else if (at >= 0) {
-#pragma unroll
-                    for (int u = 0; u < VEC; u++) v[u] = tail[(long long)(at - (pos0[i] - (TAPS - 1))) * p.channels + u];
-                } else {
-#pragma unroll
-                    for (int u = 0; u < VEC; u++) v[u] = 0.0f;
-                }
-                if (p.new_tail && j > 0) {  // the input `back` tokens ago is back + 1 ago next time
-                    float *left = p.new_tail + (long long)p.seq_slot[seq[i]] * (TAPS - 1) * p.channels + (long long)(j - 1) * p.channels + c;
-#pragma unroll
-                    for (int u = 0; u < VEC; u++) left[u] = v[u];
-                }
-#pragma unroll
-                for (int u = 0; u < VEC; u++) acc[u] = fmaf(w[u * TAPS + j], v[u], acc[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < VEC; u++) acc[u] = p.plain ? acc[u] : silu_f(acc[u]);
+        for (int i = 0; i < TOKENS; i++) {
+            seq[i] = t0 + i < p.n_tokens ? p.token_seq[t0 + i] : -1;
+            pos[i] = t0 + i < p.n_tokens ? p.token_pos[t0 + i] : 0;
         }
-        ConvVector<T, VEC>::store((T *)p.out + (long long)(t0 + i) * p.channels + c, acc);
+#pragma unroll
+        for (int i = 0; i < TOKENS + TAPS - 1; i++) {
+            const int t = t0 + i - (TAPS - 1);
+            rows[i] = make_uint4(0, 0, 0, 0);
+            if (t >= 0 && t < p.n_tokens) rows[i] = *(const uint4 *)((const T *)p.in + (long long)t * p.ld + c);
+        }
+#pragma unroll
+        for (int i = 0; i < TOKENS; i++) pos0[i] = seq[i] >= 0 ? p.seq_pos0[seq[i]] : 0;
+#pragma unroll
+        for (int i = 0; i < TOKENS; i++) {
+            if (t0 + i >= p.n_tokens) break;
+            float acc[VEC];
+#pragma unroll
+            for (int u = 0; u < VEC; u++) acc[u] = 0.0f;
+            if (seq[i] >= 0) {
+                const float *tail = p.tail + (p.new_tail || pos[i] - pos0[i] < TAPS - 1 ? (long long)p.seq_slot[seq[i]] * (TAPS - 1) * p.channels + c : 0);
+#pragma unroll
+                for (int j = 0; j < TAPS; j++) {
+                    const int back = TAPS - 1 - j, at = pos[i] - back;
+                    float v[VEC];
+                    if (at >= pos0[i]) ConvVector<T, VEC>::open(rows[i + j], v);
+                    else if (at >= 0) {
+#pragma unroll
+                        for (int u = 0; u < VEC; u++) v[u] = tail[(long long)(at - (pos0[i] - (TAPS - 1))) * p.channels + u];
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < VEC; u++) v[u] = 0.0f;
+                    }
+                    if (p.new_tail && j > 0) {  // the input `back` tokens ago is back + 1 ago next time
+                        float *left = p.new_tail + (long long)p.seq_slot[seq[i]] * (TAPS - 1) * p.channels + (long long)(j - 1) * p.channels + c;
+#pragma unroll
+                        for (int u = 0; u < VEC; u++) left[u] = v[u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < VEC; u++) acc[u] = fmaf(w[u * TAPS + j], v[u], acc[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < VEC; u++) acc[u] = p.plain ? acc[u] : silu_f(acc[u]);
+            }
+            ConvVector<T, VEC>::store((T *)p.out + (long long)(t0 + i) * p.channels + c, acc);
+        }
     }
 }
 
@@ -170,16 +176,18 @@ extern "C" int abk_short_conv(const void *in, long long ld, void *out, int dtype
     cudaStream_t s = (cudaStream_t)stream;
     const int vec = dtype == ABK_BF16 ? 8 : 4;
     if (channels % vec == 0 && ld % vec == 0 && taps >= 2 && taps <= 4 && !(((uintptr_t)in | (uintptr_t)out | (uintptr_t)w) & 15)) {
-        const int many = n_tokens < 1024 ? 1 : dtype == ABK_BF16 ? CONV_TOKENS : CONV_TOKENS / 2;
-        dim3 tiles((n_tokens + many - 1) / many, (channels / vec + 127) / 128);
-#define CONV_AS(T, VEC, TAPS, TOKENS) abk_launch(short_conv_vec_kernel<T, VEC, TAPS, TOKENS>, tiles, dim3(128), 0, s, p)
+        const int strips = (channels / vec + 127) / 128, many = n_tokens < 1024 ? 1 : dtype == ABK_BF16 ? CONV_TOKENS : CONV_TOKENS / 2;
+        const int turns = dtype == ABK_F32 && many > 1 && (long long)n_tokens / many * strips >= 2400 ? 2 : 1;
+        dim3 tiles((n_tokens + many * turns - 1) / (many * turns), strips);
+#define CONV_AS(T, VEC, TAPS, TOKENS, TURNS) abk_launch(short_conv_vec_kernel<T, VEC, TAPS, TOKENS, TURNS>, tiles, dim3(128), 0, s, p)
 #define CONV_LAUNCH(TAPS)                                                   \
     if (dtype == ABK_BF16) {                                                \
-        if (many == 1) CONV_AS(__nv_bfloat16, 8, TAPS, 1);                  \
-        else CONV_AS(__nv_bfloat16, 8, TAPS, CONV_TOKENS);                  \
+        if (many == 1) CONV_AS(__nv_bfloat16, 8, TAPS, 1, 1);               \
+        else CONV_AS(__nv_bfloat16, 8, TAPS, CONV_TOKENS, 1);               \
     } else {                                                                \
-        if (many == 1) CONV_AS(float, 4, TAPS, 1);                          \
-        else CONV_AS(float, 4, TAPS, CONV_TOKENS / 2);                      \
+        if (many == 1) CONV_AS(float, 4, TAPS, 1, 1);                       \
+        else if (turns == 1) CONV_AS(float, 4, TAPS, CONV_TOKENS / 2, 1);   \
+        else CONV_AS(float, 4, TAPS, CONV_TOKENS / 2, 2);                   \
     }
         if (taps == 2) { CONV_LAUNCH(2) } else if (taps == 3) { CONV_LAUNCH(3) } else { CONV_LAUNCH(4) }
 #undef CONV_LAUNCH

@@ -731,7 +731,7 @@ def test_activations_in_bfloat16_are_the_float32_ones_rounded(V, first):
         assert torch.equal(outs[0].bfloat16(), outs[1])
 
 
-@pytest.mark.parametrize("lens,C,taps", [((1030,), 16, 4), ((700, 2, 1, 3, 330), 24, 3), ((1025, 1), 8, 2), ((3, 1, 2), 16, 4)])
+@pytest.mark.parametrize("lens,C,taps", [((1030,), 16, 4), ((700, 2, 1, 3, 330), 24, 3), ((1025, 1), 8, 2), ((3, 1, 2), 16, 4), ((1600, 3, 2, 1, 1599), 1028, 4)])
 def test_short_convolution_of_several_tokens_a_thread(lens, C, taps):
     """Groups of tokens that cross from sequence to sequence, rows before a sequence's start and from its slot's tail, both types."""
     from abacus_b200.kernels import ops
