@@ -2,7 +2,8 @@
 // run of rows padded to whole tiles of 128, so that a tile has one expert and the product is an ordinary tiled one
 // whose weight operand is chosen per row tile.
 //
-//   moe_sort      pairs (token, k-th choice) -> places in the sorted order. Three launches: a count per expert (each
+//   moe_sort      pairs (token, k-th choice) -> places in the sorted order. Two launches (three for steps of very many
+//                 pairs or experts, whose counts and places are kernels of their own): a count per expert (each
 //                 pair draws its rank within its expert with an atomic: the order within an expert is whatever the
 //                 hardware made it, which no result depends on, a row's product being its own); the experts' first
 //                 places (runs padded to 128 rows) and the expert of every row tile (-1 beyond the last); the rows
@@ -71,7 +72,7 @@ __global__ void __launch_bounds__(256) moe_offsets_kernel(const int *counts, int
 // Both of the above, and the counts' zeros, by one CTA: a launch that may start while the kernel before still runs, in place of three that
 // may not. With the gathering, 6,002 pairs, 16 experts, rows of 2,560: 9.8 us, with the three 16.4; 300 pairs: 3.1 and 9.1.
 #define MP_THREADS 1024
-#define MP_PAIRS 32768  // pairs that one CTA counts: beyond, many do it faster
+#define MP_PAIRS 32768  // pairs that one CTA counts (moe_plans)
 __global__ void __launch_bounds__(MP_THREADS) moe_plan_kernel(const int *pair_expert, int n_pairs, int experts, int *rank, int *first,
                                                               int *tile_expert, int max_tiles) {
     extern __shared__ int mp_tiles[];  // [experts + 1] first tile of each expert; [experts] pairs
@@ -141,6 +142,12 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const __nv_bfloat16 *x,
     }
 }
 
+// Pairs of a step and experts that one CTA plans: 16 experts, 32,768 pairs, with the gathering 45.4 us by one CTA and 47.4 by many, 8 experts 45.9
+// and 47.2 (24,576: 32.9 and 36.8; all pairs of one expert 55.7 and 63.7; 64 experts 44 and 53); one CTA's shared memory and time grow with both.
+static bool moe_plans(int n_pairs, int experts) { return n_pairs <= MP_PAIRS && experts <= 4096; }
+// Kernels that abk_moe_sort launches.
+extern "C" int abk_moe_sort_kernels(int n_pairs, int experts) { return n_pairs <= 0 ? 0 : moe_plans(n_pairs, experts) ? 2 : 3; }
+
 // counts [experts], rank and place [n_pairs], first [experts], tile_expert [max_tiles] int32; sorted bfloat16
 // [max_tiles * 128, d]. max_tiles >= ceil(n_pairs / 128) + experts.
 extern "C" int abk_moe_sort(const void *x, long long ldx, int pairs_per_row, const int *pair_expert, const float *pair_scale,
@@ -151,7 +158,7 @@ extern "C" int abk_moe_sort(const void *x, long long ldx, int pairs_per_row, con
         ABK_REFUSE("moe_sort: %d row tiles do not hold %d pairs of %d experts", max_tiles, n_pairs, experts);
     if (experts > 8192) ABK_REFUSE("moe_sort: %d experts", experts);
     cudaStream_t s = (cudaStream_t)stream;
-    if (n_pairs <= MP_PAIRS && experts <= 4096) {
+    if (moe_plans(n_pairs, experts)) {
         abk_launch(moe_plan_kernel, dim3(1), dim3(MP_THREADS), (size_t)(2 * experts + 1) * sizeof(int), s, pair_expert, n_pairs, experts, rank, first,
                    tile_expert, max_tiles);
     } else {

@@ -196,6 +196,10 @@ static bool gemm_split_wins(int M, int N, int K) {
 }
 // Bytes of scratch memory with which abk_gemm_simt goes to the tensor cores (0: it does not).
 extern "C" long long abk_gemm_simt_scratch(int M, int N, int K) { return gemm_split_wins(M, N, K) ? gemm_split_scratch(M, N, K) : 0; }
+// Kernels that abk_gemm_simt launches, given that scratch memory; dtype: of x and w.
+extern "C" int abk_gemm_simt_kernels(int dtype, int M, int N, int K) {
+    return M <= 0 || N <= 0 ? 0 : gemm_split_wins(M, N, K) ? gemm_split_kernels(M, N, K, dtype == ABK_F32 ? 3 : 1) : 1;
+}
 
 // x_dtype/w_dtype/out_dtype: ABK_F32 or ABK_BF16. Supported: all-float32; bf16 x and w with bf16 or f32 out.
 // scratch: at least abk_gemm_simt_scratch bytes, or null (then every product runs on the CUDA cores); status: int32 [>= 2], word 1

@@ -479,7 +479,7 @@ static void gp_choose(int M, int N, int K, int parts, bool may_quarter, int &bn,
     const long long pairs = abk_sm_count() / 2;
     const float pieces = (float)((K + GP_K - 1) / GP_K) * (gp_steps(K) == 4 ? 1.0f : gp_steps(K) == 2 ? 1.2f : 1.6f);  // (in those of sums over 64)
     float best = 0.0f;
-    bn = 0;
+    bn = quarters = 0;
     for (const auto &t : tile) {
         if (parts == 1 && t.bn == 128) continue;  // (not built: two numbers an output in registers)
         const long long tiles = ((long long)M + t.bn - 1) / t.bn * ((N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
@@ -503,6 +503,18 @@ static long long gp_planes(int rows, int K) {  // bytes, up to a multiple of 102
 static long long gemm_split_scratch(int M, int N, int K) {
     const int n_slab = gp_slab_rows(N, K, 256), m_slab = gp_slab_rows(M, K, 128);
     return gp_planes(n_slab, K) + gp_planes(m_slab, K) + (gp_may_quarter(m_slab, n_slab) ? 4LL * GP_QUARTERS * m_slab * n_slab : 0) + 1024;
+}
+
+// Kernels that gemm_split_run launches where the sizes choose the tile.
+static int gemm_split_kernels(int M, int N, int K, int parts) {
+    const int n_slab = gp_slab_rows(N, K, 256), m_slab = gp_slab_rows(M, K, 128);
+    int kernels = 0, bn, quarters;
+    for (int m = 0; m < M; m += m_slab)
+        for (int n = 0; n < N; n += n_slab) {
+            gp_choose(M - m < m_slab ? M - m : m_slab, N - n < n_slab ? N - n : n_slab, K, parts, parts == 3 && gp_may_quarter(m_slab, n_slab), bn, quarters);
+            kernels += 2 + quarters;
+        }
+    return kernels;
 }
 
 // Where bn is 0 the sizes choose it and whether K is walked in quarters.

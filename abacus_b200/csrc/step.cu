@@ -30,6 +30,7 @@ typedef int (*QkvPrepFn)(void *, int, int, int, int, int, int, const int *, cons
                          const int *, int, int, int, void *);
 typedef int (*GemmSimtFn)(const void *, int, const void *, int, void *, int, int, int, int, long long, long long, long long,
                           void *, long long, int *, void *);
+typedef int (*GemmSimtKernelsFn)(int, int, int, int);
 typedef int (*GemmRowsFn)(const void *, const void *, void *, int, int, int, int, long long, long long, long long, void *);
 typedef int (*GemmRowsSwigluFn)(const void *, const void *, void *, int, int, int, long long, long long, long long, int,
                                 void *);
@@ -64,6 +65,7 @@ struct AbkFns {
     SwigluFn swiglu;
     QkvPrepFn qkv_prep;
     GemmSimtFn gemm_simt;
+    GemmSimtKernelsFn gemm_simt_kernels;
     GemmRowsFn gemm_rows;
     GemmRowsSwigluFn gemm_rows_swiglu;
     GemmTcFn gemm_tc;
@@ -194,6 +196,7 @@ static int linear(const AbkModel &m, const AbkStep &s, const AbkLinear &l, const
     if (tc_takes(x, ldx, l))
         return LAUNCH(f.gemm_tc, x, l.w, out, out_dtype, rows, l.n, l.k, ldx, l.ldw, ldo, m.gemm_scratch, m.gemm_tickets,
                          m.kernel_status, 0, -1, 0, -1, stream);
+    if (s.parts && f.gemm_simt_kernels) step_launches += f.gemm_simt_kernels(l.dtype, rows, l.n, l.k) - 1;  // (LAUNCH counts one)
     return LAUNCH(f.gemm_simt, x, m.dtype, l.w, l.dtype, out, out_dtype, rows, l.n, l.k, ldx, l.ldw, ldo, s.parts, s.parts_bytes,
                   m.kernel_status, stream);
 }

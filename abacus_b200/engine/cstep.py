@@ -30,7 +30,8 @@ ENABLED = os.environ.get("ABACUS_C_STEP", "1") != "0"
 # (field of AbkFns, kernel library, exported launcher) in the order of csrc/step.cu
 LAUNCHERS = [("embed", "elementwise", "abk_embed"), ("add_rmsnorm", "elementwise", "abk_add_rmsnorm"),
              ("swiglu", "elementwise", "abk_swiglu"), ("qkv_prep", "elementwise", "abk_qkv_prep"),
-             ("gemm_simt", "gemm_simt", "abk_gemm_simt"), ("gemm_rows", "gemm_rows", "abk_gemm_rows"),
+             ("gemm_simt", "gemm_simt", "abk_gemm_simt"), ("gemm_simt_kernels", "gemm_simt", "abk_gemm_simt_kernels"),
+             ("gemm_rows", "gemm_rows", "abk_gemm_rows"),
              ("gemm_rows_swiglu", "gemm_rows", "abk_gemm_rows_swiglu"), ("gemm_tc", "gemm_tc", "abk_gemm_tc"),
              ("gemm_tc_swiglu", "gemm_tc", "abk_gemm_tc_swiglu"),
              ("attention_generic", "attention_generic", "abk_attention_generic"),

@@ -290,9 +290,14 @@ def gemm_simt_scratch(m, n, k):
     return lib.abk_gemm_simt_scratch(_i(m), _i(n), _i(k))
 
 
+@functools.lru_cache(maxsize=4096)
+def _gemm_simt_kernels(dtype, m, n, k):
+    return load_module("gemm_simt").abk_gemm_simt_kernels(_i(dtype), _i(m), _i(n), _i(k))
+
+
 def gemm_simt(x, w, out, m=None):
-    """out[:m] = x[:m] . w^T in float32, any sizes (src/model.c:299 and the like): on the CUDA cores, large ones on the
-    tensor cores in parts that together hold every digit (csrc/gemm_split.cuh)."""
+    """out[:m] = x[:m] . w^T with sums in float32, any sizes (src/model.c:299 and the like): on the CUDA cores, large ones on the
+    tensor cores in bfloat16 parts (csrc/gemm_split.cuh)."""
     _need_cuda(x, w, out)
     lib = load_module("gemm_simt")
     m = x.shape[0] if m is None else m
@@ -304,7 +309,7 @@ def gemm_simt(x, w, out, m=None):
     scratch = torch.empty(size, dtype=torch.uint8, device=x.device) if size else None
     _check(lib, lib.abk_gemm_simt(_p(x), _i(_dt(x)), _p(w), _i(_dt(w)), _p(out), _i(_dt(out)), _i(m), _i(n), _i(k),
                                   _ll(x.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)), _p(scratch), _ll(size),
-                                  _p(kernel_status(x.device)), _stream()), "gemm_simt")
+                                  _p(kernel_status(x.device)), _stream()), "gemm_simt", kernels=_gemm_simt_kernels(_dt(x), m, n, k))
 
 
 def gemm_rows_takes(x, w, out, m):
@@ -1517,7 +1522,7 @@ def moe_sort(x, pairs_per_row, pair_expert, pair_scale, n_pairs, experts, scratc
     counts, first, rank = scratch[:experts], scratch[experts:2 * experts], scratch[2 * experts:]
     _check(lib, lib.abk_moe_sort(_p(x), _ll(x.stride(0)), _i(pairs_per_row), _p(pair_expert), _p(pair_scale), _i(n_pairs),
                                  _i(experts), _i(d), _p(counts), _p(rank), _p(first), _p(place), _p(tile_expert),
-                                 _i(max_tiles), _p(sorted_rows), _stream()), "moe_sort", kernels=3)
+                                 _i(max_tiles), _p(sorted_rows), _stream()), "moe_sort", kernels=lib.abk_moe_sort_kernels(_i(n_pairs), _i(experts)))
 
 
 def gemm_grouped(x, w, out, tile_expert, activation=0, limit=0.0, in_pairs=-1):

@@ -356,6 +356,36 @@ def test_argmax_takes_the_first_maximum(ops):
     assert out[1].item() == 77 and out[2].item() == 5002 and out[3].item() == 0
 
 
+def test_launches_are_counted_as_they_are(ops):
+    """ops.LAUNCHES against the kernels of a captured graph: products by size (one kernel, parts and products, sums of quarters, several
+    slabs), and pairs sorted by expert in two launches or three."""
+    from cuda.bindings import runtime
+    scratch = lambda n: torch.empty(n, dtype=torch.int32, device="cuda")
+
+    def product(m, n, k, dtype=torch.float32):
+        x, w, out = torch.zeros(m, k, dtype=dtype, device="cuda"), torch.zeros(n, k, dtype=dtype, device="cuda"), torch.empty(m, n, device="cuda")
+        return lambda: ops.gemm_simt(x, w, out)
+
+    def sort(pairs, experts):
+        tiles = -(-pairs // 128) + experts
+        args = (torch.zeros(pairs, 8, dtype=torch.bfloat16, device="cuda"), 1, torch.zeros(pairs, dtype=torch.int32, device="cuda"), None, pairs, experts,
+                scratch(2 * experts + pairs), scratch(pairs), scratch(tiles), torch.empty(tiles * 128, 8, dtype=torch.bfloat16, device="cuda"))
+        return lambda: ops.moe_sort(*args)
+
+    for call, kernels in ((product(20, 100, 512), 1), (product(500, 6144, 1024), 2), (product(500, 1024, 3072), 3), (product(100, 20000, 1024), 5),
+                          (product(500, 2048, 1022, torch.bfloat16), 2), (sort(300, 4), 2), (sort(32768, 16), 2), (sort(32769, 16), 3)):
+        call()
+        torch.cuda.synchronize()
+        graph, before = torch.cuda.CUDAGraph(keep_graph=True), ops.LAUNCHES
+        with torch.cuda.graph(graph):
+            call()
+        raw = runtime.cudaGraph_t(init_value=graph.raw_cuda_graph())
+        _, _, count = runtime.cudaGraphGetNodes(raw)
+        nodes = runtime.cudaGraphGetNodes(raw, count)[1]
+        types = [runtime.cudaGraphNodeGetType(n)[1] for n in nodes]
+        assert types.count(runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel) == kernels == ops.LAUNCHES - before
+
+
 @pytest.mark.parametrize("temp, top_k", [(0.8, 20), (1.7, 5), (0.3, 64)])
 def test_sample_topk_draws_what_the_plain_sampler_draws(ops, temp, top_k):
     rng = np.random.default_rng(3)
