@@ -183,8 +183,9 @@ class StepBatch:
             self._sent_on.add(stream)
         self._dev.copy_(self._host, non_blocking=True)
         if self.device.type == "cuda":
+            # (the event stays with the batch's device, whichever device is the current one)
             self._sent = self._sent or torch.cuda.Event()
-            self._sent.record()
+            self._sent.record(torch.cuda.current_stream(self._dev.device))
 
     def advance_on_device(self):
         """Every sequence moves one position on (a decode step follows a decode step); the tokens are

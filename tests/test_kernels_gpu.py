@@ -697,6 +697,16 @@ def test_a_steps_words_are_made_known_to_each_stream_that_copies_them(ops, monke
         assert len(sent) == straight_so_far
 
 
+def test_a_steps_event_belongs_to_the_stream_that_copies(ops, monkeypatch):
+    """The event that keeps the pinned words from being rewritten is recorded on the batch's own device: one event serves the batch for good, and
+    the current device may change between two steps."""
+    from abacus_b200.engine.batch import Sequence, StepBatch
+    batch, recorded, record = StepBatch(4, 2, 0, "cuda"), [], torch.cuda.Event.record
+    monkeypatch.setattr(torch.cuda.Event, "record", lambda self, stream=None: (recorded.append(stream), record(self, stream)))
+    batch.fill([Sequence(0, [5], 0, [])])
+    assert len(recorded) == 1 and recorded[0] is not None and recorded[0].device == batch._dev.device
+
+
 # ------------------------------------------------------------------ tensor-core matrix product
 
 def product_tolerance(want, k, out_dtype):
