@@ -87,6 +87,13 @@ class Engine:
         prompts = use_graphs and prompt_graphs and os.environ.get("ABACUS_PROMPT_GRAPHS", "1") != "0"
         self.prompt_graphs = PromptGraphs(self, from_start_only=prompt_graphs == "from_start") if prompts else None
         self._step_batch = None
+        self._graph_memory = None
+
+    def graph_memory(self):
+        """The memory pool of the engine's captured steps, by its id."""
+        if self._graph_memory is None:
+            self._graph_memory = torch.cuda.MemPool()
+        return self._graph_memory.id
 
     # ------------------------------------------------------------ sequences
     def open(self):

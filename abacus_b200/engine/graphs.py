@@ -7,6 +7,9 @@ its step from a StepBatch whose device buffers never move; each replay is preced
 small host-to-device copy of that step's indices (or, with `advance`, by a kernel that moves
 every row one position on, so that a loop can run without the host).
 
+What a forward pass allocates and frees on its way (scratch memory of float32 products) comes from one pool that all of an engine's
+graphs share: their replays follow one another on the engine's stream, and none reads what another left there.
+
 A graph holds addresses: of the workspace, the cache, the rotary tables. If the workspace has
 grown since the capture (its generation changed), the graph is captured again.
 
@@ -67,7 +70,7 @@ class DecodeGraph:
         collecting = gc.isenabled()
         gc.disable()
         try:
-            with torch.cuda.graph(self.graph):
+            with torch.cuda.graph(self.graph, pool=self.engine.graph_memory()):
                 self.logits = self.engine.forward(self.batch)
         finally:
             if collecting:

@@ -274,6 +274,45 @@ def test_a_layer_that_reads_anothers_cache_goes_the_same_way_in_c(tmp_path, rows
     assert torch.equal(*logits)
 
 
+def test_captured_steps_share_their_scratch_memory(tmp_path):
+    """Captured prompt steps of a float32 model that goes through its parts: the products' scratch memory is there once, not once a
+    graph; replays in any order give what the steps gave; graphs and engines come and go."""
+    import gc
+    from abacus_b200.engine import Engine, load_model
+    folder = folder_of(tmp_path, "B", hidden_size=1024, intermediate_size=3072, num_attention_heads=16, num_key_value_heads=8, head_dim=128,
+                       max_position_embeddings=4096)
+    model, vocab = load_model(folder, "float32"), TINY["B"]["cfg"]["vocab_size"]
+    prompts = {n: random_tokens(np.random.default_rng(n), n, vocab) for n in (620, 500, 370, 250)}  # (rows 640, 512, 384 and 256)
+
+    def step(engine, n):
+        slot = engine.open()
+        out = engine.step([(slot, prompts[n], [0, n - 1])]).clone()
+        engine.close(slot)
+        return out
+
+    eager = Engine(model, max_tokens=4096, use_graphs=False)
+    eager.cstep = None
+    want = {n: step(eager, n) for n in prompts}
+    for _ in range(2):
+        engine = Engine(model, max_tokens=4096)
+        engine.cstep = None
+        held = []
+        for n in prompts:
+            for _ in range(3):
+                assert torch.equal(step(engine, n), want[n])
+            torch.cuda.synchronize()
+            held.append(torch.cuda.memory_reserved())
+        assert engine.prompt_graphs.captured == 4 and held[-1] - held[0] < 24 << 20, held  # (of its own a graph would have 60 to 100 MB of parts and sums)
+        for n in (250, 620, 370, 500, 250):
+            assert torch.equal(step(engine, n), want[n])
+        engine.prompt_graphs.graphs.clear()  # (all graphs gone, the pool is still the engine's)
+        gc.collect()
+        engine.prompt_graphs.seen.clear()
+        for _ in range(3):
+            assert torch.equal(step(engine, 370), want[370])
+        engine.check_status()
+
+
 def test_preparing_q_k_v_in_the_neighbouring_kernels_changes_no_bit(tmp_path, monkeypatch):
     """In bfloat16 the step between the q/k/v product and attention (per-head norm, rotation, cache write) runs in the
     product's epilogue for long prompt steps and inside the attention kernel for decode steps. With both switched off
