@@ -14,12 +14,14 @@
 //              rounded, the remainder rounded, the remainder of that), and the product is taken once with each;
 //   warps 2-9  a thread a query row (four warps a group): reads its row of S, masks (only in tiles that some row does not
 //              see whole), follows the row's maximum, and writes the three parts of the row's weights over its scores.
-// While one group's rows are in the softmax the tensor cores work for the other. Bound by the softmax warps: 995 instructions a
-// warp and tile one weight at a time, two warps to a scheduler, where the products of both groups take 1,100 cycles (tensor pipe
-// 29 % of active cycles). Two weights at a time need one multiply-add, sum or remainder for both and give the same bits. Measured one
+// While one group's rows are in the softmax the tensor cores work for the other. Bound by the softmax warps: 860 instructions a
+// warp and tile (995 one weight at a time), two warps to a scheduler, where the products of both groups take 1,100 cycles (tensor pipe
+// 31 % of active cycles). Two weights at a time need one multiply-add, sum or remainder for both and give the same bits. Measured one
 // weight at a time: 3 prompts, 3,893 tokens, 32 query and 8 key heads of 128, a window of 1,024: 158 us (the warp-level kernel 377);
-// 32 heads of 192 with values of 128, no window: 191 (506); two at a time the whole layers, products and all, go from 398 to 392 and
-// from 416 to 411 us.
+// 32 heads of 192 with values of 128, no window: 191 (506). Two at a time, the kernel alone in turns with the other: 155 -> 149 us and 190 ->
+// 183; 16 query heads, one prompt of 2,048: 67.3 -> 64.1; 512 tokens, 16 heads of 192 with values of 64: 28.05 and 28.33. (The whole layers, with
+// products and the host's step, change by less than their runs differ.) The pairs cost registers: the three instantiations
+// for values of 64 spill 68 bytes a thread (3,893 tokens, 16 heads of 64, a window of 512: 68.2 -> 67.2 all the same).
 // Tensor memory: two groups of 128 columns of output and of 96 columns of scores and weights, 512 in all, so a CTA to an SM.
 // A value row beyond the sequence's end belongs to another sequence or to nothing, and a weight of zero times what is no
 // number is none: the rows are set to zero in shared memory before the tile that crosses the end is multiplied.

@@ -5,7 +5,9 @@
 // sums: K in pieces of 16, piece c to sum c % 8, each sum over its k in ascending order, then in pairs,
 // ((s0 + s1) + (s2 + s3)) + ((s4 + s5) + (s6 + s7)); up to K = 256 it is one sum over k in ascending order (a chain of that
 // length needs no cutting, and the small products of small models keep the order they had). So a row's result does not
-// depend on where its tile lies, nor on how many other rows are in the batch as long as the product goes the same way.
+// depend on where its tile lies. Nor does it on how many other rows are in the batch as long as the product goes the same way: a row of a step that
+// is large enough for the tensor cores differs from the same row alone by the two orders' rounding (some 2e-7), so a prompt in one step
+// and token by token are not bit-equal where a product has 512 inputs and more and gemm_split_wins takes the step's rows.
 // Formula: src/model.c:299, 302, 307, 309, 324 (weights are [out, in] row-major, no bias).
 //
 // A warp has one tile of outputs and one of their sums. It stages its own pieces, 16 bytes at a time by cp.async (rows of 20

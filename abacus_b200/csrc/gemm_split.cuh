@@ -27,8 +27,8 @@
 // cores 691). What is left: factors below 1e-33 whose partners are beyond 2^14, so that the element is not small.
 //
 // What bounds it: the chain between the tensor cores and the warps that add up (0.3 us a short sum), and the way of the parts from
-// the L2, 6 bytes a number, at some 30 bytes a cycle and SM (500 x 6144 x 1024 in 65 us, 9 of them for the parts; sums of 128 53, the CUDA
-// cores 197; 4000 x 6144 x 1024 in 333 us, 253, 1,349). The adding warps report to their own CTA's barrier and the pair's idle warp passes
+// the L2, 6 bytes a number, at some 30 bytes a cycle and SM (500 x 6144 x 1024 in 62 us, 9 of them for the parts; sums over 128 53, the CUDA
+// cores 197; 4000 x 6144 x 1024 in 305 us, 253, 1,349). The adding warps report to their own CTA's barrier and the pair's idle warp passes
 // that on: 16 warps' words to the other CTA's barrier, one by one, took 72 us for 63.
 //
 // Two kernels: one writes the operands' parts as three planes of bfloat16 each, the other multiplies them on pairs of CTAs. (As one kernel

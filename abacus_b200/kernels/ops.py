@@ -1050,7 +1050,7 @@ def delta_scan(qkv, decay_in, beta_in, a_log, dt_bias, state, out, batch, n_head
     decay_in float32 [tokens, heads * key] (rows of any pitch) before bias and softplus; beta_in [tokens, >= heads] (rows of any pitch)
     before the sigmoid; out float32 [tokens, heads * value], not yet normed. per_head: one decay for all key channels of a
     head; decay_in is then [tokens, >= heads] of qkv's type and dt_bias [heads]. A step of one token a sequence is one kernel;
-    else every (block of four tokens, head), or for few and long prompts (chunk of 16, head), is prepared in parallel into scratch memory from
+    else every (block of four tokens, head), or where few columns walk beside the longest prompt (chunk of 16, head), is prepared in parallel into scratch memory from
     ws (a parts.Workspace), then the sequences are walked, a block or chunk at a time (tokens_a_time 4 or 16 pins it; refused where it is not
     built). chunks (with
     per_head, for steps that bring prompts): the walk goes in chunks of 64 tokens, a triangular system a chunk solved

@@ -1,7 +1,9 @@
 """out = x . W^T, the matrix product every projection is (src/model.c:299, 302, 307, 309, 324).
 
-float32: CUDA-core kernel with a fixed summation order. bfloat16: the tcgen05
-tensor-core kernel where it takes the shape, else the CUDA-core kernel.
+float32: few rows or little to do on the CUDA cores, else on the tensor cores in bfloat16 parts (csrc/gemm_simt.cu has the rule),
+each with a summation order that goes by the inputs alone: a row's bits do not depend on the rows beside it while
+a step's rows stay on one side of the rule, and change by some 2e-7 across it. bfloat16: the tcgen05
+tensor-core kernel where it takes the shape, else the kernels of the float32 path.
 """
 import torch
 
