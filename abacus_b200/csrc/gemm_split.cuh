@@ -124,12 +124,12 @@ struct GemmSplit {
     float *quarters;  // [GP_QUARTERS][M][N]
 };
 
-template <typename T> __device__ __forceinline__ void gp_put(const GemmSplit &g, int m, int n, float v) {
-    if (sizeof(T) == 4 || g.out_dtype == ABK_F32) ((float *)g.out)[m * g.ldo + n] = v;
+__device__ __forceinline__ void gp_put(const GemmSplit &g, int m, int n, float v) {
+    if (g.out_dtype == ABK_F32) ((float *)g.out)[m * g.ldo + n] = v;
     else ((__nv_bfloat16 *)g.out)[m * g.ldo + n] = __float2bfloat16_rn(v);
 }
-template <typename T> __device__ __forceinline__ float gp_stored(const GemmSplit &g, int m, int n) {
-    if (sizeof(T) == 4 || g.out_dtype == ABK_F32) return __ldcg((const float *)g.out + m * g.ldo + n);
+__device__ __forceinline__ float gp_stored(const GemmSplit &g, int m, int n) {
+    if (g.out_dtype == ABK_F32) return __ldcg((const float *)g.out + m * g.ldo + n);
     return __bfloat162float(__ldcg((const __nv_bfloat16 *)g.out + m * g.ldo + n));
 }
 // Whether a sum has to be taken again.
@@ -194,7 +194,7 @@ template <typename T, int THREADS> __device__ __forceinline__ void gp_redo(const
     if (tid < THREADS)
 #pragma unroll
         for (int j = 0; j < 8; j++)
-            if (bad >> j & 1) gp_put<T>(g, m0 + row + j, n0 + n, a[j]);
+            if (bad >> j & 1) gp_put(g, m0 + row + j, n0 + n, a[j]);
 }
 
 // The same for the tiles of a pair's CTA (item pair, pair + pairs, ...).
@@ -205,7 +205,7 @@ template <typename T, int BN> __device__ __noinline__ void gp_redo_items(const G
         for (int m0 = item % g.m_tiles * BN; m0 < m_end; m0 += ROWS) {
             uint32_t bad = 0;
             if (threadIdx.x < THREADS && n < g.N)
-                for (int j = 0, m = m0 + threadIdx.x / 128 * 8; j < 8 && m < m_end; j++, m++) bad |= (uint32_t)gp_again(gp_stored<T>(g, m, n)) << j;
+                for (int j = 0, m = m0 + threadIdx.x / 128 * 8; j < 8 && m < m_end; j++, m++) bad |= (uint32_t)gp_again(gp_stored(g, m, n)) << j;
             if (__syncthreads_or(bad)) gp_redo<T, THREADS>(g, m0, n0, bad, smem);
         }
     }
@@ -405,7 +405,7 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
                     for (int j = 0; j < COLS; j++)
                         if (j < cols) {
                             const float v = PARTS == 3 ? total[j] : sum[j] + total[j];
-                            gp_put<T>(g, m0 + j, n, v), redo |= gp_again(v);
+                            gp_put(g, m0 + j, n, v), redo |= gp_again(v);
                         }
                 }
 #pragma unroll
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(GP_SUM_THREADS) gemm_split_sum_kernel(const __
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const float v = ((q[j][0] + q[j][1]) + q[j][2]) + q[j][3];
-            if (m + j < g.M && n < g.N) gp_put<float>(g, m + j, n, v), bad |= (uint32_t)gp_again(v) << j;
+            if (m + j < g.M && n < g.N) gp_put(g, m + j, n, v), bad |= (uint32_t)gp_again(v) << j;
         }
         if (__syncthreads_or(bad)) gp_redo<float, GP_SUM_THREADS>(g, m0, n0, bad, smem);
     }

@@ -297,6 +297,24 @@ def test_products_in_parts_refuse_a_k_without_four_quarters(ops, k):
         assert rc == (-1 if k < 193 else 0) and bool((out == (7.0 if k < 193 else k)).all()) and not status.any()
 
 
+@pytest.mark.parametrize("quarters", [0, 1])
+def test_products_in_parts_store_what_they_are_asked_to(ops, quarters):
+    """Float32 operands and bfloat16 results through the exported launcher: the float32 results rounded, and not a number beyond them."""
+    m, n, k = 70, 300, 700
+    gen, lib, status = torch.Generator(device="cuda").manual_seed(7), ops.load_module("gemm_simt"), ops.kernel_status(torch.device("cuda", 0))
+    x, w = torch.randn((m, k), generator=gen, device="cuda"), torch.randn((n, k), generator=gen, device="cuda")
+    x[5] = float("nan")
+    lib.abk_gemm_split_scratch.restype = ctypes.c_longlong
+    scratch, outs = torch.empty(lib.abk_gemm_split_scratch(m, n, k), dtype=torch.uint8, device="cuda"), []
+    for dtype in (torch.float32, torch.bfloat16):
+        room = torch.full((2 * m, n), 7, dtype=dtype, device="cuda")
+        assert lib.abk_gemm_split(ops._p(x), ops._p(w), ops._i(0), ops._p(room), ops._i(ops._dt(room)), ops._i(m), ops._i(n), ops._i(k), ops._ll(k),
+                                  ops._ll(k), ops._ll(n), ops._i(96), ops._i(quarters), ops._p(scratch), ops._p(status), ops._stream()) == 0
+        assert bool((room[m:] == 7).all())
+        outs.append(room[:m].bfloat16().nan_to_num(9))
+    assert torch.equal(*outs) and bool((outs[0][5] == 9).all()) and not status.any()
+
+
 def test_a_product_of_nothing_but_nan_takes_no_milliseconds(ops):
     """Eight times what it takes on the CUDA cores at most: the tiles are taken again by the CTAs that made them, one after the other."""
     m, n, k = 500, 6144, 1024
