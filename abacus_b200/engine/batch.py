@@ -159,7 +159,7 @@ class StepBatch:
                 setattr(self, name, whole if whole.shape[0] == n else whole[:n])
         self.sequences = list(sequences)  # host view, for mixers that walk the sequences themselves
         self.is_decode = one_each
-        self.longest = max(lens, default=0)
+        self.longest = 1 if one_each else max(lens, default=0)
         for name, p in self.plans.items():
             info = p.fill(self._layouts[name], self.sequences, h[f"plan:{name}"], self.is_decode, exact)
             self.plan[name] = PlanView(p, self._layouts[name], self._parts[f"plan:{name}"], info)

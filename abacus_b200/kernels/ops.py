@@ -291,8 +291,9 @@ def gemm_simt_scratch(m, n, k):
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_simt_kernels(dtype, m, n, k):
-    return load_module("gemm_simt").abk_gemm_simt_kernels(_i(dtype), _i(m), _i(n), _i(k))
+def _gemm_simt_plan(dtype, m, n, k):
+    """(bytes of scratch memory, kernels) of a product of these sizes."""
+    return gemm_simt_scratch(m, n, k), load_module("gemm_simt").abk_gemm_simt_kernels(_i(dtype), _i(m), _i(n), _i(k))
 
 
 def gemm_simt(x, w, out, m=None):
@@ -305,11 +306,12 @@ def gemm_simt(x, w, out, m=None):
     assert x.shape[1] == k and out.shape[1] == n and x.shape[0] >= m and out.shape[0] >= m
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     # (of the calling stream's own: freed when this returns, and given out again behind what runs on that stream)
-    size = gemm_simt_scratch(m, n, k)
+    kind = _dt(x)
+    size, kernels = _gemm_simt_plan(kind, m, n, k)
     scratch = torch.empty(size, dtype=torch.uint8, device=x.device) if size else None
-    _check(lib, lib.abk_gemm_simt(_p(x), _i(_dt(x)), _p(w), _i(_dt(w)), _p(out), _i(_dt(out)), _i(m), _i(n), _i(k),
+    _check(lib, lib.abk_gemm_simt(_p(x), _i(kind), _p(w), _i(_dt(w)), _p(out), _i(_dt(out)), _i(m), _i(n), _i(k),
                                   _ll(x.stride(0)), _ll(w.stride(0)), _ll(out.stride(0)), _p(scratch), _ll(size),
-                                  _p(kernel_status(x.device)), _stream()), "gemm_simt", kernels=_gemm_simt_kernels(_dt(x), m, n, k))
+                                  _p(kernel_status(x.device)), _stream()), "gemm_simt", kernels=kernels)
 
 
 def gemm_rows_takes(x, w, out, m):
