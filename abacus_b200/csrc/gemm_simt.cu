@@ -178,7 +178,7 @@ static int gemm_simt_launch(const void *x, const void *w, void *out, int M, int 
 }
 
 // The product on the tensor cores (gemm_split.cuh), for any M and N and K from 193 on (every quarter of K has a piece of 64). bn: rows of x in a tile (32, 64, 96, 128), quarters: pairs of CTAs take
-// quarters of K (of float32 operands only); 0, 0: by size. scratch: abk_gemm_split_scratch bytes.
+// quarters of K (not of bfloat16 operands below K = 2048, nor are there tiles of 128 then); 0, 0: by size. scratch: abk_gemm_split_scratch bytes.
 extern "C" int abk_gemm_split(const void *x, const void *w, int dtype, void *out, int out_dtype, int M, int N, int K, long long ldx, long long ldw,
                               long long ldo, int bn, int quarters, void *scratch, int *status, void *stream) {
     const GemmSplit g = {x, w, out, dtype, out_dtype, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};
@@ -192,15 +192,16 @@ extern "C" long long abk_gemm_split_scratch(int M, int N, int K) { return gemm_s
 // host side takes some 12 us more: 64 x 6144 x 1024 in 27 us against 32, 100 x 4096 x 1024 in 21 against 36, 500 x 1024 x 1024 in 20 against
 // 35; below that there is little to win (64 x 1024 x 1024: 12.8 against 13.4; 500 x 256 x 512: 10.3 against 7.9). 64 columns are one of the plain
 // kernel's tiles and a quarter of a pair's: 6300 x 64 x 1024 in 39 us against 36, x 72 in 39 against 67. Up to 64 rows are one of its tiles too, and
-// weights beyond the L2 are written and read again as parts: 33 x 40960 x 1024 in 145 against 157, x 65536 in 231 against 223.
-static bool gemm_split_wins(int M, int N, int K) {
-    return M > 32 && N > 64 && K >= 512 && (long long)M * N * K >= 400000000LL && (M > 64 || N < 65536);
+// weights beyond the L2 are written and read again as parts: 33 x 40960 x 1024 in 145 against 157, x 65536 in 231 against 223; 40 x
+// 16384 x 700 in 46 against 50, 33 x 24000 x 512 in 59 against 53. (bfloat16: 33 x 24000 x 513 in 50 against 77.)
+static bool gemm_split_wins(int dtype, int M, int N, int K) {
+    return M > 32 && N > 64 && K >= 512 && (long long)M * N * K >= 400000000LL && (dtype == ABK_BF16 || M > 64 || N < (K < 1024 ? 20000 : 65536));
 }
-// Bytes of scratch memory with which abk_gemm_simt goes to the tensor cores (0: it does not).
-extern "C" long long abk_gemm_simt_scratch(int M, int N, int K) { return gemm_split_wins(M, N, K) ? gemm_split_scratch(M, N, K) : 0; }
+// Bytes of scratch memory with which abk_gemm_simt goes to the tensor cores (0: it does not); dtype: of x and w.
+extern "C" long long abk_gemm_simt_scratch(int M, int N, int K, int dtype) { return gemm_split_wins(dtype, M, N, K) ? gemm_split_scratch(M, N, K) : 0; }
 // Kernels that abk_gemm_simt launches, given that scratch memory; dtype: of x and w.
 extern "C" int abk_gemm_simt_kernels(int dtype, int M, int N, int K) {
-    return M <= 0 || N <= 0 ? 0 : gemm_split_wins(M, N, K) ? gemm_split_kernels(M, N, K, dtype == ABK_F32 ? 3 : 1) : 1;
+    return M <= 0 || N <= 0 ? 0 : gemm_split_wins(dtype, M, N, K) ? gemm_split_kernels(M, N, K, dtype == ABK_F32 ? 3 : 1) : 1;
 }
 
 // x_dtype/w_dtype/out_dtype: ABK_F32 or ABK_BF16. Supported: all-float32; bf16 x and w with bf16 or f32 out.
@@ -214,7 +215,7 @@ extern "C" int abk_gemm_simt(const void *x, int x_dtype, const void *w, int w_dt
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
     if (N > 65535 * 64) ABK_REFUSE("gemm: %d output columns are more than one launch takes", N);
-    if (scratch && x_dtype == w_dtype && (x_dtype == ABK_BF16 || out_dtype == ABK_F32) && gemm_split_wins(M, N, K)) {
+    if (scratch && x_dtype == w_dtype && (x_dtype == ABK_BF16 || out_dtype == ABK_F32) && gemm_split_wins(x_dtype, M, N, K)) {
         if (scratch_bytes < gemm_split_scratch(M, N, K))
             ABK_REFUSE("gemm: %lld bytes of scratch memory for %d x %d x %d, which takes %lld", scratch_bytes, M, N, K, gemm_split_scratch(M, N, K));
         const GemmSplit g = {x, w, out, x_dtype, out_dtype, M, N, K, 0, 0, ldx, ldw, ldo, status, nullptr};

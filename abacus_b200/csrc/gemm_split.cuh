@@ -18,9 +18,10 @@
 // order, then its small products. That order goes by K alone: a row's result does not depend on how many other rows
 // are in the batch, whether a pair of CTAs walks all of K or a quarter, or where its tile lies.
 // bfloat16 operands (those that the tensor-core product proper refuses: rows that start anywhere) have one part. Their eight sums on the CUDA
-// cores lose less, a product being exact there too, so their short sums, over 16, are added in one running sum with what each addition rounds off
-// beside it (Knuth's two-sum), added at the end. (In float32 that takes 2048 x 1024 x 1020 from 22 us, with errors of 1.3e-7, to 68, with 0.35e-7;
-// the CUDA cores 148, 0.9e-7.)
+// cores lose less, a product being exact there too, so below K = 2048 their short sums, over 16 and from 1024 on over 32, are added in one running
+// sum with what each addition rounds off beside it (Knuth's two-sum), added at the end; from there on they go as float32 ones, over 32. Errors of
+// this and of the CUDA cores, K = 512, 1024, 2048, 3072: magnitudes 3.2 4.7 6.2 5.9 and 4.5 5.2 6.8 6.9e-8, either sign 3.5 4.6 9.5 10.9 and 6.9 8.7 11.7
+// 14.4e-8. 2048 x 1024 x 1020 in 68 us, 273 x 686 x 2768 in 21 (the CUDA cores 148 and 76; two-sums over 16 at every K 68 and 89).
 // A number that is not finite makes its products NaN in this form, and one below 1e-33 keeps fewer digits (its third part is too small for
 // bfloat16): an element that came out not finite, or below 2^-96 but not zero, is taken again with the CUDA cores' eight sums, a tile at a time and
 // behind all waits, so that no wait runs out meanwhile: 2000 x 6144 x 1024 in 170 us, with one row of NaN 400, with nothing but NaN 3,600 (the CUDA
@@ -217,8 +218,8 @@ template <> struct GpOperand<1> { typedef __nv_bfloat16 T; };
 // A tile is 256 rows of w (128 of each CTA) and BN rows of x; pair c of CTAs takes items c, c + pairs, ... An item is a tile, or
 // (QUARTERS) a quarter of K of one, whose sums go to `quarters` and are added up by the kernel behind.
 // map_w, map_x: the planes, one below the other; PARTS: 3 of float32 operands, 1 of bfloat16 ones; STEPS: of 16 of K in a
-// short sum, 1, 2 or 4.
-template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_bounds__(GP_THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w,
+// short sum, 1, 2 or 4; TWO_SUM: one running sum of all, with what its additions round off.
+template <int BN, bool QUARTERS, int PARTS, int STEPS, bool TWO_SUM> __global__ void __launch_bounds__(GP_THREADS, 1) gemm_split_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                                                const __grid_constant__ CUtensorMap map_x, const __grid_constant__ GemmSplit g) {
     using S = GpShape<BN>;
     constexpr int STAGES = S::STAGES, COLS = S::COLS, SUMS = S::SUMS, SMALLS = S::SMALLS;
@@ -341,7 +342,7 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
         // a warp has a quarter of the lanes (the weights' rows) and COLS columns (rows of x) of the accumulators
         const int lane_base = (warp & 3) * 32, col0 = (warp >> 2) * COLS;
         const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + col0;
-        float sum[COLS], total[COLS];  // of the quarter, of those before; PARTS 1: of all, and what its additions rounded off
+        float sum[COLS], total[COLS];  // of the quarter, of those before; TWO_SUM: of all, and what its additions rounded off
         const f32x2 minus = pack2(-1.0f, -1.0f);
 #pragma unroll
         for (int j = 0; j < COLS; j++) sum[j] = total[j] = 0.0f;
@@ -365,7 +366,7 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
 #pragma unroll
                         for (int j = 0; j < 8; j += 2) {
                             float *const s2 = sum + c + j, *const t2 = total + c + j;
-                            if constexpr (PARTS == 3) {
+                            if constexpr (!TWO_SUM) {
                                 s2[0] += __uint_as_float(v[j]), s2[1] += __uint_as_float(v[j + 1]);
                             } else {
                                 const f32x2 a = pack2(s2[0], s2[1]), b2 = pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
@@ -375,13 +376,15 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
                             }
                         }
                     }
-                    if (PARTS == 3 && n + 1 == sums) {
+                    if (!TWO_SUM && n + 1 == sums) {
 #pragma unroll
                         for (int c = 0; c < COLS; c += 8) {
-                            gp_tmem_ld<8>(taddr + (SUMS + quarter_i % SMALLS) * BN + c, v);
-                            tc::tmem_ld_wait();
+                            if constexpr (PARTS == 3) {
+                                gp_tmem_ld<8>(taddr + (SUMS + quarter_i % SMALLS) * BN + c, v);
+                                tc::tmem_ld_wait();
+                            }
 #pragma unroll
-                            for (int j = 0; j < 8; j++) total[c + j] += sum[c + j] + __uint_as_float(v[j]), sum[c + j] = 0.0f;
+                            for (int j = 0; j < 8; j++) total[c + j] += PARTS == 3 ? sum[c + j] + __uint_as_float(v[j]) : sum[c + j], sum[c + j] = 0.0f;
                         }
                     }
                     tc::fence_before_sync();
@@ -404,7 +407,7 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
 #pragma unroll
                     for (int j = 0; j < COLS; j++)
                         if (j < cols) {
-                            const float v = PARTS == 3 ? total[j] : sum[j] + total[j];
+                            const float v = TWO_SUM ? sum[j] + total[j] : total[j];
                             gp_put(g, m0 + j, n, v), redo |= gp_again(v);
                         }
                 }
@@ -427,7 +430,7 @@ template <int BN, bool QUARTERS, int PARTS, int STEPS> __global__ void __launch_
 
 // The four quarters' sums of every element, in order: a CTA has tiles of 16 rows and 128 columns, a thread a column and eight rows.
 #define GP_SUM_THREADS 256
-__global__ void __launch_bounds__(GP_SUM_THREADS) gemm_split_sum_kernel(const __grid_constant__ GemmSplit g) {
+template <typename T> __global__ void __launch_bounds__(GP_SUM_THREADS) gemm_split_sum_kernel(const __grid_constant__ GemmSplit g) {  // T: of the operands
     __shared__ __align__(16) float smem[GP_REDO_FLOATS(GP_SUM_THREADS)];
     constexpr int ROWS = GP_SUM_THREADS / 16;
     const long long plane = (long long)g.M * g.N;
@@ -446,28 +449,29 @@ __global__ void __launch_bounds__(GP_SUM_THREADS) gemm_split_sum_kernel(const __
             const float v = ((q[j][0] + q[j][1]) + q[j][2]) + q[j][3];
             if (m + j < g.M && n < g.N) gp_put(g, m + j, n, v), bad |= (uint32_t)gp_again(v) << j;
         }
-        if (__syncthreads_or(bad)) gp_redo<float, GP_SUM_THREADS>(g, m0, n0, bad, smem);
+        if (__syncthreads_or(bad)) gp_redo<T, GP_SUM_THREADS>(g, m0, n0, bad, smem);
     }
 }
 
-template <int BN, bool QUARTERS, int PARTS, int STEPS> static int gemm_split_launch(const CUtensorMap &map_w, const CUtensorMap &map_x, GemmSplit g, cudaStream_t s) {
+template <int BN, bool QUARTERS, int PARTS, int STEPS, bool TWO_SUM = false> static int gemm_split_launch(const CUtensorMap &map_w, const CUtensorMap &map_x, GemmSplit g, cudaStream_t s) {
     using S = GpShape<BN>;
-    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_split_kernel<BN, QUARTERS, PARTS, STEPS>, S::BYTES);
+    const cudaError_t e = abk_allow_shared_memory((const void *)gemm_split_kernel<BN, QUARTERS, PARTS, STEPS, TWO_SUM>, S::BYTES);
     if (e != cudaSuccess) return (int)e;
     const int pairs = abk_sm_count() / 2, items = QUARTERS ? g.tiles * GP_QUARTERS : g.tiles;
-    abk_launch_clusters(gemm_split_kernel<BN, QUARTERS, PARTS, STEPS>, dim3(2 * (items < pairs ? items : pairs)), dim3(GP_THREADS), S::BYTES, s, 2, map_w, map_x, g);
+    abk_launch_clusters(gemm_split_kernel<BN, QUARTERS, PARTS, STEPS, TWO_SUM>, dim3(2 * (items < pairs ? items : pairs)), dim3(GP_THREADS), S::BYTES, s, 2, map_w, map_x, g);
     const int rc = ABK_LAUNCH_RESULT();
     if (rc || !QUARTERS) return rc;
     const long long blocks = ((long long)g.M + 15) / 16 * ((g.N + 127) / 128), most = 8LL * abk_sm_count();
-    abk_launch(gemm_split_sum_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(GP_SUM_THREADS), 0, s, g);
+    abk_launch(gemm_split_sum_kernel<typename GpOperand<PARTS>::T>, dim3((unsigned)(blocks < most ? blocks : most)), dim3(GP_SUM_THREADS), 0, s, g);
     return ABK_LAUNCH_RESULT();
 }
 
 #define GP_QUARTERS_BYTES (64LL << 20)  // sums of quarters in the scratch memory at most
 static bool gp_may_quarter(int M, int N) { return 4LL * GP_QUARTERS * M * N <= GP_QUARTERS_BYTES; }
 
-// Steps of 16 of K in a short sum of float32 operands' parts.
-static int gp_steps(int K) { return K < 1024 ? 1 : K < 2048 ? 2 : 4; }
+// Steps of 16 of K in a short sum, and whether bfloat16 operands are added up by two-sums.
+static int gp_steps(int K, int parts) { return K < 1024 ? 1 : K < 2048 || parts == 1 ? 2 : 4; }
+static bool gp_two_sum(int K, int parts) { return parts == 1 && K < 2048; }
 
 // Rows of x in a tile, and whether pairs of CTAs take quarters of K: what takes least, by turns of the GPU's pairs times what a
 // piece of 64 of K takes (measured with a turn each: 1.2 us for tiles of 32 rows, 1.25, 1.35, 1.5 for 128 with sums over 64, a fifth more
@@ -477,11 +481,11 @@ static int gp_steps(int K) { return K < 1024 ? 1 : K < 2048 ? 2 : 4; }
 static void gp_choose(int M, int N, int K, int parts, bool may_quarter, int &bn, int &quarters) {
     static const struct { int bn; float us; } tile[4] = {{32, 1.2f}, {64, 1.25f}, {96, 1.35f}, {128, 1.5f}};
     const long long pairs = abk_sm_count() / 2;
-    const float pieces = (float)((K + GP_K - 1) / GP_K) * (gp_steps(K) == 4 ? 1.0f : gp_steps(K) == 2 ? 1.2f : 1.6f);  // (in those of sums over 64)
+    const float pieces = (float)((K + GP_K - 1) / GP_K) * (gp_steps(K, parts) == 4 ? 1.0f : gp_steps(K, parts) == 2 ? 1.2f : 1.6f);  // (in those of sums over 64)
     float best = 0.0f;
     bn = quarters = 0;
     for (const auto &t : tile) {
-        if (parts == 1 && t.bn == 128) continue;  // (not built: two numbers an output in registers)
+        if (gp_two_sum(K, parts) && t.bn == 128) continue;  // (not built: two numbers an output in registers)
         const long long tiles = ((long long)M + t.bn - 1) / t.bn * ((N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
         for (int q = 0; q < (may_quarter ? 2 : 1); q++) {
             const float us = q ? (float)((tiles * GP_QUARTERS + pairs - 1) / pairs) * pieces / GP_QUARTERS * t.us + 3.0f + (float)M * (float)N * 6.4e-6f
@@ -511,7 +515,7 @@ static int gemm_split_kernels(int M, int N, int K, int parts) {
     int kernels = 0, bn, quarters;
     for (int m = 0; m < M; m += m_slab)
         for (int n = 0; n < N; n += n_slab) {
-            gp_choose(M - m < m_slab ? M - m : m_slab, N - n < n_slab ? N - n : n_slab, K, parts, parts == 3 && gp_may_quarter(m_slab, n_slab), bn, quarters);
+            gp_choose(M - m < m_slab ? M - m : m_slab, N - n < n_slab ? N - n : n_slab, K, parts, !gp_two_sum(K, parts) && gp_may_quarter(m_slab, n_slab), bn, quarters);
             kernels += 2 + quarters;
         }
     return kernels;
@@ -528,7 +532,7 @@ template <typename T> static int gemm_split_run(GemmSplit g, int bn, int quarter
     g.quarters = (float *)(x_planes + gp_planes(m_slab, g.K) / 2);
     const T *const x = (const T *)g.x, *const w = (const T *)g.w;
     char *const out = (char *)g.out;
-    const bool may_quarter = parts == 3 && gp_may_quarter(m_slab, n_slab);
+    const bool may_quarter = !gp_two_sum(g.K, parts) && gp_may_quarter(m_slab, n_slab);
     const auto vec = [&](const T *from, long long ld) { return sizeof(T) == 4 && g.K % 4 == 0 && ld % 4 == 0 && !((uintptr_t)from & 15); };
     for (int m = 0; m < M; m += m_slab)
         for (int n = 0; n < N; n += n_slab) {
@@ -544,18 +548,19 @@ template <typename T> static int gemm_split_run(GemmSplit g, int bn, int quarter
             if (!b) gp_choose(g.M, g.N, g.K, parts, may_quarter, b, in_quarters);
             if (in_quarters && !may_quarter) ABK_REFUSE("gemm: no room for the quarters of %d x %d sums", g.M, g.N);
             g.m_tiles = (g.M + b - 1) / b, g.tiles = g.m_tiles * ((g.N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
-            const int steps = gp_steps(g.K);
+            const int steps = gp_steps(g.K, parts);
             CUtensorMap map_w, map_x;
             if ((rc = tmap::bf16_rows_of_128_bytes(w_planes, (long long)parts * g.N, g.K, pitch, GP_ROWS, &map_w))) return rc;
             if ((rc = tmap::bf16_rows_of_128_bytes(x_planes, (long long)parts * g.M, g.K, pitch, b / 2, &map_x))) return rc;
-#define GP_CASE(BN)                                                                                                                        \
-    case BN:                                                                                                                               \
-        if constexpr (parts == 3)                                                                                                          \
-            rc = steps == 1 ? GP_AS(BN, 1) : steps == 2 ? GP_AS(BN, 2) : GP_AS(BN, 4);                                                     \
-        else if constexpr (BN < 128) rc = gemm_split_launch<BN, false, 1, 1>(map_w, map_x, g, s);                                          \
-        else ABK_REFUSE("gemm: tiles of %d rows of bfloat16 numbers are not built", BN);                                                   \
+#define GP_AS(BN, STEPS) (in_quarters ? gemm_split_launch<BN, true, parts, STEPS>(map_w, map_x, g, s) : gemm_split_launch<BN, false, parts, STEPS>(map_w, map_x, g, s))
+#define GP_CASE(BN)                                                                                                             \
+    case BN:                                                                                                                    \
+        if constexpr (parts == 3) rc = steps == 1 ? GP_AS(BN, 1) : steps == 2 ? GP_AS(BN, 2) : GP_AS(BN, 4);                    \
+        else if (!gp_two_sum(g.K, parts)) rc = GP_AS(BN, 2);                                                                    \
+        else if constexpr (BN < 128)                                                                                            \
+            rc = steps == 1 ? gemm_split_launch<BN, false, 1, 1, true>(map_w, map_x, g, s) : gemm_split_launch<BN, false, 1, 2, true>(map_w, map_x, g, s); \
+        else ABK_REFUSE("gemm: tiles of %d rows of bfloat16 numbers are not built for K = %d", BN, g.K);                        \
         break
-#define GP_AS(BN, STEPS) (in_quarters ? gemm_split_launch<BN, true, 3, STEPS>(map_w, map_x, g, s) : gemm_split_launch<BN, false, 3, STEPS>(map_w, map_x, g, s))
             switch (b) {
                 GP_CASE(32);
                 GP_CASE(64);

@@ -258,8 +258,8 @@ class CStep:
         s.xn_final = ws.get("xn_final", (max(r, 1), d), dtype).data_ptr()
         s.partial_floats = partial_floats
         # (a smaller matrix can need more: with few columns the sums of quarters of K fit too)
-        s.parts_bytes = max([ops.gemm_simt_scratch(n, *p) for p in self.products]
-                            + [ops.gemm_simt_scratch(r, *self.head_product) if self.head_product else 0])
+        s.parts_bytes = max([ops.gemm_simt_scratch(n, *p, _dt(dtype)) for p in self.products]
+                            + [ops.gemm_simt_scratch(r, *self.head_product, _dt(dtype)) if self.head_product else 0])
         s.parts = ws.get("parts", (s.parts_bytes,), torch.uint8).data_ptr() if s.parts_bytes else None
         s.n_rows, s.n_logit_rows, s.is_decode, s.any_continuation = n, r, int(batch.is_decode), int(batch.any_continuation)
         s.max_len_after, s.position_bound, s.n_lists = batch.max_len_after, bound, len(self.plan_names)

@@ -283,17 +283,17 @@ def attention_generic(qkv, out, n_heads, n_kv_heads, head_dim, scale, window, ba
 
 
 @functools.lru_cache(maxsize=4096)
-def gemm_simt_scratch(m, n, k):
+def gemm_simt_scratch(m, n, k, dtype=F32):
     """Bytes of scratch memory with which gemm_simt runs a product of these sizes on the tensor cores (0: it does not)."""
     lib = load_module("gemm_simt")
     lib.abk_gemm_simt_scratch.restype = ctypes.c_longlong
-    return lib.abk_gemm_simt_scratch(_i(m), _i(n), _i(k))
+    return lib.abk_gemm_simt_scratch(_i(m), _i(n), _i(k), _i(dtype))
 
 
 @functools.lru_cache(maxsize=4096)
 def _gemm_simt_plan(dtype, m, n, k):
     """(bytes of scratch memory, kernels) of a product of these sizes."""
-    return gemm_simt_scratch(m, n, k), load_module("gemm_simt").abk_gemm_simt_kernels(_i(dtype), _i(m), _i(n), _i(k))
+    return gemm_simt_scratch(m, n, k, dtype), load_module("gemm_simt").abk_gemm_simt_kernels(_i(dtype), _i(m), _i(n), _i(k))
 
 
 def gemm_simt(x, w, out, m=None):

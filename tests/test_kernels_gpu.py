@@ -275,7 +275,7 @@ def test_sums_in_parts_that_are_no_numbers_or_too_small_are_taken_again(ops, m, 
     want, plain_out, others = product(clean), torch.empty(m, n, device="cuda"), [i for i in range(m) if i not in planted]
     assert lib.abk_gemm_simt(ops._p(x), ops._i(ops._dt(x)), ops._p(w), ops._i(ops._dt(w)), ops._p(plain_out), ops._i(0), ops._i(m), ops._i(n), ops._i(k),
                              ops._ll(k), ops._ll(k), ops._ll(n), None, ops._ll(0), ops._p(status), ops._stream()) == 0
-    for rows, quarters in [(0, 0)] + [(r, q) for r in (32, 64, 96, 128) for q in (0, 1) if dtype == torch.float32 or (r < 128 and not q)]:
+    for rows, quarters in [(0, 0)] + [(r, q) for r in (32, 64, 96, 128) for q in (0, 1) if dtype == torch.float32 or k >= 2048 or (r < 128 and not q)]:
         out = product(x, rows, quarters)
         assert torch.equal(out[others], want[others]), (rows, quarters)
         for i in planted:
